@@ -1417,6 +1417,12 @@ static int enqueue_ftem(pdac_ctx *ctx, double dt, cudaStream_t st, bool in_sweep
 // kernels of the corrector in one graph sweep, k_sweep_check included
 static long long sweep_kernels(const pdac_ctx *) { return 10; }
 
+// warps k_inner_team may spread a short worklist over: those resident at
+// once, or none beyond the packed ones for a member of a batch
+static int inner_spread(const pdac_ctx *ctx) {
+    return ctx->allow_coop ? 148 * PDAC_INNER_MINB(ctx->nph) * (pdac::KS / 32) : 1;
+}
+
 static int enqueue_sweep(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof) {
     Fld &F = ctx->F;
     // implicit_fluxes: momentum fluxes, stresses and drag of the current
@@ -1444,8 +1450,8 @@ static int enqueue_sweep(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof) {
         if (ctx->d3) PHASE_LAUNCH_D(nph, pdac::k_resid_test, 3, test_grid, TPB_RESID, st, ctx->P, F, dt, ctx->d_cand, ncand, wl, cnt, dirty);
         else PHASE_LAUNCH_D(nph, pdac::k_resid_test, 2, test_grid, TPB_RESID, st, ctx->P, F, dt, ctx->d_cand, ncand, wl, cnt, dirty);
         if (prof) CK(cudaEventRecord(ctx->cev[3 * col + 1], st));
-        if (ctx->d3) INNER_LAUNCH_D(nph, pdac::k_inner_team, 3, g, TPB_TEAM, st, ctx->P, F, dt, ctx->d_nit, wl, cnt, dirty);
-        else INNER_LAUNCH_D(nph, pdac::k_inner_team, 2, g, TPB_TEAM, st, ctx->P, F, dt, ctx->d_nit, wl, cnt, dirty);
+        if (ctx->d3) INNER_LAUNCH_D(nph, pdac::k_inner_team, 3, g, TPB_TEAM, st, ctx->P, F, dt, ctx->d_nit, wl, cnt, dirty, inner_spread(ctx));
+        else INNER_LAUNCH_D(nph, pdac::k_inner_team, 2, g, TPB_TEAM, st, ctx->P, F, dt, ctx->d_nit, wl, cnt, dirty, inner_spread(ctx));
         if (prof) CK(cudaEventRecord(ctx->cev[3 * col + 2], st));
     }
     // implicit_enthalpy: the enthalpy fluxes (with implicit_fluxes) and the
@@ -1744,8 +1750,8 @@ int pdac_gpu_iter_static(pdac_ctx *ctx, double dt, int *nit_out) {
             ctx->launches++;
             long team_threads = (nthr + (ctx->d3 ? 4 : 7)) / (ctx->d3 ? 5 : 8) * 32;
             int g = std::min(ctx->inner_grid, blocks(team_threads, TPB_TEAM));
-            if (ctx->d3) INNER_LAUNCH_D(nph, pdac::k_inner_team, 3, g, TPB_TEAM, st, ctx->P, F, dt, dnit, work, cnt, dirty);
-            else INNER_LAUNCH_D(nph, pdac::k_inner_team, 2, g, TPB_TEAM, st, ctx->P, F, dt, dnit, work, cnt, dirty);
+            if (ctx->d3) INNER_LAUNCH_D(nph, pdac::k_inner_team, 3, g, TPB_TEAM, st, ctx->P, F, dt, dnit, work, cnt, dirty, inner_spread(ctx));
+            else INNER_LAUNCH_D(nph, pdac::k_inner_team, 2, g, TPB_TEAM, st, ctx->P, F, dt, dnit, work, cnt, dirty, inner_spread(ctx));
             ctx->launches += 2;
         }
         CK(cudaMemcpyAsync(ctx->h_counters, wcount, 6 * sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -27,38 +27,46 @@ __device__ __forceinline__ double ldro(const double *p) {
     if (RO) return __ldg(p);
     return *p;
 }
+// the same for a stencil slot that may be the cell c itself, which this
+// launch does write (later, by the lanes of its own team)
+template <bool RO>
+__device__ __forceinline__ double ldro_self(const double *a, int idx, int c) {
+    return idx == c ? a[c] : ldro<RO>(a + idx);
+}
 
-// mass flux through one face (masf + fmas, flux_m.f:47-324), written for a
-// face on the minus side (W/S/B) or the plus side (E/N/T) of the cell.
-// dc = cell value, dm/dmm = first/second neighbour on the minus side, dp/dpp
-// on the plus side; r = radial factor of x faces in cylindrical 2D, else 1.
+// The mass flux through one face (masf + fmas, flux_m.f:47-324) in
+// coordinates mirrored about the cell: n is the cell across the face, f the
+// one beyond it, o the one on the other side of the cell c.  The reference's
+// gradients are differences along the axis; mirroring a W/S/B face flips the
+// sign of all three, which an IEEE difference, product and quotient carry
+// exactly, so both kinds of face run the same instructions (one division
+// instead of one per branch of face side and velocity sign) and give the
+// bits of the reference's expressions (a zero may change its sign).
 struct FaceGeo {
-    double inmm, inm, inp, inpp, incr_p, incr_m, r;
+    double cn, cf, co;  // 2 x reciprocal spacing of (n, c), (f, n), (c, o)
+    double iu, id;      // the MUSCL increment for flow out of the cell / into it, signed like the axis
+    double r;           // radial factor of x faces in cylindrical 2D, else 1
     bool lim_on;
 };
 
-__device__ __forceinline__ double face_mflux(const Prm &P, const FaceGeo &g, bool minus, double cs, double dc,
-                                             double dm, double dmm, double dp, double dpp, bool mus) {
-    double f;
-    if (minus) f = 0.5 * (cs - fabs(cs)) * dc * g.r + 0.5 * (cs + fabs(cs)) * dm * g.r;
-    else f = 0.5 * (cs - fabs(cs)) * dp * g.r + 0.5 * (cs + fabs(cs)) * dc * g.r;
+// cs: face velocity; out: it leaves the cell (upwind side c); d*: densities
+template <int D>
+__device__ __forceinline__ double face_mflux(const Prm &P, const FaceGeo &g, double cs, bool out, double dc,
+                                             double dn, double df, double dopp, bool mus) {
+    // the donor-cell flux: of 0.5 (cs -+ |cs|) one is cs, the other 0
+    double f = cs * (out ? dc : dn);
+    if (D == 2) f = f * g.r;
     if (!mus) return f;
-    double gradc, gradm, gradp;
-    if (minus) {
-        gradc = 2.0 * g.inm * (dc - dm);
-        gradm = 2.0 * g.inmm * (dm - dmm);
-        gradp = 2.0 * g.inp * (dp - dc);
-    } else {
-        gradm = 2.0 * g.inm * (dc - dm);
-        gradc = 2.0 * g.inp * (dp - dc);
-        gradp = 2.0 * g.inpp * (dpp - dp);
-    }
-    double erre = 0, incr = 0, lim = 0;
-    if (cs >= 0) { if (gradc != 0) erre = gradm / gradc; incr = g.incr_p; }
-    else if (cs < 0) { if (gradc != 0) erre = gradp / gradc; incr = g.incr_m; }
-    if (g.lim_on) lim = limiter(P.lm, erre, P.beta);
-    double upwnd = lim * gradc * incr;
-    return f + upwnd * cs * g.r;
+    const double gc = g.cn * (dn - dc);
+    const double gf = g.cf * (df - dn), go = g.co * (dc - dopp);
+    const double num = out ? go : gf;
+    const bool nz = gc != 0;
+    const double erre = (nz ? num : 0.0) / (nz ? gc : 1.0);
+    const double lim = g.lim_on ? limiter(P.lm, erre, P.beta) : 0.0;
+    const double upwnd = lim * gc * (out ? g.iu : g.id);
+    double t = upwnd * cs;
+    if (D == 2) t = t * g.r;
+    return f + t;
 }
 
 // Loop-invariant part of one face's phase system (matrix.f:38-328) for the
@@ -103,20 +111,18 @@ struct FaceK<NP, true> {
 // the six scalars of FaceK
 enum { FK_PNB = 0, FK_D0EPNB, FK_K1, FK_K2, FK_D1, FK_INV };
 
-// The loop-invariant density stencil of one face's mass fluxes by phase:
-// the near (cm, cp) and far (cf) neighbour values and the cell's own values
-// at loop entry (o, read by opt_inner_loop's stale slots).  SH = true keeps
-// them in this lane's column of a shared [4 NC][KS] array, as FaceK does.
+// The loop-invariant density stencil of one face's mass fluxes by phase: the
+// values of the cells n, f and o of face_mflux.  SH = true keeps them in this
+// lane's column of a shared [3 NC][KS] array, as FaceK does.
 template <int NC, bool SH>
 struct DensK;
 
 template <int NC>
 struct DensK<NC, false> {
-    double cm_[NC], cp_[NC], cf_[NC], o_[NC];
+    double n_[NC], f_[NC], o_[NC];
     __device__ __forceinline__ explicit DensK(double *) {}
-    __device__ __forceinline__ double &cm(int l) { return cm_[l]; }
-    __device__ __forceinline__ double &cp(int l) { return cp_[l]; }
-    __device__ __forceinline__ double &cf(int l) { return cf_[l]; }
+    __device__ __forceinline__ double &n(int l) { return n_[l]; }
+    __device__ __forceinline__ double &f(int l) { return f_[l]; }
     __device__ __forceinline__ double &o(int l) { return o_[l]; }
 };
 
@@ -124,10 +130,9 @@ template <int NC>
 struct DensK<NC, true> {
     double *s;  // this lane's column: element q at s[q * KS]
     __device__ __forceinline__ explicit DensK(double *col) : s(col) {}
-    __device__ __forceinline__ double &cm(int l) { return s[l * KS]; }
-    __device__ __forceinline__ double &cp(int l) { return s[(NC + l) * KS]; }
-    __device__ __forceinline__ double &cf(int l) { return s[(2 * NC + l) * KS]; }
-    __device__ __forceinline__ double &o(int l) { return s[(3 * NC + l) * KS]; }
+    __device__ __forceinline__ double &n(int l) { return s[l * KS]; }
+    __device__ __forceinline__ double &f(int l) { return s[(NC + l) * KS]; }
+    __device__ __forceinline__ double &o(int l) { return s[(2 * NC + l) * KS]; }
 };
 
 template <int NP, bool RO, class KT>
@@ -136,13 +141,14 @@ __device__ __forceinline__ void face_prepare(const Prm &P, const Fld &F, int c, 
     const int nph = nphases<NP>(P);
     const size_t n = P.ncell;
     const double *dd = dir == 0 ? P.dx : (dir == 1 ? P.dy : P.dz);
+    const double *hh = dir == 0 ? P.hx : (dir == 1 ? P.hy : P.hz);
     double grav = dir == 0 ? P.gravx : (dir == 1 ? P.gravy : P.gravz);
     const double *app = dir == 0 ? F.appu : (dir == 1 ? F.appv : F.appw);
     const double *rg = dir == 0 ? F.rug : (dir == 1 ? F.rvg : F.rwg);
     const double *rs = dir == 0 ? F.rus : (dir == 1 ? F.rvs : F.rws);
     double alpha = P.alpha, ag = P.alphagrav;
     double d0 = dd[ii], d1 = side > 0 ? dd[ii + 1] : dd[ii - 1];
-    double inv = 1.0 / (d0 + d1);
+    double inv = side > 0 ? hh[ii] : hh[ii - 1];
     int rowc = side > 0 ? c : raw;
     K.sc(FK_D1) = d1;
     K.sc(FK_INV) = inv;
@@ -150,17 +156,17 @@ __device__ __forceinline__ void face_prepare(const Prm &P, const Fld &F, int c, 
     K.sc(FK_D0EPNB) = P.pmodel == 1 ? d0 * ldro<RO>(F.ep + nb) : 0.0;
     K.sc(FK_K1) = alpha * dt * inv * 2.0;
     K.sc(FK_K2) = dt * ag * inv * grav;
-    K.brow(0) = ldro<RO>(rg + rowc);
+    K.brow(0) = __ldg(rg + rowc);
     K.d0rn(0) = d0 * ldro<RO>(F.rgp + nb);
 #pragma unroll
     for (int l = 2; l <= nph; ++l) {
-        K.brow(l - 1) = ldro<RO>(rs + (l - 2) * n + rowc);
+        K.brow(l - 1) = __ldg(rs + (l - 2) * n + rowc);
         K.d0rn(l - 1) = d0 * ldro<RO>(F.rlk + (l - 2) * n + nb);
     }
     const int nap = nph * (nph + 1) / 2;
 #pragma unroll
     for (int ls = 1; ls <= nap; ++ls)
-        K.A(ls - 1) = alpha * (d0 * ldro<RO>(app + (ls - 1) * n + nb) + d1 * ldro<RO>(app + (ls - 1) * n + c)) * inv;
+        K.A(ls - 1) = alpha * (d0 * __ldg(app + (ls - 1) * n + nb) + d1 * __ldg(app + (ls - 1) * n + c)) * inv;
 }
 
 // the in-loop assembly and solution; side as in face_system
@@ -219,22 +225,34 @@ template <int NP>
 __host__ __device__ constexpr int inner_face_rows() { return (NP > 0 && NP <= 6) ? FaceK<NP, true>::N : 0; }
 template <int NP>
 __host__ __device__ constexpr int inner_dens_rows() {
-    return (NP > 0 && NP <= PDAC_INNER_SHD_MAXP) ? 4 * (Sys<NP>::M - 1) : 0;
+    return (NP > 0 && NP <= PDAC_INNER_SHD_MAXP) ? 3 * (Sys<NP>::M - 1) : 0;
 }
 template <int NP>
 __host__ __device__ constexpr size_t inner_smem_bytes() {
     return (size_t)(inner_face_rows<NP>() + inner_dens_rows<NP>()) * KS * sizeof(double);
 }
 
-// The inner loop of cell c (outer sweep nit, 1-based) by the team of lanes
-// tb .. tb + T - 1 of this warp (lane q of the team owns face q); kcols and
-// dcols are the shared FaceK and DensK arrays.  RO as in ldro.
+// The inner loop of worklist cell c (outer sweep nit, 1-based) by the team of
+// lanes tb .. tb + T - 1 of this warp (lane q of the team owns face q); kcols
+// and dcols are the shared FaceK and DensK arrays.  RO as in ldro.
+//
+// Every lane of the warp makes this call and runs the same instructions to
+// the end: a team whose cell has converged stores it and goes on computing
+// values that nothing reads (live = false, also for the lanes that own no
+// face and for teams without a cell, which take any valid c), so that the
+// shuffles take the whole warp and teams never run apart.  What bounds the
+// loop is the dependent FP64 chain of an iteration (~1500 cycles of 8.8-cycle
+// operations, 76-cycle reciprocals and 127-cycle quotients, measured) and the
+// instructions of a warp's teams when they diverge; hence one code path for
+// all faces, velocity signs and bracketing states.
 template <int NP, int D, bool RO>
-__device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, double dt, int nit, int c, unsigned *dirty,
-                                                int q, int tb, unsigned tmask, double *kcols, double *dcols) {
+__device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, double dt, int nit, int c, bool live,
+                                                unsigned *dirty, int q, int tb, double *kcols, double *dcols) {
+    constexpr unsigned full = 0xffffffffu;
     constexpr int NC = Sys<NP>::M - 1;   // phase capacity
     constexpr bool SH = inner_face_rows<NP>() > 0;   // FaceK in shared memory (40 KB per block at NP = 6)
-    constexpr bool SHD = inner_dens_rows<NP>() > 0;  // DensK too (16 KB at NP = 4, 24 KB at NP = 6)
+    constexpr bool SHD = inner_dens_rows<NP>() > 0;  // DensK too (12 KB at NP = 4, 18 KB at NP = 6)
+    constexpr int NAX = D == 3 ? 3 : 2;  // axes; lanes q < NAX own the minus faces
     const int nph = nphases<NP>(P), ns = nph - 1;
     const size_t n = P.ncell;
     int i, j, k;
@@ -242,97 +260,101 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
     else { i = c % P.nx + 1; j = 1; k = c / P.nx + 1; }
     const int *fl = P.flag;
     // ---- this lane's face: axis, side, raw and remapped neighbours -------
-    const int a = D == 3 ? q % 3 : q % 2;
-    const bool minus = D == 3 ? q < 3 : q < 2;
+    const bool minus = q < NAX;
+    const int a = minus ? q : q - NAX;
     const int dir = D == 3 ? a : (a == 0 ? 0 : 2);
     const int ii = dir == 0 ? i : (dir == 1 ? j : k);
     const int nax = dir == 0 ? P.nx : (dir == 1 ? P.ny : P.nz);
-    int raw_m, raw_p, rm, rmm, rp, rpp;
-    if (D == 3) {
-        Raw3 R;
-        Rem3 M;
-        raw3(P, i, j, k, R);
-        rem3(P, i, j, k, R, M);
-        if (dir == 0) { raw_m = R.w; raw_p = R.e; rm = M.w; rmm = M.ww; rp = M.e; rpp = M.ee; }
-        else if (dir == 1) { raw_m = R.s; raw_p = R.n; rm = M.s; rmm = M.ss; rp = M.n; rpp = M.nn; }
-        else { raw_m = R.b; raw_p = R.t; rm = M.b; rmm = M.bb; rp = M.t; rpp = M.tt; }
-    } else {
-        Raw2 R;
-        Rem2 M;
-        raw2(P, i, k, R);
-        rem2(P, i, k, R, M);
-        if (dir == 0) { raw_m = R.w; raw_p = R.e; rm = M.w; rmm = M.ww; rp = M.e; rpp = M.ee; }
-        else { raw_m = R.b; raw_p = R.t; rm = M.b; rmm = M.bb; rp = M.t; rpp = M.tt; }
-    }
-    const int rawnb = minus ? raw_m : raw_p;
-    const bool solved = (fl[rawnb] & 1) != 0;
+    const int stride = dir == 0 ? 1 : (D == 2 ? P.nx : (dir == 1 ? P.nx : P.nx * P.ny));
+    // steps to the clamped neighbours along the axis (raw2 / raw3), in face
+    // coordinates: n across the face, f beyond it, o on the other side
+    const int toward = minus ? ii - 1 : nax - ii;  // cells to the mesh's end across the face
+    const int rawnb = minus ? c - stride * min(1, ii - 1) : c + stride * min(1, nax - ii);
+    const int rawop = minus ? c + stride * min(1, nax - ii) : c - stride * min(1, ii - 1);
+    const int rawfar = minus ? c - stride * min(2, ii - 1) : c + stride * min(2, nax - ii);
+    const int fnb = fl[rawnb];
+    // the remapped neighbours (rem2 / rem3): a wall reads as the cell itself,
+    // a wall beyond the neighbour as the neighbour (y: the remapped one), the
+    // last cell before the frame repeats the remapped neighbour
+    const int rn = is_wallf(fnb) ? c : rawnb, ro = is_wallf(fl[rawop]) ? c : rawop;
+    const int rf = toward == 1 ? rn : (is_wallf(fl[rawfar]) ? (dir == 1 ? rn : rawnb) : rawfar);
+    const bool solved = (fnb & 1) != 0;
     const int fcell = minus ? rawnb : c;  // where this face's velocity and fluxes live
     const bool mus = P.muscl > 0 && fl[c] == FLUID;
     FaceGeo g;
     {
         const double *dd = dir == 0 ? P.dx : (dir == 1 ? P.dy : P.dz);
-        int im2 = max(1, ii - 2), ip2 = min(nax, ii + 2);
-        g.inmm = 1.0 / (dd[ii - 1] + dd[im2]);
-        g.inm = 1.0 / (dd[ii] + dd[ii - 1]);
-        g.inp = 1.0 / (dd[ii] + dd[ii + 1]);
-        g.inpp = 1.0 / (dd[ii + 1] + dd[ip2]);
-        g.incr_p = minus ? 0.5 * dd[ii - 1] : 0.5 * dd[ii];
-        g.incr_m = minus ? -0.5 * dd[ii] : -0.5 * dd[ii + 1];
+        const double *hh = dir == 0 ? P.hx : (dir == 1 ? P.hy : P.hz);
+        const double hm = 2.0 * hh[ii - 1], hp = 2.0 * hh[ii];
+        g.cn = minus ? hm : hp;
+        g.co = minus ? hp : hm;
+        g.cf = 2.0 * hh[minus ? max(ii - 2, 0) : ii + 1];
+        g.iu = 0.5 * dd[ii];
+        g.id = minus ? -0.5 * dd[ii - 1] : -0.5 * dd[ii + 1];
         g.r = (D == 2 && dir == 0) ? (minus ? P.rb[i - 1] : P.rb[i]) : 1.0;
-        g.lim_on = minus ? (ii != 2 && fl[raw_m] == FLUID) : (ii != nax - 1 && fl[raw_p] == FLUID);
+        g.lim_on = toward != 1 && fnb == FLUID;
     }
     double *const gvel = dir == 0 ? F.ug : (dir == 1 ? F.vg : F.wg);
     double *const svel = dir == 0 ? F.us : (dir == 1 ? F.vs : F.ws);
+    double *const gfa = dir == 0 ? F.rgfe : (dir == 1 ? F.rgfn : F.rgft);
     double vel[NC];
     vel[0] = gvel[fcell];
 #pragma unroll
     for (int l = 2; l <= nph; ++l) vel[l - 1] = svel[(l - 2) * n + fcell];
     FaceK<NP, SH> K(kcols + threadIdx.x);
-    if (solved) face_prepare<NP, RO>(P, F, c, minus ? rm : rp, rawnb, ii, dir, minus ? -1 : +1, dt, K);
-    // mass-flux stencil of this face by phase (gas first): neighbour
-    // values, or the cell's own current value where the slot is the cell
-    const int rfar = minus ? rmm : rpp;
-    const bool sm = rm == c, sp = rp == c, sfar = rfar == c;
-    DensK<NC, SHD> Dk(dcols + threadIdx.x);
-    Dk.cm(0) = ldro<RO>(F.rgp + rm); Dk.cp(0) = ldro<RO>(F.rgp + rp); Dk.cf(0) = mus ? ldro<RO>(F.rgp + rfar) : 0.0;
-#pragma unroll
-    for (int l = 2; l <= nph; ++l) {
-        const double *D_ = F.rlk + (size_t)(l - 2) * n;
-        Dk.cm(l - 1) = ldro<RO>(D_ + rm); Dk.cp(l - 1) = ldro<RO>(D_ + rp);
-        Dk.cf(l - 1) = mus ? ldro<RO>(D_ + rfar) : 0.0;
-    }
-    // opt_inner_loop (iter.f:1255-1547) builds the density stencils once
-    // and updates only their centre: a neighbour slot remapped to the
-    // cell keeps the loop-entry value there
-    Dk.o(0) = F.rgp[c];
-#pragma unroll
-    for (int l = 2; l <= nph; ++l) Dk.o(l - 1) = F.rlk[(size_t)(l - 2) * n + c];
+    if (solved) face_prepare<NP, RO>(P, F, c, rn, rawnb, ii, dir, minus ? -1 : +1, dt, K);
+    // density stencil of this face's mass fluxes by phase (gas first).  A
+    // slot remapped to the cell reads the cell's own current value, except in
+    // opt_inner_loop (iter.f:1255-1547), which builds the stencils once and
+    // updates only their centre: there it keeps the loop-entry value, which
+    // is what this load reads
     const bool stale = P.opt == 2;
+    const bool sn = !stale && rn == c, so = !stale && ro == c, sf = !stale && rf == c, self = sn || so || sf;
+    DensK<NC, SHD> Dk(dcols + threadIdx.x);
+#pragma unroll
+    for (int l = 1; l <= nph; ++l) {
+        const double *D_ = l == 1 ? F.rgp : F.rlk + (size_t)(l - 2) * n;
+        Dk.n(l - 1) = ldro_self<RO>(D_, rn, c);
+        Dk.o(l - 1) = ldro_self<RO>(D_, ro, c);
+        Dk.f(l - 1) = mus ? ldro_self<RO>(D_, rf, c) : 0.0;
+    }
     auto mflux = [&](int ph, double own) {
-        const double slot = stale ? Dk.o(ph) : own;
-        double dm = sm ? slot : Dk.cm(ph), dp = sp ? slot : Dk.cp(ph), df = sfar ? slot : Dk.cf(ph);
-        return minus ? face_mflux(P, g, true, vel[ph], own, dm, df, dp, 0.0, mus)
-                     : face_mflux(P, g, false, vel[ph], own, dm, 0.0, dp, df, mus);
+        double dn = Dk.n(ph), df = Dk.f(ph), dopp = Dk.o(ph);
+        if (self) {
+            if (sn) dn = own;
+            if (so) dopp = own;
+            if (sf) df = own;
+        }
+        const double cs = vel[ph];
+        return face_mflux<D>(P, g, cs, (cs >= 0) != minus, own, dn, df, dopp, mus);
     };
     // ---- cell state (identical in every lane) ------------------------------
     const double rx = D == 2 ? P.inr[i] : 1.0;
     const double idx_i = P.indx[i], idz_k = P.indz[k], idy_j = D == 3 ? P.indy[j] : 0.0;
     const double rgpn_c = F.rgpn[c];
-    const CellFaces bf = cell_faces(P, c);  // faces, iter.f:259
-    auto resid = [&](double fe, double fw, double fn, double fs, double ft, double fb, double rgpc) {
-        double resx = (bf.e * fe - bf.w * fw) * idx_i * rx;
-        double resz = (bf.t * ft - bf.b * fb) * idz_k;
-        double resy = D == 3 ? (bf.n * fn - bf.s * fs) * idy_j : 0.0;
-        return rgpc - rgpn_c + dt * bf.ivf * (resx + resy + resz);
-    };
-    double dg;  // calc_res of the stored state (raw W/S/B neighbours)
-    if (D == 3) {
-        int cw = at3(P, max(i - 1, 1), j, k), cs = at3(P, i, max(j - 1, 1), k), cb = at3(P, i, j, max(k - 1, 1));
-        dg = resid(F.rgfe[c], F.rgfe[cw], F.rgfn[c], F.rgfn[cs], F.rgft[c], F.rgft[cb], F.rgp[c]);
-    } else {
-        int cw = at2(P, max(i - 1, 1), k), cb = at2(P, i, max(k - 1, 1));
-        dg = resid(F.rgfe[c], F.rgfe[cw], 0.0, 0.0, F.rgft[c], F.rgft[cb], F.rgp[c]);
+    double bq = 1.0, ivf = 1.0;  // this face's open factor and 1 / fluid fraction (faces, iter.f:259)
+    if (P.immb) {
+        const int bit = dir == 0 ? (minus ? 2 : 1) : (dir == 1 ? (minus ? 32 : 16) : (minus ? 8 : 4));
+        bq = (__ldg(P.ib_faces + c) & bit) ? 1.0 : 0.0;
+        ivf = __ldg(P.ib_ivf + c);
     }
+    const double dti = dt * ivf;
+    // the flux divergence of one phase: every lane gets the axis differences
+    // (plus face minus minus face, each times its open factor) over the cell
+    // sizes and sums them in the reference's order (x, y, z)
+    const double ida = dir == 0 ? idx_i : (dir == 1 ? idy_j : idz_k);
+    const int lmin = minus ? q + tb : q - NAX + tb;  // the minus face's lane of this lane's axis
+    auto diverg = [&](double fl_) {
+        const double w = bq * fl_;
+        double d = (w - __shfl_sync(full, w, lmin)) * ida;
+        if (D == 2 && dir == 0) d = d * rx;
+        const double dx_ = __shfl_sync(full, d, tb + NAX);
+        const double dz_ = __shfl_sync(full, d, tb + 2 * NAX - 1);
+        const double dy_ = D == 3 ? __shfl_sync(full, d, tb + NAX + 1) : 0.0;
+        return D == 3 ? dx_ + dy_ + dz_ : dx_ + dz_;
+    };
+    // calc_res of the stored state (iter.f:743-771, which sums x + y + z)
+    double dg = F.rgp[c] - rgpn_c + dti * diverg(gfa[fcell]);
     double dgorig = dg;
     const double conv = F.conv[c];
     double d3 = dg, p3 = F.p[c], abeta = F.abeta[c];
@@ -340,24 +362,20 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
     // does not change within the loop: summed once, in thermal_eosg's order
     double mg = 0;
     for (int ig = 0; ig < P.ng; ++ig) mg = mg + GAS(F.xgc, c, ig) * P.gmw[P.gas_type[ig]];
-    const double tgc = F.tg[c];
-    const double rgas_tg = P.rgas * tgc;
+    const double rgas_tg = P.rgas * F.tg[c];
     int kros = -1;
     PAdj s = {0, 0, 0, 0, 0, 0};
-    double p = F.p[c], ep = F.ep[c], rog = F.rog[c], rgp = F.rgp[c];
-    double rlk[NC], rlkn[NC], sink[NC];
+    double p = p3, ep = F.ep[c], rog, rgp;
+    double rlk[NC], rlkn[NC], snk[NC];
 #pragma unroll
     for (int is = 1; is <= ns; ++is) {
         rlk[is - 1] = F.rlk[(is - 1) * n + c];
         rlkn[is - 1] = F.rlkn[(is - 1) * n + c];
-        sink[is - 1] = F.sink[(is - 1) * n + c];
+        snk[is - 1] = dti * F.sink[(is - 1) * n + c];
     }
     double flux[NC];  // this lane's face mass flux by phase (gas first)
 #pragma unroll
     for (int l = 0; l < NC; ++l) flux[l] = 0.0;
-    // source lanes of the faces (3D: W S B E N T = 0..5; 2D: W B E T = 0..3)
-    const int lW = tb + 0, lE = tb + (D == 3 ? 3 : 2), lB = tb + (D == 3 ? 2 : 1), lT = tb + (D == 3 ? 5 : 3);
-    const int lS = tb + 1, lN = tb + 4;
     for (int loop = 1; loop <= P.inmax; ++loop) {
         if (loop > 1 || nit > 1) padjust(s, p, kros, d3, p3, P.omega, abeta);
         rog = p / rgas_tg * mg;  // thermal_eosg
@@ -370,85 +388,89 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
         double rls = 0;
 #pragma unroll
         for (int is = 1; is <= ns; ++is) {
-            double fW = __shfl_sync(tmask, flux[is], lW), fE = __shfl_sync(tmask, flux[is], lE);
-            double fB = __shfl_sync(tmask, flux[is], lB), fT = __shfl_sync(tmask, flux[is], lT);
-            double fS = 0, fN = 0;
-            if (D == 3) { fS = __shfl_sync(tmask, flux[is], lS); fN = __shfl_sync(tmask, flux[is], lN); }
-            double rlkx = (bf.e * fE - bf.w * fW) * idx_i * rx;
-            double rlkz = (bf.t * fT - bf.b * fB) * idz_k;
-            double rlky = D == 3 ? (bf.n * fN - bf.s * fS) * idy_j : 0.0;
-            double t = rlkn[is - 1] - dt * bf.ivf * (rlkx + rlky + rlkz);
-            t = t + dt * bf.ivf * sink[is - 1];
+            double t = rlkn[is - 1] - dti * diverg(flux[is]);
+            t = t + snk[is - 1];
             double v = fmax(0.0, t);
             rlk[is - 1] = v;
             rls = rls + v * P.inrl[is];
         }
         ep = 1.0 - rls;
-        if (rls > 1.0 && q == 0) atomicAdd(&F.counters[2], 1);
+        if (rls > 1.0 && q == 0 && live) atomicAdd(&F.counters[2], 1);
         rgp = ep * rog;
         // gas mass flux and continuity residual (iter.f:597-771)
         flux[0] = mflux(0, rgp);
-        {
-            double fW = __shfl_sync(tmask, flux[0], lW), fE = __shfl_sync(tmask, flux[0], lE);
-            double fB = __shfl_sync(tmask, flux[0], lB), fT = __shfl_sync(tmask, flux[0], lT);
-            double fS = 0, fN = 0;
-            if (D == 3) { fS = __shfl_sync(tmask, flux[0], lS); fN = __shfl_sync(tmask, flux[0], lN); }
-            dg = resid(fE, fW, fN, fS, fT, fB, rgp);
-        }
+        dg = rgp - rgpn_c + dti * diverg(flux[0]);
+        bool done = loop == P.inmax;
         if (fabs(dg) > conv || fabs(dg) >= fabs(dgorig)) {
             if (nit == 1 && loop == 1) dgorig = dg;
             d3 = dg;
         } else if (fabs(dg) <= conv) {
-            break;
+            done = true;
         }
-    }
-    // ---- final values -----------------------------------------------------
-    {
-        // face mass fluxes (every face, as calc_*_mass_flux writes them)
-        double *gfa = dir == 0 ? F.rgfe : (dir == 1 ? F.rgfn : F.rgft);
-        double *sfa = dir == 0 ? F.rsfe : (dir == 1 ? F.rsfn : F.rsft);
-        gfa[fcell] = flux[0];
+        if (live && done) {
+            // the cell's final values: face mass fluxes (every face, as
+            // calc_*_mass_flux writes them), velocities, cell state
+            double *sfa = dir == 0 ? F.rsfe : (dir == 1 ? F.rsfn : F.rsft);
+            gfa[fcell] = flux[0];
 #pragma unroll
-        for (int is = 1; is <= ns; ++is) sfa[(size_t)(is - 1) * n + fcell] = flux[is];
-        if (solved) {
-            gvel[fcell] = vel[0];
+            for (int is = 1; is <= ns; ++is) sfa[(size_t)(is - 1) * n + fcell] = flux[is];
+            if (solved) {
+                gvel[fcell] = vel[0];
 #pragma unroll
-            for (int l = 2; l <= nph; ++l) svel[(l - 2) * n + fcell] = vel[l - 1];
+                for (int l = 2; l <= nph; ++l) svel[(l - 2) * n + fcell] = vel[l - 1];
+            }
+            mark_dirty(dirty, rawnb);
+            if (q == 0) {
+                F.p[c] = p; F.rog[c] = rog; F.rgp[c] = rgp; F.ep[c] = ep;
+#pragma unroll
+                for (int is = 1; is <= ns; ++is) F.rlk[(is - 1) * n + c] = rlk[is - 1];
+                F.abeta[c] = abeta;
+                mark_dirty(dirty, c);
+            }
+            live = false;
         }
-        mark_dirty(dirty, rawnb);
-    }
-    if (q == 0) {
-        F.p[c] = p; F.rog[c] = rog; F.rgp[c] = rgp; F.ep[c] = ep;
-#pragma unroll
-        for (int is = 1; is <= ns; ++is) F.rlk[(is - 1) * n + c] = rlk[is - 1];
-        F.abeta[c] = abeta;
-        mark_dirty(dirty, c);
+        if (!__any_sync(full, live)) break;
     }
 }
 
-// the inner loop of the worklist's nwork cells (outer sweep nit, 1-based)
-// by the warps warp, warp + nwarps, ... of the launch; RO as in ldro
+// the inner loop of the worklist's nwork cells (outer sweep nit, 1-based) by
+// the warps warp, warp + nwarps, ... of the launch, cpw <= teams per warp
+// cells at a time; every lane of a warp makes the call.  RO as in ldro.
 template <int NP, int D, bool RO>
 __device__ __forceinline__ void inner_team_run(const Prm &P, const Fld &F, double dt, int nit, const int *list,
-                                               int nwork, unsigned *dirty, int warp, int nwarps) {
+                                               int nwork, unsigned *dirty, int warp, int nwarps, int cpw) {
     constexpr int T = D == 3 ? 6 : 4;    // lanes per cell
-    constexpr int TPW = 32 / T;          // teams per warp (3D: 5, lanes 30 and 31 idle)
+    constexpr int TPW = 32 / T;          // teams per warp (3D: 5, lanes 30 and 31 own no face)
     const int lane = threadIdx.x & 31, tw = lane / T;
-    if (tw >= TPW) return;  // idle lanes take no part in any team
     const int q = lane - tw * T, tb = tw * T;
-    const unsigned tmask = ((1u << T) - 1u) << tb;
     extern __shared__ __align__(16) double inner_smem[];
     double *const kcols = inner_smem;                              // [FaceK rows][KS]
-    double *const dcols = inner_smem + inner_face_rows<NP>() * KS;  // [4 NC][KS]
-    for (int w = warp * TPW + tw; w < nwork; w += nwarps * TPW)
-        inner_team_cell<NP, D, RO>(P, F, dt, nit, list[w], dirty, q, tb, tmask, kcols, dcols);
+    double *const dcols = inner_smem + inner_face_rows<NP>() * KS;  // [3 NC][KS]
+    for (int w0 = warp * cpw; w0 < nwork; w0 += nwarps * cpw) {
+        const bool live = tw < TPW && tw < cpw && w0 + tw < nwork;
+        inner_team_cell<NP, D, RO>(P, F, dt, nit, list[live ? w0 + tw : w0], live, dirty, q, tb, kcols, dcols);
+    }
+}
+
+// cells per warp of a worklist of nwork cells: while the list leaves warps
+// idle each cell gets a warp of its own as far as they reach, since teams of
+// one warp share its issue slots and wait for the slowest.  nwarps: the warps
+// the launch may count on (one when other launches fill the device, as the
+// other members of a batch do: 24 members with their cells spread out ran
+// 5 % slower than packed)
+template <int D>
+__device__ __forceinline__ int cells_per_warp(int nwork, int nwarps) {
+    constexpr int TPW = 32 / (D == 3 ? 6 : 4);
+    return min(TPW, max(1, (nwork + nwarps - 1) / nwarps));
 }
 
 template <int NP, int D>
 __global__ void __launch_bounds__(128, PDAC_INNER_MINB(NP)) k_inner_team(Prm P, Fld F, double dt, const int *nitp, const int *list,
-                                                                     const int *count, unsigned *dirty) {
+                                                                     const int *count, unsigned *dirty, int spread) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    inner_team_run<NP, D, true>(P, F, dt, *nitp, list, *count, dirty, warp, nwarps);
+    const int nwork = *count;
+    inner_team_run<NP, D, true>(P, F, dt, *nitp, list, nwork, dirty, warp, nwarps,
+                                cells_per_warp<D>(nwork, min(nwarps, spread)));
 }
 
 // Residual test of one colour phase (iter.f:241-319) in two launches.
@@ -595,7 +617,7 @@ __device__ __forceinline__ void fused_phase(const Prm &P, const Fld &F, double d
             if (lane == 0) base = atomicAdd(wcount + colour, nwork);
             base = __shfl_sync(0xffffffffu, base, 0);
             if (unconv) work[base + __popc(um & ((1u << lane) - 1u))] = c;
-            inner_team_run<NP, D, RO>(P, F, dt, nit, mylist, nwork, dirty, 0, 1);
+            inner_team_run<NP, D, RO>(P, F, dt, nit, mylist, nwork, dirty, 0, 1, 32 / (D == 3 ? 6 : 4));
         }
         __syncwarp();  // the list is read before the next word overwrites it
     }

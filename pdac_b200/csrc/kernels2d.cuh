@@ -677,44 +677,49 @@ __device__ __forceinline__ void calc_eps_2d(const Prm &P, const Fld &F, const Ra
 // padjust + newp, iter.f:997-1109 (bracketing state in registers)
 struct PAdj { double dp, d1, d2, p1, p2, d12; };
 
+// The two secant quotients are formed once for every bracketing state (the
+// 1 / (d1 - d2) of the first bracket takes the place of the second), so that
+// cells in different states run the same instructions; an unused quotient is
+// dropped by the selects.
 __device__ __forceinline__ void padjust(PAdj &s, double &p, int &kros, double d3, double &p3, double omega, double &abeta) {
-    if (kros != 3) {
+    const bool brk = kros == 3;  // bracketed before this call
+    if (!brk) {
         if (d3 > 0.0) {
             s.d1 = d3; s.p1 = p3;
-            if (kros == -1) kros = 0;
-            else if (kros == 1) kros = 2;
+            kros = kros == -1 ? 0 : (kros == 1 ? 2 : kros);
         } else if (d3 <= 0.0) {
             s.d2 = d3; s.p2 = p3;
-            if (kros == -1) kros = 1;
-            else if (kros == 0) kros = 2;
+            kros = kros == -1 ? 1 : (kros == 0 ? 2 : kros);
         }
-        if (kros == 2) {
-            s.d12 = 1.0 / (s.d1 - s.d2);
-            p = (s.d1 * s.p2 - s.d2 * s.p1) * s.d12;
-            abeta = (s.p1 - s.p2) * s.d12;
+    }
+    if (kros >= 2) {
+        const double d1 = s.d1, d2 = s.d2, p1 = s.p1, p2 = s.p2;
+        const double qb = (brk ? d2 * p3 - d3 * p2 : 1.0) / (brk ? d2 - d3 : d1 - d2);
+        if (brk) {
+            const bool ne = d1 != d3, opp = d1 * d3 <= 0.0;
+            const double qa = (ne ? d1 * p3 - d3 * p1 : 0.0) / (ne ? d1 - d3 : 1.0);
+            const double h1 = 0.5 * (p1 + p3), h2 = 0.5 * (p2 + p3);
+            double pa = qa, pb = qb;
+            if (opp) {
+                if (d2 == d3 || pb < p3 || pb > p1) pb = h1;
+            } else {
+                if (!ne || pa < p2 || pa > p3) pa = h2;
+            }
+            p = 0.5 * (pa + pb);
+            if (d3 > 0.0) { s.d1 = d3; s.p1 = p3; }
+            else { s.d2 = d3; s.p2 = p3; }
+        } else {
+            s.d12 = qb;
+            p = (d1 * p2 - d2 * p1) * s.d12;
+            abeta = (p1 - p2) * s.d12;
             kros = 3;
-        } else if (kros < 2) {
-            s.dp = -d3 * abeta;
-            s.dp = s.dp * omega;
-            double sg = copysign(1.0, d3);
-            if (-s.dp * sg > 2.5e-1 * p3) s.dp = -2.5e-1 * sg * p3;
-            p = p + s.dp;
         }
     } else {
-        double d1 = s.d1, d2 = s.d2, p1 = s.p1, p2 = s.p2, pa = 0, pb = 0;
-        if (d1 != d3) pa = (d1 * p3 - d3 * p1) / (d1 - d3);
-        if (d1 * d3 <= 0.0) {
-            if (d2 != d3) pb = (d2 * p3 - d3 * p2) / (d2 - d3);
-            else pb = 0.5 * (p1 + p3);
-            if (pb < p3 || pb > p1) pb = 0.5 * (p1 + p3);
-        } else {
-            if (d1 == d3) pa = 0.5 * (p2 + p3);
-            if (pa < p2 || pa > p3) pa = 0.5 * (p2 + p3);
-            pb = (d2 * p3 - d3 * p2) / (d2 - d3);
-        }
-        p = 0.5 * (pa + pb);
-        if (d3 > 0.0) { s.d1 = d3; s.p1 = p3; }
-        else { s.d2 = d3; s.p2 = p3; }
+        s.dp = -d3 * abeta;
+        s.dp = s.dp * omega;
+        double sg = copysign(1.0, d3);
+        if (-s.dp * sg > 2.5e-1 * p3) s.dp = -2.5e-1 * sg * p3;
+        p = p + s.dp;
     }
     p3 = p;
 }

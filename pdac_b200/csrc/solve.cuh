@@ -41,10 +41,13 @@ __device__ __forceinline__ void gauss_jordan_t(const Prm &P, double (&a)[M][M], 
             double div = 1.0 / a[l][l];
 #pragma unroll
             for (int lj = l + 1; lj <= nph; ++lj) a[l][lj] = a[l][lj] * div;
-            b[l] = b[l] * div;
+            // the reference's elimination also visits row l itself, with a
+            // multiplier of 0: that changes nothing but a -0 into a 0
+            b[l] = b[l] * div + 0.0;
             a[l][l] = 0.0;
 #pragma unroll
             for (int li = 1; li <= nph; ++li) {
+                if (li == l) continue;
                 double amul = a[li][l];
 #pragma unroll
                 for (int lj = l + 1; lj <= nph; ++lj) a[li][lj] = a[li][lj] - amul * a[l][lj];
