@@ -139,6 +139,7 @@ struct Fld {
     double *rgfe, *rgfn, *rgft, *rsfe, *rsfn, *rsft, *conv, *abeta;
     double *egfe, *egfn, *egft, *esfe, *esfn, *esft, *rhg, *rhs;
     double *yfe, *yfn, *yft;
+    double *fk;  // face records of iter (face_rec, solve.cuh), axis-major; null: none
     double *sink;
     double *smag, *mugt, *kapgt, *must;  // sub-grid model (turbo.f:10-14); must (ncell, ns)
     double *dyn, *delt, *scoeff;         // dynamic model: per-cell work blocks, filter width, cdyn

@@ -43,6 +43,7 @@ struct pdac_ctx {
     double *d_vfact = nullptr, *d_vfact0 = nullptr;
     double *d_app0u = nullptr, *d_app0v = nullptr, *d_app0w = nullptr;
     double *d_partial = nullptr;
+    double *d_fk = nullptr;  // face records of iter where mf cannot hold them
     int nvent = 0;
     std::string err;
     cudaEvent_t ev[16];
@@ -965,6 +966,21 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     // per-class blocks inside a slot are exactly ncell apart, as the
     // reference's (ncell, n) column-major arrays; the stride pads slot ends
     F.counters = ctx->d_counters;
+    // the face records of iter (solve.cuh), for the phase counts whose inner
+    // loop reads them and while tilde, which rewrites the terms they are made
+    // of, does not run inside the sweeps.  In 3D they take the place of the
+    // momentum fluxes and stresses (mf and vis, neighbours in the arena),
+    // which tilde is done with when iter starts and rewrites before it reads
+    // them again; where they do not fit there (six phases) and in 2D they get
+    // memory of their own, and if there is none left the inner loop forms the
+    // terms itself
+    F.fk = nullptr;
+    if (!t1 && !cfg->implicit_fluxes && (ctx->nph <= 4 || ctx->nph == 6)) {
+        const size_t need = (size_t)pdac::face_rec(ctx->nph) * (ctx->d3 ? 3 : 2) * n;
+        if (ctx->d3 && need <= stride * 12 * ctx->nph) F.fk = F.mf;
+        else if (cudaMalloc(&ctx->d_fk, need * sizeof(double)) == cudaSuccess) F.fk = ctx->d_fk;
+        else (void)cudaGetLastError();
+    }
     if (lt) {
         // turbulence_setup (turbo.f:42-108): smag = lm^2 with the
         // Smagorinsky length lm = cmut delta, delta = sqrt(dz dx) in 2D and
@@ -1095,6 +1111,7 @@ int pdac_gpu_destroy(pdac_ctx *ctx) {
     cudaFreeHost(ctx->h_nit);
     cudaFree(ctx->d_cand);
     cudaFree(ctx->d_partial);
+    cudaFree(ctx->d_fk);
     cudaFree(ctx->d_sinkbuf);
     cudaFree(ctx->d_ring);
     cudaFree(ctx->d_wave_idx);

@@ -71,45 +71,62 @@ __device__ __forceinline__ double face_mflux(const Prm &P, const FaceGeo &g, dou
 
 // Loop-invariant part of one face's phase system (matrix.f:38-328) for the
 // cell's inner loop: everything that does not depend on the cell's own p,
-// ep, rgp and rlk, evaluated once with the operations of face_system so that
-// the in-loop assembly (face_assemble) reproduces face_system bit for bit:
-// A(ls) = alpha (d0 app(nb) + d1 app(c)) / (d0 + d1) by interphase index,
-// brow(l) the tilde momenta of the face (gas first), d0rn(l) = d0 x the
-// neighbour bulk densities (l = 0: d0 rgp(nb)), and six scalars.  Two
-// storage forms with one interface: SH = true keeps them in this lane's
-// column of a shared [N][KS] array (blocks of KS threads), which frees ~50
-// registers of the inner loop for a third resident block per SM; SH = false
-// (the generic phase count, whose array would not fit) keeps them in
-// registers.
+// ep, rgp and rlk, evaluated once so that the in-loop assembly
+// (face_assemble) gives the bits of the predictor's (face_solve): the face's
+// record (rec: interphase terms by interphase index, then the tilde momenta
+// of its row, gas first) and seven scalars.  Two storage forms: SH = true
+// keeps them as 16-byte pairs in this lane's column of a shared [N][KS]
+// array (blocks of KS threads), which frees ~50 registers of the inner loop
+// for a third resident block per SM and lets the record arrive by
+// asynchronous copies; SH = false (the generic phase count, whose array
+// would not fit) keeps them in registers.
 constexpr int KS = 128;  // threads per block of every kernel running the inner loop
+
+// the seven scalars of FaceK (and one of padding)
+enum { FK_PNB = 0, FK_D0EPNB, FK_K1, FK_K2, FK_D1, FK_INV, FK_D0, FK_N };
 
 template <int NP, bool SH>
 struct FaceK;
 
 template <int NP>
 struct FaceK<NP, false> {
-    static constexpr int M = Sys<NP>::M, NA = M * (M - 1) / 2;
-    double A_[NA], brow_[M - 1], d0rn_[M - 1], sc_[6];
+    static constexpr int M = Sys<NP>::M, R = (M * (M - 1) / 2 + M) / 2 * 2;
+    double rec_[R], sc_[FK_N + 1];
     __device__ __forceinline__ explicit FaceK(double *) {}
-    __device__ __forceinline__ double &A(int i) { return A_[i]; }
-    __device__ __forceinline__ double &brow(int l) { return brow_[l]; }
-    __device__ __forceinline__ double &d0rn(int l) { return d0rn_[l]; }
+    __device__ __forceinline__ void set(int i, double v) { rec_[i] = v; }
+    __device__ __forceinline__ void get(double (&v)[R]) const {
+#pragma unroll
+        for (int i = 0; i < R; ++i) v[i] = rec_[i];
+    }
     __device__ __forceinline__ double &sc(int q) { return sc_[q]; }
 };
 
 template <int NP>
 struct FaceK<NP, true> {
-    static constexpr int M = Sys<NP>::M, NA = M * (M - 1) / 2, N = NA + 2 * (M - 1) + 6;
-    double *s;  // this lane's column: element q at s[q * KS]
-    __device__ __forceinline__ explicit FaceK(double *col) : s(col) {}
-    __device__ __forceinline__ double &A(int i) { return s[i * KS]; }
-    __device__ __forceinline__ double &brow(int l) { return s[(NA + l) * KS]; }
-    __device__ __forceinline__ double &d0rn(int l) { return s[(NA + M - 1 + l) * KS]; }
-    __device__ __forceinline__ double &sc(int q) { return s[(NA + 2 * (M - 1) + q) * KS]; }
+    static constexpr int R = face_rec(NP), N = R + FK_N + 1;
+    double *s;  // this lane's column: element q at s[q / 2 * 2 * KS + q % 2]
+    __device__ __forceinline__ explicit FaceK(double *cols) : s(cols + 2 * threadIdx.x) {}
+    __device__ __forceinline__ void set(int i, double v) { s[i / 2 * 2 * KS + i % 2] = v; }
+    __device__ __forceinline__ void get(double (&v)[R]) const {
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) {
+            const double2 w = *reinterpret_cast<const double2 *>(s + i * 2 * KS);
+            v[2 * i] = w.x;
+            v[2 * i + 1] = w.y;
+        }
+    }
+    // the record from global memory, 16 bytes at a time past the L1 (no cell
+    // of the colour shares a face with another); fetched() ends the wait
+    __device__ __forceinline__ void fetch(const double *rec) const {
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) {
+            const unsigned dst = (unsigned)__cvta_generic_to_shared(s + i * 2 * KS);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(rec + 2 * i) : "memory");
+        }
+    }
+    __device__ __forceinline__ void fetched() const { asm volatile("cp.async.wait_all;" ::: "memory"); }
+    __device__ __forceinline__ double &sc(int q) { return s[(R + q) / 2 * 2 * KS + (R + q) % 2]; }
 };
-
-// the six scalars of FaceK
-enum { FK_PNB = 0, FK_D0EPNB, FK_K1, FK_K2, FK_D1, FK_INV };
 
 // The loop-invariant density stencil of one face's mass fluxes by phase: the
 // values of the cells n, f and o of face_mflux.  SH = true keeps them in this
@@ -135,69 +152,81 @@ struct DensK<NC, true> {
     __device__ __forceinline__ double &o(int l) { return s[(2 * NC + l) * KS]; }
 };
 
-template <int NP, bool RO, class KT>
-__device__ __forceinline__ void face_prepare(const Prm &P, const Fld &F, int c, int nb, int raw, int ii, int dir,
+// Fills K for the face of cell c whose row is held by cell rowc (c itself on
+// the plus side, the neighbour on the minus side), by axis q = dir (3D) or
+// 0 / 1 (2D): the record through an asynchronous copy, or, where iter keeps
+// none (F.fk null or a generic phase count), from the interphase terms and
+// tilde momenta.
+template <int NP, bool RO, bool SH, class KT>
+__device__ __forceinline__ void face_prepare(const Prm &P, const Fld &F, int c, int nb, int rowc, int ii, int dir,
                                              int side, double dt, KT &K) {
     const int nph = nphases<NP>(P);
     const size_t n = P.ncell;
     const double *dd = dir == 0 ? P.dx : (dir == 1 ? P.dy : P.dz);
     const double *hh = dir == 0 ? P.hx : (dir == 1 ? P.hy : P.hz);
-    double grav = dir == 0 ? P.gravx : (dir == 1 ? P.gravy : P.gravz);
-    const double *app = dir == 0 ? F.appu : (dir == 1 ? F.appv : F.appw);
-    const double *rg = dir == 0 ? F.rug : (dir == 1 ? F.rvg : F.rwg);
-    const double *rs = dir == 0 ? F.rus : (dir == 1 ? F.rvs : F.rws);
-    double alpha = P.alpha, ag = P.alphagrav;
-    double d0 = dd[ii], d1 = side > 0 ? dd[ii + 1] : dd[ii - 1];
-    double inv = side > 0 ? hh[ii] : hh[ii - 1];
-    int rowc = side > 0 ? c : raw;
+    const double d0 = dd[ii], d1 = side > 0 ? dd[ii + 1] : dd[ii - 1];
+    const double inv = side > 0 ? hh[ii] : hh[ii - 1];
+    bool rec = false;
+    if constexpr (SH) {
+        if (F.fk) {
+            K.fetch(face_rec_ptr<NP>(P, F, P.d3 ? dir : dir / 2, rowc));
+            rec = true;
+        }
+    }
+    if (!rec) {
+        const double *app = dir == 0 ? F.appu : (dir == 1 ? F.appv : F.appw);
+        const double *rg = dir == 0 ? F.rug : (dir == 1 ? F.rvg : F.rwg);
+        const double *rs = dir == 0 ? F.rus : (dir == 1 ? F.rvs : F.rws);
+        const int nap = nph * (nph + 1) / 2;
+#pragma unroll
+        for (int ls = 1; ls <= nap; ++ls)
+            K.set(ls - 1, P.alpha * (d0 * __ldg(app + (ls - 1) * n + nb) + d1 * __ldg(app + (ls - 1) * n + c)) * inv);
+        K.set(nap, __ldg(rg + rowc));
+#pragma unroll
+        for (int l = 2; l <= nph; ++l) K.set(nap + l - 1, __ldg(rs + (l - 2) * n + rowc));
+    }
+    K.sc(FK_D0) = d0;
     K.sc(FK_D1) = d1;
     K.sc(FK_INV) = inv;
     K.sc(FK_PNB) = ldro<RO>(F.p + nb);
     K.sc(FK_D0EPNB) = P.pmodel == 1 ? d0 * ldro<RO>(F.ep + nb) : 0.0;
-    K.sc(FK_K1) = alpha * dt * inv * 2.0;
-    K.sc(FK_K2) = dt * ag * inv * grav;
-    K.brow(0) = __ldg(rg + rowc);
-    K.d0rn(0) = d0 * ldro<RO>(F.rgp + nb);
-#pragma unroll
-    for (int l = 2; l <= nph; ++l) {
-        K.brow(l - 1) = __ldg(rs + (l - 2) * n + rowc);
-        K.d0rn(l - 1) = d0 * ldro<RO>(F.rlk + (l - 2) * n + nb);
-    }
-    const int nap = nph * (nph + 1) / 2;
-#pragma unroll
-    for (int ls = 1; ls <= nap; ++ls)
-        K.A(ls - 1) = alpha * (d0 * __ldg(app + (ls - 1) * n + nb) + d1 * __ldg(app + (ls - 1) * n + c)) * inv;
+    K.sc(FK_K1) = P.alpha * dt * inv * 2.0;
+    K.sc(FK_K2) = dt * P.alphagrav * inv * (dir == 0 ? P.gravx : (dir == 1 ? P.gravy : P.gravz));
 }
 
-// the in-loop assembly and solution; side as in face_system
-template <int NP, class KT>
-__device__ __forceinline__ void face_assemble(const Prm &P, KT &K, int side, double pc, double epc,
+// the in-loop assembly and solution: K and Dk of the face, the cell's
+// current p, ep, rgp and rlk; side +1 for E/N/T, -1 for W/S/B faces
+template <int NP, class KT, class DT>
+__device__ __forceinline__ void face_assemble(const Prm &P, KT &K, DT &Dk, int side, double pc, double epc,
                                               double rgpc, const double *rlkc, double *v) {
     constexpr int M = Sys<NP>::M;
-    const int nph = nphases<NP>(P);
-    double a[M][M], b[M];
-    double d1 = K.sc(FK_D1), inv = K.sc(FK_INV), pnb = K.sc(FK_PNB), K1 = K.sc(FK_K1), K2 = K.sc(FK_K2);
+    const int nph = nphases<NP>(P), nap = nph * (nph + 1) / 2;
+    double a[M][M], b[M], rec[KT::R];
+    K.get(rec);
+    const double d0 = K.sc(FK_D0), d1 = K.sc(FK_D1), inv = K.sc(FK_INV), pnb = K.sc(FK_PNB);
+    const double K1 = K.sc(FK_K1), K2 = K.sc(FK_K2);
     double dp = side > 0 ? pc - pnb : pnb - pc;
     double ep_f = 1.0;
     if (P.pmodel == 1) ep_f = (K.sc(FK_D0EPNB) + d1 * epc) * inv;
-    b[1] = K.brow(0) + K1 * ep_f * dp;
-    b[1] = b[1] + K2 * (K.d0rn(0) + d1 * rgpc);
-    a[1][1] = K.A(0) + (K.d0rn(0) + d1 * rgpc) * inv;
+    b[1] = rec[nap] + K1 * ep_f * dp;
+    const double rgf = d0 * Dk.n(0) + d1 * rgpc;
+    b[1] = b[1] + K2 * rgf;
+    a[1][1] = rec[0] + rgf * inv;
 #pragma unroll
     for (int l = 2; l <= nph; ++l) {
-        double rc = rlkc[l - 2];
+        const double rf = d0 * Dk.n(l - 1) + d1 * rlkc[l - 2];
         double eps_f = 0.0;
-        if (P.pmodel == 1) eps_f = (K.d0rn(l - 1) + d1 * rc) * inv * P.inrl[l - 1];
-        b[l] = K.brow(l - 1) + K1 * eps_f * dp;
-        b[l] = b[l] + K2 * (K.d0rn(l - 1) + d1 * rc);
+        if (P.pmodel == 1) eps_f = rf * inv * P.inrl[l - 1];
+        b[l] = rec[nap + l - 1] + K1 * eps_f * dp;
+        b[l] = b[l] + K2 * rf;
         int ls1 = l * (l - 1) / 2;
 #pragma unroll
         for (int ll = 1; ll <= l; ++ll) {
-            double val = K.A(ls1 + ll - 1);
+            double val = rec[ls1 + ll - 1];
             a[l][ll] = val;
             a[ll][l] = val;
         }
-        a[l][l] = a[l][l] + (K.d0rn(l - 1) + d1 * rc) * inv;
+        a[l][l] = a[l][l] + rf * inv;
     }
     gauss_jordan_t<NP>(P, a, b);
 #pragma unroll
@@ -301,8 +330,8 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
     vel[0] = gvel[fcell];
 #pragma unroll
     for (int l = 2; l <= nph; ++l) vel[l - 1] = svel[(l - 2) * n + fcell];
-    FaceK<NP, SH> K(kcols + threadIdx.x);
-    if (solved) face_prepare<NP, RO>(P, F, c, rn, rawnb, ii, dir, minus ? -1 : +1, dt, K);
+    FaceK<NP, SH> K(kcols);
+    if (solved) face_prepare<NP, RO, SH>(P, F, c, rn, fcell, ii, dir, minus ? -1 : +1, dt, K);
     // density stencil of this face's mass fluxes by phase (gas first).  A
     // slot remapped to the cell reads the cell's own current value, except in
     // opt_inner_loop (iter.f:1255-1547), which builds the stencils once and
@@ -376,12 +405,13 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
     double flux[NC];  // this lane's face mass flux by phase (gas first)
 #pragma unroll
     for (int l = 0; l < NC; ++l) flux[l] = 0.0;
+    if constexpr (SH) K.fetched();
     for (int loop = 1; loop <= P.inmax; ++loop) {
         if (loop > 1 || nit > 1) padjust(s, p, kros, d3, p3, P.omega, abeta);
         rog = p / rgas_tg * mg;  // thermal_eosg
         rgp = ep * rog;
         // this lane's face system (matrix.f:351-630)
-        if (solved) face_assemble<NP>(P, K, minus ? -1 : +1, p, ep, rgp, rlk, vel);
+        if (solved) face_assemble<NP>(P, K, Dk, minus ? -1 : +1, p, ep, rgp, rlk, vel);
         // particle mass fluxes and volume fractions (iter.f:778-994)
 #pragma unroll
         for (int is = 1; is <= ns; ++is) flux[is] = mflux(is, rlk[is - 1]);

@@ -588,8 +588,8 @@ __global__ void k_predictor2d(Prm P, Fld F, double dt) {
     Rem2 M;
     raw2(P, i, k, R);
     rem2(P, i, k, R, M);
-    face_solve<NP>(P, F, c, M.e, R.e, i, 0, +1, dt);
-    face_solve<NP>(P, F, c, M.t, R.t, k, 2, +1, dt);
+    face_solve<NP>(P, F, c, M.e, R.e, i, 0, dt);
+    face_solve<NP>(P, F, c, M.t, R.t, k, 2, dt);
 }
 
 // gas mass flux of one cell over its four faces (calc_gas_mass_flux,

@@ -546,9 +546,9 @@ __global__ void k_predictor3d(Prm P, Fld F, double dt) {
     Rem3 M;
     raw3(P, i, j, k, R);
     rem3(P, i, j, k, R, M);
-    face_solve<NP>(P, F, c, M.e, R.e, i, 0, +1, dt);
-    face_solve<NP>(P, F, c, M.n, R.n, j, 1, +1, dt);
-    face_solve<NP>(P, F, c, M.t, R.t, k, 2, +1, dt);
+    face_solve<NP>(P, F, c, M.e, R.e, i, 0, dt);
+    face_solve<NP>(P, F, c, M.n, R.n, j, 1, dt);
+    face_solve<NP>(P, F, c, M.t, R.t, k, 2, dt);
 }
 
 // mass flux of one cell over its six faces (calc_gas_mass_flux and

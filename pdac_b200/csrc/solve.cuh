@@ -57,17 +57,28 @@ __device__ __forceinline__ void gauss_jordan_t(const Prm &P, double (&a)[M][M], 
     }
 }
 
-// Phase matrix of one face, matrix.f:38-328, solved (matrix.f:351-630) into
-// the face velocities v[0..nph-1] (gas first).  dir 0/1/2 = x/y/z; side +1 =
-// the E/N/T face of cell c (assemble_matrix), side -1 = its W/S/B face
-// (assemble_all_matrix).  nb = remapped face neighbour, raw = raw face
-// neighbour (whose row holds the tilde momentum of a W/S/B face), ii = the
-// cell's index along dir.  The cell's own p, ep, rgp and rlk come in
-// registers; neighbour values and the tilde terms are read-only here.
+// Doubles of one face record (F.fk): the face's interphase terms
+// alpha (d0 app(nb) + d1 app(c)) / (d0 + d1) by interphase index, then the
+// tilde momenta of its row (gas first), padded to whole 16-byte pairs.
+__host__ __device__ constexpr int face_rec(int nph) { return (nph * (nph + 1) / 2 + nph + 1) / 2 * 2; }
+// the record of the E/N/T face of cell c along axis q (0 = x, last = z)
 template <int NP>
-__device__ __forceinline__ void face_system(const Prm &P, const Fld &F, int c, int nb, int raw, int ii, int dir,
-                                            int side, double dt, double pc, double epc, double rgpc,
-                                            const double *rlkc, double *v) {
+__device__ __forceinline__ double *face_rec_ptr(const Prm &P, const Fld &F, int q, int c) {
+    return F.fk + ((size_t)q * P.ncell + c) * face_rec(NP);
+}
+
+// The predictor's face solution (iter.f:135-145): the phase matrix of the
+// E/N/T face of cell c along dir (matrix.f:38-328), solved
+// (matrix.f:351-630), its velocities stored, when the raw face neighbour is
+// fluid.  nb = remapped face neighbour, ii = the cell's index along dir.
+// Writes the face's record, which the inner loop of either of its cells
+// reads for the rest of iter: neither the interphase terms nor the tilde
+// momenta change there, and a face between two fluid cells has the same
+// terms seen from both.
+template <int NP>
+__device__ __forceinline__ void face_solve(const Prm &P, const Fld &F, int c, int nb, int raw, int ii, int dir,
+                                           double dt) {
+    if (!(P.flag[raw] & 1)) return;
     constexpr int M = Sys<NP>::M;
     const int nph = nphases<NP>(P);
     const size_t n = P.ncell;
@@ -78,59 +89,53 @@ __device__ __forceinline__ void face_system(const Prm &P, const Fld &F, int c, i
     const double *rs = dir == 0 ? F.rus : (dir == 1 ? F.rvs : F.rws);
     double alpha = P.alpha, ag = P.alphagrav;
     double a[M][M], b[M];
-    // side +1: d0 = d(ii), d1 = d(ii+1); side -1: d0 = d(ii), d1 = d(ii-1)
-    double d0 = dd[ii], d1 = side > 0 ? dd[ii + 1] : dd[ii - 1];
-    double inv = 1.0 / (d0 + d1);
-    int rowc = side > 0 ? c : raw;
-    double pnb = __ldg(F.p + nb), rgpnb = __ldg(F.rgp + nb);
-    double dp = side > 0 ? pc - pnb : pnb - pc;
+    double d0 = dd[ii], d1 = dd[ii + 1];
+    double inv = dir == 0 ? P.hx[ii] : (dir == 1 ? P.hy[ii] : P.hz[ii]);
+    constexpr int RS = NP > 0 ? face_rec(NP) : 2, NA = NP * (NP + 1) / 2;
+    double rec[RS];
+    if (NP > 0) rec[RS - 1] = 0.0;  // the padding, where there is one
+    double pnb = __ldg(F.p + nb), rgpnb = __ldg(F.rgp + nb), rgpc = F.rgp[c];
+    double dp = F.p[c] - pnb;
     double ep_f = 1.0;
-    if (P.pmodel == 1) ep_f = (d0 * __ldg(F.ep + nb) + d1 * epc) * inv;
-    b[1] = __ldg(rg + rowc) + alpha * dt * inv * 2.0 * ep_f * dp;
+    if (P.pmodel == 1) ep_f = (d0 * __ldg(F.ep + nb) + d1 * F.ep[c]) * inv;
+    const double r1 = __ldg(rg + c);
+    if (NP > 0) rec[NA] = r1;
+    b[1] = r1 + alpha * dt * inv * 2.0 * ep_f * dp;
     b[1] = b[1] + dt * ag * inv * grav * (d0 * rgpnb + d1 * rgpc);
     a[1][1] = alpha * (d0 * __ldg(app + nb) + d1 * __ldg(app + c)) * inv;
+    if (NP > 0) rec[0] = a[1][1];
     a[1][1] = a[1][1] + (d0 * rgpnb + d1 * rgpc) * inv;
 #pragma unroll
     for (int l = 2; l <= nph; ++l) {
-        double rn = __ldg(F.rlk + (l - 2) * n + nb), rc = rlkc[l - 2];
+        double rn = __ldg(F.rlk + (l - 2) * n + nb), rc = F.rlk[(l - 2) * n + c];
         double eps_f = 0.0;
         if (P.pmodel == 1) eps_f = (d0 * rn + d1 * rc) * inv * P.inrl[l - 1];
-        b[l] = __ldg(rs + (l - 2) * n + rowc) + alpha * dt * inv * 2.0 * eps_f * dp;
+        const double rl = __ldg(rs + (l - 2) * n + c);
+        if (NP > 0) rec[NA + l - 1] = rl;
+        b[l] = rl + alpha * dt * inv * 2.0 * eps_f * dp;
         b[l] = b[l] + dt * ag * inv * grav * (d0 * rn + d1 * rc);
         int ls1 = l * (l - 1) / 2;
 #pragma unroll
         for (int ll = 1; ll <= l; ++ll) {
             int ls = ls1 + ll;
             double val = alpha * (d0 * __ldg(app + (ls - 1) * n + nb) + d1 * __ldg(app + (ls - 1) * n + c)) * inv;
+            if (NP > 0) rec[ls - 1] = val;
             a[l][ll] = val;
             a[ll][l] = val;
         }
         a[l][l] = a[l][l] + (d0 * rn + d1 * rc) * inv;
     }
+    if (NP > 0 && F.fk) {
+        double2 *w = reinterpret_cast<double2 *>(face_rec_ptr<NP>(P, F, P.d3 ? dir : dir / 2, c));
+#pragma unroll
+        for (int q = 0; q < RS / 2; ++q) w[q] = make_double2(rec[2 * q], rec[2 * q + 1]);
+    }
     gauss_jordan_t<NP>(P, a, b);
-#pragma unroll
-    for (int l = 1; l <= nph; ++l) v[l - 1] = b[l];
-}
-
-// face_system with the cell's state read from and the velocities stored to
-// memory, when the raw face neighbour is fluid (the predictor, iter.f:135-145)
-template <int NP>
-__device__ __forceinline__ void face_solve(const Prm &P, const Fld &F, int c, int nb, int raw, int ii, int dir,
-                                           int side, double dt) {
-    if (!(P.flag[raw] & 1)) return;
-    constexpr int M = Sys<NP>::M;
-    const int nph = nphases<NP>(P);
-    const size_t n = P.ncell;
-    double rlkc[M - 1], v[M - 1];
-#pragma unroll
-    for (int l = 2; l <= nph; ++l) rlkc[l - 2] = F.rlk[(l - 2) * n + c];
-    face_system<NP>(P, F, c, nb, raw, ii, dir, side, dt, F.p[c], F.ep[c], F.rgp[c], rlkc, v);
-    int store = side > 0 ? c : raw;
     double *g = dir == 0 ? F.ug : (dir == 1 ? F.vg : F.wg);
     double *s = dir == 0 ? F.us : (dir == 1 ? F.vs : F.ws);
-    g[store] = v[0];
+    g[c] = b[1];
 #pragma unroll
-    for (int l = 2; l <= nph; ++l) s[(l - 2) * n + store] = v[l - 1];
+    for (int l = 2; l <= nph; ++l) s[(l - 2) * n + c] = b[l];
 }
 
 // value of a stencil slot: the cell's own current value where the (remapped)
