@@ -399,7 +399,8 @@ int pdac_gpu_elapsed(pdac_ctx *ctx, int a, int b, double *ms);
  *   [1] planes of a tiled block's march up k;
  *   [2] blocks of the corrector's inner-loop kernel;
  *   [3] blocks of its residual-test kernel;
- *   [4] cells per block of the one-launch sweep loop of small domains.
+ *   [4] cells per block of the sweep loop on a cooperative grid (not used
+ *       by the 2D meshes whose sweep loop runs on one cluster).
  * None of them changes a result: only the speed.
  * pdac_gpu_autotune times candidates on the context's current state and
  * installs the fastest: the momentum-flux pass directly (it rewrites the
@@ -425,8 +426,9 @@ int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin);
  * with the members' kernels running concurrently on the device.  A member on
  * the semi-implicit path (time_integration = 0, rungekut = 1, no implicit-
  * flux modes, cstop unset, more than one gas) takes its whole step as
- * graph nodes -- boundary to ftem, the outer sweep loop as a conditional
- * node, its outcome copied back once -- and all such members' nodes form
+ * graph nodes -- boundary to ftem, the outer sweep loop as one kernel on a
+ * thread-block cluster (small 2D meshes) or a conditional node, its outcome
+ * copied back once -- and all such members' nodes form
  * ONE CUDA graph (independent branches), launched once per batch step by
  * the calling thread (rebuilt after a member's launch shapes change; one
  * graph per member if that graph cannot be instantiated); the other
@@ -434,11 +436,11 @@ int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin);
  * threads (<= 0: one per such member).  Both give the member's results of
  * pdac_gpu_step, bit for bit; pdac_gpu_phase_times is not updated by a
  * graph step.  While in a batch, members run without cooperative launches
- * (the small-domain sweep loop and the explicit solver's wavefront take
- * their multi-launch forms, with the same results), so that no two
- * cooperative grids share the device.  The batch does not own the members: create, upload and download
- * them with the per-context calls, never while a batch step runs, and
- * destroy the batch before them.  A member appears once.
+ * (the sweep loop on a grid and the explicit solver's wavefront take their
+ * multi-launch forms, with the same results), so that no two cooperative
+ * grids share the device.  The batch does not own the members: create,
+ * upload and download them with the per-context calls, never while a batch
+ * step runs, and destroy the batch before them.  A member appears once.
  * pdac_gpu_batch_step fills nit[m] and status[m] (either may be NULL) for
  * every member, steps every member whatever the others return, and returns
  * the first non-zero member status (its message in

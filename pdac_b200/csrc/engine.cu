@@ -67,7 +67,7 @@ struct pdac_ctx {
     long long step_launches = 0;
     int *d_status = nullptr, *h_status = nullptr;
     unsigned *d_dirty = nullptr;                 // corrector active set, one bit per cell
-    int *d_cand = nullptr;                       // candidate cells of one colour phase
+    unsigned *d_cmask = nullptr;                 // fluid cells per colour, the active set's words
     int inner_grid = 0;
     int *d_nit = nullptr, *h_nit = nullptr;  // outer sweep number (device, pinned host)
     // the outer sweep loop as a graph: a conditional WHILE node whose body is
@@ -76,16 +76,18 @@ struct pdac_ctx {
     cudaGraphExec_t it_exec = nullptr;
     double it_dt = 0.0;
     long long it_per_sweep = 10;  // kernels of one sweep of that graph
-    // small domains: the whole sweep loop as one cooperative launch of
-    // coop_blocks blocks (0: the graph), coop_cpb cells per block, at most
-    // coop_max_blocks blocks resident at once
+    // the form of iter's sweep loop (setup_sweep_loop): one launch on a
+    // cluster of cluster_blocks blocks, else one cooperative launch of
+    // coop_blocks blocks (coop_cpb cells per block, at most coop_max_blocks
+    // resident at once), else (both 0) the graph
     int coop_blocks = 0, coop_cpb = 1024, coop_max_blocks = 0;
+    int cluster_blocks = 0;
     // grid of the residual-test kernels (0: half the inner-loop grid)
     int test_grid = 0;
-    // cooperative launches (the small-domain sweep loop, the explicit
-    // solver's wavefront) only when the context is not stepped alongside
-    // others: a batch turns them off in its members, so that no two
-    // cooperative grids are in flight on the device at once
+    // cooperative launches (the sweep loop, the explicit solver's wavefront)
+    // only when the context is not stepped alongside others: a batch turns
+    // them off in its members, so that no two cooperative grids are in
+    // flight on the device at once (see coop_lock)
     bool allow_coop = true;
     std::vector<double> sweep_log;  // per colour phase when profiling: sweep, colour, worklist, tested, ms x2
     bool prof = false;
@@ -263,8 +265,14 @@ static cudaError_t set_inner_attrs_np() {
     const int sm = (int)pdac::inner_smem_bytes<NP>();
     cudaError_t e = cudaFuncSetAttribute(pdac::k_inner_team<NP, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(pdac::k_inner_team<NP, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(pdac::k_iter_coop<NP, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(pdac::k_iter_coop<NP, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    auto loop = [&](auto kernel, bool cluster) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pdac::sweep_smem_bytes<NP>());
+        if (cluster && e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    };
+    loop(pdac::k_sweep_loop<NP, 2, false>, false);
+    loop(pdac::k_sweep_loop<NP, 3, false>, false);
+    loop(pdac::k_sweep_loop<NP, 2, true>, true);
     return e;
 }
 static cudaError_t set_inner_attrs() {
@@ -599,76 +607,117 @@ int setup_wave(pdac_ctx *ctx, const int *flag) {
 
 }  // namespace
 
-// Domains of at most this many cells run iter's sweep loop as one
-// cooperative launch (k_iter_coop): their colour phases are a few
-// microseconds of work each, less than the launch of a graph node.
-#ifndef PDAC_COOP_MAX_CELLS
-#define PDAC_COOP_MAX_CELLS (1 << 18)
+// 2D meshes of at most this many cells run iter's sweep loop on one cluster
+// of 16 blocks: their colour phases hold a few hundred cells, and the
+// hardware's cluster barrier costs a fraction of a grid-wide one.  Measured
+// (ms of a burst, cluster against grid): 128 x 192 35.9 / 38.1, 251 x 383
+// 35.5 / 38.9, 384 x 640 125.8 / 95.2 (its worklists outgrow the cluster's 64
+// warps); 3D meshes have long worklists from the start (24^3 10.5 / 7.4) and
+// always take the grid.
+#ifndef PDAC_CLUSTER_MAX_CELLS
+#define PDAC_CLUSTER_MAX_CELLS (1 << 17)
 #endif
-#ifndef PDAC_COOP_CELLS_PER_BLOCK
-#define PDAC_COOP_CELLS_PER_BLOCK 1024
-#endif
+constexpr int CLUSTER_BLOCKS = 16;
 
+// the sweep loop in one launch on stream st
 template <int NP>
-static cudaError_t launch_iter_coop_np(pdac_ctx *ctx, double dt, cudaStream_t st, const pdac::SweepWork &W) {
+static cudaError_t launch_sweep_loop_np(pdac_ctx *ctx, double dt, cudaStream_t st, const pdac::SweepWork &W) {
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    lc.gridDim = dim3(ctx->coop_blocks);
+    const bool cl = ctx->cluster_blocks > 0;
+    if (cl) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = ctx->cluster_blocks;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    lc.gridDim = dim3(cl ? ctx->cluster_blocks : ctx->coop_blocks);
     lc.blockDim = dim3(TPB_TEAM);
-    lc.dynamicSmemBytes = pdac::inner_smem_bytes<NP>();
+    lc.dynamicSmemBytes = pdac::sweep_smem_bytes<NP>();
     lc.stream = st;
     lc.attrs = at;
     lc.numAttrs = 1;
-    if (ctx->d3) return cudaLaunchKernelEx(&lc, pdac::k_iter_coop<NP, 3>, ctx->P, ctx->F, dt, W, ctx->cfg.maxout);
-    return cudaLaunchKernelEx(&lc, pdac::k_iter_coop<NP, 2>, ctx->P, ctx->F, dt, W, ctx->cfg.maxout);
+    const int mo = ctx->cfg.maxout;
+    if (ctx->d3) return cudaLaunchKernelEx(&lc, pdac::k_sweep_loop<NP, 3, false>, ctx->P, ctx->F, dt, W, mo);
+    return cl ? cudaLaunchKernelEx(&lc, pdac::k_sweep_loop<NP, 2, true>, ctx->P, ctx->F, dt, W, mo)
+              : cudaLaunchKernelEx(&lc, pdac::k_sweep_loop<NP, 2, false>, ctx->P, ctx->F, dt, W, mo);
 }
 
-static cudaError_t launch_iter_coop(pdac_ctx *ctx, double dt, cudaStream_t st, const pdac::SweepWork &W) {
+static cudaError_t launch_sweep_loop(pdac_ctx *ctx, double dt, cudaStream_t st) {
+    const pdac::SweepWork W{ctx->d_wcount, ctx->d_wcount + 9, ctx->d_work, ctx->d_dirty, ctx->d_cmask, ctx->d_nit, ctx->work_stride};
     switch (ctx->nph) {
-        case 2: return launch_iter_coop_np<2>(ctx, dt, st, W);
-        case 3: return launch_iter_coop_np<3>(ctx, dt, st, W);
-        case 4: return launch_iter_coop_np<4>(ctx, dt, st, W);
-        case 6: return launch_iter_coop_np<6>(ctx, dt, st, W);
-        default: return launch_iter_coop_np<0>(ctx, dt, st, W);
+        case 2: return launch_sweep_loop_np<2>(ctx, dt, st, W);
+        case 3: return launch_sweep_loop_np<3>(ctx, dt, st, W);
+        case 4: return launch_sweep_loop_np<4>(ctx, dt, st, W);
+        case 6: return launch_sweep_loop_np<6>(ctx, dt, st, W);
+        default: return launch_sweep_loop_np<0>(ctx, dt, st, W);
     }
 }
 
-// the cooperative grid of a small domain: one block of 128 threads per
-// PDAC_COOP_CELLS_PER_BLOCK cells, within what the device holds at once
-// (measured on the 128 x 192 2D plume: 1024 and 256 cells per block run
-// the step in 6.43 ms, 4096 in 7.46 ms, 64 in 6.76 ms)
-static int setup_iter_coop(pdac_ctx *ctx) {
-    ctx->coop_blocks = 0;
-    if ((long)ctx->ncell > PDAC_COOP_MAX_CELLS) return PDAC_OK;
-    int dev = 0, coop = 0, nsm = 0, occ = 0;
+// the blocks of the two one-launch forms the device holds at once
+template <int NP, int D>
+static cudaError_t sweep_loop_room(int nsm, int &grid_blocks, int &clusters) {
+    const size_t sm = pdac::sweep_smem_bytes<NP>();
+    int occ = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_sweep_loop<NP, D, false>, TPB_TEAM, sm);
+    grid_blocks = occ * nsm;
+    clusters = 0;
+    if (e != cudaSuccess || D == 3) return e;
+    cudaLaunchConfig_t lc = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CLUSTER_BLOCKS;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    lc.gridDim = dim3(CLUSTER_BLOCKS);
+    lc.blockDim = dim3(TPB_TEAM);
+    lc.dynamicSmemBytes = sm;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    return cudaOccupancyMaxActiveClusters(&clusters, pdac::k_sweep_loop<NP, 2, true>, &lc);
+}
+
+// The form of the sweep loop.  One launch whose blocks stay resident spares
+// each colour phase its two launches, which the barriers between the residual
+// tests and the inner loop replace: a cluster for the 2D meshes above, a
+// cooperative grid for all others (one block per 64 cells up to what the
+// device holds in 3D, per 1024 in 2D, where the worklists are short and a
+// barrier over fewer blocks is quicker: 384 x 640 95.2 ms against 98.9 with
+// 64).  Against the graph of launches the grid took 128 x 128 x 96 from 85.2
+// to 76.5 ms a burst and 256 x 256 x 192 from 506.7 to 469.8.  The graph runs
+// what the cooperative grid may not (members of a batch, implicit modes).
+static int setup_sweep_loop(pdac_ctx *ctx) {
+    ctx->coop_blocks = ctx->cluster_blocks = 0;
+    int dev = 0, coop = 0, nsm = 0, clusters = 0, room = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    if (!coop) return PDAC_OK;
-    auto occ_of = [&](auto kernel, size_t smem) {
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, TPB_TEAM, smem);
-    };
-    cudaError_t e;
     switch (ctx->nph) {
-        case 2: e = ctx->d3 ? occ_of(pdac::k_iter_coop<2, 3>, pdac::inner_smem_bytes<2>())
-                            : occ_of(pdac::k_iter_coop<2, 2>, pdac::inner_smem_bytes<2>()); break;
-        case 3: e = ctx->d3 ? occ_of(pdac::k_iter_coop<3, 3>, pdac::inner_smem_bytes<3>())
-                            : occ_of(pdac::k_iter_coop<3, 2>, pdac::inner_smem_bytes<3>()); break;
-        case 4: e = ctx->d3 ? occ_of(pdac::k_iter_coop<4, 3>, pdac::inner_smem_bytes<4>())
-                            : occ_of(pdac::k_iter_coop<4, 2>, pdac::inner_smem_bytes<4>()); break;
-        case 6: e = ctx->d3 ? occ_of(pdac::k_iter_coop<6, 3>, pdac::inner_smem_bytes<6>())
-                            : occ_of(pdac::k_iter_coop<6, 2>, pdac::inner_smem_bytes<6>()); break;
-        default: e = ctx->d3 ? occ_of(pdac::k_iter_coop<0, 3>, pdac::inner_smem_bytes<0>())
-                             : occ_of(pdac::k_iter_coop<0, 2>, pdac::inner_smem_bytes<0>()); break;
+        case 2: CK((ctx->d3 ? sweep_loop_room<2, 3> : sweep_loop_room<2, 2>)(nsm, room, clusters)); break;
+        case 3: CK((ctx->d3 ? sweep_loop_room<3, 3> : sweep_loop_room<3, 2>)(nsm, room, clusters)); break;
+        case 4: CK((ctx->d3 ? sweep_loop_room<4, 3> : sweep_loop_room<4, 2>)(nsm, room, clusters)); break;
+        case 6: CK((ctx->d3 ? sweep_loop_room<6, 3> : sweep_loop_room<6, 2>)(nsm, room, clusters)); break;
+        default: CK((ctx->d3 ? sweep_loop_room<0, 3> : sweep_loop_room<0, 2>)(nsm, room, clusters)); break;
     }
-    CK(e);
-    ctx->coop_cpb = PDAC_COOP_CELLS_PER_BLOCK;
-    ctx->coop_max_blocks = occ * nsm;
+    if (!ctx->d3 && (long)ctx->ncell <= PDAC_CLUSTER_MAX_CELLS && clusters > 0) ctx->cluster_blocks = CLUSTER_BLOCKS;
+    if (!coop) return PDAC_OK;
+    ctx->coop_cpb = ctx->d3 ? 64 : 1024;
+    ctx->coop_max_blocks = room;
     const int want = std::max(1, (int)((ctx->ncell + ctx->coop_cpb - 1) / ctx->coop_cpb));
     ctx->coop_blocks = std::min(want, ctx->coop_max_blocks);
     return PDAC_OK;
+}
+
+// Held while a cooperative grid of this library is in flight on a device:
+// contexts may be stepped from several host threads, and two such grids at
+// once could each hold part of the device and wait for the rest.  iter takes
+// the graph form instead of waiting.
+static std::mutex &coop_lock() {
+    static std::mutex mu[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
+    return mu[dev % 64];
 }
 
 extern "C" {
@@ -890,7 +939,9 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     CK(cudaMallocHost(&ctx->h_status, 4 * sizeof(int)));
     CK(cudaMalloc(&ctx->d_wcount, 16 * sizeof(int)));
     CK(cudaMalloc(&ctx->d_dirty, ((size_t)n + 31) / 32 * sizeof(unsigned)));
-    CK(cudaMalloc(&ctx->d_cand, (size_t)n * sizeof(int)));
+    CK(cudaMalloc(&ctx->d_cmask, (size_t)3 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
+    pdac::k_colour_masks<<<blocks(((long)n + 31) / 32), TPB, 0, ctx->stream>>>(P, ctx->d_cmask);
+    CK(cudaGetLastError());
     {
         int dev = 0, nsm = 148;
         CK(cudaGetDevice(&dev));
@@ -1042,7 +1093,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
         int st = setup_wave(ctx, cfg->flag);
         if (st) return st;
     } else {
-        int st = setup_iter_coop(ctx);
+        int st = setup_sweep_loop(ctx);
         if (st) return st;
     }
     if (cfg->isink > 0) {
@@ -1109,7 +1160,7 @@ int pdac_gpu_destroy(pdac_ctx *ctx) {
     if (ctx->ex_graph) cudaGraphDestroy(ctx->ex_graph);
     cudaFree(ctx->d_nit);
     cudaFreeHost(ctx->h_nit);
-    cudaFree(ctx->d_cand);
+    cudaFree(ctx->d_cmask);
     cudaFree(ctx->d_partial);
     cudaFree(ctx->d_fk);
     cudaFree(ctx->d_sinkbuf);
@@ -1429,10 +1480,10 @@ static int enqueue_htilde(pdac_ctx *ctx, double dt, cudaStream_t st);
 static int enqueue_ftem(pdac_ctx *ctx, double dt, cudaStream_t st, bool in_sweep);
 
 // one outer sweep of the corrector (iter.f:241-410): three colour phases of
-// candidate collection, residual test and inner loop; the sweep number is
-// read on the device from d_nit
+// residual test and inner loop; the sweep number is read on the device from
+// d_nit
 // kernels of the corrector in one graph sweep, k_sweep_check included
-static long long sweep_kernels(const pdac_ctx *) { return 10; }
+static long long sweep_kernels(const pdac_ctx *) { return 7; }
 
 // warps k_inner_team may spread a short worklist over: those resident at
 // once, or none beyond the packed ones for a member of a batch
@@ -1449,7 +1500,7 @@ static int enqueue_sweep(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof) {
         if (s) return s;
     }
     const int nph = ctx->nph;
-    const size_t n = ctx->ncell, nwords = (n + 31) / 32;
+    const size_t nwords = ((size_t)ctx->ncell + 31) / 32;
     const long nthr = (long)((ctx->nx + 2) / 3) * ctx->ny * ctx->nz;
     const int test_grid = ctx->test_grid > 0 ? ctx->test_grid : std::max(1, ctx->inner_grid / 2);
     // one team of lanes per worklist cell (5 teams of 6 lanes per warp in
@@ -1460,12 +1511,12 @@ static int enqueue_sweep(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof) {
     // [col] worklist length, [3 + col] cells tested, [6 + col] candidates, of colour col
     CK(cudaMemsetAsync(ctx->d_wcount, 0, 9 * sizeof(int), st));
     for (int col = 0; col < 3; ++col) {
-        int *cnt = ctx->d_wcount + col, *ncand = ctx->d_wcount + 6 + col;
+        int *cnt = ctx->d_wcount + col;
         if (prof) CK(cudaEventRecord(ctx->cev[3 * col], st));
-        pdac::k_resid_collect<<<blocks((long)nwords, TPB_RESID), TPB_RESID, 0, st>>>(ctx->P, col, dirty, ctx->d_cand, ncand);
+        const unsigned *cmask = ctx->d_cmask + (size_t)col * nwords;
         int *wl = ctx->d_work + col * ctx->work_stride;
-        if (ctx->d3) PHASE_LAUNCH_D(nph, pdac::k_resid_test, 3, test_grid, TPB_RESID, st, ctx->P, F, dt, ctx->d_cand, ncand, wl, cnt, dirty);
-        else PHASE_LAUNCH_D(nph, pdac::k_resid_test, 2, test_grid, TPB_RESID, st, ctx->P, F, dt, ctx->d_cand, ncand, wl, cnt, dirty);
+        if (ctx->d3) PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 3, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, dirty, wl, cnt);
+        else PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 2, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, dirty, wl, cnt);
         if (prof) CK(cudaEventRecord(ctx->cev[3 * col + 1], st));
         if (ctx->d3) INNER_LAUNCH_D(nph, pdac::k_inner_team, 3, g, TPB_TEAM, st, ctx->P, F, dt, ctx->d_nit, wl, cnt, dirty, inner_spread(ctx));
         else INNER_LAUNCH_D(nph, pdac::k_inner_team, 2, g, TPB_TEAM, st, ctx->P, F, dt, ctx->d_nit, wl, cnt, dirty, inner_spread(ctx));
@@ -1570,13 +1621,21 @@ int pdac_gpu_iter(pdac_ctx *ctx, double dt, int *nit_out) {
     // every cell is tested in the first sweep
     CK(cudaMemsetAsync(ctx->d_dirty, 0xff, (n + 31) / 32 * sizeof(unsigned), st));
     int nit;
-    const bool coop = ctx->coop_blocks > 0 && ctx->allow_coop && !ctx->cfg.implicit_fluxes && !ctx->cfg.implicit_enthalpy;
-    if (!ctx->prof && coop) {
-        // small domain: the sweep loop in one cooperative launch
-        pdac::SweepWork W{ctx->d_wcount, ctx->d_cand, ctx->d_work, ctx->d_dirty, ctx->d_nit, ctx->work_stride};
-        CK(launch_iter_coop(ctx, dt, st, W));
+    const bool explicit_modes = !ctx->cfg.implicit_fluxes && !ctx->cfg.implicit_enthalpy;
+    std::unique_lock<std::mutex> lk;
+    bool one = false;  // the sweep loop in one launch
+    if (!ctx->prof && explicit_modes) {
+        one = ctx->cluster_blocks > 0;
+        if (!one && ctx->coop_blocks > 0 && ctx->allow_coop) {
+            lk = std::unique_lock<std::mutex>(coop_lock(), std::try_to_lock);
+            one = lk.owns_lock();
+        }
+    }
+    if (one) {
+        CK(launch_sweep_loop(ctx, dt, st));
         CK(cudaMemcpyAsync(ctx->h_nit, ctx->d_nit, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if (lk.owns_lock()) lk.unlock();
         nit = *ctx->h_nit;
         ctx->sweeps += std::min(nit, ctx->cfg.maxout);
         ctx->launches++;
@@ -1603,7 +1662,7 @@ int pdac_gpu_iter(pdac_ctx *ctx, double dt, int *nit_out) {
             CK(cudaMemcpyAsync(ctx->d_nit, ctx->h_nit, sizeof(int), cudaMemcpyHostToDevice, st));
             int s = enqueue_sweep(ctx, dt, st, true);
             if (s) return s;
-            ctx->launches += 9;
+            ctx->launches += 6;
             CK(cudaMemcpyAsync(ctx->h_counters, ctx->d_wcount, 6 * sizeof(int), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             ctx->sweeps++;
@@ -1731,7 +1790,6 @@ int pdac_gpu_iter_static(pdac_ctx *ctx, double dt, int *nit_out) {
     int *wcount = reinterpret_cast<int *>(base);
     int *dnit = wcount + 12;  // sweep number, read by the inner loop
     int *work = reinterpret_cast<int *>(base + 256);
-    int *cand = reinterpret_cast<int *>(base + 256 + work_bytes);
     unsigned *dirty = reinterpret_cast<unsigned *>(base + 256 + 2 * work_bytes);
     cudaStream_t st = ctx->stream;
     Fld &F = ctx->F;
@@ -1760,11 +1818,10 @@ int pdac_gpu_iter_static(pdac_ctx *ctx, double dt, int *nit_out) {
         CK(cudaMemcpyAsync(dnit, ctx->h_nit, sizeof(int), cudaMemcpyHostToDevice, st));
         CK(cudaMemsetAsync(wcount, 0, 9 * sizeof(int), st));
         for (int col = 0; col < 3; ++col) {
-            int *cnt = wcount + col, *ncand = wcount + 6 + col;
-            pdac::k_resid_collect<<<blocks((long)nwords, TPB_RESID), TPB_RESID, 0, st>>>(ctx->P, col, dirty, cand, ncand);
-            if (ctx->d3) PHASE_LAUNCH_D(nph, pdac::k_resid_test, 3, test_grid, TPB_RESID, st, ctx->P, F, dt, cand, ncand, work, cnt, dirty);
-            else PHASE_LAUNCH_D(nph, pdac::k_resid_test, 2, test_grid, TPB_RESID, st, ctx->P, F, dt, cand, ncand, work, cnt, dirty);
-            ctx->launches++;
+            int *cnt = wcount + col;
+            const unsigned *cmask = ctx->d_cmask + (size_t)col * nwords;
+            if (ctx->d3) PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 3, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, dirty, work, cnt);
+            else PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 2, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, dirty, work, cnt);
             long team_threads = (nthr + (ctx->d3 ? 4 : 7)) / (ctx->d3 ? 5 : 8) * 32;
             int g = std::min(ctx->inner_grid, blocks(team_threads, TPB_TEAM));
             if (ctx->d3) INNER_LAUNCH_D(nph, pdac::k_inner_team, 3, g, TPB_TEAM, st, ctx->P, F, dt, dnit, work, cnt, dirty, inner_spread(ctx));
@@ -2087,6 +2144,8 @@ int pdac_gpu_explicit_iter(pdac_ctx *ctx, double dt) {
     if (ctx->ti != 1) return fail(ctx, PDAC_ERR_CONFIG, "explicit_iter: the context runs time_integration = 0");
     cudaStream_t st = ctx->stream;
     CK(cudaEventRecord(ctx->ev[6], st));
+    std::unique_lock<std::mutex> lk(coop_lock(), std::defer_lock);
+    if (ctx->wave_grid_blocks > 0 && ctx->allow_coop) lk.lock();  // until the stream is idle below
     if (ctx->prof) {
         ctx->launches += enqueue_explicit(ctx, dt, st, true);
         CK(cudaGetLastError());
@@ -2408,18 +2467,21 @@ int pdac_gpu_autotune(pdac_ctx *ctx, const char *cache_path, int *out, int nout)
                                       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess
                                   ? PDAC_OK
                                   : fail(ctx, PDAC_ERR_CUDA, "autotune: device query");
-        const bool coop = ctx->coop_max_blocks > 0 && ctx->allow_coop && !ctx->cfg.implicit_fluxes &&
-                          !ctx->cfg.implicit_enthalpy;
+        const bool one_launch = !ctx->cfg.implicit_fluxes && !ctx->cfg.implicit_enthalpy;
+        const bool cluster = one_launch && ctx->cluster_blocks > 0;  // nothing to tune
+        const bool coop = one_launch && ctx->coop_max_blocks > 0 && ctx->allow_coop;
         float best_ms = 1e30f;
-        if (!status && coop) {
-            for (int cpb : {256, 512, 1024, 2048}) {
+        if (!status && coop && !cluster) {
+            for (int cpb : {64, 256, 1024, 4096}) {
+                // as many blocks as the candidate before: nothing new
+                if (cpb > 64 && (long)ctx->coop_max_blocks * cpb <= (long)ctx->ncell) continue;
                 Tuning t = best;
                 t.coop_cpb = cpb;
                 float ms = 0;
                 if ((status = time_step(t, ms))) break;
                 if (ms < best_ms) { best_ms = ms; best = t; }
             }
-        } else if (!status) {
+        } else if (!status && !cluster) {
             for (int mult : {4, 8, 16, 32}) {
                 Tuning t = best;
                 t.inner_grid = nsm * mult;
@@ -2982,26 +3044,39 @@ static int add_step_nodes(pdac_ctx *ctx, cudaGraph_t g) {
     e = cudaGraphAddChildGraphNode(&pre, g, nullptr, 0, part);
     cudaGraphDestroy(part);
     CK(e);
-    // the sweep loop
-    cudaGraphConditionalHandle loop;
-    CK(cudaGraphConditionalHandleCreate(&loop, g, 1, cudaGraphCondAssignDefault));
-    alignas(cudaGraphNodeParams) unsigned char cp_storage[sizeof(cudaGraphNodeParams)] = {};
-    cudaGraphNodeParams &cp = *reinterpret_cast<cudaGraphNodeParams *>(cp_storage);
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = loop;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    CK(cudaGraphAddNode(&loop_node, g, &pre, 1, &cp));
-    CK(cudaStreamBeginCaptureToGraph(st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    const long long mid = ctx->launches;
-    s = enqueue_sweep(ctx, dt, st, false);
-    ctx->it_per_sweep = sweep_kernels(ctx) + (ctx->launches - mid);
-    ctx->launches = mid;
-    if (!s) pdac::k_sweep_check<<<1, 1, 0, st>>>(ctx->d_wcount, ctx->d_nit, ctx->cfg.maxout, loop);
-    cudaGraph_t body = nullptr;
-    e = cudaStreamEndCapture(st, &body);
-    if (s) { ctx->launches = before; return s; }
-    CK(e);
+    // the sweep loop: one kernel on a cluster, or a WHILE node
+    if (ctx->cluster_blocks > 0) {
+        CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
+        const cudaError_t el = launch_sweep_loop(ctx, dt, st);
+        e = cudaStreamEndCapture(st, &part);
+        CK(el);
+        CK(e);
+        e = cudaGraphAddChildGraphNode(&loop_node, g, &pre, 1, part);
+        cudaGraphDestroy(part);
+        CK(e);
+        ctx->it_per_sweep = 0;
+        ctx->launches++;
+    } else {
+        cudaGraphConditionalHandle loop;
+        CK(cudaGraphConditionalHandleCreate(&loop, g, 1, cudaGraphCondAssignDefault));
+        alignas(cudaGraphNodeParams) unsigned char cp_storage[sizeof(cudaGraphNodeParams)] = {};
+        cudaGraphNodeParams &cp = *reinterpret_cast<cudaGraphNodeParams *>(cp_storage);
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = loop;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        CK(cudaGraphAddNode(&loop_node, g, &pre, 1, &cp));
+        CK(cudaStreamBeginCaptureToGraph(st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+        const long long mid = ctx->launches;
+        s = enqueue_sweep(ctx, dt, st, false);
+        ctx->it_per_sweep = sweep_kernels(ctx) + (ctx->launches - mid);
+        ctx->launches = mid;
+        if (!s) pdac::k_sweep_check<<<1, 1, 0, st>>>(ctx->d_wcount, ctx->d_nit, ctx->cfg.maxout, loop);
+        cudaGraph_t body = nullptr;
+        e = cudaStreamEndCapture(st, &body);
+        if (s) { ctx->launches = before; return s; }
+        CK(e);
+    }
     // the kernels after it
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
     s = enqueue_step_post(ctx, dt, st);

@@ -260,6 +260,11 @@ template <int NP>
 __host__ __device__ constexpr size_t inner_smem_bytes() {
     return (size_t)(inner_face_rows<NP>() + inner_dens_rows<NP>()) * KS * sizeof(double);
 }
+// k_sweep_loop's, which holds the warps' scan lists in the same place
+template <int NP>
+__host__ __device__ constexpr size_t sweep_smem_bytes() {
+    return inner_smem_bytes<NP>() > KS / 32 * 352 * sizeof(int) ? inner_smem_bytes<NP>() : KS / 32 * 352 * sizeof(int);
+}
 
 // The inner loop of worklist cell c (outer sweep nit, 1-based) by the team of
 // lanes tb .. tb + T - 1 of this warp (lane q of the team owns face q); kcols
@@ -503,50 +508,31 @@ __global__ void __launch_bounds__(128, PDAC_INNER_MINB(NP)) k_inner_team(Prm P, 
                                 cells_per_warp<D>(nwork, min(nwarps, spread)));
 }
 
-// Residual test of one colour phase (iter.f:241-319) in two launches.
+// Residual test of one colour phase (iter.f:241-319).
 // The active set is one bit per cell: the test of a cell reads only its own
 // p/rog/rgp and the mass fluxes of its faces, which change only when the
 // cell or a face neighbour runs the inner loop; such a run sets the bits of
 // those cells (mark_dirty).  A converged test rewrites the cell's volume
-// fractions (calc_eps, from the same fluxes) and rgp = ep rog: if that
+// fractions (calc_eps, from the same fluxes and rgp = ep rog): if that
 // changes rgp, the next test computes a different residual, so the cell
 // keeps its bit; otherwise a clean cell would recompute exactly the values
-// it holds, and it is not tested.  k_resid_collect turns the set bits of
-// one colour's fluid cells into a candidate list (clearing them, and the
-// bits of non-fluid cells, which are never tested); k_resid_test tests each
-// candidate: a converged cell updates its volume fractions and rgp, an
-// unconverged one goes to the worklist of k_inner_team.
-// candidates of one colour: the block's threads take consecutive words of
-// the bitmask, block-uniform rounds over the grid (one round when the grid
-// covers the words)
-template <int TPBK>
-__device__ __forceinline__ void collect_phase(const Prm &P, int colour, unsigned *dirty, int *cand, int *ncand) {
+// it holds, and it is not tested.  cmask holds, per colour, the bits of the
+// colour's fluid cells in the same words (k_colour_masks, set up once): a
+// word's candidates are its active bits under the mask, and the bits that
+// runs set on non-fluid neighbours are never looked at.
+__global__ void k_colour_masks(Prm P, unsigned *cmask) {
     const unsigned nwords = ((unsigned)P.ncell + 31u) / 32u;
-    for (unsigned base = blockIdx.x * (unsigned)TPBK; base < nwords; base += gridDim.x * (unsigned)TPBK) {
-    unsigned t = base + threadIdx.x;
-    int mine[32], nmine = 0;
-    if (t < nwords) {
-        unsigned w = dirty[t], keep = w;
-        while (w) {
-            int b = __ffs(w) - 1;
-            w &= w - 1u;
-            int c = (int)(32u * t) + b;
-            if (c >= P.ncell) break;
-            if (!(P.flag[c] & 1)) { keep &= ~(1u << b); continue; }
-            int i = c % P.nx + 1, r = c / P.nx, j = r % P.ny + 1, k = r / P.ny + 1;
-            if ((i + j + k) % 3 != colour) continue;
-            keep &= ~(1u << b);
-            mine[nmine++] = c;
-        }
-        if (keep != dirty[t]) dirty[t] = keep;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nwords) return;
+    unsigned m[3] = {0u, 0u, 0u};
+    for (int b = 0; b < 32; ++b) {
+        const int c = (int)(32u * t) + b;
+        if (c >= P.ncell) break;
+        if (!(P.flag[c] & 1)) continue;
+        const int i = c % P.nx + 1, r = c / P.nx, j = r % P.ny + 1, k = r / P.ny + 1;
+        m[(i + j + k) % 3] |= 1u << b;
     }
-    block_append_n<TPBK, 32>(cand, ncand, mine, nmine, nullptr, 0);
-    }
-}
-
-__global__ void __launch_bounds__(TPB_RESID) k_resid_collect(Prm P, int colour, unsigned *dirty, int *cand,
-                                                             int *ncand) {
-    collect_phase<TPB_RESID>(P, colour, dirty, cand, ncand);
+    for (int q = 0; q < 3; ++q) cmask[(size_t)q * nwords + t] = m[q];
 }
 
 // the residual test of cell c (iter.f:241-319): a converged cell updates its
@@ -578,119 +564,135 @@ __device__ __forceinline__ bool test_cell(const Prm &P, const Fld &F, double dt,
     return true;
 }
 
-// the residual test of the len candidates, block-uniform rounds
-template <int TPBK, int NP, int D>
-__device__ __forceinline__ void test_phase(const Prm &P, const Fld &F, double dt, const int *cand, int len, int *work,
-                                           int *count, unsigned *dirty) {
-    for (int base = blockIdx.x * TPBK; base < len; base += gridDim.x * TPBK) {
-        int idx = base + threadIdx.x, c = -1, nmine = 0;
-        if (idx < len) {
-            c = cand[idx];
-            nmine = test_cell<NP, D>(P, F, dt, c, dirty) ? 1 : 0;
+// One colour's residual tests by the warps warp, warp + nwarps, ... of a
+// launch: each takes 32 words of the active set at a time, moves their
+// candidates (clearing their bits) to its list in shared memory, tests them
+// 32 at a time and appends the unconverged ones to the worklist.  The active
+// cells sit close together (the plume's front), so consecutive words go to
+// different warps: word by word while one round covers the mesh, else in
+// groups of eight (one 32-byte sector).  slist: SCAN_LIST ints per warp.
+// Collecting and testing in one pass took the two launches' fixed cost
+// (about 12 us) down to one's.
+constexpr int SCAN_LIST = 32 * 11;  // a colour has at most 11 cells in a word of 32
+template <int NP, int D>
+__device__ __forceinline__ void scan_phase(const Prm &P, const Fld &F, double dt, const unsigned *cmask,
+                                           unsigned *dirty, int *work, int *count, int *tested, unsigned warp,
+                                           unsigned nwarps, int *slist) {
+    constexpr unsigned full = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u, nwords = ((unsigned)P.ncell + 31u) / 32u;
+    const unsigned gs = nwords <= 32u * nwarps ? 1u : 8u, gpi = 32u / gs;  // words per group, groups per round
+    int ntest = 0;
+    for (unsigned g0 = 0; (size_t)g0 * nwarps * gs < nwords; g0 += gpi) {
+        const unsigned t = ((g0 + lane / gs) * nwarps + warp) * gs + lane % gs;
+        unsigned w = 0;
+        if (t < nwords) {
+            w = __ldcg(dirty + t) & __ldg(cmask + t);
+            if (w) atomicAnd(dirty + t, ~w);
         }
-        block_append_n<TPBK, 1>(work, count, &c, nmine, count + 3, idx < len ? 1 : 0);
+        int incl = __popc(w);
+        const int mine = incl;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(full, incl, o);
+            if (lane >= (unsigned)o) incl += v;
+        }
+        const int total = __shfl_sync(full, incl, 31);
+        if (total == 0) continue;
+        for (int off = incl - mine; w; w &= w - 1u) slist[off++] = (int)(32u * t) + __ffs(w) - 1;
+        __syncwarp();
+        for (int base = 0; base < total; base += 32) {
+            const int idx = base + (int)lane;
+            int c = -1;
+            bool u = false;
+            if (idx < total) {
+                c = slist[idx];
+                u = test_cell<NP, D>(P, F, dt, c, dirty);
+            }
+            const unsigned um = __ballot_sync(full, u);
+            if (um) {
+                int at = 0;
+                if (lane == 0) at = atomicAdd(count, __popc(um));
+                at = __shfl_sync(full, at, 0);
+                if (u) work[at + __popc(um & ((1u << lane) - 1u))] = c;
+            }
+        }
+        ntest += total;
+        __syncwarp();  // the list is read before the next round overwrites it
     }
+    if (tested && lane == 0 && ntest) atomicAdd(tested, ntest);
 }
 
 template <int NP, int D>
-__global__ void __launch_bounds__(TPB_RESID) k_resid_test(Prm P, Fld F, double dt, const int *cand, const int *ncand,
-                                                          int *work, int *count, unsigned *dirty) {
-    test_phase<TPB_RESID, NP, D>(P, F, dt, cand, *ncand, work, count, dirty);
+__global__ void __launch_bounds__(TPB_RESID) k_resid_scan(Prm P, Fld F, double dt, const unsigned *cmask,
+                                                          unsigned *dirty, int *work, int *count) {
+    __shared__ int slist[TPB_RESID / 32][SCAN_LIST];
+    const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    scan_phase<NP, D>(P, F, dt, cmask, dirty, work, count, count + 3, warp, nwarps, slist[threadIdx.x >> 5]);
 }
 
-// One colour phase of the cooperative sweep loop in one pass: collect, test
-// and inner loop fused, with one grid barrier after it instead of three.
-// Each warp takes one word of the active set (32 consecutive cells) at a time:
-// lane b tests the cell of bit b when that bit is set and the cell is a
-// fluid cell of the colour, the unconverged cells (at most 11 of the 32 are
-// of one colour) go to a warp-local list in shared memory, and the warp's
-// teams run their inner loops.  Cells of one colour share no stencil data,
-// so testing and iterating them in this order gives the bits of the
-// three-launch form.  The colour's set bits of a word are cleared
-// atomically before its cells are tested: other warps set bits of the
-// neighbouring cells meanwhile.  Appends the unconverged cells to the
-// colour's worklist (work, wcount[col] long; the cells the last sweep left
-// unconverged, as pdac_gpu_unconverged_cells reports them) and adds the
-// tested ones to wcount[3 + col].  RO as in ldro.
-template <int NP, int D, bool RO>
-__device__ __forceinline__ void fused_phase(const Prm &P, const Fld &F, double dt, int nit, int colour,
-                                            unsigned *dirty, int *wcount, int *work, unsigned warp, unsigned nwarps) {
-    const int lane = threadIdx.x & 31;
-    __shared__ int wlist[KS / 32][32];
-    int *const mylist = wlist[threadIdx.x >> 5];
-    const unsigned nwords = ((unsigned)P.ncell + 31u) / 32u;
-    int ntest_sum = 0;
-    for (unsigned t = warp; t < nwords; t += nwarps) {  // uniform across the warp
-        const unsigned w = __ldcg(dirty + t);
-        const int c = (int)(32u * t) + lane;
-        bool cand = false, clear = false;
-        if (((w >> lane) & 1u) && c < P.ncell) {
-            if (!(P.flag[c] & 1)) {
-                clear = true;  // a non-fluid cell is never tested
-            } else {
-                int i = c % P.nx + 1, r = c / P.nx, j = r % P.ny + 1, k = r / P.ny + 1;
-                cand = (i + j + k) % 3 == colour;
-                clear = cand;
-            }
-        }
-        const unsigned cm = __ballot_sync(0xffffffffu, clear);
-        if (lane == 0 && cm) atomicAnd(dirty + t, ~cm);
-        __syncwarp();
-        const bool unconv = cand && test_cell<NP, D>(P, F, dt, c, dirty);
-        const unsigned um = __ballot_sync(0xffffffffu, unconv);
-        if (unconv) mylist[__popc(um & ((1u << lane) - 1u))] = c;
-        ntest_sum += __popc(__ballot_sync(0xffffffffu, cand));
-        __syncwarp();
-        const int nwork = __popc(um);
-        if (nwork) {
-            int base = 0;
-            if (lane == 0) base = atomicAdd(wcount + colour, nwork);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (unconv) work[base + __popc(um & ((1u << lane) - 1u))] = c;
-            inner_team_run<NP, D, RO>(P, F, dt, nit, mylist, nwork, dirty, 0, 1, 32 / (D == 3 ? 6 : 4));
-        }
-        __syncwarp();  // the list is read before the next word overwrites it
-    }
-    if (lane == 0 && ntest_sum) atomicAdd(wcount + 3 + colour, ntest_sum);
-}
-
-// The whole outer sweep loop of iter (iter.f:204-410) in one cooperative
-// launch, for small domains: the colour phases (fused_phase: collect, test
-// and inner loop in one pass) follow each other across grid-wide barriers
-// instead of launches.
-// Every thread of the grid takes every barrier the same number of times:
-// the loop ends on counters that all threads read after the same barrier.
+// The whole outer sweep loop of iter (iter.f:204-410) in one launch whose
+// blocks are all resident: the colour phases' residual tests and inner loops
+// follow each other across barriers instead of launches.  Two forms of
+// barrier: CLUSTER = true runs the mesh on one thread-block cluster with the
+// hardware's cluster barrier (the blocks of a cluster are always scheduled
+// together, so any number of such launches may share the device);
+// CLUSTER = false runs it on a cooperative grid.
+// Every thread takes every barrier the same number of times: the loop ends
+// on counters that all threads read after the same barrier.
 struct SweepWork {
-    int *wcount;      // [col] worklist length, [3 + col] cells tested, [6 + col] candidates
-    int *cand, *work; // candidate list of one colour phase; worklists, colour col at work + col * wstride
+    int *wcount;      // on return: [col] worklist length of the last sweep
+    int *counts;      // two sets of three worklist lengths, for odd and even sweeps
+    int *work;        // worklists, colour col at work + col * wstride
     unsigned *dirty;  // active set, one bit per cell
+    const unsigned *cmask;  // colour masks
     int *nit;         // the sweep count on return, as the graph's k_sweep_check leaves it
     long wstride;     // ints per colour's worklist
 };
 
-template <int NP, int D>
-__global__ void __launch_bounds__(128, PDAC_INNER_MINB(NP)) k_iter_coop(Prm P, Fld F, double dt, SweepWork W, int maxout) {
+template <int NP, int D, bool CLUSTER>
+__global__ void __launch_bounds__(KS, PDAC_INNER_MINB(NP)) k_sweep_loop(Prm P, Fld F, double dt, SweepWork W, int maxout) {
     namespace cg = cooperative_groups;
-    cg::grid_group g = cg::this_grid();
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    auto barrier = [] {
+        __syncwarp();
+        if (CLUSTER) cg::this_cluster().sync();
+        else cg::this_grid().sync();
+    };
+    extern __shared__ __align__(16) double inner_smem[];
+    const int wid = threadIdx.x >> 5, warp = blockIdx.x * (KS / 32) + wid, nwarps = gridDim.x * (KS / 32);
+    const unsigned nwords = ((unsigned)P.ncell + 31u) / 32u;
+    // the scan's list and the inner loop's columns are never live together
+    int *const slist = reinterpret_cast<int *>(inner_smem) + wid * SCAN_LIST;
     int nit = 1;
+    if (blockIdx.x == 0 && threadIdx.x < 6) W.counts[threadIdx.x] = 0;
+    barrier();
     for (;;) {
-        if (blockIdx.x == 0 && threadIdx.x < 9) W.wcount[threadIdx.x] = 0;
-        g.sync();
+        int *const cnt = W.counts + 3 * (nit & 1), *const other = W.counts + 3 * (~nit & 1);
         for (int col = 0; col < 3; ++col) {
-            fused_phase<NP, D, false>(P, F, dt, nit, col, W.dirty, W.wcount, W.work + col * W.wstride, warp, nwarps);
-            g.sync();
+            int *const work = W.work + col * W.wstride;
+            scan_phase<NP, D>(P, F, dt, W.cmask + (size_t)col * nwords, W.dirty, work, cnt + col, nullptr, warp,
+                              nwarps, slist);
+            barrier();
+            const int nwork = __ldcg(cnt + col);
+            // the next sweep's lengths: last read before this sweep's first barrier
+            if (col == 1 && blockIdx.x == 0 && threadIdx.x < 3) other[threadIdx.x] = 0;
+            if (nwork)
+                inner_team_run<NP, D, false>(P, F, dt, nit, work, nwork, W.dirty, warp, nwarps,
+                                             cells_per_warp<D>(nwork, nwarps));
+            barrier();
         }
-        const long unconverged = (long)__ldcg(W.wcount) + __ldcg(W.wcount + 1) + __ldcg(W.wcount + 2);
-        if (unconverged == 0) break;
-        if (nit >= maxout) {
-            nit = maxout + 1;
-            break;
+        const int n0 = __ldcg(cnt), n1 = __ldcg(cnt + 1), n2 = __ldcg(cnt + 2);
+        const bool conv = (long)n0 + n1 + n2 == 0;
+        if (conv || nit >= maxout) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                W.wcount[0] = n0;
+                W.wcount[1] = n1;
+                W.wcount[2] = n2;
+                *W.nit = conv ? nit : maxout + 1;
+            }
+            return;
         }
         ++nit;
-        g.sync();  // every thread has read the counters before they are cleared
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) *W.nit = nit;
 }
 
 // End of one outer sweep on the device (iter.f:388-410): with no unconverged
