@@ -33,8 +33,9 @@ extern "C" {
                                        the state after a step                */
 #define PDAC_ERR_ARG            6   /* bad argument (NULL, size, name)        */
 #define PDAC_ERR_BOUNDARY       7   /* inoutflow.f:99,143: rls >= 1 on a BC   */
-#define PDAC_ERR_TIMEOUT        8   /* reserved: no kernel of this build waits
-                                       on a flag, so none can time out       */
+#define PDAC_ERR_TIMEOUT        8   /* explicit_iter: a bounded wait of the
+                                       gas-enthalpy wavefront ran out (no
+                                       regular run meets this)               */
 
 /* ---- cell flags, grid.f:45-58 ----------------------------------------- */
 #define PDAC_FLUID        1

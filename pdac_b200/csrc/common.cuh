@@ -50,6 +50,11 @@ struct Prm {
     double gravx, gravy, gravz, void_fraction;
     double atm_ygc[PDAC_MAXG];
     double gmw[8], mmugs[8], mmugek[8];
+    // per gas of the run, in its order: the specific-heat polynomial
+    // (hcapgs.f:33-85), the molar weight as a divisor, and with icpc = 0 the
+    // fixed value that replaces the polynomial (0: none)
+    double hcp[PDAC_MAXG][4], hfix[PDAC_MAXG];
+    pdac_fp::Recip hmw[PDAC_MAXG];
     double rgas, gammaair;
     double dk[PDAC_MAXP], rl[PDAC_MAXP], inrl[PDAC_MAXP], phis[PDAC_MAXP], cmus[PDAC_MAXP];
     double cps[PDAC_MAXP], kap[PDAC_MAXP], plim[PDAC_MAXP], phi[PDAC_MAXP];

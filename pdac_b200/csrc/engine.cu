@@ -139,10 +139,10 @@ struct pdac_ctx {
     // shared-memory tiled 3D stencil passes: tile shape (index into
     // TILE_SHAPES) and planes per block of the march up k
     int tile_shape = 0, tile_kchunk = 32;
-    int *d_wave_idx = nullptr;    // order, src[3], start
+    int *d_wave_idx = nullptr;    // order, pos_of, code
     double *d_wave_rec = nullptr; // records and pnew
-    int wave_grid_blocks = 0;
-    bool wave_one = false;
+    int wave_tiles = 0;     // tiles of the gas-enthalpy wavefront (0: a launch per hyperplane)
+    bool wave_one = false;  // one column per thread
 };
 
 namespace {
@@ -284,6 +284,24 @@ static cudaError_t set_inner_attrs() {
     return e;
 }
 
+// the specific-heat tables of the run's gases (hcapgs.f:33-85, the
+// polynomials of hcapg1) in their order; again when a restart file brings
+// other gases
+void set_gas_tables(pdac_ctx *ctx) {
+    static const double cp[7][4] = {
+        {2.811e1, -3.68e-6, 1.746e-5, -1.065e-8}, {3.115e1, -1.357e-2, 2.680e-5, -1.168e-8},
+        {1.980e1, 7.344e-2, -5.602e-5, 1.715e-8}, {2.714e1, 9.274e-3, -1.381e-5, 7.645e-9},
+        {3.224e1, 1.924e-3, 1.055e-5, -3.596e-9}, {3.0413e1, -1.059e-2, 2.458e-5, -1.135e-8},
+        {2.385e1, 6.699e-2, -4.961e-5, 1.328e-8}};
+    Prm &P = ctx->P;
+    for (int ig = 0; ig < ctx->ng; ++ig) {
+        const int g = P.gas_type[ig];
+        for (int q = 0; q < 4; ++q) P.hcp[ig][q] = cp[g - 1][q];
+        P.hmw[ig] = pdac_fp::recip(P.gmw[g]);
+        P.hfix[ig] = P.icpc == 0 && g == 5 ? 1810.0 : (P.icpc == 0 && g == 6 ? 1004.0 : 0.0);
+    }
+}
+
 // setup.f:551-616 and particles.f:35-79: gas and particle constants
 void set_constants(pdac_ctx *ctx) {
     Prm &P = ctx->P;
@@ -292,6 +310,7 @@ void set_constants(pdac_ctx *ctx) {
     double s[8] = {0, 3.467, 3.798, 3.941, 2.827, 2.641, 3.711, 4.112};
     double e[8] = {0, 106.7, 71.4, 195.2, 59.7, 809.1, 78.6, 335.4};
     for (int q = 0; q < 8; ++q) { P.gmw[q] = g[q] * 1.0e-3; P.mmugs[q] = s[q]; P.mmugek[q] = e[q]; }
+    set_gas_tables(ctx);
     P.rgas = 8.31432;
     P.gammaair = 1.4;
     for (int is = 1; is <= ctx->ns; ++is) {
@@ -516,92 +535,99 @@ void boundary_levels(const pdac_cfg *c, std::vector<int> &items, std::vector<int
     starts.push_back((int)lev.size());
 }
 
-// The records of the explicit solver's gas-enthalpy wavefront (fixed by the
-// cell flags): interior fluid cells in hyperplane order d = i + j + k (i + k
-// in 2D), cell order within a hyperplane; empty hyperplanes are dropped, as
-// no cell depends on one.  Also picks the cooperative grid.
+// The tiles and records of the explicit solver's gas-enthalpy wavefront
+// (k_rk3_wave_tile; fixed by the cell flags).  Tiles of 16 x 4 columns
+// (measured, both stages and their records, 128 x 128 x 96 / 224 x 208 x 161:
+// 16 x 4 2.0 / 5.7 ms, 8 x 8 2.3 / 6.7, 16 x 8 2.4 / 7.1, 16 x 16 2.5 / 6.9);
+// where those are more than the device holds at once (about 57000 columns),
+// tiles of 1024 and 2048 columns, several per thread.  2D meshes have one row
+// of columns: one tile up to 256 of them, which needs no exchange through L2
+// and no cooperative launch (128 x 192: 0.63 ms, three tiles of 64 0.84), else
+// tiles of 64.
 int setup_wave(pdac_ctx *ctx, const int *flag) {
     const int nx = ctx->nx, ny = ctx->d3 ? ctx->ny : 1, nz = ctx->nz, n = ctx->ncell;
     const int jlo = ctx->d3 ? 2 : 1, jhi = ctx->d3 ? ny - 1 : 1;
-    const int dmin = 2 + jlo + 2, dmax = (nx - 1) + jhi + (nz - 1);
-    const int nd = dmax - dmin + 1;
-    std::vector<int> count(nd + 1, 0), pos_of(n, -1);
+    const int ni = nx - 2, nj = jhi - jlo + 1, nk = nz - 2;
+    ctx->wave_tiles = 0;
+    if (ni < 1 || nj < 1 || nk < 1) return PDAC_OK;
+    int dev = 0, coop = 0, nsm = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    auto room = [&](bool one, int threads, int tt) {
+        int occ = 0;
+        const size_t sm = 2 * (size_t)tt * sizeof(double);
+        if (ctx->d3)
+            (void)(one ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<3, true, true>, threads, sm)
+                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<3, false, true>, threads, sm));
+        else
+            (void)(one ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<2, true, true>, threads, sm)
+                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<2, false, true>, threads, sm));
+        return occ * nsm;
+    };
+    const int shapes3[][2] = {{16, 4}, {32, 32}, {64, 32}}, shapes2[][2] = {{1, 64}, {1, 1024}, {1, 2048}};
+    pdac::Wave &W = ctx->W;
+    int tiles = 0;
+    bool one = true;
+    if (!ctx->d3 && nk <= 256) {
+        W.tj = 1;
+        W.tk = (nk + 31) / 32 * 32;
+        tiles = 1;  // with one column per thread
+    } else {
+        for (int q = 0; q < 3 && coop; ++q) {
+            W.tj = ctx->d3 ? shapes3[q][0] : shapes2[q][0];
+            W.tk = ctx->d3 ? shapes3[q][1] : shapes2[q][1];
+            one = W.tj * W.tk <= 256;
+            const int m = ((nj + W.tj - 1) / W.tj) * ((nk + W.tk - 1) / W.tk);
+            if (m <= room(one, std::min(512, W.tj * W.tk), W.tj * W.tk)) { tiles = m; break; }
+        }
+    }
+    if (tiles == 1 && !one) tiles = 0;  // cannot be: several columns a thread come with many tiles
+    if (!tiles) return PDAC_OK;
+    W.tt = W.tj * W.tk;
+    W.ntj = (nj + W.tj - 1) / W.tj;
+    W.steps = ni + W.tj + W.tk - 2;
+    const long long np = (long long)tiles * W.steps * W.tt;
+    if (np > 0x7fffffffLL) return PDAC_OK;
+    W.npos = (int)np;
+    std::vector<int> order(np, -1), pos_of(n, -1);
+    std::vector<unsigned char> code(np, 0);
     auto each = [&](auto fn) {
         for (int k = 2; k <= nz - 1; ++k)
             for (int j = jlo; j <= jhi; ++j)
                 for (int i = 2; i <= nx - 1; ++i) {
-                    int c = (i - 1) + nx * ((j - 1) + ny * (k - 1));
-                    if (flag[c] & 1) fn(c, i + j + k - dmin);
+                    const int c = (i - 1) + nx * ((j - 1) + ny * (k - 1));
+                    if (flag[c] & 1) fn(c, i, j, k);
                 }
     };
-    each([&](int, int q) { count[q + 1]++; });
-    std::vector<int> first(nd + 1, 0);
-    for (int q = 0; q < nd; ++q) first[q + 1] = first[q] + count[q + 1];
-    const int np = first[nd];
-    std::vector<int> order(std::max(np, 1), 0), fill(first.begin(), first.end() - 1);
-    each([&](int c, int q) {
-        pos_of[c] = fill[q];
-        order[fill[q]++] = c;
+    each([&](int c, int i, int j, int k) {
+        const int J = (j - jlo) / W.tj, jl = (j - jlo) % W.tj, K = (k - 2) / W.tk, kl = (k - 2) % W.tk;
+        const int tile = J + W.ntj * K, s = (i - 2) + jl + kl, p = (tile * W.steps + s) * W.tt + jl + W.tj * kl;
+        pos_of[c] = p;
+        order[p] = c;
     });
-    std::vector<int> start;
-    int widest = 0;
-    for (int q = 0; q < nd; ++q)
-        if (first[q + 1] > first[q]) {
-            start.push_back(first[q]);
-            widest = std::max(widest, first[q + 1] - first[q]);
-        }
-    const int nplanes = (int)start.size();
-    start.push_back(np);
-    start.push_back(np);  // read one past the last hyperplane by the prefetch guard
-    std::vector<int> src(3 * (size_t)std::max(np, 1), -1);
-    for (int p = 0; p < np; ++p) {
-        const int c = order[p];
-        src[p] = pos_of[c - 1];
-        if (ctx->d3) src[(size_t)np + p] = pos_of[c - nx];
-        src[2 * (size_t)np + p] = pos_of[c - nx * ny];
-    }
-    const size_t ni = order.size() + src.size() + start.size() + pos_of.size();
-    CK(cudaMalloc(&ctx->d_wave_idx, ni * sizeof(int)));
-    int *o = ctx->d_wave_idx, *s = o + order.size(), *st = s + src.size(), *po = st + start.size();
+    each([&](int c, int, int, int) {
+        int m = pdac::WC_REC;
+        if (pos_of[c - 1] >= 0) m |= pdac::WC_W;
+        if (ctx->d3 && pos_of[c - nx] >= 0) m |= pdac::WC_S;
+        if (pos_of[c - nx * ny] >= 0) m |= pdac::WC_B;
+        code[pos_of[c]] = (unsigned char)m;
+    });
+    CK(cudaMalloc(&ctx->d_wave_idx, (order.size() + pos_of.size()) * sizeof(int) + code.size()));
+    int *o = ctx->d_wave_idx, *po = o + order.size();
+    unsigned char *cd = reinterpret_cast<unsigned char *>(po + pos_of.size());
     CK(cudaMemcpy(o, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(s, src.data(), src.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(st, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(po, pos_of.data(), pos_of.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(cd, code.data(), code.size(), cudaMemcpyHostToDevice));
     const size_t nrec = (size_t)(pdac::WR_YG + ctx->ng) + 1;  // the fields and pnew
-    CK(cudaMalloc(&ctx->d_wave_rec, nrec * std::max(np, 1) * sizeof(double)));
-    pdac::Wave &W = ctx->W;
+    CK(cudaMalloc(&ctx->d_wave_rec, nrec * np * sizeof(double)));
     W.order = o;
     W.pos_of = po;
-    W.src = s;
-    W.start = st;
+    W.code = cd;
     W.rec = ctx->d_wave_rec;
-    W.pnew = ctx->d_wave_rec + (nrec - 1) * std::max(np, 1);
-    W.npos = np;
-    W.nplanes = nplanes;
-    W.dmin = dmin;
-    // a cooperative grid of co-resident blocks: one record per thread and
-    // hyperplane when the device holds enough blocks for the widest one
-    int dev = 0, coop = 0, nsm = 0, occ1 = 0, occn = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    ctx->wave_grid_blocks = 0;
-    ctx->wave_one = false;
-    if (!coop || np == 0) return PDAC_OK;
-    if (ctx->d3) {
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, pdac::k_rk3_wave_rec<3, true>, TPB, 0));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occn, pdac::k_rk3_wave_rec<3, false>, TPB, 0));
-    } else {
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, pdac::k_rk3_wave_rec<2, true>, TPB, 0));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occn, pdac::k_rk3_wave_rec<2, false>, TPB, 0));
-    }
-    const int need = blocks(widest);
-    if (need <= occ1 * nsm) {
-        ctx->wave_grid_blocks = need;
-        ctx->wave_one = true;
-    } else {
-        ctx->wave_grid_blocks = occn * nsm;
-    }
+    W.pnew = ctx->d_wave_rec + (nrec - 1) * np;
+    ctx->wave_tiles = tiles;
+    ctx->wave_one = one;
     return PDAC_OK;
 }
 
@@ -2060,30 +2086,36 @@ static long long enqueue_explicit(pdac_ctx *ctx, double dt, cudaStream_t st, boo
         else PHASE_LAUNCH_D(nph, pdac::k_rk3_stage, 2, blocks(n), TPB, st, P, F, K, dt, stage);
         L++;
         mark();
-        // gas-enthalpy wavefront over the hyperplanes i + j + k = d of the
-        // interior (2 <= i <= nx - 1 ...), in increasing d: records, one
-        // cooperative launch over all hyperplanes, scatter of the results
-        if (ctx->wave_grid_blocks > 0 && ctx->allow_coop) {
+        // gas-enthalpy wavefront: records, one launch over all tiles,
+        // scatter of the results; in a batch, where a cooperative launch is
+        // not allowed, meshes of several tiles take a launch per hyperplane
+        // i + j + k = d of the interior (2 <= i <= nx - 1 ...), in increasing d
+        if (ctx->wave_tiles == 1 || (ctx->wave_tiles > 1 && ctx->allow_coop)) {
             const pdac::Wave &W = ctx->W;
             const int rb = blocks(W.npos);
+            int *gave_up = ctx->d_counters + 6;
             cudaLaunchConfig_t lc = {};
             cudaLaunchAttribute at[1];
             at[0].id = cudaLaunchAttributeCooperative;
             at[0].val.cooperative = 1;
-            lc.gridDim = dim3(ctx->wave_grid_blocks);
-            lc.blockDim = dim3(TPB);
+            lc.gridDim = dim3(ctx->wave_tiles);
+            lc.blockDim = dim3(std::min(512, W.tt));
+            lc.dynamicSmemBytes = 2 * (size_t)W.tt * sizeof(double);
             lc.stream = st;
             lc.attrs = at;
-            lc.numAttrs = 1;
+            const bool multi = ctx->wave_tiles > 1;
+            lc.numAttrs = multi ? 1 : 0;
             if (ctx->d3) {
                 pdac::k_rk3_wave_pre<3><<<blocks(n), TPB, 0, st>>>(P, F, K, W, dt, stage);
-                if (ctx->wave_one) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_rec<3, true>, P, W, dt, stage);
-                else cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_rec<3, false>, P, W, dt, stage);
+                if (!multi) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<3, true, false>, P, W, dt, stage, gave_up);
+                else if (ctx->wave_one) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<3, true, true>, P, W, dt, stage, gave_up);
+                else cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<3, false, true>, P, W, dt, stage, gave_up);
                 pdac::k_rk3_wave_post<3><<<rb, TPB, 0, st>>>(P, F, K, W, stage);
             } else {
                 pdac::k_rk3_wave_pre<2><<<blocks(n), TPB, 0, st>>>(P, F, K, W, dt, stage);
-                if (ctx->wave_one) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_rec<2, true>, P, W, dt, stage);
-                else cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_rec<2, false>, P, W, dt, stage);
+                if (!multi) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<2, true, false>, P, W, dt, stage, gave_up);
+                else if (ctx->wave_one) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<2, true, true>, P, W, dt, stage, gave_up);
+                else cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<2, false, true>, P, W, dt, stage, gave_up);
                 pdac::k_rk3_wave_post<2><<<rb, TPB, 0, st>>>(P, F, K, W, stage);
             }
             L += 3;
@@ -2145,7 +2177,7 @@ int pdac_gpu_explicit_iter(pdac_ctx *ctx, double dt) {
     cudaStream_t st = ctx->stream;
     CK(cudaEventRecord(ctx->ev[6], st));
     std::unique_lock<std::mutex> lk(coop_lock(), std::defer_lock);
-    if (ctx->wave_grid_blocks > 0 && ctx->allow_coop) lk.lock();  // until the stream is idle below
+    if (ctx->wave_tiles > 1 && ctx->allow_coop) lk.lock();  // until the stream is idle below
     if (ctx->prof) {
         ctx->launches += enqueue_explicit(ctx, dt, st, true);
         CK(cudaGetLastError());
@@ -2158,7 +2190,7 @@ int pdac_gpu_explicit_iter(pdac_ctx *ctx, double dt) {
         ctx->launches += ctx->ex_launches;
     }
     CK(cudaEventRecord(ctx->ev[7], st));
-    CK(cudaMemcpyAsync(ctx->h_counters + 1, ctx->d_counters + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(ctx->h_counters + 1, ctx->d_counters + 1, 6 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (ctx->prof) {
         float t[8];
@@ -2168,6 +2200,10 @@ int pdac_gpu_explicit_iter(pdac_ctx *ctx, double dt) {
         ctx->ex_ms[2] += t[2] + t[5];
         ctx->ex_ms[3] += t[7];
         ctx->ex_calls++;
+    }
+    if (ctx->h_counters[6]) {
+        CK(cudaMemsetAsync(ctx->d_counters + 6, 0, sizeof(int), st));
+        return fail(ctx, PDAC_ERR_TIMEOUT, "explicit_iter: the gas-enthalpy wavefront gave up waiting for a pressure");
     }
     // explicit_solver.f:1214-1215 stops the run on more than one failure
     if (ctx->h_counters[1] > 1) return fail(ctx, PDAC_ERR_EOS, "explicit_iter: caloric equation of state failed");
@@ -2599,6 +2635,7 @@ int pdac_gpu_read_restart(pdac_ctx *ctx, const char *path, double *time, int *nf
     if (regas) {
         // kernels and captured graphs carry the gas table by value
         for (int ig = 0; ig < ctx->ng; ++ig) ctx->cfg.gas_type[ig] = ctx->P.gas_type[ig] = gt[ig];
+        set_gas_tables(ctx);
         if (ctx->it_exec) { cudaGraphExecDestroy(ctx->it_exec); ctx->it_exec = nullptr; }
         if (ctx->it_graph) { cudaGraphDestroy(ctx->it_graph); ctx->it_graph = nullptr; }
         if (ctx->ex_exec) { cudaGraphExecDestroy(ctx->ex_exec); ctx->ex_exec = nullptr; }

@@ -880,7 +880,7 @@ __global__ void k_ftem3d(Prm P, Fld F, double dt) {
     F.sieg[c] = bt[1];
     for (int is = 1; is <= ns; ++is) SOL(F.sies, c, is) = bt[is + 1];
     double yg[PDAC_MAXG];
-    for (int ig = 0; ig < P.ng; ++ig) yg[ig] = GAS(F.ygc, c, ig);
+    load_ygc(P, F, c, yg);
     double tg = F.tg[c], cg;
     int info = caloric_eosg(P, cg, tg, yg, bt[1]);
     F.tg[c] = tg;

@@ -481,15 +481,40 @@ __device__ __forceinline__ void mole(const Prm &P, double *xg, const double *yg)
     for (int ig = 0; ig < P.ng; ++ig) xg[ig] = yg[ig] / P.gmw[P.gas_type[ig]] * molinv;
 }
 
-// eosg.f:139-223 (fixed-point caloric inversion, <= 2000 iterations)
+// hcapgs.f:33-85 for gas ig of the run: hcapg1's polynomial with the signs in
+// the coefficients, its powers given
+__device__ __forceinline__ double hcap_of(const Prm &P, int ig, double t1, double t2, double t3) {
+    double c = P.hcp[ig][0] + P.hcp[ig][1] * t1 + P.hcp[ig][2] * t2 + P.hcp[ig][3] * t3;
+    c = pdac_fp::div_by(c, P.hmw[ig]);
+    return P.hfix[ig] != 0.0 ? P.hfix[ig] : c;
+}
+
+// the cell's gas mass fractions, in registers (constant indices)
+__device__ __forceinline__ void load_ygc(const Prm &P, const Fld &F, int c, double *yg) {
+#pragma unroll
+    for (int ig = 0; ig < PDAC_MAXG; ++ig) yg[ig] = ig < P.ng ? F.ygc[(size_t)ig * P.ncell + c] : 0.0;
+}
+
+// eosg.f:139-223 (fixed-point caloric inversion, <= 2000 iterations).  yg
+// stays in registers (constant indices).  Every iteration is one dependent
+// chain -- powers, polynomial, molar weight, sum over the gases, quotient,
+// test -- so it holds one division (sieg / cgas): the one by the molar weight
+// goes by div_by, the one of the test by rel_change_within, ~270 cycles
+// instead of ~480.
 __device__ __forceinline__ int caloric_eosg(const Prm &P, double &cgas, double &tg, const double *yg, double sieg) {
     int info = 1;
     for (int ii = 1; ii <= 2000; ++ii) {
-        double tgnn = tg;
-        cgas = 0;
-        for (int ig = 0; ig < P.ng; ++ig) cgas = hcapg1(P, P.gas_type[ig], tg) * yg[ig] + cgas;
-        tg = 0.0 + (sieg - 0.0) / cgas;
-        if (fabs((tgnn - tg) / tgnn) <= 1.0e-8) { info = 0; break; }
+        const double tgnn = tg;
+        const double t1 = (P.icpc <= 1) ? P.tref : tg, t2 = t1 * t1, t3 = t1 * t2;
+        double cs = 0;
+#pragma unroll
+        for (int ig = 0; ig < PDAC_MAXG; ++ig) {
+            if (ig >= P.ng) break;
+            cs = hcap_of(P, ig, t1, t2, t3) * yg[ig] + cs;
+        }
+        cgas = cs;
+        tg = 0.0 + (sieg - 0.0) / cs;
+        if (pdac_fp::rel_change_within(tgnn, tg, 1.0e-8)) { info = 0; break; }
     }
     if (tg <= 0.0) info = 1;
     return info;

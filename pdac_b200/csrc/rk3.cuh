@@ -596,7 +596,7 @@ __global__ void k_rk3_wave(Prm P, Fld F, RkF K, double dt, int stage, int d, int
     double tmp = 1.0 / rgpnew;
     double sieg = siegtmp * tmp;
     double yg[PDAC_MAXG];
-    for (int ig = 0; ig < P.ng; ++ig) yg[ig] = GAS(F.ygc, c, ig);
+    load_ygc(P, F, c, yg);
     double tg = F.tg[c], cg;
     caloric_eosg(P, cg, tg, yg, sieg);
     double mg = 0.0;
@@ -614,34 +614,42 @@ __global__ void k_rk3_wave(Prm P, Fld F, RkF K, double dt, int stage, int d, int
     for (int is = 1; is <= P.ns; ++is) F.rlk[(size_t)(is - 1) * n + c] = K.xrlk[(size_t)(is - 1) * n + c];
 }
 
-// ---- the wavefront on hyperplane-ordered records -----------------------------
+// ---- the wavefront on records in tile order ------------------------------
 // Of a cell's gas-enthalpy update only the pressures of its west, south and
 // bottom neighbours come from the wavefront itself; everything else is known
 // once the stage kernel has run.  k_rk3_wave_pre computes those parts once
-// per stage in parallel and stores them as records ordered hyperplane by
-// hyperplane (interior fluid cells only), so that the wavefront reads them
-// coalesced and takes the three neighbour pressures from the previous
-// hyperplane's slice of pnew, which stays in L2.  The arithmetic and its
-// order are those of rhs_gas_enth and k_rk3_wave.
+// per stage in parallel and stores them as records; k_rk3_wave_tile runs the
+// recurrence over them.  The arithmetic and its order are those of
+// rhs_gas_enth and k_rk3_wave.
+//
+// The columns (j, k) of the interior are dealt out to tiles of tj x tk, one
+// block each; the block's thread of column (jl, kl) solves cell i = 2 + s -
+// jl - kl of its column in step s, so a step is a hyperplane of the tile, and
+// its records lie one after the other: record (tile, s, t) at (tile steps +
+// s) tt + t.
 struct Wave {
-    const int *order;   // record position -> cell
-    const int *pos_of;  // cell -> record position, -1 for cells without a record
-    const int *src;     // [3][npos]: record of the W / S / B neighbour when it is a fluid cell, else -1
-    const int *start;   // hyperplane dmin + q holds records start[q] .. start[q + 1] - 1
-    double *rec;        // [WR_YG + ng][npos]
-    double *pnew;       // new pressure per record
-    int npos, nplanes, dmin;
+    const int *order;           // record position -> cell, -1 where there is none
+    const int *pos_of;          // cell -> record position, -1 for cells without a record
+    const unsigned char *code;  // per position: WC_REC a record, WC_W/S/B its neighbour's pressure is the wavefront's
+    double *rec;                // [WR_YG + ng][npos]
+    double *pnew;               // new pressure per record
+    int npos, tj, tk, tt, ntj, steps;
 };
+enum { WC_REC = 1, WC_W = 2, WC_S = 4, WC_B = 8 };
 // record fields; the wavefront's results (WR_O*) are stored in record order
 // too and scattered to the cell arrays by k_rk3_wave_post
 enum { WR_OR, WR_OSIEG, WR_OTG, WR_OCG, WR_AX, WR_AY, WR_AZ, WR_PE, WR_PN, WR_PT, WR_PW, WR_PS, WR_PB, WR_R0, WR_EP,
        WR_SP, WR_INV, WR_TG, WR_ROG, WR_MG, WR_YG };
 
+// the word a reader in another tile takes for a pressure that is not there
+// yet: a NaN with a payload that no operation produces
+constexpr unsigned long long WAVE_EMPTY = 0x7ff4deadbeef0001ull;
+
 // the non-recurrent part of every record, then the commit of the values
 // k_rk3_stage parked (nothing of this stage reads the old ones afterwards).
 // One thread per cell in cell order, so that the reads coalesce; the record
-// stores scatter, but the records of one hyperplane's neighbouring cells
-// (i - 1, j + 1, k) are written a few rows apart in time and meet in L2.
+// stores scatter, but those of neighbouring rows are written a few rows apart
+// in time and meet in L2.
 template <int D>
 __global__ void k_rk3_wave_pre(Prm P, Fld F, RkF K, Wave W, double dt, int stage) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -655,9 +663,10 @@ __global__ void k_rk3_wave_pre(Prm P, Fld F, RkF K, Wave W, double dt, int stage
     auto R = [&](int f) -> double & { return W.rec[(size_t)f * np + pos]; };
     const double *dx = P.dx, *dz = P.dz;
     // lower-face gas velocities as the wavefront sees them: new (parked)
-    // where that neighbour is a record, committed one hyperplane earlier
-    const double ugw = W.src[pos] >= 0 ? K.xug[q.rw] : F.ug[q.rw];
-    const double wgb = W.src[2 * np + pos] >= 0 ? K.xwg[q.rb] : F.wg[q.rb];
+    // where that neighbour is a record, committed one step earlier
+    const int code = W.code[pos];
+    const double ugw = code & WC_W ? K.xug[q.rw] : F.ug[q.rw];
+    const double wgb = code & WC_B ? K.xwg[q.rb] : F.wg[q.rb];
     double indxc = 1.0 / (dx[i] + (dx[i + 1] + dx[i - 1]) * 0.5);
     double indyc = 0.0;
     double indzc = 1.0 / (dz[k] + (dz[k + 1] + dz[k - 1]) * 0.5);
@@ -665,7 +674,7 @@ __global__ void k_rk3_wave_pre(Prm P, Fld F, RkF K, Wave W, double dt, int stage
     double vgc = 0.0;
     double wgc = 0.5 * (F.wg[c] + wgb);
     if (D == 3) {
-        const double vgs = W.src[np + pos] >= 0 ? K.xvg[q.rs] : F.vg[q.rs];
+        const double vgs = code & WC_S ? K.xvg[q.rs] : F.vg[q.rs];
         indyc = 1.0 / (P.dy[j] + (P.dy[j + 1] + P.dy[j - 1]) * 0.5);
         vgc = 0.5 * (F.vg[c] + vgs);
     }
@@ -696,6 +705,7 @@ __global__ void k_rk3_wave_pre(Prm P, Fld F, RkF K, Wave W, double dt, int stage
     double mg = 0.0;
     for (int ig = 0; ig < P.ng; ++ig) mg = mg + GAS(F.xgc, c, ig) * P.gmw[P.gas_type[ig]];
     R(WR_MG) = mg;
+    W.pnew[pos] = __longlong_as_double((long long)WAVE_EMPTY);
     for (int ig = 0; ig < P.ng; ++ig) R(WR_YG + ig) = GAS(F.ygc, c, ig);
     F.rgp[c] = K.xrgp[c];
     F.ep[c] = K.xep[c];
@@ -708,7 +718,6 @@ __global__ void k_rk3_wave_pre(Prm P, Fld F, RkF K, Wave W, double dt, int stage
 // the inputs of one record
 struct WaveIn {
     double ax, ay, az, pe, pn, pt, pw, ps, pb, r0, ep, sp, inv, tg, rog, mg, yg[PDAC_MAXG];
-    int sw, ss, sb;
 };
 
 template <int D>
@@ -720,77 +729,153 @@ __device__ __forceinline__ void wave_load(const Prm &P, const Wave &W, int pos, 
     v.pw = R(WR_PW); v.ps = D == 3 ? R(WR_PS) : 0.0; v.pb = R(WR_PB);
     v.r0 = R(WR_R0); v.ep = R(WR_EP); v.sp = R(WR_SP); v.inv = R(WR_INV); v.tg = R(WR_TG); v.rog = R(WR_ROG);
     v.mg = R(WR_MG);
-    for (int ig = 0; ig < P.ng; ++ig) v.yg[ig] = R(WR_YG + ig);
-    v.sw = W.src[pos]; v.ss = D == 3 ? W.src[np + pos] : -1; v.sb = W.src[2 * np + pos];
+#pragma unroll
+    for (int ig = 0; ig < PDAC_MAXG; ++ig) v.yg[ig] = ig < P.ng ? R(WR_YG + ig) : 0.0;
 }
 
-// the recurrent part: neighbour pressures, right-hand side, enthalpy,
-// temperature and pressure of one record; stores in record order only
-template <int D>
-__device__ __forceinline__ void wave_solve(const Prm &P, const Wave &W, const WaveIn &v, int pos, double a1dt,
-                                           double a2dt, int stage) {
-    const double pw = v.sw >= 0 ? __ldcg(W.pnew + v.sw) : v.pw;
-    const double pb = v.sb >= 0 ? __ldcg(W.pnew + v.sb) : v.pb;
+// a pressure another tile may still be writing, and its writing: single
+// 8-byte words through L2; no other access of the kernel touches them, so no
+// ordering is needed and none is asked of the compiler
+__device__ __forceinline__ unsigned long long wave_look(const double *p) {
+    unsigned long long x;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x) : "l"(p));
+    return x;
+}
+__device__ __forceinline__ void wave_publish(double *p, double v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(__double_as_longlong(v)));
+}
+
+// the recurrent part of one record: from its west, south and bottom
+// pressures the right-hand side, enthalpy, temperature and pressure, which it
+// returns; stores in record order only.  MULTI: other tiles read the pressure
+template <int D, bool MULTI>
+__device__ __forceinline__ double wave_solve(const Prm &P, const Wave &W, const WaveIn &v, int pos, double pw,
+                                             double ps, double pb, double a1dt, double a2dt, int stage) {
     double dpxyz = 0.0;
     dpxyz = dpxyz + v.ax * (v.pe - pw);
-    if (D == 3) {
-        const double ps = v.ss >= 0 ? __ldcg(W.pnew + v.ss) : v.ps;
-        dpxyz = dpxyz + v.ay * (v.pn - ps);
-    } else {
-        dpxyz = dpxyz + 0.0;
-    }
+    if (D == 3) dpxyz = dpxyz + v.ay * (v.pn - ps);
+    else dpxyz = dpxyz + 0.0;
     dpxyz = dpxyz + v.az * (v.pt - pb);
     const double r = v.r0 + v.ep * dpxyz;
     const double siegtmp = stage == 1 ? v.sp + a1dt * r + a2dt * 0.0 : v.sp + a2dt * r;
     const double sieg = siegtmp * v.inv;
     double tg = v.tg, cg;
+    const pdac_fp::Recip mg = pdac_fp::recip(v.mg);
     caloric_eosg(P, cg, tg, v.yg, sieg);
-    const double p = v.rog * tg * P.rgas / v.mg;
+    const double p = pdac_fp::div_by(v.rog * tg * P.rgas, mg);
+    if (MULTI) wave_publish(W.pnew + pos, p);
+    else W.pnew[pos] = p;
     const size_t np = W.npos;
-    __stcg(W.pnew + pos, p);
     W.rec[(size_t)WR_OR * np + pos] = r;
     W.rec[(size_t)WR_OSIEG * np + pos] = sieg;
     W.rec[(size_t)WR_OTG * np + pos] = tg;
     W.rec[(size_t)WR_OCG * np + pos] = cg;
+    return p;
 }
 
-// every hyperplane of a stage in one cooperative launch over the records: a
-// grid-wide barrier separates the hyperplanes (all blocks are co-resident,
-// so it always completes) and the neighbour pressures of the previous
-// hyperplane are read past L1.  When the grid covers the widest hyperplane
-// (ONE) a thread holds at most one record per hyperplane and loads the next
-// one before the barrier, which leaves only the three neighbour pressures on
-// the critical path after it.
-template <int D, bool ONE>
-__global__ void __launch_bounds__(128) k_rk3_wave_rec(Prm P, Wave W, double dt, int stage) {
-    namespace cg = cooperative_groups;
-    cg::grid_group g = cg::this_grid();
-    const int nthr = gridDim.x * blockDim.x;
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+constexpr int WAVE_LOOKS = 1 << 22;  // the limit of one wait: a second or two
+
+// The wavefront of a stage in one launch, a block per tile.  The west
+// pressure of a cell is its thread's previous one, the south and bottom ones
+// are its neighbours' of the previous step, through shared memory and one
+// block barrier a step; the tile's first columns take theirs from the tiles
+// to the south and below, through L2.  What bounds it is one record's
+// dependent chain (the caloric iteration) per step over nx + ny + nz steps:
+// with every hyperplane of the mesh spread over the device and separated by a
+// grid-wide barrier a step of 128 x 128 x 96 took 4.6 us, of which about 3 the
+// exchange (a wait for the single pressures through L2 took as long); here an
+// exchange between tiles costs its latency once per tile, not once per step,
+// since a tile that runs behind its neighbours finds their pressures there
+// (looked for one step ahead).  Both stages with their records, before and
+// now: 128 x 192 1.99 -> 0.63 ms, 128 x 128 x 96 3.85 -> 2.0, 224 x 208 x 161
+// 9.6 -> 5.7.
+//
+// A tile waits only for tiles of lower index and all blocks are resident (a
+// cooperative launch, unless there is one tile), so the waits end: a pressure
+// word holds WAVE_EMPTY from k_rk3_wave_pre until its record is solved.  Each
+// wait is bounded all the same; one that runs out sets *gave_up, on which the
+// other waits give up too and every block leaves after its next barrier.
+// ONE: a thread per column, which loads the next step's record while this one
+// is solved; else a thread takes several columns in turn.
+// MULTI: there is more than one tile.
+template <int D, bool ONE, bool MULTI>
+__global__ void __launch_bounds__(ONE ? 256 : 512) k_rk3_wave_tile(Prm P, Wave W, double dt, int stage, int *gave_up) {
+    extern __shared__ double sp[];  // [2][tt]
+    const int tt = W.tt, tile = blockIdx.x, steps = W.steps;
     const double a1dt = (stage == 1 ? 1.0 : 0.25) * dt, a2dt = (stage == 1 ? 0.0 : 0.25) * dt;
-    if (ONE) {
-        WaveIn v;
-        int pos = W.start[0] + tid;
-        bool have = pos < W.start[1];
-        if (have) wave_load<D>(P, W, pos, v);
-        for (int q = 0; q < W.nplanes; ++q) {
-            if (have) wave_solve<D>(P, W, v, pos, a1dt, a2dt, stage);
-            if (q + 1 < W.nplanes) {
-                pos = W.start[q + 1] + tid;
-                have = pos < W.start[q + 2];
-                if (have) wave_load<D>(P, W, pos, v);
+    const int base = tile * steps * tt;
+    // from a position to its southern / bottom neighbour's in the next tile
+    const int off_s = (W.tj - 1 - steps) * tt + W.tj - 1;
+    const int off_b = (W.tk - 1 - W.ntj * steps) * tt + W.tj * (W.tk - 1);
+    auto wait = [&](const double *p, unsigned long long x, bool &lost) {
+        for (int q = 0; x == WAVE_EMPTY; ++q) {
+            x = wave_look(p);
+            if (q >= WAVE_LOOKS || ((q & 1023) == 1023 && *(volatile int *)gave_up)) {
+                lost = true;
+                break;
             }
-            g.sync();
         }
+        return __longlong_as_double((long long)x);
+    };
+    if (ONE) {
+        const int t = threadIdx.x, jl = t % W.tj, kl = t / W.tj;
+        const bool south = jl == 0, below = kl == 0;
+        int pos = base + t, code = W.code[pos], code1 = steps > 1 ? W.code[pos + tt] : 0;
+        unsigned long long es = WAVE_EMPTY, eb = WAVE_EMPTY;  // looked for one step ahead
+        double pown = 0.0;
+        // step s on record v while the next one arrives in w
+        auto step = [&](int s, WaveIn &v, WaveIn &w) {
+            const int npos = pos + tt, code2 = s + 2 < steps ? W.code[npos + tt] : 0;
+            unsigned long long ns = WAVE_EMPTY, nb = WAVE_EMPTY;
+            if (code1 & WC_REC) wave_load<D>(P, W, npos, w);
+            if (MULTI && (code1 & WC_S) && south) ns = wave_look(W.pnew + npos + off_s);
+            if (MULTI && (code1 & WC_B) && below) nb = wave_look(W.pnew + npos + off_b);
+            bool lost = false;
+            if (code & WC_REC) {
+                const double *prev = sp + ((s + 1) & 1) * tt;
+                double ps = v.ps, pb = v.pb;
+                if (code & WC_S) ps = MULTI && south ? wait(W.pnew + pos + off_s, es, lost) : prev[t - 1];
+                if (code & WC_B) pb = MULTI && below ? wait(W.pnew + pos + off_b, eb, lost) : prev[t - W.tj];
+                pown = wave_solve<D, MULTI>(P, W, v, pos, code & WC_W ? pown : v.pw, ps, pb, a1dt, a2dt, stage);
+                sp[(s & 1) * tt + t] = pown;
+            }
+            pos = npos;
+            code = code1;
+            code1 = code2;
+            es = ns;
+            eb = nb;
+            if (MULTI) return __syncthreads_or(lost) != 0;
+            __syncthreads();
+            return false;
+        };
+        WaveIn v, w;
+        if (code & WC_REC) wave_load<D>(P, W, pos, v);
+        bool lost = false;
+        for (int s = 0; s < steps && !lost; s += 2) {
+            lost = step(s, v, w);
+            if (!lost && s + 1 < steps) lost = step(s + 1, w, v);
+        }
+        if (lost && t == 0) atomicExch(gave_up, 1);
     } else {
-        for (int q = 0; q < W.nplanes; ++q) {
-            const int end = W.start[q + 1];
-            for (int pos = W.start[q] + tid; pos < end; pos += nthr) {
+        for (int s = 0; s < steps; ++s) {
+            bool lost = false;
+            for (int t = threadIdx.x; t < tt; t += blockDim.x) {
+                const int pos = base + s * tt + t, code = W.code[pos];
+                if (!(code & WC_REC)) continue;
+                const int jl = t % W.tj, kl = t / W.tj;
                 WaveIn v;
                 wave_load<D>(P, W, pos, v);
-                wave_solve<D>(P, W, v, pos, a1dt, a2dt, stage);
+                const double *prev = sp + ((s + 1) & 1) * tt;
+                double ps = v.ps, pb = v.pb;
+                if (code & WC_S) ps = jl == 0 ? wait(W.pnew + pos + off_s, WAVE_EMPTY, lost) : prev[t - 1];
+                if (code & WC_B) pb = kl == 0 ? wait(W.pnew + pos + off_b, WAVE_EMPTY, lost) : prev[t - W.tj];
+                sp[(s & 1) * tt + t] =
+                    wave_solve<D, MULTI>(P, W, v, pos, code & WC_W ? prev[t] : v.pw, ps, pb, a1dt, a2dt, stage);
             }
-            g.sync();
+            if (__syncthreads_or(lost)) {
+                if (threadIdx.x == 0) atomicExch(gave_up, 1);
+                return;
+            }
         }
     }
 }
@@ -802,6 +887,7 @@ __global__ void k_rk3_wave_post(Prm P, Fld F, RkF K, Wave W, int stage) {
     if (pos >= W.npos) return;
     const size_t np = W.npos, n = P.ncell;
     const int c = W.order[pos], e0 = (D == 3 ? 4 : 3) * P.nph;
+    if (c < 0) return;
     (stage == 1 ? K.k1 : K.k2)[(size_t)e0 * n + c] = W.rec[(size_t)WR_OR * np + pos];
     F.sieg[c] = W.rec[(size_t)WR_OSIEG * np + pos];
     F.tg[c] = W.rec[(size_t)WR_OTG * np + pos];
@@ -996,7 +1082,7 @@ __global__ void k_rk3_solve(Prm P, Fld F, RkF K, double dt) {
     }
     // closure: caloric_eosg, caloric_eosl, volume fraction, density, pressure
     double yg[PDAC_MAXG];
-    for (int ig = 0; ig < P.ng; ++ig) yg[ig] = GAS(F.ygc, c, ig);
+    load_ygc(P, F, c, yg);
     double tg = F.tg[c], cg;
     int info = caloric_eosg(P, cg, tg, yg, sieg);
     F.sieg[c] = sieg;
