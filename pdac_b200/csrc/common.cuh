@@ -73,6 +73,9 @@ struct Prm {
     unsigned long long mnx, mny;
     const double *p_atm, *t_atm;
     const int *flag;
+    // 3D with MUSCL: one bit per cell whose flux stencils need no look at the
+    // flags (k_simple_mask); null: none
+    const unsigned *simple;
     // immersed boundaries (immb.f, ghost.f:2888-3345); immb = 0: none, and
     // every face factor below reads as 1
     int immb;

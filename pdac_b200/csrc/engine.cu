@@ -68,6 +68,10 @@ struct pdac_ctx {
     int *d_status = nullptr, *h_status = nullptr;
     unsigned *d_dirty = nullptr;                 // corrector active set, one bit per cell
     unsigned *d_cmask = nullptr;                 // fluid cells per colour, the active set's words
+    // 3D with MUSCL: the mask of simple cells (P.simple) and the list of the
+    // other fluid cells
+    unsigned *d_simple = nullptr;
+    int *d_rest = nullptr, nrest = 0;
     int inner_grid = 0;
     int *d_nit = nullptr, *h_nit = nullptr;  // outer sweep number (device, pinned host)
     // the outer sweep loop as a graph: a conditional WHILE node whose body is
@@ -148,13 +152,22 @@ struct pdac_ctx {
 namespace {
 
 // forms of the 3D momentum-flux pass (launch_mom_tile): 0 = one thread per
-// (cell, phase) and component, three launches (k_tilde_flux3d<0|1|2>, the
-// stencils gathered through L1); 1..4 = the shared-memory tiled pass
-// k_mom_flux3d_tile with 32 x 4, 32 x 8, 16 x 8 or 64 x 2 cells (i x j) per
-// block.  Measured on the 256 x 256 x 192 plume (the autotuner picks per
-// run): form 0 took 8.2 ms per tilde, the 32 x 4 tile ~9 ms -- its threads
-// run all three components between two barriers at 12 warps per SM
+// (cell, phase, component), the simple cells and the others in a launch each
+// (k_tilde_flux3d, the stencils gathered through L1); 1..4 = the
+// shared-memory tiled pass k_mom_flux3d_tile with 32 x 4, 32 x 8, 16 x 8 or
+// 64 x 2 cells (i x j) per block.  Measured (the autotuner picks per run): on
+// 128 x 128 x 96 form 0 takes 0.80 ms per tilde (1.16 before the simple cells
+// had a pass of their own); on 256 x 256 x 192 it took 8.2 then and the 32 x 4
+// tile ~9 ms -- its threads run all three components between two barriers at
+// 12 warps per SM
 const int N_TILE_SHAPES = 5;
+
+// the cells of the general flux and stress passes: those the simple pass
+// leaves (list), or all n cells of the mesh (list null) without one
+struct RestCells {
+    const int *list;
+    int n;
+};
 
 // set_attr: raise the kernel's dynamic shared-memory limit (done once per
 // context at create, outside any stream capture); else launch it
@@ -171,7 +184,7 @@ cudaError_t launch_mom_tile_t(const pdac::Prm &P, const pdac::Fld &F, int nph, i
 
 template <typename Real>
 cudaError_t launch_mom_tile(const pdac::Prm &P, const pdac::Fld &F, int nph, int shape, int kchunk, cudaStream_t st,
-                            bool set_attr = false) {
+                            RestCells rest, bool set_attr = false) {
     // the tiled pass reads its stencils from shared memory and does not
     // apply the immersed-boundary velocity masks: immersed boundaries use form 0
     if (P.immb && !set_attr) shape = 0;
@@ -182,23 +195,22 @@ cudaError_t launch_mom_tile(const pdac::Prm &P, const pdac::Fld &F, int nph, int
         case 4: return launch_mom_tile_t<64, 2, Real>(P, F, nph, kchunk, st, set_attr);
         default: {
             if (set_attr) return cudaSuccess;
-            const long nt = (long)P.ncell * nph;
-            const int g = (int)((nt + 127) / 128);
-            pdac::k_tilde_flux3d<0, Real><<<g, 128, 0, st>>>(P, F);
-            pdac::k_tilde_flux3d<1, Real><<<g, 128, 0, st>>>(P, F);
-            pdac::k_tilde_flux3d<2, Real><<<g, 128, 0, st>>>(P, F);
+            if (P.simple)
+                pdac::k_tilde_flux3d<Real, true><<<dim3(3 * ((P.ncell + 127) / 128), nph), 128, 0, st>>>(P, F, nullptr, 0);
+            if (rest.n > 0)
+                pdac::k_tilde_flux3d<Real, false><<<dim3(3 * ((rest.n + 127) / 128), nph), 128, 0, st>>>(P, F, rest.list, rest.n);
             return cudaGetLastError();
         }
     }
 }
 
 // kernel launches of one momentum-flux pass of form shape
-inline int mom_launches(int shape) { return shape == 0 ? 3 : 1; }
+inline int mom_launches(int shape) { return shape == 0 ? 2 : 1; }
 
 cudaError_t set_tile_attrs(const pdac::Prm &P, const pdac::Fld &F) {
     for (int s = 0; s < N_TILE_SHAPES; ++s) {
-        cudaError_t e = launch_mom_tile<double>(P, F, 1, s, 1, nullptr, true);
-        if (e == cudaSuccess) e = launch_mom_tile<float>(P, F, 1, s, 1, nullptr, true);
+        cudaError_t e = launch_mom_tile<double>(P, F, 1, s, 1, nullptr, RestCells{}, true);
+        if (e == cudaSuccess) e = launch_mom_tile<float>(P, F, 1, s, 1, nullptr, RestCells{}, true);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -211,6 +223,23 @@ int fail(pdac_ctx *c, int code, const std::string &msg) {
     if (c) c->err = msg;
     return code;
 }
+
+// the general passes' cells of a context, and kernel launches over a 3D
+// stencil pass KERNEL(SIMPLE): the simple cells, then the others; gy: grid.y
+RestCells rest_cells(const pdac_ctx *c) {
+    return c->P.simple ? RestCells{c->d_rest, c->nrest} : RestCells{nullptr, c->ncell};
+}
+#define STENCIL_LAUNCH(ctx, gy, st, KSIMPLE, KREST, ...)                                                          \
+    do {                                                                                                         \
+        const RestCells rc_ = rest_cells(ctx);                                                                   \
+        if ((ctx)->P.simple)                                                                                     \
+            KSIMPLE<<<dim3(((ctx)->ncell + 127) / 128, gy), 128, 0, st>>>((ctx)->P, (ctx)->F, __VA_ARGS__ nullptr, 0), \
+                (ctx)->launches++;                                                                               \
+        if (rc_.n > 0)                                                                                           \
+            KREST<<<dim3((rc_.n + 127) / 128, gy), 128, 0, st>>>((ctx)->P, (ctx)->F, __VA_ARGS__ rc_.list, rc_.n), \
+                (ctx)->launches++;                                                                               \
+    } while (0)
+#define PDAC_COMMA ,
 
 #define CK(x)                                                                                  \
     do {                                                                                       \
@@ -966,6 +995,18 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     CK(cudaMalloc(&ctx->d_wcount, 16 * sizeof(int)));
     CK(cudaMalloc(&ctx->d_dirty, ((size_t)n + 31) / 32 * sizeof(unsigned)));
     CK(cudaMalloc(&ctx->d_cmask, (size_t)3 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
+    if (ctx->d3 && P.muscl > 0) {
+        CK(cudaMalloc(&ctx->d_simple, ((size_t)n + 31) / 32 * sizeof(unsigned)));
+        pdac::k_simple_mask<<<blocks(((long)n + 31) / 32), TPB, 0, ctx->stream>>>(P, ctx->d_simple);
+        P.simple = ctx->d_simple;
+        CK(cudaMemsetAsync(ctx->d_nonfinite, 0, sizeof(int), ctx->stream));  // counts here
+        pdac::k_rest_list<<<blocks(n, 256), 256, 0, ctx->stream>>>(P, ctx->d_nonfinite, nullptr);
+        CK(cudaMemcpyAsync(&ctx->nrest, ctx->d_nonfinite, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        CK(cudaMalloc(&ctx->d_rest, (size_t)std::max(1, ctx->nrest) * sizeof(int)));
+        CK(cudaMemsetAsync(ctx->d_nonfinite, 0, sizeof(int), ctx->stream));
+        pdac::k_rest_list<<<blocks(n, 256), 256, 0, ctx->stream>>>(P, ctx->d_nonfinite, ctx->d_rest);
+    }
     pdac::k_colour_masks<<<blocks(((long)n + 31) / 32), TPB, 0, ctx->stream>>>(P, ctx->d_cmask);
     CK(cudaGetLastError());
     {
@@ -1187,6 +1228,8 @@ int pdac_gpu_destroy(pdac_ctx *ctx) {
     cudaFree(ctx->d_nit);
     cudaFreeHost(ctx->h_nit);
     cudaFree(ctx->d_cmask);
+    cudaFree(ctx->d_simple);
+    cudaFree(ctx->d_rest);
     cudaFree(ctx->d_partial);
     cudaFree(ctx->d_fk);
     cudaFree(ctx->d_sinkbuf);
@@ -1469,10 +1512,9 @@ static int enqueue_tilde(pdac_ctx *ctx, double dt, cudaStream_t st) {
     if (s) return s;
     if (ctx->d3) {
         CK(cudaMemsetAsync(F.mf, 0, n * 9 * (ns + 1) * sizeof(double), st));
-        pdac::k_visc3d<<<blocks((long)n * (ns + 1)), TPB, 0, st>>>(ctx->P, F);
-        ctx->launches++;
-        if (ctx->P.mixed) CK(launch_mom_tile<float>(ctx->P, F, ctx->nph, ctx->tile_shape, ctx->tile_kchunk, st));
-        else CK(launch_mom_tile<double>(ctx->P, F, ctx->nph, ctx->tile_shape, ctx->tile_kchunk, st));
+        STENCIL_LAUNCH(ctx, ctx->nph, st, pdac::k_visc3d<true>, pdac::k_visc3d<false>, );
+        if (ctx->P.mixed) CK(launch_mom_tile<float>(ctx->P, F, ctx->nph, ctx->tile_shape, ctx->tile_kchunk, st, rest_cells(ctx)));
+        else CK(launch_mom_tile<double>(ctx->P, F, ctx->nph, ctx->tile_shape, ctx->tile_kchunk, st, rest_cells(ctx)));
         ctx->launches += mom_launches(ctx->tile_shape);
         PHASE_LAUNCH(ctx->nph, pdac::k_tilde3d, blocks(n), TPB, st, ctx->P, F, dt, ctx->d_app0u, ctx->d_app0v, ctx->d_app0w);
         ctx->launches++;
@@ -1637,7 +1679,8 @@ int pdac_gpu_iter(pdac_ctx *ctx, double dt, int *nit_out) {
     int nph = ctx->nph;
     if (ctx->d3) {
         PHASE_LAUNCH(nph, pdac::k_predictor3d, blocks(n), TPB, st, ctx->P, F, dt);
-        pdac::k_mflux_init3d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);
+        STENCIL_LAUNCH(ctx, 1, st, pdac::k_mflux_init3d<true>, pdac::k_mflux_init3d<false>, dt PDAC_COMMA);
+        ctx->launches--;  // counted below
     } else {
         PHASE_LAUNCH(nph, pdac::k_predictor2d, blocks(n), TPB, st, ctx->P, F, dt);
         pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);
@@ -1827,7 +1870,8 @@ int pdac_gpu_iter_static(pdac_ctx *ctx, double dt, int *nit_out) {
     int nph = ctx->nph;
     if (ctx->d3) {
         PHASE_LAUNCH(nph, pdac::k_predictor3d, blocks(n), TPB, st, ctx->P, F, dt);
-        pdac::k_mflux_init3d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);
+        STENCIL_LAUNCH(ctx, 1, st, pdac::k_mflux_init3d<true>, pdac::k_mflux_init3d<false>, dt PDAC_COMMA);
+        ctx->launches--;  // counted below
     } else {
         PHASE_LAUNCH(nph, pdac::k_predictor2d, blocks(n), TPB, st, ctx->P, F, dt);
         pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);
@@ -1876,8 +1920,8 @@ static int enqueue_ygas(pdac_ctx *ctx, double dt, cudaStream_t st) {
     for (double *a : {ctx->F.yfe, ctx->F.yfn, ctx->F.yft})
         if (a) CK(cudaMemsetAsync(a, 0, n * ctx->ng * sizeof(double), st));
     if (ctx->d3) {
-        (ctx->P.mixed ? pdac::k_ygas_flux3d<float> : pdac::k_ygas_flux3d<double>)<<<blocks(n), TPB, 0, st>>>(ctx->P, ctx->F),
-            ctx->launches++;
+        if (ctx->P.mixed) STENCIL_LAUNCH(ctx, 1, st, (pdac::k_ygas_flux3d<float, true>), (pdac::k_ygas_flux3d<float, false>), );
+        else STENCIL_LAUNCH(ctx, 1, st, (pdac::k_ygas_flux3d<double, true>), (pdac::k_ygas_flux3d<double, false>), );
         pdac::k_ygas3d<<<blocks(n), TPB, 0, st>>>(ctx->P, ctx->F, dt), ctx->launches++;
     } else {
         (ctx->P.mixed ? pdac::k_ygas_flux2d<float> : pdac::k_ygas_flux2d<double>)<<<blocks(n), TPB, 0, st>>>(ctx->P, ctx->F),
@@ -1916,9 +1960,10 @@ static int enqueue_htilde(pdac_ctx *ctx, double dt, cudaStream_t st) {
         if (a) CK(cudaMemsetAsync(a, 0, n * ns * sizeof(double), st));
     accumulate_conductivity(ctx, st);
     if (ctx->d3) {
-        (ctx->P.mixed ? pdac::k_htilde_flux3d<true, float> : pdac::k_htilde_flux3d<true, double>)<<<blocks(n), TPB, 0, st>>>(
-            ctx->P, F),
-            ctx->launches++;
+        if (ctx->P.mixed)
+            STENCIL_LAUNCH(ctx, ctx->nph, st, (pdac::k_htilde_flux3d<true, float, true>), (pdac::k_htilde_flux3d<true, float, false>), );
+        else
+            STENCIL_LAUNCH(ctx, ctx->nph, st, (pdac::k_htilde_flux3d<true, double, true>), (pdac::k_htilde_flux3d<true, double, false>), );
         pdac::k_htilde3d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt), ctx->launches++;
     } else {
         (ctx->P.mixed ? pdac::k_htilde_flux2d<true, float> : pdac::k_htilde_flux2d<true, double>)<<<blocks(n), TPB, 0, st>>>(
@@ -1991,7 +2036,8 @@ int pdac_gpu_initialize_fieldn(pdac_ctx *ctx) {
     if (ctx->d3) {
         PHASE_LAUNCH_D(ctx->nph, pdac::k_rk3_fieldn, 3, blocks(n), TPB, st, ctx->P, F, ctx->K, ctx->cfg.dt);
         if (int s = accumulate_viscosities(ctx, st)) return s;
-        pdac::k_visc3d<<<blocks((long)n * (ns + 1)), TPB, 0, st>>>(ctx->P, F);
+        STENCIL_LAUNCH(ctx, ctx->nph, st, pdac::k_visc3d<true>, pdac::k_visc3d<false>, );
+        ctx->launches--;  // counted below
     } else {
         PHASE_LAUNCH_D(ctx->nph, pdac::k_rk3_fieldn, 2, blocks(n), TPB, st, ctx->P, F, ctx->K, ctx->cfg.dt);
         if (int s = accumulate_viscosities(ctx, st)) return s;
@@ -2055,23 +2101,26 @@ static long long enqueue_explicit(pdac_ctx *ctx, double dt, cudaStream_t st, boo
             L++;
         }
         if (ctx->d3) {
+            const long long before = ctx->launches;
             if (P.mixed) {
-                pdac::k_rk3_mflux<3, float><<<blocks(n), TPB, 0, st>>>(P, F);
-                (void)launch_mom_tile<float>(P, F, nph, ctx->tile_shape, ctx->tile_kchunk, st);
-                pdac::k_htilde_flux3d<false, float><<<blocks(n), TPB, 0, st>>>(P, F);
+                STENCIL_LAUNCH(ctx, nph, st, (pdac::k_rk3_mflux<3, float, true>), (pdac::k_rk3_mflux<3, float, false>), );
+                (void)launch_mom_tile<float>(P, F, nph, ctx->tile_shape, ctx->tile_kchunk, st, rest_cells(ctx));
+                STENCIL_LAUNCH(ctx, nph, st, (pdac::k_htilde_flux3d<false, float, true>), (pdac::k_htilde_flux3d<false, float, false>), );
             } else {
-                pdac::k_rk3_mflux<3><<<blocks(n), TPB, 0, st>>>(P, F);
-                (void)launch_mom_tile<double>(P, F, nph, ctx->tile_shape, ctx->tile_kchunk, st);
-                pdac::k_htilde_flux3d<false><<<blocks(n), TPB, 0, st>>>(P, F);
+                STENCIL_LAUNCH(ctx, nph, st, (pdac::k_rk3_mflux<3, double, true>), (pdac::k_rk3_mflux<3, double, false>), );
+                (void)launch_mom_tile<double>(P, F, nph, ctx->tile_shape, ctx->tile_kchunk, st, rest_cells(ctx));
+                STENCIL_LAUNCH(ctx, nph, st, (pdac::k_htilde_flux3d<false, double, true>), (pdac::k_htilde_flux3d<false, double, false>), );
             }
-            L += 2 + mom_launches(ctx->tile_shape);
+            L += ctx->launches - before;
+            ctx->launches = before;  // the caller adds L
+            L += mom_launches(ctx->tile_shape);
         } else {
             if (P.mixed) {
-                pdac::k_rk3_mflux<2, float><<<blocks(n), TPB, 0, st>>>(P, F);
+                pdac::k_rk3_mflux<2, float, false><<<blocks(n), TPB, 0, st>>>(P, F, nullptr, 0);
                 pdac::k_tilde_flux2d<float><<<blocks(n), TPB, 0, st>>>(P, F);
                 pdac::k_htilde_flux2d<false, float><<<blocks(n), TPB, 0, st>>>(P, F);
             } else {
-                pdac::k_rk3_mflux<2><<<blocks(n), TPB, 0, st>>>(P, F);
+                pdac::k_rk3_mflux<2, double, false><<<blocks(n), TPB, 0, st>>>(P, F, nullptr, 0);
                 pdac::k_tilde_flux2d<<<blocks(n), TPB, 0, st>>>(P, F);
                 pdac::k_htilde_flux2d<false><<<blocks(n), TPB, 0, st>>>(P, F);
             }
@@ -2435,8 +2484,8 @@ int pdac_gpu_autotune(pdac_ctx *ctx, const char *cache_path, int *out, int nout)
             for (int kc : chunks) {
                 if (kc < 1 || kc > ctx->nz || (shape == 0 && kc != chunks[1])) continue;  // form 0 has no chunks
                 auto launch = [&]() {
-                    return ctx->P.mixed ? launch_mom_tile<float>(ctx->P, ctx->F, ctx->nph, shape, kc, st)
-                                        : launch_mom_tile<double>(ctx->P, ctx->F, ctx->nph, shape, kc, st);
+                    return ctx->P.mixed ? launch_mom_tile<float>(ctx->P, ctx->F, ctx->nph, shape, kc, st, rest_cells(ctx))
+                                        : launch_mom_tile<double>(ctx->P, ctx->F, ctx->nph, shape, kc, st, rest_cells(ctx));
                 };
                 cudaError_t e = launch();
                 if (e == cudaSuccess) e = cudaEventRecord(a, st);
@@ -3022,7 +3071,8 @@ static int enqueue_step_pre(pdac_ctx *ctx, double dt, cudaStream_t st) {
     const int nph = ctx->nph;
     if (ctx->d3) {
         PHASE_LAUNCH(nph, pdac::k_predictor3d, blocks(n), TPB, st, ctx->P, F, dt);
-        pdac::k_mflux_init3d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);
+        STENCIL_LAUNCH(ctx, 1, st, pdac::k_mflux_init3d<true>, pdac::k_mflux_init3d<false>, dt PDAC_COMMA);
+        ctx->launches--;  // counted below
     } else {
         PHASE_LAUNCH(nph, pdac::k_predictor2d, blocks(n), TPB, st, ctx->P, F, dt);
         pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);

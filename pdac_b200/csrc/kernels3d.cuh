@@ -246,24 +246,44 @@ __global__ void k_fieldn3d(Prm P, Fld F) {
 // ---------------------------------------------------------------------------
 // tilde momentum fluxes, compute_all_fluxes_tilde tilde.f:850-1326 (3D)
 // ---------------------------------------------------------------------------
-// one thread per (cell, phase) for one momentum component COMP (0 = x,
-// 1 = y, 2 = z): consecutive threads take consecutive cells of one phase.
-// Real is the arithmetic type: double, or float in the mixed-precision mode
-// (the FP64 state is converted as it is read; fluxes are stored in FP64).
-template <int COMP, typename Real = double>
-__global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_tilde_flux3d(Prm P, Fld F) {
-    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (unsigned)P.ncell * (unsigned)(P.ns + 1)) return;
-    int ph = (int)(t / (unsigned)P.ncell), c = (int)(t % (unsigned)P.ncell);
-    if (!fluid(P, c)) return;
-    int i, j, k;
-    ijk_of(P, c, i, j, k);
-    Raw3 R;
-    Rem3 M;
-    raw3(P, i, j, k, R);
-    rem3(P, i, j, k, R, M);
-    bool dw = !fluid(P, R.w), ds = !fluid(P, R.s), db = !fluid(P, R.b);
-    bool mus = P.muscl > 0 && P.flag[c] == FLUID;
+// The cell of a flux or stress thread: with SIMPLE the pass covers the simple
+// cells, thread t taking cell t if it is one, else the cells of the list
+// (list null: every fluid cell).  false: nothing to do.
+//
+// Most of a mesh is simple, and there the index work (clamped neighbours, 25
+// flag reads, remapping, per-face conditions) was most of the instructions:
+// the momentum pass of 128 x 128 x 96 issued ~1140 a thread and component,
+// bound by issue at 24 % of the FP64 pipe.  Splitting the pass in two launches
+// keeps the general path's registers out of the simple one.
+template <bool SIMPLE>
+__device__ __forceinline__ bool stencil_cell(const Prm &P, unsigned t, const int *list, int nlist, int &c, int &i,
+                                             int &j, int &k, Raw3 &R, Rem3 &M) {
+    if (SIMPLE) {
+        if (t >= (unsigned)P.ncell || !is_simple(P, (int)t)) return false;
+        c = (int)t;
+        raw3_simple(P, c, R);
+        rem3_simple(R, M);
+        ijk_of(P, c, i, j, k);
+    } else {
+        if (t >= (unsigned)nlist) return false;
+        c = list ? list[t] : (int)t;
+        if (!fluid(P, c)) return false;
+        ijk_of(P, c, i, j, k);
+        raw3(P, i, j, k, R);
+        rem3(P, i, j, k, R, M);
+    }
+    return true;
+}
+
+// the fluxes of one momentum component COMP (0 = x, 1 = y, 2 = z) of one
+// phase of one cell.  Real is the arithmetic type: double, or float in the
+// mixed-precision mode (the FP64 state is converted as it is read; fluxes are
+// stored in FP64).
+template <int COMP, typename Real, bool SIMPLE>
+__device__ __forceinline__ void tilde_flux_cell(const Prm &P, const Fld &F, int ph, int c, int i, int j, int k,
+                                                const Raw3 &R, const Rem3 &M) {
+    const bool dw = !SIMPLE && !fluid(P, R.w), ds = !SIMPLE && !fluid(P, R.s), db = !SIMPLE && !fluid(P, R.b);
+    const bool mus = SIMPLE || (P.muscl > 0 && P.flag[c] == FLUID);
     size_t n = P.ncell;
     size_t off = (size_t)(ph > 0 ? ph - 1 : 0) * n;
     const double *U = ph == 0 ? F.ug : F.us + off;
@@ -274,26 +294,42 @@ __global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_tilde_flux3d(Prm P, Fld
     rnb3(u, U, R);
     rnb3(v, V, R);
     rnb3(w, W, R);
-    if (ib_masked(P, c)) { ib_mask3(P, u, R, 1); ib_mask3(P, v, R, 16); ib_mask3(P, w, R, 4); }
+    if (!SIMPLE && ib_masked(P, c)) { ib_mask3(P, u, R, 1); ib_mask3(P, v, R, 16); ib_mask3(P, w, R, 4); }
     nb3(d, D, R, M);
     F6T<Real> f = {0, 0, 0, 0, 0, 0};
     if (COMP == 0) {  // x momentum
         interp_x3(P, d, i, ds3);
         flu_3d(P, f, dw, ds, db, ds3, u, v, w, i);
-        if (mus && i != P.nx - 1) muscl_flu_3d(P, f, ds3, u, v, w, i, j, k);
+        if (mus && (SIMPLE || i != P.nx - 1)) muscl_flu_3d(P, f, ds3, u, v, w, i, j, k);
     } else if (COMP == 1) {  // y momentum
         interp_y3(P, d, j, ds3);
         flv_3d(P, f, dw, ds, db, ds3, u, v, w, j);
-        if (mus && j != P.ny - 1) muscl_flv_3d(P, f, ds3, u, v, w, i, j, k);
+        if (mus && (SIMPLE || j != P.ny - 1)) muscl_flv_3d(P, f, ds3, u, v, w, i, j, k);
     } else {  // z momentum
         interp_z3(P, d, k, ds3);
         flw_3d(P, f, dw, ds, db, ds3, u, v, w, k);
-        if (mus && k != P.nz - 1) muscl_flw_3d(P, f, ds3, u, v, w, i, j, k);
+        if (mus && (SIMPLE || k != P.nz - 1)) muscl_flw_3d(P, f, ds3, u, v, w, i, j, k);
     }
     MFX(ph, COMP, 0)[c] = f.e; MFX(ph, COMP, 1)[c] = f.n; MFX(ph, COMP, 2)[c] = f.t;
     if (dw) MFX(ph, COMP, 0)[R.w] = f.w;
     if (ds) MFX(ph, COMP, 1)[R.s] = f.s;
     if (db) MFX(ph, COMP, 2)[R.b] = f.b;
+}
+
+// one thread per (cell, phase, component): blocks of consecutive cells, the
+// three components of the same cells next to each other (they read the same
+// fields), phase in blockIdx.y
+template <typename Real, bool SIMPLE>
+__global__ void __launch_bounds__(128, SIMPLE ? (sizeof(Real) == 8 ? 5 : 7) : PDAC_FLUX_MINB) k_tilde_flux3d(Prm P, Fld F, const int *list, int nlist) {
+    const unsigned comp = blockIdx.x % 3u, t = (blockIdx.x / 3u) * blockDim.x + threadIdx.x;
+    const int ph = blockIdx.y;
+    int c, i, j, k;
+    Raw3 R;
+    Rem3 M;
+    if (!stencil_cell<SIMPLE>(P, t, list, nlist, c, i, j, k, R, M)) return;
+    if (comp == 0) tilde_flux_cell<0, Real, SIMPLE>(P, F, ph, c, i, j, k, R, M);
+    else if (comp == 1) tilde_flux_cell<1, Real, SIMPLE>(P, F, ph, c, i, j, k, R, M);
+    else tilde_flux_cell<2, Real, SIMPLE>(P, F, ph, c, i, j, k, R, M);
 }
 
 // tilde mesh loop, tilde.f:276-848 (3D), with stress3D, kdrags/sdrag and
@@ -302,18 +338,14 @@ __global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_tilde_flux3d(Prm P, Fld
 // viscous stress divergence of one phase of one cell (viscg / viscs,
 // visc.f:150-291, stress3D visc.f:293-559) with the particle repulsion term
 // (tilde.f:362-416); one thread per (cell, phase), consecutive threads take
-// consecutive cells of one phase
-__global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_visc3d(Prm P, Fld F) {
-    unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (unsigned)P.ncell * (unsigned)(P.ns + 1)) return;
-    int ph = (int)(t / (unsigned)P.ncell), c = (int)(t % (unsigned)P.ncell);
-    if (!fluid(P, c)) return;
-    int i, j, k;
-    ijk_of(P, c, i, j, k);
+// consecutive cells of one phase (blockIdx.y)
+template <bool SIMPLE>
+__global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_visc3d(Prm P, Fld F, const int *list, int nlist) {
+    const int ph = blockIdx.y;
+    int c, i, j, k;
     Raw3 R;
     Rem3 M;
-    raw3(P, i, j, k, R);
-    rem3(P, i, j, k, R, M);
+    if (!stencil_cell<SIMPLE>(P, blockIdx.x * blockDim.x + threadIdx.x, list, nlist, c, i, j, k, R, M)) return;
     const double *dx = P.dx, *dy = P.dy, *dz = P.dz;
     size_t n = P.ncell;
     size_t off = (size_t)(ph > 0 ? ph - 1 : 0) * n;
@@ -553,19 +585,21 @@ __global__ void k_predictor3d(Prm P, Fld F, double dt) {
 
 // mass flux of one cell over its six faces (calc_gas_mass_flux and
 // calc_part_mass_flux, iter.f:597-925): densities remapped, velocities raw
+template <bool SIMPLE>
 __device__ __forceinline__ void cell_massflux3d(const Prm &P, const double *D, const double *U, const double *V,
                                                 const double *W, const Raw3 &R, const Rem3 &M, int i, int j, int k,
                                                 F6d &f) {
     S3 d;
     first_nb3(d, D, R, M);
-    bool mus = P.muscl > 0 && P.flag[R.c] == FLUID;
+    const bool mus = SIMPLE || (P.muscl > 0 && P.flag[R.c] == FLUID);
     if (mus) third_nb3(d, D, M);
-    const int *fl = P.flag;
-    massflux_3d(P, d, U[R.w], U[R.c], V[R.s], V[R.c], W[R.b], W[R.c], i, j, k, mus, fl[R.w], fl[R.e], fl[R.s],
-                fl[R.n], fl[R.b], fl[R.t], f);
+    auto fl = [&](int q) { return SIMPLE ? (int)FLUID : P.flag[q]; };
+    massflux_3d(P, d, U[R.w], U[R.c], V[R.s], V[R.c], W[R.b], W[R.c], i, j, k, mus, fl(R.w), fl(R.e), fl(R.s),
+                fl(R.n), fl(R.b), fl(R.t), f);
 }
 
 // betas, iter.f:1112-1248 (3D)
+template <bool SIMPLE>
 __device__ __forceinline__ void betas_3d(const Prm &P, const Fld &F, const Raw3 &R, const Rem3 &M, int i, int j, int k,
                                          double dt, double &cnv, double &abt) {
     const double *dx = P.dx, *dy = P.dy, *dz = P.dz;
@@ -573,14 +607,17 @@ __device__ __forceinline__ void betas_3d(const Prm &P, const Fld &F, const Raw3 
     double indxp = P.hx[i], indxm = P.hx[i - 1];
     double indzp = P.hz[k], indzm = P.hz[k - 1];
     double indyp = P.hy[j], indym = P.hy[j - 1];
-    auto open = [](int f) { return f == BL_CELL || f == FLUID || f == DOME || f == IMMB || f == FREE_IO || f == ZERO_GRAD; };
-    const int *fl = P.flag;
-    double iep_e = open(fl[R.e]) ? (dx[i + 1] * F.ep[c] + dx[i] * F.ep[M.e]) * indxp * indxp * 2.0 : 0.0;
-    double iep_w = open(fl[R.w]) ? (dx[i - 1] * F.ep[c] + dx[i] * F.ep[M.w]) * indxm * indxm * 2.0 : 0.0;
-    double iep_t = open(fl[R.t]) ? (dz[k + 1] * F.ep[c] + dz[k] * F.ep[M.t]) * indzp * indzp * 2.0 : 0.0;
-    double iep_b = open(fl[R.b]) ? (dz[k - 1] * F.ep[c] + dz[k] * F.ep[M.b]) * indzm * indzm * 2.0 : 0.0;
-    double iep_n = open(fl[R.n]) ? (dy[j + 1] * F.ep[c] + dy[j] * F.ep[M.n]) * indyp * indyp * 2.0 : 0.0;
-    double iep_s = open(fl[R.s]) ? (dy[j - 1] * F.ep[c] + dy[j] * F.ep[M.s]) * indym * indym * 2.0 : 0.0;
+    auto open = [&](int q) {
+        if (SIMPLE) return true;
+        const int f = P.flag[q];
+        return f == BL_CELL || f == FLUID || f == DOME || f == IMMB || f == FREE_IO || f == ZERO_GRAD;
+    };
+    double iep_e = open(R.e) ? (dx[i + 1] * F.ep[c] + dx[i] * F.ep[M.e]) * indxp * indxp * 2.0 : 0.0;
+    double iep_w = open(R.w) ? (dx[i - 1] * F.ep[c] + dx[i] * F.ep[M.w]) * indxm * indxm * 2.0 : 0.0;
+    double iep_t = open(R.t) ? (dz[k + 1] * F.ep[c] + dz[k] * F.ep[M.t]) * indzp * indzp * 2.0 : 0.0;
+    double iep_b = open(R.b) ? (dz[k - 1] * F.ep[c] + dz[k] * F.ep[M.b]) * indzm * indzm * 2.0 : 0.0;
+    double iep_n = open(R.n) ? (dy[j + 1] * F.ep[c] + dy[j] * F.ep[M.n]) * indyp * indyp * 2.0 : 0.0;
+    double iep_s = open(R.s) ? (dy[j - 1] * F.ep[c] + dy[j] * F.ep[M.s]) * indym * indym * 2.0 : 0.0;
     double iepx = (1.0 * iep_e + 1.0 * iep_w) * P.indx[i] * 1.0;
     double iepz = (iep_t + iep_b) * P.indz[k];
     double iepy = (iep_n + iep_s) * P.indy[j];
@@ -593,24 +630,23 @@ __device__ __forceinline__ void betas_3d(const Prm &P, const Fld &F, const Raw3 
 
 // initial gas mass fluxes + betas (iter.f:170-191): a face shared by two
 // fluid cells ends with the value of the later cell in the reference loop
-__global__ void k_mflux_init3d(Prm P, Fld F, double dt) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.ncell || !fluid(P, c)) return;
-    int i, j, k;
-    ijk_of(P, c, i, j, k);
+template <bool SIMPLE>
+__global__ void __launch_bounds__(128) k_mflux_init3d(Prm P, Fld F, double dt, const int *list, int nlist) {
+    int c, i, j, k;
     Raw3 R;
     Rem3 M;
-    raw3(P, i, j, k, R);
-    rem3(P, i, j, k, R, M);
+    if (!stencil_cell<SIMPLE>(P, blockIdx.x * blockDim.x + threadIdx.x, list, nlist, c, i, j, k, R, M)) return;
     F6d f;
-    cell_massflux3d(P, F.rgp, F.ug, F.vg, F.wg, R, M, i, j, k, f);
+    cell_massflux3d<SIMPLE>(P, F.rgp, F.ug, F.vg, F.wg, R, M, i, j, k, f);
     F.rgfe[R.w] = f.w;
     F.rgfn[R.s] = f.s;
     F.rgft[R.b] = f.b;
-    if (!fluid(P, R.e)) F.rgfe[c] = f.e;
-    if (!fluid(P, R.n)) F.rgfn[c] = f.n;
-    if (!fluid(P, R.t)) F.rgft[c] = f.t;
-    betas_3d(P, F, R, M, i, j, k, dt, F.conv[c], F.abeta[c]);
+    if (!SIMPLE) {
+        if (!fluid(P, R.e)) F.rgfe[c] = f.e;
+        if (!fluid(P, R.n)) F.rgfn[c] = f.n;
+        if (!fluid(P, R.t)) F.rgft[c] = f.t;
+    }
+    betas_3d<SIMPLE>(P, F, R, M, i, j, k, dt, F.conv[c], F.abeta[c]);
 }
 
 // calc_res, iter.f:743-771 (3D)
@@ -648,18 +684,14 @@ __device__ __forceinline__ void calc_eps_3d(const Prm &P, const Fld &F, const Ra
 // ---------------------------------------------------------------------------
 // ygas, ygas.f:27-325 (3D)
 // ---------------------------------------------------------------------------
-template <typename Real = double>
-__global__ void __launch_bounds__(128, PDAC_SCALAR_FLUX_MINB) k_ygas_flux3d(Prm P, Fld F) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.ncell || !fluid(P, c)) return;
-    int i, j, k;
-    ijk_of(P, c, i, j, k);
+template <typename Real, bool SIMPLE>
+__global__ void __launch_bounds__(128, sizeof(Real) == 8 ? 5 : PDAC_SCALAR_FLUX_MINB) k_ygas_flux3d(Prm P, Fld F, const int *list, int nlist) {
+    int c, i, j, k;
     Raw3 R;
     Rem3 M;
-    raw3(P, i, j, k, R);
-    rem3(P, i, j, k, R, M);
-    bool dw = !fluid(P, R.w), ds = !fluid(P, R.s), db = !fluid(P, R.b);
-    bool mus = P.muscl > 0 && P.flag[c] == FLUID;
+    if (!stencil_cell<SIMPLE>(P, blockIdx.x * blockDim.x + threadIdx.x, list, nlist, c, i, j, k, R, M)) return;
+    const bool dw = !SIMPLE && !fluid(P, R.w), ds = !SIMPLE && !fluid(P, R.s), db = !SIMPLE && !fluid(P, R.b);
+    const bool mus = SIMPLE || (P.muscl > 0 && P.flag[c] == FLUID);
     S3T<Real> d;
     first_nb3(d, F.rgp, R, M);
     if (mus) third_nb3(d, F.rgp, M);
@@ -717,21 +749,20 @@ __global__ void k_ygas3d(Prm P, Fld F, double dt) {
 // htilde, htilde.f:25-575 (3D)
 // ---------------------------------------------------------------------------
 // GRAV as in k_htilde_flux2d
-template <bool GRAV, typename Real = double>
-__global__ void __launch_bounds__(128, PDAC_SCALAR_FLUX_MINB) k_htilde_flux3d(Prm P, Fld F) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.ncell || !fluid(P, c)) return;
-    int i, j, k;
-    ijk_of(P, c, i, j, k);
+// one thread per (cell, phase), phase in blockIdx.y
+template <bool GRAV, typename Real, bool SIMPLE>
+__global__ void __launch_bounds__(128, sizeof(Real) == 8 ? 7 : PDAC_SCALAR_FLUX_MINB) k_htilde_flux3d(Prm P, Fld F, const int *list, int nlist) {
+    int c, i, j, k;
     Raw3 R;
     Rem3 M;
-    raw3(P, i, j, k, R);
-    rem3(P, i, j, k, R, M);
-    bool dw = !fluid(P, R.w), ds = !fluid(P, R.s), db = !fluid(P, R.b);
-    bool mus = P.muscl > 0 && P.flag[c] == FLUID;
-    bool hw = P.flag[R.w] != 1, hs = P.flag[R.s] != 1, hb = P.flag[R.b] != 1;  // hotc.f tests the flag value
+    if (!stencil_cell<SIMPLE>(P, blockIdx.x * blockDim.x + threadIdx.x, list, nlist, c, i, j, k, R, M)) return;
+    const bool dw = !SIMPLE && !fluid(P, R.w), ds = !SIMPLE && !fluid(P, R.s), db = !SIMPLE && !fluid(P, R.b);
+    const bool mus = SIMPLE || (P.muscl > 0 && P.flag[c] == FLUID);
+    // hotc.f tests the flag value
+    const bool hw = !SIMPLE && P.flag[R.w] != 1, hs = !SIMPLE && P.flag[R.s] != 1, hb = !SIMPLE && P.flag[R.b] != 1;
     size_t n = P.ncell;
-    for (int ph = 0; ph <= P.ns; ++ph) {
+    {
+        const int ph = blockIdx.y;
         size_t off = (size_t)(ph > 0 ? ph - 1 : 0) * n;
         const double *EN = ph == 0 ? F.sieg : F.sies + off;
         const double *DE = ph == 0 ? F.rgp : F.rlk + off;

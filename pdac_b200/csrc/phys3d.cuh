@@ -87,6 +87,74 @@ __device__ __forceinline__ void rem3(const Prm &P, int i, int j, int k, const Ra
     rem3_fl(P, P.flag, i, j, k, R, M);
 }
 
+// The neighbours of a simple cell: its stencils stay inside the mesh and meet
+// no wall, so raw and remapped neighbours are the plain offsets.
+__device__ __forceinline__ void raw3_simple(const Prm &P, int c, Raw3 &R) {
+    const int y = P.nx, z = P.nx * P.ny;
+    R.c = c;
+    R.e = c + 1; R.w = c - 1; R.n = c + y; R.s = c - y; R.t = c + z; R.b = c - z;
+    R.ee = c + 2; R.ww = c - 2; R.nn = c + 2 * y; R.ss = c - 2 * y; R.tt = c + 2 * z; R.bb = c - 2 * z;
+    R.en = R.n + 1; R.wn = R.n - 1; R.es = R.s + 1; R.ws = R.s - 1;
+    R.et = R.t + 1; R.wt = R.t - 1; R.nt = R.t + y; R.st = R.t - y;
+    R.eb = R.b + 1; R.wb = R.b - 1; R.nb = R.b + y; R.sb = R.b - y;
+    R.eet = R.t + 2; R.een = R.n + 2; R.enn = R.nn + 1; R.nnt = R.t + 2 * y; R.ett = R.tt + 1; R.ntt = R.tt + y;
+    R.eee = c + 3; R.nnn = R.nn + y; R.ttt = R.tt + z;
+}
+__device__ __forceinline__ void rem3_simple(const Raw3 &R, Rem3 &M) {
+    M.e = R.e; M.w = R.w; M.n = R.n; M.s = R.s; M.t = R.t; M.b = R.b;
+    M.ee = R.ee; M.ww = R.ww; M.nn = R.nn; M.ss = R.ss; M.tt = R.tt; M.bb = R.bb;
+    M.eb = R.eb; M.wb = R.wb; M.nb = R.nb; M.sb = R.sb;
+    M.eet = R.eet; M.een = R.een; M.enn = R.enn; M.nnt = R.nnt; M.ett = R.ett; M.ntt = R.ntt;
+    M.eee = R.eee; M.nnn = R.nnn; M.ttt = R.ttt;
+}
+__device__ __forceinline__ bool is_simple(const Prm &P, int c) { return (__ldg(P.simple + (c >> 5)) >> (c & 31)) & 1u; }
+
+// The mask of simple cells, for every stencil of the flux and stress passes:
+// a fluid cell (flag 1, so MUSCL is on and no immersed-boundary mask applies)
+// three cells or more from the mesh's ends, its six face neighbours flag 1
+// too (every limiter on, no face this cell owns towards a non-fluid one), and
+// no wall at any offset the passes read.
+__global__ void k_simple_mask(Prm P, unsigned *mask) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ((unsigned)P.ncell + 31u) / 32u) return;
+    unsigned m = 0;
+    const int *fl = P.flag;
+    for (int b = 0; b < 32; ++b) {
+        const int c = (int)(32u * t) + b;
+        if (c >= P.ncell) break;
+        if (fl[c] != FLUID) continue;
+        const int i = c % P.nx + 1, r = c / P.nx, j = r % P.ny + 1, k = r / P.ny + 1;
+        if (i < 3 || i > P.nx - 3 || j < 3 || j > P.ny - 3 || k < 3 || k > P.nz - 3) continue;
+        Raw3 R;
+        raw3_simple(P, c, R);
+        const int face[6] = {R.e, R.w, R.n, R.s, R.t, R.b};
+        const int rest[27] = {R.ee, R.ww, R.nn, R.ss, R.tt, R.bb, R.en, R.wn, R.es, R.ws, R.et, R.wt, R.nt, R.st,
+                              R.eb, R.wb, R.nb, R.sb, R.eet, R.een, R.enn, R.nnt, R.ett, R.ntt, R.eee, R.nnn, R.ttt};
+        bool ok = true;
+        for (int q : face) ok = ok && fl[q] == FLUID;
+        for (int q : rest) ok = ok && !is_wallf(fl[q]);
+        if (ok) m |= 1u << b;
+    }
+    mask[t] = m;
+}
+// the fluid cells that are not simple: counted, then listed (roughly in cell
+// order, one block's at a time)
+__global__ void k_rest_list(Prm P, int *count, int *list) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    __shared__ int n[32], base;
+    const bool in = c < P.ncell && (P.flag[c] & 1) && !is_simple(P, c);
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (lane == 0) n[wid] = __popc(m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int tot = 0;
+        for (int w = 0; w < (int)blockDim.x / 32; ++w) { const int v = n[w]; n[w] = tot; tot += v; }
+        base = tot ? atomicAdd(count, tot) : 0;
+    }
+    __syncthreads();
+    if (in && list) list[base + n[wid] + __popc(m & ((1u << lane) - 1u))] = c;
+}
+
 template <typename Real>
 struct S3T {
     Real c, e, w, n, s, t, b, ee, ww, nn, ss, tt, bb;
@@ -191,16 +259,36 @@ template <typename Real>
 struct F6T { Real e, n, t, w, s, b; };
 using F6d = F6T<double>;
 
+// The donor-cell flux 0.5 (cs - |cs|) dn un + 0.5 (cs + |cs|) dc uc of a face
+// whose plus side is n: of the two weights one is cs and the other 0 (exactly:
+// halving and doubling are), so only the upwind product is formed.
+template <typename Real>
+__device__ __forceinline__ Real donor(Real cs, Real dc, Real uc, Real dn, Real un) {
+    const bool p = cs >= 0;
+    return cs * (p ? dc : dn) * (p ? uc : un);
+}
+template <typename Real>
+__device__ __forceinline__ Real donor(Real cs, Real dc, Real dn) {
+    return cs * (cs >= 0 ? dc : dn);
+}
+// the same flux in the order of flw (flux_w.f): 0.5 dc uc (cs + |cs|) + ...
+template <typename Real>
+__device__ __forceinline__ Real donor_w(Real cs, Real dc, Real uc, Real dn, Real un) {
+    const bool p = cs >= 0;
+    return Real(0.5) * (p ? dc : dn) * (p ? uc : un) * (cs + cs);
+}
+
 // one limited face correction: shared by the momentum, mass and scalar MUSCL
-// routines, which differ only in the gradients and increments they pass
+// routines, which differ only in the gradients and increments they pass.  One
+// quotient for both signs of the velocity, so that a warp whose faces differ
+// in it does not divide twice.
 template <typename Real>
 __device__ __forceinline__ void muscl_face(int lt, double beta, Real &fx, Real cs, Real gradc, Real gradm,
                                            Real gradp, Real incr_p, Real incr_m, bool lim_on) {
-    Real erre = 0, incr = 0, lim = 0;
-    if (cs >= 0) { if (gradc != 0) erre = gradm / gradc; incr = incr_p; }
-    else if (cs < 0) { if (gradc != 0) erre = gradp / gradc; incr = incr_m; }
-    if (lim_on) lim = limiter(lt, erre, beta);
-    Real upwnd = lim * gradc * incr;
+    const bool p = cs >= 0, nz = gradc != 0;
+    const Real erre = (nz ? (p ? gradm : gradp) : Real(0)) / (nz ? gradc : Real(1));
+    const Real lim = lim_on ? limiter(lt, erre, beta) : Real(0);
+    const Real upwnd = lim * gradc * (p ? incr_p : incr_m);
     fx = fx + upwnd * cs;
 }
 
@@ -209,15 +297,15 @@ __device__ __forceinline__ void flu_3d(const Prm &P, F6T<Real> &f, bool dw, bool
                                        const S3T<Real> &v, const S3T<Real> &w, int i) {
     const Real *dx = Met<Real>::dx(P);
     Real indxp = Met<Real>::hx(P)[i], cs;
-    if (dw) { cs = Real(0.5) * (u.c + u.w); f.w = Real(0.5) * (cs - fabs(cs)) * d.c * u.c + Real(0.5) * (cs + fabs(cs)) * d.w * u.w; }
-    if (ds) { cs = (dx[i + 1] * v.s + dx[i] * v.es) * indxp; f.s = Real(0.5) * (cs - fabs(cs)) * d.c * u.c + Real(0.5) * (cs + fabs(cs)) * d.s * u.s; }
-    if (db) { cs = (dx[i + 1] * w.b + dx[i] * w.eb) * indxp; f.b = Real(0.5) * (cs - fabs(cs)) * d.c * u.c + Real(0.5) * (cs + fabs(cs)) * d.b * u.b; }
+    if (dw) { cs = Real(0.5) * (u.c + u.w); f.w = donor(cs, d.w, u.w, d.c, u.c); }
+    if (ds) { cs = (dx[i + 1] * v.s + dx[i] * v.es) * indxp; f.s = donor(cs, d.s, u.s, d.c, u.c); }
+    if (db) { cs = (dx[i + 1] * w.b + dx[i] * w.eb) * indxp; f.b = donor(cs, d.b, u.b, d.c, u.c); }
     cs = Real(0.5) * (u.c + u.e);
-    f.e = Real(0.5) * (cs - fabs(cs)) * d.e * u.e + Real(0.5) * (cs + fabs(cs)) * d.c * u.c;
+    f.e = donor(cs, d.c, u.c, d.e, u.e);
     cs = (dx[i + 1] * v.c + dx[i] * v.e) * indxp;
-    f.n = Real(0.5) * (cs - fabs(cs)) * d.n * u.n + Real(0.5) * (cs + fabs(cs)) * d.c * u.c;
+    f.n = donor(cs, d.c, u.c, d.n, u.n);
     cs = (dx[i + 1] * w.c + dx[i] * w.e) * indxp;
-    f.t = Real(0.5) * (cs - fabs(cs)) * d.t * u.t + Real(0.5) * (cs + fabs(cs)) * d.c * u.c;
+    f.t = donor(cs, d.c, u.c, d.t, u.t);
 }
 template <typename Real>
 __device__ __forceinline__ void muscl_flu_3d(const Prm &P, F6T<Real> &f, const S3T<Real> &d, const S3T<Real> &u, const S3T<Real> &v, const S3T<Real> &w,
@@ -245,15 +333,15 @@ __device__ __forceinline__ void flv_3d(const Prm &P, F6T<Real> &f, bool dw, bool
                                        const S3T<Real> &v, const S3T<Real> &w, int j) {
     const Real *dy = Met<Real>::dy(P);
     Real indyp = Met<Real>::hy(P)[j], cs;
-    if (dw) { cs = (u.wn * dy[j] + u.w * dy[j + 1]) * indyp; f.w = Real(0.5) * (cs - fabs(cs)) * d.c * v.c + Real(0.5) * (cs + fabs(cs)) * d.w * v.w; }
-    if (ds) { cs = Real(0.5) * (v.c + v.s); f.s = Real(0.5) * (cs - fabs(cs)) * d.c * v.c + Real(0.5) * (cs + fabs(cs)) * d.s * v.s; }
-    if (db) { cs = (w.nb * dy[j] + w.b * dy[j + 1]) * indyp; f.b = Real(0.5) * (cs - fabs(cs)) * d.c * v.c + Real(0.5) * (cs + fabs(cs)) * d.b * v.b; }
+    if (dw) { cs = (u.wn * dy[j] + u.w * dy[j + 1]) * indyp; f.w = donor(cs, d.w, v.w, d.c, v.c); }
+    if (ds) { cs = Real(0.5) * (v.c + v.s); f.s = donor(cs, d.s, v.s, d.c, v.c); }
+    if (db) { cs = (w.nb * dy[j] + w.b * dy[j + 1]) * indyp; f.b = donor(cs, d.b, v.b, d.c, v.c); }
     cs = indyp * (u.c * dy[j + 1] + u.n * dy[j]);
-    f.e = Real(0.5) * (cs - fabs(cs)) * d.e * v.e + Real(0.5) * (cs + fabs(cs)) * d.c * v.c;
+    f.e = donor(cs, d.c, v.c, d.e, v.e);
     cs = Real(0.5) * (v.n + v.c);
-    f.n = Real(0.5) * (cs - fabs(cs)) * d.n * v.n + Real(0.5) * (cs + fabs(cs)) * d.c * v.c;
+    f.n = donor(cs, d.c, v.c, d.n, v.n);
     cs = indyp * (w.c * dy[j + 1] + w.n * dy[j]);
-    f.t = Real(0.5) * (cs - fabs(cs)) * d.t * v.t + Real(0.5) * (cs + fabs(cs)) * d.c * v.c;
+    f.t = donor(cs, d.c, v.c, d.t, v.t);
 }
 template <typename Real>
 __device__ __forceinline__ void muscl_flv_3d(const Prm &P, F6T<Real> &f, const S3T<Real> &d, const S3T<Real> &u, const S3T<Real> &v, const S3T<Real> &w,
@@ -281,15 +369,15 @@ __device__ __forceinline__ void flw_3d(const Prm &P, F6T<Real> &f, bool dw, bool
                                        const S3T<Real> &v, const S3T<Real> &w, int k) {
     const Real *dz = Met<Real>::dz(P);
     Real indzp = Met<Real>::hz(P)[k], cs;
-    if (dw) { cs = (dz[k + 1] * u.w + dz[k] * u.wt) * indzp; f.w = Real(0.5) * d.w * w.w * (cs + fabs(cs)) + Real(0.5) * d.c * w.c * (cs - fabs(cs)); }
-    if (ds) { cs = (dz[k + 1] * v.s + dz[k] * v.st) * indzp; f.s = Real(0.5) * d.s * w.s * (cs + fabs(cs)) + Real(0.5) * d.c * w.c * (cs - fabs(cs)); }
-    if (db) { cs = Real(0.5) * (w.b + w.c); f.b = Real(0.5) * d.b * w.b * (cs + fabs(cs)) + Real(0.5) * d.c * w.c * (cs - fabs(cs)); }
+    if (dw) { cs = (dz[k + 1] * u.w + dz[k] * u.wt) * indzp; f.w = donor_w(cs, d.w, w.w, d.c, w.c); }
+    if (ds) { cs = (dz[k + 1] * v.s + dz[k] * v.st) * indzp; f.s = donor_w(cs, d.s, w.s, d.c, w.c); }
+    if (db) { cs = Real(0.5) * (w.b + w.c); f.b = donor_w(cs, d.b, w.b, d.c, w.c); }
     cs = (dz[k + 1] * u.c + dz[k] * u.t) * indzp;
-    f.e = Real(0.5) * d.c * w.c * (cs + fabs(cs)) + Real(0.5) * d.e * w.e * (cs - fabs(cs));
+    f.e = donor_w(cs, d.c, w.c, d.e, w.e);
     cs = (dz[k + 1] * v.c + dz[k] * v.t) * indzp;
-    f.n = Real(0.5) * d.c * w.c * (cs + fabs(cs)) + Real(0.5) * d.n * w.n * (cs - fabs(cs));
+    f.n = donor_w(cs, d.c, w.c, d.n, w.n);
     cs = Real(0.5) * (w.c + w.t);
-    f.t = Real(0.5) * d.c * w.c * (cs + fabs(cs)) + Real(0.5) * d.t * w.t * (cs - fabs(cs));
+    f.t = donor_w(cs, d.c, w.c, d.t, w.t);
 }
 template <typename Real>
 __device__ __forceinline__ void muscl_flw_3d(const Prm &P, F6T<Real> &f, const S3T<Real> &d, const S3T<Real> &u, const S3T<Real> &v, const S3T<Real> &w,
@@ -319,12 +407,12 @@ __device__ __forceinline__ void massflux_3d(const Prm &P, const S3T<Real> &d, Re
                                             Real wb, Real wc, int i, int j, int k, bool muscl_on, int flw, int fle,
                                             int fls, int fln, int flb, int flt, F6T<Real> &f) {
     Real cs;
-    cs = uw; f.w = Real(0.5) * (cs - fabs(cs)) * d.c + Real(0.5) * (cs + fabs(cs)) * d.w;
-    cs = vs; f.s = Real(0.5) * (cs - fabs(cs)) * d.c + Real(0.5) * (cs + fabs(cs)) * d.s;
-    cs = wb; f.b = Real(0.5) * (cs - fabs(cs)) * d.c + Real(0.5) * (cs + fabs(cs)) * d.b;
-    cs = uc; f.e = Real(0.5) * (cs - fabs(cs)) * d.e + Real(0.5) * (cs + fabs(cs)) * d.c;
-    cs = vc; f.n = Real(0.5) * (cs - fabs(cs)) * d.n + Real(0.5) * (cs + fabs(cs)) * d.c;
-    cs = wc; f.t = Real(0.5) * (cs - fabs(cs)) * d.t + Real(0.5) * (cs + fabs(cs)) * d.c;
+    cs = uw; f.w = donor(cs, d.w, d.c);
+    cs = vs; f.s = donor(cs, d.s, d.c);
+    cs = wb; f.b = donor(cs, d.b, d.c);
+    cs = uc; f.e = donor(cs, d.c, d.e);
+    cs = vc; f.n = donor(cs, d.c, d.n);
+    cs = wc; f.t = donor(cs, d.c, d.t);
     if (!muscl_on) return;
     const Real *dx = Met<Real>::dx(P), *dy = Met<Real>::dy(P), *dz = Met<Real>::dz(P);
     int im2 = max(1, i - 2), ip2 = min(P.nx, i + 2), jm2 = max(1, j - 2), jp2 = min(P.ny, j + 2);
@@ -352,12 +440,12 @@ template <typename Real>
 __device__ __forceinline__ void fsc_3d(const Prm &P, F6T<Real> &f, bool dw, bool ds, bool db, const S3T<Real> &d, const S3T<Real> &fl,
                                        Real uw, Real uc, Real vs, Real vc, Real wb, Real wc) {
     Real cs;
-    if (dw) { cs = uw; f.w = Real(0.5) * (cs - fabs(cs)) * d.c * fl.c + Real(0.5) * (cs + fabs(cs)) * d.w * fl.w; }
-    if (ds) { cs = vs; f.s = Real(0.5) * (cs - fabs(cs)) * d.c * fl.c + Real(0.5) * (cs + fabs(cs)) * d.s * fl.s; }
-    if (db) { cs = wb; f.b = Real(0.5) * (cs - fabs(cs)) * d.c * fl.c + Real(0.5) * (cs + fabs(cs)) * d.b * fl.b; }
-    cs = uc; f.e = Real(0.5) * (cs - fabs(cs)) * d.e * fl.e + Real(0.5) * (cs + fabs(cs)) * d.c * fl.c;
-    cs = vc; f.n = Real(0.5) * (cs - fabs(cs)) * d.n * fl.n + Real(0.5) * (cs + fabs(cs)) * d.c * fl.c;
-    cs = wc; f.t = Real(0.5) * (cs - fabs(cs)) * d.t * fl.t + Real(0.5) * (cs + fabs(cs)) * d.c * fl.c;
+    if (dw) { cs = uw; f.w = donor(cs, d.w, fl.w, d.c, fl.c); }
+    if (ds) { cs = vs; f.s = donor(cs, d.s, fl.s, d.c, fl.c); }
+    if (db) { cs = wb; f.b = donor(cs, d.b, fl.b, d.c, fl.c); }
+    cs = uc; f.e = donor(cs, d.c, fl.c, d.e, fl.e);
+    cs = vc; f.n = donor(cs, d.c, fl.c, d.n, fl.n);
+    cs = wc; f.t = donor(cs, d.c, fl.c, d.t, fl.t);
 }
 template <typename Real>
 __device__ __forceinline__ void muscl_fsc_3d(const Prm &P, F6T<Real> &f, const S3T<Real> &d, const S3T<Real> &fl, Real uc, Real vc,

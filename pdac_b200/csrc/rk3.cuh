@@ -404,21 +404,20 @@ __global__ void k_visc2d(Prm P, Fld F) {
 // cell of the reference loop, so this thread writes its W/S/B faces always
 // and its E/N/T faces only towards non-fluid cells.
 // Real as in k_tilde_flux3d (float only in 3D).
-template <int D, typename Real = double>
-__global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_rk3_mflux(Prm P, Fld F) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= P.ncell || !fluid(P, c)) return;
+// In 3D one thread per (cell, phase), phase in blockIdx.y; SIMPLE, list and
+// nlist as in k_tilde_flux3d.
+template <int D, typename Real, bool SIMPLE>
+__global__ void __launch_bounds__(128, SIMPLE ? 7 : PDAC_FLUX_MINB) k_rk3_mflux(Prm P, Fld F, const int *list, int nlist) {
     const size_t n = P.ncell;
-    const bool mus = P.muscl > 0 && P.flag[c] == FLUID;
-    const int *fl = P.flag;
     if (D == 3) {
-        int i, j, k;
-        ijk_of(P, c, i, j, k);
+        int c, i, j, k;
         Raw3 R;
         Rem3 M;
-        raw3(P, i, j, k, R);
-        rem3(P, i, j, k, R, M);
-        for (int ph = 0; ph <= P.ns; ++ph) {
+        if (!stencil_cell<SIMPLE>(P, blockIdx.x * blockDim.x + threadIdx.x, list, nlist, c, i, j, k, R, M)) return;
+        const bool mus = SIMPLE || (P.muscl > 0 && P.flag[c] == FLUID);
+        auto fl = [&](int q) { return SIMPLE ? (int)FLUID : P.flag[q]; };
+        {
+            const int ph = blockIdx.y;
             size_t off = (size_t)(ph > 0 ? ph - 1 : 0) * n;
             const double *Dn = ph == 0 ? F.rgp : F.rlk + off;
             const double *U = ph == 0 ? F.ug : F.us + off;
@@ -434,16 +433,22 @@ __global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_rk3_mflux(Prm P, Fld F)
                 d.ww = 0.0; d.ss = 0.0; d.bb = 0.0;
             }
             F6T<Real> f;
-            massflux_3d(P, d, Real(U[R.w]), Real(U[c]), Real(V[R.s]), Real(V[c]), Real(W[R.b]), Real(W[c]), i, j, k, mus, fl[R.w], fl[R.e], fl[R.s], fl[R.n],
-                        fl[R.b], fl[R.t], f);
+            massflux_3d(P, d, Real(U[R.w]), Real(U[c]), Real(V[R.s]), Real(V[c]), Real(W[R.b]), Real(W[c]), i, j, k, mus, fl(R.w), fl(R.e), fl(R.s), fl(R.n),
+                        fl(R.b), fl(R.t), f);
             fe[R.w] = f.w;
             fn[R.s] = f.s;
             ft[R.b] = f.b;
-            if (!fluid(P, R.e)) fe[c] = f.e;
-            if (!fluid(P, R.n)) fn[c] = f.n;
-            if (!fluid(P, R.t)) ft[c] = f.t;
+            if (!SIMPLE) {
+                if (!fluid(P, R.e)) fe[c] = f.e;
+                if (!fluid(P, R.n)) fn[c] = f.n;
+                if (!fluid(P, R.t)) ft[c] = f.t;
+            }
         }
     } else {
+        const int c = blockIdx.x * blockDim.x + threadIdx.x;
+        if (c >= P.ncell || !fluid(P, c)) return;
+        const bool mus = P.muscl > 0 && P.flag[c] == FLUID;
+        const int *fl = P.flag;
         int i = c % P.nx + 1, k = c / P.nx + 1;
         Raw2 R;
         Rem2 M;
