@@ -55,6 +55,11 @@ struct Prm {
     // fixed value that replaces the polynomial (0: none)
     double hcp[PDAC_MAXG][4], hfix[PDAC_MAXG];
     pdac_fp::Recip hmw[PDAC_MAXG];
+    // and of the gas viscosity (visc.f:37-148): 1000 x molar weight, squared
+    // collision diameter, the energy parameter as a divisor, and per pair the
+    // factors of the mixture rule that hold no temperature
+    double vm[PDAC_MAXG], vs2[PDAC_MAXG], vpw[PDAC_MAXG][PDAC_MAXG], vs8[PDAC_MAXG][PDAC_MAXG];
+    pdac_fp::Recip vek[PDAC_MAXG];
     double rgas, gammaair;
     double dk[PDAC_MAXP], rl[PDAC_MAXP], inrl[PDAC_MAXP], phis[PDAC_MAXP], cmus[PDAC_MAXP];
     double cps[PDAC_MAXP], kap[PDAC_MAXP], plim[PDAC_MAXP], phi[PDAC_MAXP];

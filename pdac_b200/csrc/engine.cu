@@ -328,6 +328,14 @@ void set_gas_tables(pdac_ctx *ctx) {
         for (int q = 0; q < 4; ++q) P.hcp[ig][q] = cp[g - 1][q];
         P.hmw[ig] = pdac_fp::recip(P.gmw[g]);
         P.hfix[ig] = P.icpc == 0 && g == 5 ? 1810.0 : (P.icpc == 0 && g == 6 ? 1004.0 : 0.0);
+        P.vm[ig] = 1.0e3 * P.gmw[g];
+        P.vs2[ig] = P.mmugs[g] * P.mmugs[g];
+        P.vek[ig] = pdac_fp::recip(P.mmugek[g]);
+        for (int jg = 0; jg < ctx->ng; ++jg) {
+            const double aa = P.gmw[g] / P.gmw[P.gas_type[jg]];
+            P.vpw[ig][jg] = pdac_fp::pow(aa, -0.25);
+            P.vs8[ig][jg] = std::sqrt(8.0 * (1.0 + aa));
+        }
     }
 }
 
@@ -1995,8 +2003,8 @@ __global__ void k_eos_sticky(int *counters) {
 
 static int enqueue_ftem(pdac_ctx *ctx, double dt, cudaStream_t st, bool in_sweep) {
     CK(cudaMemsetAsync(ctx->d_counters + 1, 0, sizeof(int), st));
-    if (ctx->d3) pdac::k_ftem3d<<<blocks(ctx->ncell), TPB, 0, st>>>(ctx->P, ctx->F, dt);
-    else pdac::k_ftem2d<<<blocks(ctx->ncell), TPB, 0, st>>>(ctx->P, ctx->F, dt);
+    if (ctx->d3) PHASE_LAUNCH(ctx->nph, pdac::k_ftem3d, blocks(ctx->ncell), TPB, st, ctx->P, ctx->F, dt);
+    else PHASE_LAUNCH(ctx->nph, pdac::k_ftem2d, blocks(ctx->ncell), TPB, st, ctx->P, ctx->F, dt);
     ctx->launches++;
     if (in_sweep) pdac::k_eos_sticky<<<1, 1, 0, st>>>(ctx->d_counters);
     CK(cudaGetLastError());

@@ -26,6 +26,7 @@
 // the C library over the ranges the path uses).
 #pragma once
 #include <cmath>
+#include <cstring>
 #include <limits>
 
 #include "fpmath_tables.h"
@@ -80,9 +81,11 @@ PDAC_FP_FN bool rel_change_within(double a, double b, double tol) {
 #ifdef __CUDACC__
 __constant__ const double kExp2Tab[64] = PDAC_EXP2_TABLE;
 __constant__ const double kLogTab[258] = PDAC_LOG_TABLE;
+__constant__ const double kInvFTab[129] = PDAC_LOG_INVF_TABLE;
 #endif
 static const double hExp2Tab[64] = PDAC_EXP2_TABLE;
 static const double hLogTab[258] = PDAC_LOG_TABLE;
+static const double hInvFTab[129] = PDAC_LOG_INVF_TABLE;
 
 PDAC_FP_FN double exp2_tab(int q) {
 #ifdef __CUDA_ARCH__
@@ -96,6 +99,13 @@ PDAC_FP_FN double log_tab(int q) {
     return kLogTab[q];
 #else
     return hLogTab[q];
+#endif
+}
+PDAC_FP_FN double invf_tab(int q) {
+#ifdef __CUDA_ARCH__
+    return kInvFTab[q];
+#else
+    return hInvFTab[q];
 #endif
 }
 
@@ -128,6 +138,44 @@ PDAC_FP_FN double frexp_(double x, int *e) {
 #endif
 }
 
+// v 2^m, as ldexp: where the result is normal the product with the power of
+// two, whose bits are m + 1023 in the exponent field, is exact (v in [1/2, 4))
+PDAC_FP_FN double scale2(double v, int m) {
+    if (m < -1020 || m > 1020) return ldexp_(v, m);
+    const unsigned long long b = (unsigned long long)(m + 1023) << 52;
+    double p;
+#ifdef __CUDA_ARCH__
+    p = __longlong_as_double((long long)b);
+#else
+    std::memcpy(&p, &b, 8);
+#endif
+    return v * p;
+}
+// x = 2^e y with y in [1, 2), for finite x > 0
+PDAC_FP_FN double split2(double x, int &e) {
+    unsigned long long b;
+#ifdef __CUDA_ARCH__
+    b = (unsigned long long)__double_as_longlong(x);
+#else
+    std::memcpy(&b, &x, 8);
+#endif
+    const int f = (int)(b >> 52);
+    if (f == 0) {  // subnormal
+        const double y = frexp_(x, &e);
+        e = e - 1;
+        return y * 2.0;
+    }
+    e = f - 1023;
+    b = (b & 0x000fffffffffffffull) | 0x3ff0000000000000ull;
+    double y;
+#ifdef __CUDA_ARCH__
+    y = __longlong_as_double((long long)b);
+#else
+    std::memcpy(&y, &b, 8);
+#endif
+    return y;
+}
+
 // exp(zh + zl) for |zl| no larger than an ulp or so of zh
 PDAC_FP_FN double exp_dd(double zh, double zl) {
     if (zh != zh) return zh;
@@ -145,7 +193,7 @@ PDAC_FP_FN double exp_dd(double zh, double zl) {
     const double p = r + q;
     const double th = exp2_tab(2 * j), tl = exp2_tab(2 * j + 1);
     const double s = th + tl;
-    return ldexp_(th + (tl + s * p), m);
+    return scale2(th + (tl + s * p), m);
 }
 
 PDAC_FP_FN double exp(double x) { return exp_dd(x, 0.0); }
@@ -153,15 +201,21 @@ PDAC_FP_FN double exp(double x) { return exp_dd(x, 0.0); }
 // log x as hi + lo, for finite x > 0
 PDAC_FP_FN void log_dd(double x, double &hi, double &lo) {
     int e;
-    double y = frexp_(x, &e);  // y in [0.5, 1)
-    y = y * 2.0;
-    e = e - 1;  // x = 2^e y, y in [1, 2)
+    const double y = split2(x, e);
     int j = (int)rint_((y - 1.0) * 128.0);
     j = j < 0 ? 0 : (j > 128 ? 128 : j);  // y in [1, 2) gives 0 .. 128; the table has 129 entries
     const double F = 1.0 + (double)j * 0x1.0p-7;
     const double f = y - F;                    // exact: |f| <= 1/256
-    const double g = f / F;                    // f/F = g + gl
-    const double gl = fma_(-g, F, f) / F;
+    // f/F = g + gl: both quotients by the tabulated 1/F as in div_by (f is 0 or
+    // a multiple of 2^-52, so no operand comes near the ends of the range)
+    const double iF = invf_tab(j);
+    double g = f * iF;
+    g = fma_(fma_(-F, g, f), iF, g);
+    g = fma_(fma_(-F, g, f), iF, g);
+    const double d = fma_(-g, F, f);
+    double gl = d * iF;
+    gl = fma_(fma_(-F, gl, d), iF, gl);
+    gl = fma_(fma_(-F, gl, d), iF, gl);
     // log1p(g) - g to degree 6 in g; |g| <= 1/256, the first term left out is
     // below 3e-18
     const double poly = g * g * (-0x1.0p-1 + g * (0x1.5555555555555p-2 + g * (-0x1.0p-2 + g * (0x1.999999999999ap-3 +
@@ -203,5 +257,34 @@ PDAC_FP_FN double pow(double x, double y) {
     }
     return negate ? -r : r;
 }
+
+// pow of one base to several exponents: its logarithm once.  y finite, not 0
+// and not an integer.
+struct PowOf {
+    double x, lh, ll;
+    bool plain;
+};
+PDAC_FP_FN PowOf pow_of(double x) {
+    PowOf b = {x, 0.0, 0.0, x > 0.0 && x < std::numeric_limits<double>::infinity() && x != 1.0};
+    if (b.plain) log_dd(x, b.lh, b.ll);
+    return b;
+}
+PDAC_FP_FN double pow_log(double lh, double ll, double y) {
+    const double zh = y * lh;
+    return exp_dd(zh, fma_(y, lh, -zh) + y * ll);
+}
+PDAC_FP_FN double pow(const PowOf &b, double y) {
+    if (b.plain) return pow_log(b.lh, b.ll, y);
+    if (b.x == 1.0) return 1.0;
+    if (b.x != b.x) return b.x + y;
+    if (b.x < 0.0) return std::numeric_limits<double>::quiet_NaN();
+    if (b.x == 0.0) return y > 0.0 ? 0.0 : std::numeric_limits<double>::infinity();
+    return y > 0.0 ? b.x : 0.0;
+}
+
+// pow(10, y): log 10 as log_dd(10) gives it
+#define PDAC_LOGDD_10_HI 0x1.26bb1bbb55516p+1
+#define PDAC_LOGDD_10_LO -0x1.f48ad494ea4p-53
+PDAC_FP_FN double pow10(double y) { return pow_log(PDAC_LOGDD_10_HI, PDAC_LOGDD_10_LO, y); }
 
 }  // namespace pdac_fp

@@ -46,6 +46,10 @@ def main():
     out.append("#define PDAC_LOG_TABLE { \\")
     out += [f"    {lit(h)}, {lit(l)}, \\" for h, l in rows]
     out += ["}", ""]
+    out.append("// 1 / (1 + j/128), j = 0 .. 128, rounded to nearest")
+    out.append("#define PDAC_LOG_INVF_TABLE { \\")
+    out += [f"    {lit(128.0 / (128.0 + j))}, \\" for j in range(129)]
+    out += ["}", ""]
     print("\n".join(out))
 
 

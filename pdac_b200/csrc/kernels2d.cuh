@@ -272,10 +272,8 @@ __global__ void k_fieldn2d(Prm P, Fld F) {
         SOL(F.rlkn, c, is) = SOL(F.rlk, c, is);
         SOL(F.siesn, c, is) = SOL(F.sies, c, is);
     }
-    double xg[PDAC_MAXG];
-    for (int ig = 0; ig < P.ng; ++ig) xg[ig] = GAS(F.xgc, c, ig);
     double mu, ka;
-    viscon(P, mu, ka, xg, F.tg[c]);
+    viscon(P, F, c, mu, ka);
     F.mug[c] = mu;
     F.kapg[c] = ka;
 }
@@ -465,6 +463,7 @@ __global__ void k_tilde2d(Prm P, Fld F, double dt, const double *app0u, const do
     double rwg = F.rwgn[c] + dt * t_;
     double rus[PDAC_MAXP], rws[PDAC_MAXP], kpgv[PDAC_MAXP];
     const double a_rep = -8.76, b_rep = -0.27;
+    const double ep265 = P.drag_model == 1 ? kdrags_ep(F.ep[c]) : 0.0;
     for (int is = 1; is <= ns; ++is) {
         double pvx = 0, pvz = 0;
         if (P.part_viscosity) {
@@ -477,10 +476,10 @@ __global__ void k_tilde2d(Prm P, Fld F, double dt, const double *app0u, const do
             if (P.repulsive_model == 1) {
                 double rc = rl[c], re = rl[ijke], rt = rl[ijkt];
                 double epsx = (dx[i + 1] * rc + dx[i] * re) * indxp * ir;
-                double gepx = pdac_fp::pow(10.0, -a_rep * epsx + b_rep);
+                double gepx = pdac_fp::pow10(-a_rep * epsx + b_rep);
                 pvx = pvx - gepx * indxp * 2.0 * (re - rc) * ir;
                 double epsz = (dz[k + 1] * rc + dz[k] * rt) * indzp * ir;
-                double gepz = pdac_fp::pow(10.0, -a_rep * epsz + b_rep);
+                double gepz = pdac_fp::pow10(-a_rep * epsz + b_rep);
                 pvz = pvz - gepz * indzp * 2.0 * (rt - rc) * ir;
             }
         }
@@ -507,7 +506,7 @@ __global__ void k_tilde2d(Prm P, Fld F, double dt, const double *app0u, const do
         rws[is] = rws[is] + dt * SOL(F.sink, c, is) * SOL(F.ws, c, is);
         double dugs = ((F.ug[c] - SOL(F.us, c, is)) + (F.ug[imjk] - SOL(F.us, imjk, is))) * 0.5;
         double dwgs = ((F.wg[c] - SOL(F.ws, c, is)) + (F.wg[ijkm] - SOL(F.ws, ijkm, is))) * 0.5;
-        kpgv[is] = drag_coeff(P, dugs, 0.0, dwgs, F.ep[c], F.rgp[c], SOL(F.rlk, c, is), F.mug[c], is);
+        kpgv[is] = drag_coeff(P, dugs, 0.0, dwgs, F.ep[c], F.rgp[c], SOL(F.rlk, c, is), F.mug[c], is, ep265);
     }
     // inter, drag.f:173-246
     double au[PDAC_MAXP * (PDAC_MAXP + 1) / 2 + 1], aw[PDAC_MAXP * (PDAC_MAXP + 1) / 2 + 1];
@@ -884,7 +883,70 @@ __global__ void k_htilde2d(Prm P, Fld F, double dt) {
 // ---------------------------------------------------------------------------
 // ftem, ftem.f:19-248 (2D)
 // ---------------------------------------------------------------------------
-__global__ void k_ftem2d(Prm P, Fld F, double dt) {
+// The enthalpy system of one cell and the new temperatures (ftem.f:112-199,
+// invdm :201-248), shared by the 2D and 3D passes: the matrix couples the gas
+// with each class only, so its first row, first column and diagonal are all
+// of it, in registers for a known phase count.  bg: the gas right-hand side
+// without the exchange; slip(is, du, dv, dw) the velocity differences;
+// work(is) the work of gravity on a class.
+template <int NP, class SLIP, class WORK>
+__device__ __forceinline__ void ftem_cell(const Prm &P, const Fld &F, int c, double dt, double bg, SLIP slip, WORK work) {
+    constexpr int M = Sys<NP>::M;
+    const int nph = nphases<NP>(P), ns = nph - 1;
+    const double alpha = P.alpha;
+    double a11 = F.rgp[c], b1 = bg;
+    double row[M], col[M], diag[M], bt[M];  // at[1][is], at[is][1], at[is][is], bt[is], is = class + 1
+    const double cgc = F.cg[c], tgc = F.tg[c], mug = F.mug[c], kapg = F.kapg[c], rog = F.rog[c];
+    const double pranumexp = hvs_prandtl(mug, kapg, cgc);
+#pragma unroll
+    for (int is = 1; is <= ns; ++is) {
+        const int is1 = is + 1;
+        double du, dv, dw;
+        slip(is, du, dv, dw);
+        const double rlk = SOL(F.rlk, c, is), tsc = SOL(F.ts, c, is);
+        const double hv = hvs(P, rlk, rog, du, dv, dw, mug, kapg, is, pranumexp);
+        const double qg = alpha * dt * hv / cgc, qs = alpha * dt * hv / P.cps[is];
+        a11 = a11 + qg;
+        row[is1] = -qs;
+        col[is1] = -qg;
+        diag[is1] = rlk + qs;
+        b1 = b1 + (1.0 - alpha) * dt * hv * tsc - (1.0 - alpha) * dt * hv * tgc;
+        bt[is1] = SOL(F.rlkn, c, is) * SOL(F.siesn, c, is) + SOL(F.rhs, c, is) + work(is) +
+                  (1.0 - alpha) * dt * hv * tgc - (1.0 - alpha) * dt * hv * tsc;
+    }
+#pragma unroll
+    for (int is = nph; is >= 2; --is) {
+        if (fabs(diag[is]) < P.flim) {
+            row[is] = 0.0; col[is] = 0.0; bt[is] = 0.0;
+        } else {
+            double div = 1.0 / diag[is];
+            col[is] = col[is] * div;
+            bt[is] = bt[is] * div;
+            b1 = b1 - row[is] * bt[is];
+            a11 = a11 - row[is] * col[is];
+        }
+    }
+    b1 = b1 / a11;
+    F.sieg[c] = b1;
+    double yg[PDAC_MAXG];
+    load_ygc(P, F, c, yg);
+    double tg = tgc, cg;
+    int info = caloric_eosg(P, cg, tg, yg, b1);
+    F.tg[c] = tg;
+    F.cg[c] = cg;
+#pragma unroll
+    for (int is = 1; is <= ns; ++is) {
+        const double b = bt[is + 1] - col[is + 1] * b1;
+        SOL(F.sies, c, is) = b;
+        const double t = 0.0 + (b - 0.0) / P.cps[is];
+        SOL(F.ts, c, is) = t;
+        if (t < 0.0) info++;
+    }
+    if (info) atomicAdd(&F.counters[1], info);
+}
+
+template <int NP>
+__global__ void __launch_bounds__(128) k_ftem2d(Prm P, Fld F, double dt) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.ncell || !fluid(P, c)) return;
     int i = c % P.nx + 1, k = c / P.nx + 1;
@@ -893,8 +955,6 @@ __global__ void k_ftem2d(Prm P, Fld F, double dt) {
     raw2(P, i, k, R);
     rem2(P, i, k, R, M);
     const double *dx = P.dx, *dz = P.dz;
-    int ns = P.ns, nph = P.nph;
-    double alpha = P.alpha;
     int imjk = R.w, ijkm = R.b;
     double indxc = 1.0 / (dx[i] + (dx[i + 1] + dx[i - 1]) * 0.5);
     double indzc = 1.0 / (dz[k] + (dz[k + 1] + dz[k - 1]) * 0.5);
@@ -907,52 +967,14 @@ __global__ void k_ftem2d(Prm P, Fld F, double dt) {
     dpxyz = dpxyz + dt * indzc * wgc * (F.p[M.t] - F.p[M.b]);
     double deltap = F.ep[c] * (F.p[c] - F.pn[c] + dpxyz);
     double workg = F.rgp[c] * (F.ug[c] * P.gravx + F.wg[c] * P.gravz);
-    double at[PDAC_MAXP + 1][PDAC_MAXP + 1], bt[PDAC_MAXP + 1];
-    at[1][1] = F.rgp[c];
-    bt[1] = F.siegn[c] * F.rgpn[c] + F.rhg[c] + deltap + workg - 0.0;
-    double cgc = F.cg[c];
-    for (int is = 1; is <= ns; ++is) {
-        int is1 = is + 1;
-        double dugs = ((F.ug[c] - SOL(F.us, c, is)) + (F.ug[imjk] - SOL(F.us, imjk, is))) * 0.5;
-        double dwgs = ((F.wg[c] - SOL(F.ws, c, is)) + (F.wg[ijkm] - SOL(F.ws, ijkm, is))) * 0.5;
-        double hv = hvs(P, SOL(F.rlk, c, is), F.rog[c], dugs, 0.0, dwgs, F.mug[c], F.kapg[c], cgc, is);
-        double works = SOL(F.rlk, c, is) * (SOL(F.us, c, is) * P.gravx + SOL(F.ws, c, is) * P.gravz);
-        double ck = P.cps[is];
-        at[1][1] = at[1][1] + alpha * dt * hv / cgc;
-        at[1][is1] = -alpha * dt * hv / ck;
-        at[is1][1] = -alpha * dt * hv / cgc;
-        at[is1][is1] = SOL(F.rlk, c, is) + alpha * dt * hv / ck;
-        bt[1] = bt[1] + (1.0 - alpha) * dt * hv * SOL(F.ts, c, is) - (1.0 - alpha) * dt * hv * F.tg[c];
-        bt[is1] = SOL(F.rlkn, c, is) * SOL(F.siesn, c, is) + SOL(F.rhs, c, is) + works +
-                  (1.0 - alpha) * dt * hv * F.tg[c] - (1.0 - alpha) * dt * hv * SOL(F.ts, c, is);
-    }
-    for (int is = nph; is >= 2; --is) {
-        if (fabs(at[is][is]) < P.flim) {
-            at[1][is] = 0.0; at[is][1] = 0.0; bt[is] = 0.0;
-        } else {
-            double div = 1.0 / at[is][is];
-            at[is][1] = at[is][1] * div;
-            bt[is] = bt[is] * div;
-            bt[1] = bt[1] - at[1][is] * bt[is];
-            at[1][1] = at[1][1] - at[1][is] * at[is][1];
-        }
-    }
-    bt[1] = bt[1] / at[1][1];
-    for (int is = 2; is <= nph; ++is) bt[is] = bt[is] - at[is][1] * bt[1];
-    F.sieg[c] = bt[1];
-    for (int is = 1; is <= ns; ++is) SOL(F.sies, c, is) = bt[is + 1];
-    double yg[PDAC_MAXG];
-    load_ygc(P, F, c, yg);
-    double tg = F.tg[c], cg;
-    int info = caloric_eosg(P, cg, tg, yg, bt[1]);
-    F.tg[c] = tg;
-    F.cg[c] = cg;
-    for (int is = 1; is <= ns; ++is) {
-        double t = 0.0 + (bt[is + 1] - 0.0) / P.cps[is];
-        SOL(F.ts, c, is) = t;
-        if (t < 0.0) info++;
-    }
-    if (info) atomicAdd(&F.counters[1], info);
+    const double bg = F.siegn[c] * F.rgpn[c] + F.rhg[c] + deltap + workg - 0.0;
+    auto slip = [&](int is, double &du, double &dv, double &dw) {
+        du = ((F.ug[c] - SOL(F.us, c, is)) + (F.ug[imjk] - SOL(F.us, imjk, is))) * 0.5;
+        dv = 0.0;
+        dw = ((F.wg[c] - SOL(F.ws, c, is)) + (F.wg[ijkm] - SOL(F.ws, ijkm, is))) * 0.5;
+    };
+    auto work = [&](int is) { return SOL(F.rlk, c, is) * (SOL(F.us, c, is) * P.gravx + SOL(F.ws, c, is) * P.gravz); };
+    ftem_cell<NP>(P, F, c, dt, bg, slip, work);
 }
 
 // deterministic two-pass reduction of the mass totals (residuals.f:14-130)

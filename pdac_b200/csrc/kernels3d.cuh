@@ -235,10 +235,8 @@ __global__ void k_fieldn3d(Prm P, Fld F) {
         SOL(F.rlkn, c, is) = SOL(F.rlk, c, is);
         SOL(F.siesn, c, is) = SOL(F.sies, c, is);
     }
-    double xg[PDAC_MAXG];
-    for (int ig = 0; ig < P.ng; ++ig) xg[ig] = GAS(F.xgc, c, ig);
     double mu, ka;
-    viscon(P, mu, ka, xg, F.tg[c]);
+    viscon(P, F, c, mu, ka);
     F.mug[c] = mu;
     F.kapg[c] = ka;
 }
@@ -370,13 +368,13 @@ __global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_visc3d(Prm P, Fld F, co
         if (P.repulsive_model == 1) {
             double rc = rl[c], re = rl[ijke], rn = rl[ijkn], rt = rl[ijkt];
             double epsx = (dx[i + 1] * rc + dx[i] * re) * indxp * ir;
-            double gepx = pdac_fp::pow(10.0, -a_rep * epsx + b_rep);
+            double gepx = pdac_fp::pow10(-a_rep * epsx + b_rep);
             vx = vx - gepx * indxp * 2.0 * (re - rc) * ir;
             double epsz = (dz[k + 1] * rc + dz[k] * rt) * indzp * ir;
-            double gepz = pdac_fp::pow(10.0, -a_rep * epsz + b_rep);
+            double gepz = pdac_fp::pow10(-a_rep * epsz + b_rep);
             vz = vz - gepz * indzp * 2.0 * (rt - rc) * ir;
             double epsy = (dy[j + 1] * rc + dy[j] * rn) * indyp * ir;
-            double gepy = pdac_fp::pow(10.0, -a_rep * epsy + b_rep);
+            double gepy = pdac_fp::pow10(-a_rep * epsy + b_rep);
             vy = vy - gepy * indyp * 2.0 * (rn - rc) * ir;
         }
     }
@@ -405,6 +403,7 @@ __global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_tilde3d(Prm P, Fld F, d
     double indxp = P.hx[i], indyp = P.hy[j], indzp = P.hz[k];
     double rr[MP][3];
     double kpgv[MP];
+    const double ep265 = P.drag_model == 1 ? kdrags_ep(F.ep[c]) : 0.0;
 #pragma unroll
     for (int ph = 0; ph <= ns; ++ph) {
         size_t off = (size_t)(ph > 0 ? ph - 1 : 0) * n;
@@ -470,7 +469,7 @@ __global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_tilde3d(Prm P, Fld F, d
             double dugs = ((F.ug[c] - SOL(F.us, c, is)) + (F.ug[imjk] - SOL(F.us, imjk, is))) * 0.5;
             double dwgs = ((F.wg[c] - SOL(F.ws, c, is)) + (F.wg[ijkm] - SOL(F.ws, ijkm, is))) * 0.5;
             double dvgs = ((F.vg[c] - SOL(F.vs, c, is)) + (F.vg[ijmk] - SOL(F.vs, ijmk, is))) * 0.5;
-            kpgv[is] = drag_coeff(P, dugs, dvgs, dwgs, F.ep[c], F.rgp[c], SOL(F.rlk, c, is), F.mug[c], is);
+            kpgv[is] = drag_coeff(P, dugs, dvgs, dwgs, F.ep[c], F.rgp[c], SOL(F.rlk, c, is), F.mug[c], is, ep265);
         }
     }
     // inter, drag.f:173-246
@@ -551,14 +550,14 @@ __global__ void __launch_bounds__(128, PDAC_FLUX_MINB) k_tilde3d(Prm P, Fld F, d
         }
     }
     if (P.immb) {
-        double rs[MP];
+        double rs[MP], kp[MP];  // copies: the branch indexes them in memory
         const int nb3[3] = {M.e, M.n, M.t}, nm3[3] = {R.w, R.s, R.b};
         const double *d3[3] = {P.dx, P.dy, P.dz};
         const int q3[3] = {i, j, k};
         for (int ax = 0; ax < 3; ++ax) {
-            for (int is = 1; is <= ns; ++is) rs[is] = rr[is][ax];
+            for (int is = 1; is <= ns; ++is) { rs[is] = rr[is][ax]; kp[is] = kpgv[is]; }
             const double dm = d3[ax][q3[ax]], dp = d3[ax][q3[ax] + 1];
-            ib_force(P, F, c, ax, nb3[ax], nm3[ax], dm, dp, 1.0 / (dm + dp), dt, kpgv, rr[0][ax], rs);
+            ib_force(P, F, c, ax, nb3[ax], nm3[ax], dm, dp, 1.0 / (dm + dp), dt, kp, rr[0][ax], rs);
             for (int is = 1; is <= ns; ++is) rr[is][ax] = rs[is];
         }
     }
@@ -847,7 +846,8 @@ __global__ void k_htilde3d(Prm P, Fld F, double dt) {
 // ---------------------------------------------------------------------------
 // ftem, ftem.f:19-248 (3D)
 // ---------------------------------------------------------------------------
-__global__ void k_ftem3d(Prm P, Fld F, double dt) {
+template <int NP>
+__global__ void __launch_bounds__(128) k_ftem3d(Prm P, Fld F, double dt) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= P.ncell || !fluid(P, c)) return;
     int i, j, k;
@@ -857,8 +857,6 @@ __global__ void k_ftem3d(Prm P, Fld F, double dt) {
     raw3(P, i, j, k, R);
     rem3(P, i, j, k, R, M);
     const double *dx = P.dx, *dy = P.dy, *dz = P.dz;
-    int ns = P.ns, nph = P.nph;
-    double alpha = P.alpha;
     int imjk = R.w, ijmk = R.s, ijkm = R.b;
     double indxc = 1.0 / (dx[i] + (dx[i + 1] + dx[i - 1]) * 0.5);
     double indzc = 1.0 / (dz[k] + (dz[k + 1] + dz[k - 1]) * 0.5);
@@ -874,54 +872,17 @@ __global__ void k_ftem3d(Prm P, Fld F, double dt) {
     double deltap = F.ep[c] * (F.p[c] - F.pn[c] + dpxyz);
     double workg = F.rgp[c] * (F.ug[c] * P.gravx + F.wg[c] * P.gravz);
     workg = workg + F.vg[c] * P.gravy;  // ftem.f:120 adds the y term without the density factor
-    double at[PDAC_MAXP + 1][PDAC_MAXP + 1], bt[PDAC_MAXP + 1];
-    at[1][1] = F.rgp[c];
-    bt[1] = F.siegn[c] * F.rgpn[c] + F.rhg[c] + deltap + workg - 0.0;
-    double cgc = F.cg[c];
-    for (int is = 1; is <= ns; ++is) {
-        int is1 = is + 1;
-        double dugs = ((F.ug[c] - SOL(F.us, c, is)) + (F.ug[imjk] - SOL(F.us, imjk, is))) * 0.5;
-        double dwgs = ((F.wg[c] - SOL(F.ws, c, is)) + (F.wg[ijkm] - SOL(F.ws, ijkm, is))) * 0.5;
-        double dvgs = ((F.vg[c] - SOL(F.vs, c, is)) + (F.vg[ijmk] - SOL(F.vs, ijmk, is))) * 0.5;
-        double hv = hvs(P, SOL(F.rlk, c, is), F.rog[c], dugs, dvgs, dwgs, F.mug[c], F.kapg[c], cgc, is);
+    const double bg = F.siegn[c] * F.rgpn[c] + F.rhg[c] + deltap + workg - 0.0;
+    auto slip = [&](int is, double &du, double &dv, double &dw) {
+        du = ((F.ug[c] - SOL(F.us, c, is)) + (F.ug[imjk] - SOL(F.us, imjk, is))) * 0.5;
+        dv = ((F.vg[c] - SOL(F.vs, c, is)) + (F.vg[ijmk] - SOL(F.vs, ijmk, is))) * 0.5;
+        dw = ((F.wg[c] - SOL(F.ws, c, is)) + (F.wg[ijkm] - SOL(F.ws, ijkm, is))) * 0.5;
+    };
+    auto work = [&](int is) {
         double works = SOL(F.rlk, c, is) * (SOL(F.us, c, is) * P.gravx + SOL(F.ws, c, is) * P.gravz);
-        works = works + SOL(F.vs, c, is) * P.gravy;
-        double ck = P.cps[is];
-        at[1][1] = at[1][1] + alpha * dt * hv / cgc;
-        at[1][is1] = -alpha * dt * hv / ck;
-        at[is1][1] = -alpha * dt * hv / cgc;
-        at[is1][is1] = SOL(F.rlk, c, is) + alpha * dt * hv / ck;
-        bt[1] = bt[1] + (1.0 - alpha) * dt * hv * SOL(F.ts, c, is) - (1.0 - alpha) * dt * hv * F.tg[c];
-        bt[is1] = SOL(F.rlkn, c, is) * SOL(F.siesn, c, is) + SOL(F.rhs, c, is) + works +
-                  (1.0 - alpha) * dt * hv * F.tg[c] - (1.0 - alpha) * dt * hv * SOL(F.ts, c, is);
-    }
-    for (int is = nph; is >= 2; --is) {
-        if (fabs(at[is][is]) < P.flim) {
-            at[1][is] = 0.0; at[is][1] = 0.0; bt[is] = 0.0;
-        } else {
-            double div = 1.0 / at[is][is];
-            at[is][1] = at[is][1] * div;
-            bt[is] = bt[is] * div;
-            bt[1] = bt[1] - at[1][is] * bt[is];
-            at[1][1] = at[1][1] - at[1][is] * at[is][1];
-        }
-    }
-    bt[1] = bt[1] / at[1][1];
-    for (int is = 2; is <= nph; ++is) bt[is] = bt[is] - at[is][1] * bt[1];
-    F.sieg[c] = bt[1];
-    for (int is = 1; is <= ns; ++is) SOL(F.sies, c, is) = bt[is + 1];
-    double yg[PDAC_MAXG];
-    load_ygc(P, F, c, yg);
-    double tg = F.tg[c], cg;
-    int info = caloric_eosg(P, cg, tg, yg, bt[1]);
-    F.tg[c] = tg;
-    F.cg[c] = cg;
-    for (int is = 1; is <= ns; ++is) {
-        double t = 0.0 + (bt[is + 1] - 0.0) / P.cps[is];
-        SOL(F.ts, c, is) = t;
-        if (t < 0.0) info++;
-    }
-    if (info) atomicAdd(&F.counters[1], info);
+        return works + SOL(F.vs, c, is) * P.gravy;
+    };
+    ftem_cell<NP>(P, F, c, dt, bg, slip, work);
 }
 
 }  // namespace pdac

@@ -405,47 +405,66 @@ __device__ __forceinline__ void hotc_2d(const Prm &P, Real &hfe, Real &hft, Real
 }
 
 // ---- closures ----------------------------------------------------------------
-// visc.f:37-148
-__device__ __forceinline__ void viscon(const Prm &P, double &mu, double &kap, const double *xg, double tg) {
-    double mmug[PDAC_MAXG], ckg[PDAC_MAXG];
-    for (int ig = 0; ig < P.ng; ++ig) {
-        int g = P.gas_type[ig];
-        double tst = tg / P.mmugek[g];
+// visc.f:37-148.  NG: the number of gases, 0 = the run's (arrays in local
+// memory).  What depends on the pair of gases only comes from tables made on
+// the host with the same functions (vm, vs2, vek, vpw, vs8; set_gas_tables).
+template <int NG>
+__device__ __forceinline__ void viscon_n(const Prm &P, double &mu, double &kap, const double *xg, double tg) {
+    const int ng = NG > 0 ? NG : P.ng;
+    double mmug[NG > 0 ? NG : PDAC_MAXG], ckg[NG > 0 ? NG : PDAC_MAXG];
+#pragma unroll
+    for (int ig = 0; ig < ng; ++ig) {
+        double tst = pdac_fp::div_by(tg, P.vek[ig]);
         double om = 1.16145 * pdac_fp::pow(tst, -0.14874) + 0.52487 * pdac_fp::exp(-0.77320 * tst) + 2.16178 * pdac_fp::exp(-2.43787 * tst);
-        double m = 1.0e3 * P.gmw[g];
-        double v = 26.69 * sqrt(m * tg) / (P.mmugs[g] * P.mmugs[g] * om);
+        double v = 26.69 * sqrt(P.vm[ig] * tg) / (P.vs2[ig] * om);
         mmug[ig] = v * 1.0e-7;
     }
     double t1 = tg, t2 = t1 * tg, t3 = t2 * tg;
-    double tr = tg / 132.5;
-    double trm1 = 1.0 / tr, trm2 = trm1 * trm1, trm3 = trm2 * trm1, trm4 = trm3 * trm1, trsrt = sqrt(tr);
-    for (int ig = 0; ig < P.ng; ++ig) {
+#pragma unroll
+    for (int ig = 0; ig < ng; ++ig) {
         switch (P.gas_type[ig]) {
         case 1: ckg[ig] = -3.273e-4 + 9.966e-5 * t1 - 3.743e-8 * t2 + 9.732e-12 * t3; break;
         case 2: ckg[ig] = 3.919e-4 + 9.816e-5 * t1 - 5.067e-8 * t2 + 1.504e-11 * t3; break;
         case 3: ckg[ig] = -7.215e-3 + 8.015e-5 * t1 + 5.477e-9 * t2 - 1.053e-11 * t3; break;
         case 4: ckg[ig] = 8.099e-3 + 6.689e-4 * t1 - 4.158e-7 * t2 + 1.562e-10 * t3; break;
         case 5: ckg[ig] = 7.341e-3 - 1.013e-5 * t1 + 1.801e-7 * t2 - 9.100e-11 * t3; break;
-        case 6: ckg[ig] = 25.9778e-3 * (0.2395 * tr + 6.4977e-3 * trsrt + 1.0 - 1.92615 * trm1 + 2.00383 * trm2 -
-                                        1.07553 * trm3 + 0.229414 * trm4); break;
+        case 6: {
+            double tr = tg / 132.5;
+            double trm1 = 1.0 / tr, trm2 = trm1 * trm1, trm3 = trm2 * trm1, trm4 = trm3 * trm1, trsrt = sqrt(tr);
+            ckg[ig] = 25.9778e-3 * (0.2395 * tr + 6.4977e-3 * trsrt + 1.0 - 1.92615 * trm1 + 2.00383 * trm2 -
+                                    1.07553 * trm3 + 0.229414 * trm4);
+            break;
+        }
         default: ckg[ig] = -8.086e-3 + 6.344e-5 * t1 - 1.382e-8 * t2 + 2.303e-12 * t3; break;
         }
     }
     mu = 0; kap = 0;
-    for (int ig = 0; ig < P.ng; ++ig) {
-        int g = P.gas_type[ig];
+#pragma unroll
+    for (int ig = 0; ig < ng; ++ig) {
         double sum = 0;
-        for (int jg = 0; jg < P.ng; ++jg) {
-            int h = P.gas_type[jg];
-            double aa = P.gmw[g] / P.gmw[h];
+#pragma unroll
+        for (int jg = 0; jg < ng; ++jg) {
             double bb = mmug[ig] / mmug[jg];
-            double cc = 1.0 + sqrt(bb) * pdac_fp::pow(aa, -0.25);
-            double phij = cc * cc / sqrt(8.0 * (1.0 + aa));
+            double cc = 1.0 + sqrt(bb) * P.vpw[ig][jg];
+            double phij = cc * cc / P.vs8[ig][jg];
             sum = sum + xg[jg] * phij;
         }
         double suminv = 1.0 / sum;
         mu = mu + xg[ig] * mmug[ig] * suminv;
         kap = kap + xg[ig] * ckg[ig] * suminv;
+    }
+}
+// the gas of cell c
+__device__ __forceinline__ void viscon(const Prm &P, const Fld &F, int c, double &mu, double &kap) {
+    const double *x = F.xgc + c;
+    const size_t n = P.ncell;
+    if (P.ng == 2) {
+        const double xg[2] = {x[0], x[n]};
+        viscon_n<2>(P, mu, kap, xg, F.tg[c]);
+    } else {
+        double xg[PDAC_MAXG];
+        for (int ig = 0; ig < P.ng; ++ig) xg[ig] = x[(size_t)ig * n];
+        viscon_n<0>(P, mu, kap, xg, F.tg[c]);
     }
 }
 
@@ -520,9 +539,12 @@ __device__ __forceinline__ int caloric_eosg(const Prm &P, double &cgas, double &
     return info;
 }
 
-// drag.f:60-157 (kdrags)
+// drag.f:60-157 (kdrags); ep265 = pow(ep, -2.65) of the cell (kdrags_ep)
+__device__ __forceinline__ double kdrags_ep(double ep) {
+    return ep < 0.8 ? 0.0 : pdac_fp::pow(ep, (double)(-2.65f));
+}
 __device__ __forceinline__ double kdrags(const Prm &P, double du, double dv, double dw, double ep, double rgp, double rlk,
-                                         double mug, int is) {
+                                         double mug, int is, double ep265) {
     double vrel = sqrt(du * du + dv * dv + dw * dw);
     double drag;
     {
@@ -538,7 +560,7 @@ __device__ __forceinline__ double kdrags(const Prm &P, double du, double dv, dou
             else dc = (double)0.43828814f;
             dc = fmin(dc, 1.0e4);
             drag = 0.75 * dc * eps / (P.dk[is] * P.phis[is]) * rgp * vrel;
-            drag = drag * pdac_fp::pow(ep, (double)(-2.65f));
+            drag = drag * ep265;
         }
     }
     return drag;
@@ -568,41 +590,45 @@ __device__ __forceinline__ double sdrag(const Prm &P, double du, double dv, doub
 
 // the drag law the run selects (tilde.f:617-623)
 __device__ __forceinline__ double drag_coeff(const Prm &P, double du, double dv, double dw, double ep, double rgp, double rlk,
-                                             double mug, int is) {
-    return P.drag_model == 1 ? kdrags(P, du, dv, dw, ep, rgp, rlk, mug, is) : sdrag(P, du, dv, dw, ep, rgp, rlk, mug, is);
+                                             double mug, int is, double ep265) {
+    return P.drag_model == 1 ? kdrags(P, du, dv, dw, ep, rgp, rlk, mug, is, ep265) : sdrag(P, du, dv, dw, ep, rgp, rlk, mug, is);
 }
 
 // drag.f:248-298
+// (the larger and the smaller class by selection, so that rlkc stays in
+// registers)
 __device__ __forceinline__ double ppdrag(const Prm &P, const double *rlkc, int k, int kk) {
-    int k1, k2;
-    if (P.dk[k - 1] >= P.dk[kk - 1]) { k1 = k - 1; k2 = kk - 1; }
-    else { k1 = kk - 1; k2 = k - 1; }
-    double ep1 = rlkc[k1] * P.inrl[k1], ep2 = rlkc[k2] * P.inrl[k2], epsum = ep1 + ep2;
+    const int a = k - 1, b = kk - 1;
+    const bool big = P.dk[a] >= P.dk[b];
+    const double epa = rlkc[a] * P.inrl[a], epb = rlkc[b] * P.inrl[b];
+    const double ep1 = big ? epa : epb, ep2 = big ? epb : epa, epsum = ep1 + ep2;
     if (ep1 > 0 && ep2 > 0) {
         double xbar = ep1 / epsum, epkl;
-        if (xbar <= P.philim[k - 1][kk - 1]) epkl = P.epsl[k - 1][kk - 1] * xbar + P.phi[k2];
-        else epkl = P.epsu[k - 1][kk - 1] * (1.0 - xbar) + P.phi[k1];
+        if (xbar <= P.philim[a][b]) epkl = P.epsl[a][b] * xbar + (big ? P.phi[b] : P.phi[a]);
+        else epkl = P.epsu[a][b] * (1.0 - xbar) + (big ? P.phi[a] : P.phi[b]);
         double espo = 1.0 / 3.0;
         double m1 = pdac_fp::pow(epkl, espo), m2 = pdac_fp::pow(epsum, espo);
         double effe = (3.0 * m1 + m2) / (2.0 * (m1 - m2));
-        return 1.0 * (1.0 + 1.0) * rlkc[k - 1] * rlkc[kk - 1] * P.dkf[k - 1][kk - 1] * effe;
+        return 1.0 * (1.0 + 1.0) * rlkc[a] * rlkc[b] * P.dkf[a][b] * effe;
     }
     return 0.0;
 }
 
-// hvs.f:9-83
+// hvs.f:9-83; pranumexp = the cell's Prandtl number to the power 1/3
+__device__ __forceinline__ double hvs_prandtl(double mug, double kapg, double cg) {
+    return pdac_fp::pow(cg * mug / kapg, 1.0 / 3.0);
+}
 __device__ __forceinline__ double hvs(const Prm &P, double rlk, double rog, double du, double dv, double dw, double mug,
-                                      double kapg, double cg, int k) {
+                                      double kapg, int k, double pranumexp) {
     if (rlk <= 0.0) return 0.0;
     double eps = rlk * P.inrl[k];
     double eps2 = eps * eps;
     double asurf = 6.0 * kapg * eps / (P.dk[k] * P.dk[k]);
     double vrel = sqrt(du * du + dv * dv + dw * dw);
     double reynum = P.dk[k] * vrel * rog / mug;
-    double pranum = cg * mug / kapg;
-    double pranumexp = pdac_fp::pow(pranum, 1.0 / 3.0);
-    double nusselt = (2.0 + 5.0 * eps2) * (1.0 + 0.7 * pdac_fp::pow(reynum, 0.2) * pranumexp);
-    nusselt = nusselt + (0.13 + 1.2 * eps2) * pdac_fp::pow(reynum, 0.7) * pranumexp;
+    const pdac_fp::PowOf re = pdac_fp::pow_of(reynum);
+    double nusselt = (2.0 + 5.0 * eps2) * (1.0 + 0.7 * pdac_fp::pow(re, 0.2) * pranumexp);
+    nusselt = nusselt + (0.13 + 1.2 * eps2) * pdac_fp::pow(re, 0.7) * pranumexp;
     return nusselt * asurf;
 }
 

@@ -256,13 +256,13 @@ __device__ __forceinline__ void phys_coeff(const Prm &P, const Fld &F, const RkF
     constexpr int MA = MP * (MP + 1) / 2 + 1;
     const int c = q.c, ns = nphases<NP>(P) - 1, nph = ns + 1;
     const size_t n = P.ncell;
-    double xg[PDAC_MAXG];
-    for (int ig = 0; ig < P.ng; ++ig) xg[ig] = GAS(F.xgc, c, ig);
     double mu, ka;
-    viscon(P, mu, ka, xg, F.tg[c]);
+    viscon(P, F, c, mu, ka);
     F.mug[c] = mu;
     F.kapg[c] = ka;
     double kp[MP], rlkc[MP];
+    const double ep265 = kdrags_ep(F.ep[c]), pranumexp = hvs_prandtl(mu, ka, F.cg[c]);
+#pragma unroll
     for (int is = 1; is <= ns; ++is) {
         size_t off = (size_t)(is - 1) * n;
         double dugs = ((F.ug[c] - F.us[off + c]) + (F.ug[q.rw] - F.us[off + q.rw])) * 0.5;
@@ -270,16 +270,18 @@ __device__ __forceinline__ void phys_coeff(const Prm &P, const Fld &F, const RkF
         double dvgs = 0.0;
         if (D == 3) dvgs = ((F.vg[c] - F.vs[off + c]) + (F.vg[q.rs] - F.vs[off + q.rs])) * 0.5;
         rlkc[is] = F.rlk[off + c];
-        K.hv[off + c] = hvs(P, rlkc[is], F.rog[c], dugs, dvgs, dwgs, mu, ka, F.cg[c], is);
-        kp[is] = kdrags(P, dugs, dvgs, dwgs, F.ep[c], F.rgp[c], rlkc[is], mu, is);
+        K.hv[off + c] = hvs(P, rlkc[is], F.rog[c], dugs, dvgs, dwgs, mu, ka, is, pranumexp);
+        kp[is] = kdrags(P, dugs, dvgs, dwgs, F.ep[c], F.rgp[c], rlkc[is], mu, is, ep265);
     }
     double au[MA], av[MA], aw[MA];
     int ks = 0;
+#pragma unroll
     for (int k1 = 1; k1 <= nph; ++k1) {
         if (k1 == 1) {
             ks++;
             au[ks] = 0; av[ks] = 0; aw[ks] = 0;
         } else {
+#pragma unroll
             for (int kk = 1; kk <= k1; ++kk) {
                 ks++;
                 if (kk == 1) {
@@ -301,12 +303,15 @@ __device__ __forceinline__ void phys_coeff(const Prm &P, const Fld &F, const RkF
             }
         }
     }
+#pragma unroll
     for (int k1 = 1; k1 <= nph; ++k1) {
         double sx = 0, sy = 0, sz = 0;
+#pragma unroll
         for (int kk = 1; kk <= k1; ++kk) {
             int t = kk + k1 * (k1 - 1) / 2;
             sx = sx + au[t]; sy = sy + av[t]; sz = sz + aw[t];
         }
+#pragma unroll
         for (int kk = k1; kk <= nph; ++kk) {
             int t = k1 + kk * (kk - 1) / 2;
             sx = sx + au[t]; sy = sy + av[t]; sz = sz + aw[t];
@@ -315,6 +320,7 @@ __device__ __forceinline__ void phys_coeff(const Prm &P, const Fld &F, const RkF
         au[t] = -sx; av[t] = -sy; aw[t] = -sz;
     }
     const int nap = nph * (nph + 1) / 2;
+#pragma unroll
     for (int t = 1; t <= nap; ++t) {
         APP(F.appu, c, t) = au[t];
         APP(F.appw, c, t) = aw[t];
@@ -386,10 +392,10 @@ __global__ void k_visc2d(Prm P, Fld F) {
             double indxp = P.hx[i], indzp = P.hz[k];
             double rc = rl[c], re = rl[M.e], rt = rl[M.t];
             double epsx = (dx[i + 1] * rc + dx[i] * re) * indxp * ir;
-            double gepx = pdac_fp::pow(10.0, -a_rep * epsx + b_rep);
+            double gepx = pdac_fp::pow10(-a_rep * epsx + b_rep);
             vx = vx - gepx * indxp * 2.0 * (re - rc) * ir;
             double epsz = (dz[k + 1] * rc + dz[k] * rt) * indzp * ir;
-            double gepz = pdac_fp::pow(10.0, -a_rep * epsz + b_rep);
+            double gepz = pdac_fp::pow10(-a_rep * epsz + b_rep);
             vz = vz - gepz * indzp * 2.0 * (rt - rc) * ir;
         }
     }
