@@ -294,14 +294,13 @@ static cudaError_t set_inner_attrs_np() {
     const int sm = (int)pdac::inner_smem_bytes<NP>();
     cudaError_t e = cudaFuncSetAttribute(pdac::k_inner_team<NP, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(pdac::k_inner_team<NP, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    auto loop = [&](auto kernel, bool cluster) {
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pdac::sweep_smem_bytes<NP>());
-        if (cluster && e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    auto loop = [&](auto kernel, size_t smem) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     };
-    loop(pdac::k_sweep_loop<NP, 2, false>, false);
-    loop(pdac::k_sweep_loop<NP, 3, false>, false);
-    loop(pdac::k_sweep_loop<NP, 2, true>, true);
+    loop(pdac::k_sweep_grid<NP, 2>, pdac::sweep_smem_bytes<NP>());
+    loop(pdac::k_sweep_grid<NP, 3>, pdac::sweep_smem_bytes<NP>());
+    loop(pdac::k_sweep_cluster<NP>, pdac::cluster_smem_bytes<NP>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(pdac::k_sweep_cluster<NP>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 static cudaError_t set_inner_attrs() {
@@ -673,14 +672,15 @@ int setup_wave(pdac_ctx *ctx, const int *flag) {
 // 2D meshes of at most this many cells run iter's sweep loop on one cluster
 // of 16 blocks: their colour phases hold a few hundred cells, and the
 // hardware's cluster barrier costs a fraction of a grid-wide one.  Measured
-// (ms of a burst, cluster against grid): 128 x 192 35.9 / 38.1, 251 x 383
-// 35.5 / 38.9, 384 x 640 125.8 / 95.2 (its worklists outgrow the cluster's 64
-// warps); 3D meshes have long worklists from the start (24^3 10.5 / 7.4) and
-// always take the grid.
+// (ms of a burst, cluster against grid): 24 x 33 2.8 / 4.5, 128 x 192 33.3 /
+// 38.8, 251 x 383 30.8 / 38.3, 359 x 363 35.4 / 42.9, 200 x 300 with five
+// classes 61.6 / 71.6.  Far above the limit the cluster's 128 warps are short
+// of the worklists; 3D meshes have long ones from the start and always take
+// the grid.
 #ifndef PDAC_CLUSTER_MAX_CELLS
 #define PDAC_CLUSTER_MAX_CELLS (1 << 17)
 #endif
-constexpr int CLUSTER_BLOCKS = 16;
+static_assert(PDAC_CLUSTER_MAX_CELLS / 32 <= pdac::CLUSTER * pdac::KC, "a word of the active set for every thread");
 
 // the sweep loop in one launch on stream st
 template <int NP>
@@ -697,15 +697,15 @@ static cudaError_t launch_sweep_loop_np(pdac_ctx *ctx, double dt, cudaStream_t s
         at[0].val.cooperative = 1;
     }
     lc.gridDim = dim3(cl ? ctx->cluster_blocks : ctx->coop_blocks);
-    lc.blockDim = dim3(TPB_TEAM);
-    lc.dynamicSmemBytes = pdac::sweep_smem_bytes<NP>();
+    lc.blockDim = dim3(cl ? pdac::KC : TPB_TEAM);
+    lc.dynamicSmemBytes = cl ? pdac::cluster_smem_bytes<NP>() : pdac::sweep_smem_bytes<NP>();
     lc.stream = st;
     lc.attrs = at;
     lc.numAttrs = 1;
     const int mo = ctx->cfg.maxout;
-    if (ctx->d3) return cudaLaunchKernelEx(&lc, pdac::k_sweep_loop<NP, 3, false>, ctx->P, ctx->F, dt, W, mo);
-    return cl ? cudaLaunchKernelEx(&lc, pdac::k_sweep_loop<NP, 2, true>, ctx->P, ctx->F, dt, W, mo)
-              : cudaLaunchKernelEx(&lc, pdac::k_sweep_loop<NP, 2, false>, ctx->P, ctx->F, dt, W, mo);
+    if (ctx->d3) return cudaLaunchKernelEx(&lc, pdac::k_sweep_grid<NP, 3>, ctx->P, ctx->F, dt, W, mo);
+    return cl ? cudaLaunchKernelEx(&lc, pdac::k_sweep_cluster<NP>, ctx->P, ctx->F, dt, W, mo)
+              : cudaLaunchKernelEx(&lc, pdac::k_sweep_grid<NP, 2>, ctx->P, ctx->F, dt, W, mo);
 }
 
 static cudaError_t launch_sweep_loop(pdac_ctx *ctx, double dt, cudaStream_t st) {
@@ -724,21 +724,21 @@ template <int NP, int D>
 static cudaError_t sweep_loop_room(int nsm, int &grid_blocks, int &clusters) {
     const size_t sm = pdac::sweep_smem_bytes<NP>();
     int occ = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_sweep_loop<NP, D, false>, TPB_TEAM, sm);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_sweep_grid<NP, D>, TPB_TEAM, sm);
     grid_blocks = occ * nsm;
     clusters = 0;
     if (e != cudaSuccess || D == 3) return e;
     cudaLaunchConfig_t lc = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CLUSTER_BLOCKS;
+    at[0].val.clusterDim.x = pdac::CLUSTER;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    lc.gridDim = dim3(CLUSTER_BLOCKS);
-    lc.blockDim = dim3(TPB_TEAM);
-    lc.dynamicSmemBytes = sm;
+    lc.gridDim = dim3(pdac::CLUSTER);
+    lc.blockDim = dim3(pdac::KC);
+    lc.dynamicSmemBytes = pdac::cluster_smem_bytes<NP>();
     lc.attrs = at;
     lc.numAttrs = 1;
-    return cudaOccupancyMaxActiveClusters(&clusters, pdac::k_sweep_loop<NP, 2, true>, &lc);
+    return cudaOccupancyMaxActiveClusters(&clusters, pdac::k_sweep_cluster<NP>, &lc);
 }
 
 // The form of the sweep loop.  One launch whose blocks stay resident spares
@@ -763,7 +763,7 @@ static int setup_sweep_loop(pdac_ctx *ctx) {
         case 6: CK((ctx->d3 ? sweep_loop_room<6, 3> : sweep_loop_room<6, 2>)(nsm, room, clusters)); break;
         default: CK((ctx->d3 ? sweep_loop_room<0, 3> : sweep_loop_room<0, 2>)(nsm, room, clusters)); break;
     }
-    if (!ctx->d3 && (long)ctx->ncell <= PDAC_CLUSTER_MAX_CELLS && clusters > 0) ctx->cluster_blocks = CLUSTER_BLOCKS;
+    if (!ctx->d3 && (long)ctx->ncell <= PDAC_CLUSTER_MAX_CELLS && clusters > 0) ctx->cluster_blocks = pdac::CLUSTER;
     if (!coop) return PDAC_OK;
     ctx->coop_cpb = ctx->d3 ? 64 : 1024;
     ctx->coop_max_blocks = room;
@@ -1002,7 +1002,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     CK(cudaMallocHost(&ctx->h_status, 4 * sizeof(int)));
     CK(cudaMalloc(&ctx->d_wcount, 16 * sizeof(int)));
     CK(cudaMalloc(&ctx->d_dirty, ((size_t)n + 31) / 32 * sizeof(unsigned)));
-    CK(cudaMalloc(&ctx->d_cmask, (size_t)3 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
+    CK(cudaMalloc(&ctx->d_cmask, (size_t)4 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
     if (ctx->d3 && P.muscl > 0) {
         CK(cudaMalloc(&ctx->d_simple, ((size_t)n + 31) / 32 * sizeof(unsigned)));
         pdac::k_simple_mask<<<blocks(((long)n + 31) / 32), TPB, 0, ctx->stream>>>(P, ctx->d_simple);
@@ -1591,8 +1591,8 @@ static int enqueue_sweep(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof) {
         if (prof) CK(cudaEventRecord(ctx->cev[3 * col], st));
         const unsigned *cmask = ctx->d_cmask + (size_t)col * nwords;
         int *wl = ctx->d_work + col * ctx->work_stride;
-        if (ctx->d3) PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 3, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, dirty, wl, cnt);
-        else PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 2, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, dirty, wl, cnt);
+        if (ctx->d3) PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 3, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, ctx->d_cmask + 3 * nwords, dirty, wl, cnt);
+        else PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 2, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, ctx->d_cmask + 3 * nwords, dirty, wl, cnt);
         if (prof) CK(cudaEventRecord(ctx->cev[3 * col + 1], st));
         if (ctx->d3) INNER_LAUNCH_D(nph, pdac::k_inner_team, 3, g, TPB_TEAM, st, ctx->P, F, dt, ctx->d_nit, wl, cnt, dirty, inner_spread(ctx));
         else INNER_LAUNCH_D(nph, pdac::k_inner_team, 2, g, TPB_TEAM, st, ctx->P, F, dt, ctx->d_nit, wl, cnt, dirty, inner_spread(ctx));
@@ -1804,6 +1804,7 @@ int pdac_gpu_unconverged_cells(pdac_ctx *ctx, int *ijk, long *n_inout) {
         if (cnt[c]) CK(cudaMemcpy(ijk + at, ctx->d_work + c * ctx->work_stride, cnt[c] * sizeof(int), cudaMemcpyDeviceToHost));
         at += cnt[c];
     }
+    for (long q = 0; q < total; ++q) ijk[q] &= 0x7fffffff;  // without the plain bit of a worklist entry
     std::sort(ijk, ijk + total);
     *n_inout = total;
     return PDAC_OK;
@@ -1898,8 +1899,8 @@ int pdac_gpu_iter_static(pdac_ctx *ctx, double dt, int *nit_out) {
         for (int col = 0; col < 3; ++col) {
             int *cnt = wcount + col;
             const unsigned *cmask = ctx->d_cmask + (size_t)col * nwords;
-            if (ctx->d3) PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 3, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, dirty, work, cnt);
-            else PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 2, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, dirty, work, cnt);
+            if (ctx->d3) PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 3, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, ctx->d_cmask + 3 * nwords, dirty, work, cnt);
+            else PHASE_LAUNCH_D(nph, pdac::k_resid_scan, 2, test_grid, TPB_RESID, st, ctx->P, F, dt, cmask, ctx->d_cmask + 3 * nwords, dirty, work, cnt);
             long team_threads = (nthr + (ctx->d3 ? 4 : 7)) / (ctx->d3 ? 5 : 8) * 32;
             int g = std::min(ctx->inner_grid, blocks(team_threads, TPB_TEAM));
             if (ctx->d3) INNER_LAUNCH_D(nph, pdac::k_inner_team, 3, g, TPB_TEAM, st, ctx->P, F, dt, dnit, work, cnt, dirty, inner_spread(ctx));

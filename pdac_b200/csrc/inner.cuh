@@ -105,7 +105,7 @@ template <int NP>
 struct FaceK<NP, true> {
     static constexpr int R = face_rec(NP), N = R + FK_N + 1;
     double *s;  // this lane's column: element q at s[q / 2 * 2 * KS + q % 2]
-    __device__ __forceinline__ explicit FaceK(double *cols) : s(cols + 2 * threadIdx.x) {}
+    __device__ __forceinline__ explicit FaceK(double *cols) : s(cols + 2 * (threadIdx.x % KS)) {}
     __device__ __forceinline__ void set(int i, double v) { s[i / 2 * 2 * KS + i % 2] = v; }
     __device__ __forceinline__ void get(double (&v)[R]) const {
 #pragma unroll
@@ -260,13 +260,19 @@ template <int NP>
 __host__ __device__ constexpr size_t inner_smem_bytes() {
     return (size_t)(inner_face_rows<NP>() + inner_dens_rows<NP>()) * KS * sizeof(double);
 }
-// k_sweep_loop's, which holds the warps' scan lists in the same place
+// the sweep loops', which hold the warps' scan lists in the same place
 template <int NP>
-__host__ __device__ constexpr size_t sweep_smem_bytes() {
-    return inner_smem_bytes<NP>() > KS / 32 * 352 * sizeof(int) ? inner_smem_bytes<NP>() : KS / 32 * 352 * sizeof(int);
+__host__ __device__ constexpr size_t sweep_smem_bytes(int threads = KS) {
+    return (size_t)threads / KS * (inner_smem_bytes<NP>() > KS / 32 * 352 * sizeof(int) ? inner_smem_bytes<NP>() : KS / 32 * 352 * sizeof(int));
 }
 
-// The inner loop of worklist cell c (outer sweep nit, 1-based) by the team of
+// A worklist entry is a cell, with the top bit set for a plain one: a cell
+// whose face stencils meet no wall and stay two cells from the mesh's ends
+// (k_colour_masks), so that no flag need be read to know its neighbours --
+// one dependent trip to L2 less before the values themselves are asked for.
+__device__ __forceinline__ int entry_cell(int e) { return e & 0x7fffffff; }
+
+// The inner loop of worklist entry e (outer sweep nit, 1-based) by the team of
 // lanes tb .. tb + T - 1 of this warp (lane q of the team owns face q); kcols
 // and dcols are the shared FaceK and DensK arrays.  RO as in ldro.
 //
@@ -280,7 +286,7 @@ __host__ __device__ constexpr size_t sweep_smem_bytes() {
 // instructions of a warp's teams when they diverge; hence one code path for
 // all faces, velocity signs and bracketing states.
 template <int NP, int D, bool RO>
-__device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, double dt, int nit, int c, bool live,
+__device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, double dt, int nit, int e, bool live,
                                                 unsigned *dirty, int q, int tb, double *kcols, double *dcols) {
     constexpr unsigned full = 0xffffffffu;
     constexpr int NC = Sys<NP>::M - 1;   // phase capacity
@@ -289,6 +295,8 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
     constexpr int NAX = D == 3 ? 3 : 2;  // axes; lanes q < NAX own the minus faces
     const int nph = nphases<NP>(P), ns = nph - 1;
     const size_t n = P.ncell;
+    const int c = entry_cell(e);
+    const bool plain = e < 0;
     int i, j, k;
     if (D == 3) ijk_of(P, c, i, j, k);
     else { i = c % P.nx + 1; j = 1; k = c / P.nx + 1; }
@@ -306,15 +314,20 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
     const int rawnb = minus ? c - stride * min(1, ii - 1) : c + stride * min(1, nax - ii);
     const int rawop = minus ? c + stride * min(1, nax - ii) : c - stride * min(1, ii - 1);
     const int rawfar = minus ? c - stride * min(2, ii - 1) : c + stride * min(2, nax - ii);
-    const int fnb = fl[rawnb];
     // the remapped neighbours (rem2 / rem3): a wall reads as the cell itself,
     // a wall beyond the neighbour as the neighbour (y: the remapped one), the
     // last cell before the frame repeats the remapped neighbour
-    const int rn = is_wallf(fnb) ? c : rawnb, ro = is_wallf(fl[rawop]) ? c : rawop;
-    const int rf = toward == 1 ? rn : (is_wallf(fl[rawfar]) ? (dir == 1 ? rn : rawnb) : rawfar);
+    int fnb = FLUID, rn = rawnb, ro = rawop, rf = rawfar;
+    bool mus = P.muscl > 0;
+    if (!plain) {
+        fnb = fl[rawnb];
+        rn = is_wallf(fnb) ? c : rawnb;
+        ro = is_wallf(fl[rawop]) ? c : rawop;
+        rf = toward == 1 ? rn : (is_wallf(fl[rawfar]) ? (dir == 1 ? rn : rawnb) : rawfar);
+        mus = mus && fl[c] == FLUID;
+    }
     const bool solved = (fnb & 1) != 0;
     const int fcell = minus ? rawnb : c;  // where this face's velocity and fluxes live
-    const bool mus = P.muscl > 0 && fl[c] == FLUID;
     FaceGeo g;
     {
         const double *dd = dir == 0 ? P.dx : (dir == 1 ? P.dy : P.dz);
@@ -344,7 +357,7 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
     // is what this load reads
     const bool stale = P.opt == 2;
     const bool sn = !stale && rn == c, so = !stale && ro == c, sf = !stale && rf == c, self = sn || so || sf;
-    DensK<NC, SHD> Dk(dcols + threadIdx.x);
+    DensK<NC, SHD> Dk(dcols + threadIdx.x % KS);
 #pragma unroll
     for (int l = 1; l <= nph; ++l) {
         const double *D_ = l == 1 ? F.rgp : F.rlk + (size_t)(l - 2) * n;
@@ -396,7 +409,7 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
     // does not change within the loop: summed once, in thermal_eosg's order
     double mg = 0;
     for (int ig = 0; ig < P.ng; ++ig) mg = mg + GAS(F.xgc, c, ig) * P.gmw[P.gas_type[ig]];
-    const double rgas_tg = P.rgas * F.tg[c];
+    const pdac_fp::Recip rgas_tg = pdac_fp::recip(P.rgas * F.tg[c]);
     int kros = -1;
     PAdj s = {0, 0, 0, 0, 0, 0};
     double p = p3, ep = F.ep[c], rog, rgp;
@@ -413,7 +426,7 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
     if constexpr (SH) K.fetched();
     for (int loop = 1; loop <= P.inmax; ++loop) {
         if (loop > 1 || nit > 1) padjust(s, p, kros, d3, p3, P.omega, abeta);
-        rog = p / rgas_tg * mg;  // thermal_eosg
+        rog = pdac_fp::div_by(p, rgas_tg) * mg;  // thermal_eosg
         rgp = ep * rog;
         // this lane's face system (matrix.f:351-630)
         if (solved) face_assemble<NP>(P, K, Dk, minus ? -1 : +1, p, ep, rgp, rlk, vel);
@@ -479,8 +492,9 @@ __device__ __forceinline__ void inner_team_run(const Prm &P, const Fld &F, doubl
     const int lane = threadIdx.x & 31, tw = lane / T;
     const int q = lane - tw * T, tb = tw * T;
     extern __shared__ __align__(16) double inner_smem[];
-    double *const kcols = inner_smem;                              // [FaceK rows][KS]
-    double *const dcols = inner_smem + inner_face_rows<NP>() * KS;  // [3 NC][KS]
+    // every KS threads have columns of their own: [FaceK rows][KS], [3 NC][KS]
+    double *const kcols = inner_smem + threadIdx.x / KS * (inner_smem_bytes<NP>() / sizeof(double));
+    double *const dcols = kcols + inner_face_rows<NP>() * KS;
     for (int w0 = warp * cpw; w0 < nwork; w0 += nwarps * cpw) {
         const bool live = tw < TPW && tw < cpw && w0 + tw < nwork;
         inner_team_cell<NP, D, RO>(P, F, dt, nit, list[live ? w0 + tw : w0], live, dirty, q, tb, kcols, dcols);
@@ -519,27 +533,72 @@ __global__ void __launch_bounds__(128, PDAC_INNER_MINB(NP)) k_inner_team(Prm P, 
 // it holds, and it is not tested.  cmask holds, per colour, the bits of the
 // colour's fluid cells in the same words (k_colour_masks, set up once): a
 // word's candidates are its active bits under the mask, and the bits that
-// runs set on non-fluid neighbours are never looked at.
+// runs set on non-fluid neighbours are never looked at.  A fourth mask holds
+// the plain cells (worklist entries above): flag 1 like all their face
+// neighbours, no wall two cells away and none of those beyond the frame.
 __global__ void k_colour_masks(Prm P, unsigned *cmask) {
     const unsigned nwords = ((unsigned)P.ncell + 31u) / 32u;
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nwords) return;
-    unsigned m[3] = {0u, 0u, 0u};
+    unsigned m[4] = {0u, 0u, 0u, 0u};
     for (int b = 0; b < 32; ++b) {
         const int c = (int)(32u * t) + b;
         if (c >= P.ncell) break;
         if (!(P.flag[c] & 1)) continue;
         const int i = c % P.nx + 1, r = c / P.nx, j = r % P.ny + 1, k = r / P.ny + 1;
         m[(i + j + k) % 3] |= 1u << b;
+        auto axis = [&](int ii, int nax, int stride) {
+            return ii >= 3 && ii <= nax - 2 && P.flag[c - stride] == FLUID && P.flag[c + stride] == FLUID &&
+                   !is_wallf(P.flag[c - 2 * stride]) && !is_wallf(P.flag[c + 2 * stride]);
+        };
+        if (P.flag[c] == FLUID && axis(i, P.nx, 1) && axis(k, P.nz, P.nx * P.ny) && (!P.d3 || axis(j, P.ny, P.nx)))
+            m[3] |= 1u << b;
     }
-    for (int q = 0; q < 3; ++q) cmask[(size_t)q * nwords + t] = m[q];
+    for (int q = 0; q < 4; ++q) cmask[(size_t)q * nwords + t] = m[q];
 }
 
 // the residual test of cell c (iter.f:241-319): a converged cell updates its
 // volume fractions and rgp (keeping its active-set bit if rgp changed);
 // returns true for an unconverged cell, which goes to the inner loop
-template <int NP, int D>
+// EAGER (2D, a known phase count) asks for what a converged cell needs
+// together with its residual: one trip to L2 instead of two, for more traffic
+template <int NP, int D, bool EAGER>
 __device__ __forceinline__ bool test_cell(const Prm &P, const Fld &F, double dt, int c, unsigned *dirty) {
+    if constexpr (EAGER && D == 2 && NP > 0) {
+        constexpr int ns = NP - 1;
+        const int i = c % P.nx + 1, k = c / P.nx + 1;
+        const int cw = at2(P, max(i - 1, 1), k), cb = at2(P, i, max(k - 1, 1));
+        const CellFaces b = cell_faces(P, c);
+        double fe[ns], fw[ns], ft[ns], fb[ns], ln[ns], sk[ns];
+#pragma unroll
+        for (int is = 1; is <= ns; ++is) {
+            fe[is - 1] = SOL(F.rsfe, c, is); fw[is - 1] = SOL(F.rsfe, cw, is);
+            ft[is - 1] = SOL(F.rsft, c, is); fb[is - 1] = SOL(F.rsft, cb, is);
+            ln[is - 1] = SOL(F.rlkn, c, is); sk[is - 1] = SOL(F.sink, c, is);
+        }
+        const double old = F.rgp[c], rog = F.rog[c], conv = F.conv[c];
+        const double resx = (b.e * F.rgfe[c] - b.w * F.rgfe[cw]) * P.indx[i] * P.inr[i];
+        const double resz = (b.t * F.rgft[c] - b.b * F.rgft[cb]) * P.indz[k];
+        const double dg = old - F.rgpn[c] + dt * b.ivf * (resx + 0.0 + resz);
+        if (!(fabs(dg) <= conv)) return true;
+        double rls = 0;
+#pragma unroll
+        for (int is = 1; is <= ns; ++is) {
+            const double rx = (b.e * fe[is - 1] - b.w * fw[is - 1]) * P.indx[i] * P.inr[i];
+            const double rz = (b.t * ft[is - 1] - b.b * fb[is - 1]) * P.indz[k];
+            double t = ln[is - 1] - dt * b.ivf * (rx + 0.0 + rz);
+            t = t + dt * b.ivf * sk[is - 1];
+            const double v = fmax(0.0, t);
+            SOL(F.rlk, c, is) = v;
+            rls = rls + v * P.inrl[is];
+        }
+        const double ep = 1.0 - rls, rgp = ep * rog;
+        if (rls > 1.0) atomicAdd(&F.counters[2], 1);
+        F.ep[c] = ep;
+        F.rgp[c] = rgp;
+        if (__double_as_longlong(rgp) != __double_as_longlong(old)) mark_dirty(dirty, c);
+        return false;
+    }
     double dg;
     if (D == 3) {
         int i, j, k;
@@ -574,69 +633,82 @@ __device__ __forceinline__ bool test_cell(const Prm &P, const Fld &F, double dt,
 // Collecting and testing in one pass took the two launches' fixed cost
 // (about 12 us) down to one's.
 constexpr int SCAN_LIST = 32 * 11;  // a colour has at most 11 cells in a word of 32
+
+// one warp's round: lane's word t (of words) of the active set under its
+// colour mask, its candidates tested; put(um, lane, u, e) takes the unconverged
+// ones (um: the ballot of u).  Returns the number tested.
+template <int NP, int D, bool EAGER, class PUT>
+__device__ __forceinline__ int scan_round(const Prm &P, const Fld &F, double dt, const unsigned *cmask,
+                                          const unsigned *plain, unsigned *dirty, unsigned t, unsigned nwords,
+                                          int *slist, PUT put) {
+    constexpr unsigned full = 0xffffffffu;
+    const unsigned lane = threadIdx.x & 31u;
+    unsigned w = 0, pl = 0;
+    if (t < nwords) {
+        w = __ldcg(dirty + t) & __ldg(cmask + t);
+        pl = __ldg(plain + t);
+        if (w) atomicAnd(dirty + t, ~w);
+    }
+    int incl = __popc(w);
+    const int mine = incl;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(full, incl, o);
+        if (lane >= (unsigned)o) incl += v;
+    }
+    const int total = __shfl_sync(full, incl, 31);
+    if (total == 0) return 0;
+    for (int off = incl - mine; w; w &= w - 1u) {
+        const int b = __ffs(w) - 1;
+        slist[off++] = (int)(32u * t + (unsigned)b | (pl >> b & 1u) << 31);
+    }
+    __syncwarp();
+    for (int base = 0; base < total; base += 32) {
+        const int idx = base + (int)lane;
+        int e = 0;
+        bool u = false;
+        if (idx < total) {
+            e = slist[idx];
+            u = test_cell<NP, D, EAGER>(P, F, dt, entry_cell(e), dirty);
+        }
+        const unsigned um = __ballot_sync(full, u);
+        if (um) put(um, lane, u, e);
+    }
+    __syncwarp();  // the list is read before the next round overwrites it
+    return total;
+}
+
 template <int NP, int D>
 __device__ __forceinline__ void scan_phase(const Prm &P, const Fld &F, double dt, const unsigned *cmask,
-                                           unsigned *dirty, int *work, int *count, int *tested, unsigned warp,
-                                           unsigned nwarps, int *slist) {
-    constexpr unsigned full = 0xffffffffu;
+                                           const unsigned *plain, unsigned *dirty, int *work, int *count, int *tested,
+                                           unsigned warp, unsigned nwarps, int *slist) {
     const unsigned lane = threadIdx.x & 31u, nwords = ((unsigned)P.ncell + 31u) / 32u;
     const unsigned gs = nwords <= 32u * nwarps ? 1u : 8u, gpi = 32u / gs;  // words per group, groups per round
     int ntest = 0;
     for (unsigned g0 = 0; (size_t)g0 * nwarps * gs < nwords; g0 += gpi) {
         const unsigned t = ((g0 + lane / gs) * nwarps + warp) * gs + lane % gs;
-        unsigned w = 0;
-        if (t < nwords) {
-            w = __ldcg(dirty + t) & __ldg(cmask + t);
-            if (w) atomicAnd(dirty + t, ~w);
-        }
-        int incl = __popc(w);
-        const int mine = incl;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(full, incl, o);
-            if (lane >= (unsigned)o) incl += v;
-        }
-        const int total = __shfl_sync(full, incl, 31);
-        if (total == 0) continue;
-        for (int off = incl - mine; w; w &= w - 1u) slist[off++] = (int)(32u * t) + __ffs(w) - 1;
-        __syncwarp();
-        for (int base = 0; base < total; base += 32) {
-            const int idx = base + (int)lane;
-            int c = -1;
-            bool u = false;
-            if (idx < total) {
-                c = slist[idx];
-                u = test_cell<NP, D>(P, F, dt, c, dirty);
-            }
-            const unsigned um = __ballot_sync(full, u);
-            if (um) {
-                int at = 0;
-                if (lane == 0) at = atomicAdd(count, __popc(um));
-                at = __shfl_sync(full, at, 0);
-                if (u) work[at + __popc(um & ((1u << lane) - 1u))] = c;
-            }
-        }
-        ntest += total;
-        __syncwarp();  // the list is read before the next round overwrites it
+        ntest += scan_round<NP, D, false>(P, F, dt, cmask, plain, dirty, t, nwords, slist,
+                                          [&](unsigned um, unsigned ln, bool u, int e) {
+                                              int at = 0;
+                                              if (ln == 0) at = atomicAdd(count, __popc(um));
+                                              at = __shfl_sync(0xffffffffu, at, 0);
+                                              if (u) work[at + __popc(um & ((1u << ln) - 1u))] = e;
+                                          });
     }
     if (tested && lane == 0 && ntest) atomicAdd(tested, ntest);
 }
 
 template <int NP, int D>
 __global__ void __launch_bounds__(TPB_RESID) k_resid_scan(Prm P, Fld F, double dt, const unsigned *cmask,
-                                                          unsigned *dirty, int *work, int *count) {
+                                                          const unsigned *plain, unsigned *dirty, int *work, int *count) {
     __shared__ int slist[TPB_RESID / 32][SCAN_LIST];
     const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    scan_phase<NP, D>(P, F, dt, cmask, dirty, work, count, count + 3, warp, nwarps, slist[threadIdx.x >> 5]);
+    scan_phase<NP, D>(P, F, dt, cmask, plain, dirty, work, count, count + 3, warp, nwarps, slist[threadIdx.x >> 5]);
 }
 
 // The whole outer sweep loop of iter (iter.f:204-410) in one launch whose
 // blocks are all resident: the colour phases' residual tests and inner loops
-// follow each other across barriers instead of launches.  Two forms of
-// barrier: CLUSTER = true runs the mesh on one thread-block cluster with the
-// hardware's cluster barrier (the blocks of a cluster are always scheduled
-// together, so any number of such launches may share the device);
-// CLUSTER = false runs it on a cooperative grid.
+// follow each other across barriers instead of launches.
 // Every thread takes every barrier the same number of times: the loop ends
 // on counters that all threads read after the same barrier.
 struct SweepWork {
@@ -644,33 +716,44 @@ struct SweepWork {
     int *counts;      // two sets of three worklist lengths, for odd and even sweeps
     int *work;        // worklists, colour col at work + col * wstride
     unsigned *dirty;  // active set, one bit per cell
-    const unsigned *cmask;  // colour masks
+    const unsigned *cmask;  // the three colour masks and the plain mask
     int *nit;         // the sweep count on return, as the graph's k_sweep_check leaves it
     long wstride;     // ints per colour's worklist
 };
 
-template <int NP, int D, bool CLUSTER>
-__global__ void __launch_bounds__(KS, PDAC_INNER_MINB(NP)) k_sweep_loop(Prm P, Fld F, double dt, SweepWork W, int maxout) {
-    namespace cg = cooperative_groups;
-    auto barrier = [] {
-        __syncwarp();
-        if (CLUSTER) cg::this_cluster().sync();
-        else cg::this_grid().sync();
-    };
+// after a sweep's last barrier: its worklist lengths; true when the loop ends
+__device__ __forceinline__ bool sweep_ends(const SweepWork &W, const int *cnt, int nit, int maxout) {
+    const int n0 = __ldcg(cnt), n1 = __ldcg(cnt + 1), n2 = __ldcg(cnt + 2);
+    const bool conv = (long)n0 + n1 + n2 == 0;
+    if (!conv && nit < maxout) return false;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        W.wcount[0] = n0;
+        W.wcount[1] = n1;
+        W.wcount[2] = n2;
+        *W.nit = conv ? nit : maxout + 1;
+    }
+    return true;
+}
+
+// on a cooperative grid: the unconverged cells of a phase go to one worklist,
+// from which all warps take theirs, a grid-wide barrier after either half
+template <int NP, int D>
+__global__ void __launch_bounds__(KS, PDAC_INNER_MINB(NP)) k_sweep_grid(Prm P, Fld F, double dt, SweepWork W, int maxout) {
+    auto barrier = [] { cooperative_groups::this_grid().sync(); };
     extern __shared__ __align__(16) double inner_smem[];
     const int wid = threadIdx.x >> 5, warp = blockIdx.x * (KS / 32) + wid, nwarps = gridDim.x * (KS / 32);
     const unsigned nwords = ((unsigned)P.ncell + 31u) / 32u;
     // the scan's list and the inner loop's columns are never live together
     int *const slist = reinterpret_cast<int *>(inner_smem) + wid * SCAN_LIST;
-    int nit = 1;
     if (blockIdx.x == 0 && threadIdx.x < 6) W.counts[threadIdx.x] = 0;
     barrier();
-    for (;;) {
+    for (int nit = 1;; ++nit) {
         int *const cnt = W.counts + 3 * (nit & 1), *const other = W.counts + 3 * (~nit & 1);
         for (int col = 0; col < 3; ++col) {
             int *const work = W.work + col * W.wstride;
-            scan_phase<NP, D>(P, F, dt, W.cmask + (size_t)col * nwords, W.dirty, work, cnt + col, nullptr, warp,
-                              nwarps, slist);
+            scan_phase<NP, D>(P, F, dt, W.cmask + (size_t)col * nwords, W.cmask + (size_t)3 * nwords, W.dirty, work,
+                              cnt + col, nullptr, warp, nwarps, slist);
+            __syncwarp();
             barrier();
             const int nwork = __ldcg(cnt + col);
             // the next sweep's lengths: last read before this sweep's first barrier
@@ -678,20 +761,76 @@ __global__ void __launch_bounds__(KS, PDAC_INNER_MINB(NP)) k_sweep_loop(Prm P, F
             if (nwork)
                 inner_team_run<NP, D, false>(P, F, dt, nit, work, nwork, W.dirty, warp, nwarps,
                                              cells_per_warp<D>(nwork, nwarps));
+            __syncwarp();
             barrier();
         }
-        const int n0 = __ldcg(cnt), n1 = __ldcg(cnt + 1), n2 = __ldcg(cnt + 2);
-        const bool conv = (long)n0 + n1 + n2 == 0;
-        if (conv || nit >= maxout) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
-                W.wcount[0] = n0;
-                W.wcount[1] = n1;
-                W.wcount[2] = n2;
-                *W.nit = conv ? nit : maxout + 1;
+        if (sweep_ends(W, cnt, nit, maxout)) return;
+    }
+}
+
+// On one thread-block cluster, for small 2D meshes, whose phases hold a few
+// hundred cells: what bounds a phase is the number of dependent trips to L2
+// on its way (0.3 to 0.5 us each; the inner loop itself is one or three
+// iterations of 0.75 us).  So a block keeps the unconverged cells of its own
+// words in shared memory -- no global list, count or second barrier between
+// test and inner loop -- and the words of a neighbourhood are dealt out to
+// different blocks: of every CLUSTER consecutive words each block has one,
+// turned by 7 from one group to the next, so that a front running down the
+// columns of a mesh of any width meets all blocks.  The hardware schedules a
+// cluster's blocks together, so any number of such launches may share the
+// device.  Ten steps of 128 x 192: 35.0 ms with a common worklist, 32.2 here.
+// Eight warps a block hide one another's trips where a phase has more cells
+// than the cluster has warps: five steps of 251 x 383, 38.0 ms with four
+// (36.3 with the common worklist), 30.8 with eight; 128 x 192 the same.
+constexpr int CLUSTER = 16, KC = 256;  // blocks; their threads, each with a word of the active set at most
+template <int NP>
+__host__ __device__ constexpr size_t cluster_smem_bytes() {
+    return sweep_smem_bytes<NP>(KC) + KC * 11 * sizeof(int);
+}
+template <int NP>
+__global__ void __launch_bounds__(KC, 1) k_sweep_cluster(Prm P, Fld F, double dt, SweepWork W, int maxout) {
+    extern __shared__ __align__(16) double inner_smem[];
+    __shared__ int nmine, base;
+    int *const mine = reinterpret_cast<int *>(reinterpret_cast<char *>(inner_smem) + sweep_smem_bytes<NP>(KC));
+    const unsigned lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const unsigned nwords = ((unsigned)P.ncell + 31u) / 32u, b = blockIdx.x;
+    int *const slist = reinterpret_cast<int *>(inner_smem) + wid * SCAN_LIST;
+    auto barrier = [] {
+        __syncwarp();
+        cooperative_groups::this_cluster().sync();
+    };
+    if (b == 0 && threadIdx.x < 6) W.counts[threadIdx.x] = 0;
+    if (threadIdx.x == 0) nmine = 0;
+    barrier();
+    for (int nit = 1;; ++nit) {
+        int *const cnt = W.counts + 3 * (nit & 1), *const other = W.counts + 3 * (~nit & 1);
+        for (int col = 0; col < 3; ++col) {
+            const unsigned g = wid + KC / 32 * lane;  // this thread's group of CLUSTER words
+            scan_round<NP, 2, true>(P, F, dt, W.cmask + (size_t)col * nwords, W.cmask + (size_t)3 * nwords, W.dirty,
+                                    g * CLUSTER + ((b + 7u * g) & (CLUSTER - 1u)), nwords, slist,
+                                    [&](unsigned um, unsigned ln, bool u, int e) {
+                                        int at = 0;
+                                        if (ln == 0) at = atomicAdd(&nmine, __popc(um));
+                                        at = __shfl_sync(0xffffffffu, at, 0);
+                                        if (u) mine[at + __popc(um & ((1u << ln) - 1u))] = e;
+                                    });
+            __syncthreads();
+            const int nwork = nmine;
+            if (threadIdx.x == 0 && nwork) base = atomicAdd(cnt + col, nwork);
+            if (nit == maxout && nwork) {  // the cells a loop without convergence reports
+                __syncthreads();
+                for (int q = threadIdx.x; q < nwork; q += KC) W.work[col * W.wstride + base + q] = mine[q];
             }
-            return;
+            // the next sweep's lengths: last read before this sweep's first barrier
+            if (col == 1 && b == 0 && threadIdx.x < 3) other[threadIdx.x] = 0;
+            if (nwork)
+                inner_team_run<NP, 2, false>(P, F, dt, nit, mine, nwork, W.dirty, wid, KC / 32,
+                                             cells_per_warp<2>(nwork, KC / 32));
+            __syncthreads();  // the list and its length are done with
+            if (threadIdx.x == 0) nmine = 0;
+            barrier();
         }
-        ++nit;
+        if (sweep_ends(W, cnt, nit, maxout)) return;
     }
 }
 

@@ -6,7 +6,8 @@ takes the launches.  Every form runs the same cells in the same colour order,
 so after each step the sweep counts, the unconverged cells and every state
 array are equal, bit for bit.  The meshes put the active set's last word, the
 colours' first cells and the worklists (shorter and longer than one round of
-the warps) at odd places; the last 2D one lies above the cluster's limit.
+the warps) at odd places; 364 x 361 lies above the cluster's limit and 359 x
+363 just below it.
 """
 import numpy as np
 import pytest
@@ -15,6 +16,7 @@ pytestmark = pytest.mark.gpu
 
 MESHES = [
     ("2d", 5, 7, 1, 2), ("2d", 13, 33, 1, 2), ("2d", 31, 65, 2, 3), ("2d", 97, 129, 3, 2), ("2d", 364, 361, 2, 2),
+    ("2d", 41, 50, 4, 2), ("2d", 37, 43, 5, 2), ("2d", 359, 363, 1, 2),
     ("3d", (6, 5, 7), None, 1, 2), ("3d", (11, 13, 9), None, 3, 3), ("3d", (33, 31, 35), None, 2, 3),
     ("3d", (17, 16, 15), None, 4, 2), ("3d", (20, 18, 17), None, 5, 2), ("3d", (66, 61, 70), None, 3, 2),
 ]
@@ -54,6 +56,27 @@ def test_sweep_loop_forms_agree(kind, a, b, ns, steps):
             assert np.array_equal(e.unconverged_cells(), cells)
     for e in (one, launches, grid):
         e.close()
+
+
+@pytest.mark.parametrize("kind,a,b,ns", [("2d", 97, 129, 2), ("2d", 23, 31, 5), ("3d", (33, 31, 35), None, 2)])
+def test_forms_agree_on_a_loop_that_ends_unconverged(kind, a, b, ns):
+    from pdac_b200.engine import Engine
+    from pdac_b200.setup_state import Case
+    deck = _deck(kind, a, b, ns)
+    deck.set("numeric", maxout=3)
+    deck.set("control", cstop=0)
+    case = Case(deck)
+    one, launches = Engine(case), Engine(case)
+    launches.reset_stats(True)
+    for sweep in (1, 2):
+        assert one.step(sweep) == launches.step(sweep) == 4
+        cells = launches.unconverged_cells()
+        assert cells.size > 0 and np.array_equal(one.unconverged_cells(), cells)
+        got, want = one.download(), launches.download()
+        for name in want:
+            assert np.array_equal(got[name], want[name]), f"step {sweep}: {name}"
+    one.close()
+    launches.close()
 
 
 def test_two_threads_step_their_own_contexts():
