@@ -66,7 +66,7 @@ struct pdac_ctx {
     long graph_gen = 0;  // bumped whenever captured launch shapes go stale (put_tuning)
     long long step_launches = 0;
     int *d_status = nullptr, *h_status = nullptr;
-    unsigned *d_dirty = nullptr;                 // corrector active set, one bit per cell
+    unsigned *d_dirty = nullptr;                 // corrector active set, one bit per cell; then as many for its expected long cells
     unsigned *d_cmask = nullptr;                 // fluid cells per colour, the active set's words
     // 3D with MUSCL: the mask of simple cells (P.simple) and the list of the
     // other fluid cells
@@ -709,7 +709,7 @@ static cudaError_t launch_sweep_loop_np(pdac_ctx *ctx, double dt, cudaStream_t s
 }
 
 static cudaError_t launch_sweep_loop(pdac_ctx *ctx, double dt, cudaStream_t st) {
-    const pdac::SweepWork W{ctx->d_wcount, ctx->d_wcount + 9, ctx->d_work, ctx->d_dirty, ctx->d_cmask, ctx->d_nit, ctx->work_stride};
+    const pdac::SweepWork W{ctx->d_wcount, reinterpret_cast<unsigned long long *>(ctx->d_wcount + 10), ctx->d_work, ctx->d_dirty, ctx->d_cmask, ctx->d_nit, ctx->work_stride};
     switch (ctx->nph) {
         case 2: return launch_sweep_loop_np<2>(ctx, dt, st, W);
         case 3: return launch_sweep_loop_np<3>(ctx, dt, st, W);
@@ -1000,8 +1000,8 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     CK(cudaMallocHost(&ctx->h_nonfinite, sizeof(int)));
     CK(cudaMalloc(&ctx->d_status, 4 * sizeof(int)));
     CK(cudaMallocHost(&ctx->h_status, 4 * sizeof(int)));
-    CK(cudaMalloc(&ctx->d_wcount, 16 * sizeof(int)));
-    CK(cudaMalloc(&ctx->d_dirty, ((size_t)n + 31) / 32 * sizeof(unsigned)));
+    CK(cudaMalloc(&ctx->d_wcount, 24 * sizeof(int)));
+    CK(cudaMalloc(&ctx->d_dirty, (size_t)2 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
     CK(cudaMalloc(&ctx->d_cmask, (size_t)4 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
     if (ctx->d3 && P.muscl > 0) {
         CK(cudaMalloc(&ctx->d_simple, ((size_t)n + 31) / 32 * sizeof(unsigned)));
@@ -1696,7 +1696,7 @@ int pdac_gpu_iter(pdac_ctx *ctx, double dt, int *nit_out) {
     ctx->launches += 2;
     CK(cudaGetLastError());
     // every cell is tested in the first sweep
-    CK(cudaMemsetAsync(ctx->d_dirty, 0xff, (n + 31) / 32 * sizeof(unsigned), st));
+    CK(cudaMemsetAsync(ctx->d_dirty, 0xff, 2 * ((n + 31) / 32) * sizeof(unsigned), st));
     int nit;
     const bool explicit_modes = !ctx->cfg.implicit_fluxes && !ctx->cfg.implicit_enthalpy;
     std::unique_lock<std::mutex> lk;
@@ -1804,7 +1804,7 @@ int pdac_gpu_unconverged_cells(pdac_ctx *ctx, int *ijk, long *n_inout) {
         if (cnt[c]) CK(cudaMemcpy(ijk + at, ctx->d_work + c * ctx->work_stride, cnt[c] * sizeof(int), cudaMemcpyDeviceToHost));
         at += cnt[c];
     }
-    for (long q = 0; q < total; ++q) ijk[q] &= 0x7fffffff;  // without the plain bit of a worklist entry
+    for (long q = 0; q < total; ++q) ijk[q] &= pdac::ENTRY_LONG - 1;  // without a worklist entry's marks
     std::sort(ijk, ijk + total);
     *n_inout = total;
     return PDAC_OK;
@@ -3086,7 +3086,7 @@ static int enqueue_step_pre(pdac_ctx *ctx, double dt, cudaStream_t st) {
         PHASE_LAUNCH(nph, pdac::k_predictor2d, blocks(n), TPB, st, ctx->P, F, dt);
         pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);
     }
-    CK(cudaMemsetAsync(ctx->d_dirty, 0xff, (n + 31) / 32 * sizeof(unsigned), st));
+    CK(cudaMemsetAsync(ctx->d_dirty, 0xff, 2 * ((n + 31) / 32) * sizeof(unsigned), st));
     pdac::k_set_int<<<1, 1, 0, st>>>(ctx->d_nit, 1);
     ctx->launches += 3;
     CK(cudaGetLastError());

@@ -270,7 +270,14 @@ __host__ __device__ constexpr size_t sweep_smem_bytes(int threads = KS) {
 // whose face stencils meet no wall and stay two cells from the mesh's ends
 // (k_colour_masks), so that no flag need be read to know its neighbours --
 // one dependent trip to L2 less before the values themselves are asked for.
-__device__ __forceinline__ int entry_cell(int e) { return e & 0x7fffffff; }
+// The next bit is set for a cell that is expected to take several iterations:
+// about half the cells take one and half take three, and a cell that took one
+// the last time takes three the next, and the other way round (95 of 100 on
+// the plumes).  The bits of the expectation follow the active set's words; it
+// decides only which cells share a warp.
+constexpr int ENTRY_LONG = 1 << 30;
+__device__ __forceinline__ int entry_cell(int e) { return e & (ENTRY_LONG - 1); }
+__device__ __forceinline__ unsigned *expect_long(const Prm &P, unsigned *dirty) { return dirty + ((unsigned)P.ncell + 31u) / 32u; }
 
 // The inner loop of worklist entry e (outer sweep nit, 1-based) by the team of
 // lanes tb .. tb + T - 1 of this warp (lane q of the team owns face q); kcols
@@ -285,7 +292,7 @@ __device__ __forceinline__ int entry_cell(int e) { return e & 0x7fffffff; }
 // operations, 76-cycle reciprocals and 127-cycle quotients, measured) and the
 // instructions of a warp's teams when they diverge; hence one code path for
 // all faces, velocity signs and bracketing states.
-template <int NP, int D, bool RO>
+template <int NP, int D, bool RO, bool SPLIT>
 __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, double dt, int nit, int e, bool live,
                                                 unsigned *dirty, int q, int tb, double *kcols, double *dcols) {
     constexpr unsigned full = 0xffffffffu;
@@ -474,6 +481,11 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
                 for (int is = 1; is <= ns; ++is) F.rlk[(is - 1) * n + c] = rlk[is - 1];
                 F.abeta[c] = abeta;
                 mark_dirty(dirty, c);
+                if (SPLIT && nit > 1 && (loop == 1) != ((e & ENTRY_LONG) != 0)) {
+                    unsigned *const w = expect_long(P, dirty) + (c >> 5);
+                    if (loop == 1) atomicOr(w, 1u << (c & 31));
+                    else atomicAnd(w, ~(1u << (c & 31)));
+                }
             }
             live = false;
         }
@@ -484,9 +496,16 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
 // the inner loop of the worklist's nwork cells (outer sweep nit, 1-based) by
 // the warps warp, warp + nwarps, ... of the launch, cpw <= teams per warp
 // cells at a time; every lane of a warp makes the call.  RO as in ldro.
-template <int NP, int D, bool RO>
+// SPLIT: the first nlong entries from the list's front are the expected long
+// ones, the others stand backwards from entry last; no warp holds both, so
+// that a warp of short cells ends after one iteration (a warp of five mixed
+// ones hardly ever does).  Four steps of 128 x 128 x 96 with four phases 72.0
+// -> 69.3 ms; three of its hills with six 95.8 -> 90.9; four of 256 x 256 x
+// 192 432 -> 424, with every long cell first 443.
+template <int NP, int D, bool RO, bool SPLIT = false>
 __device__ __forceinline__ void inner_team_run(const Prm &P, const Fld &F, double dt, int nit, const int *list,
-                                               int nwork, unsigned *dirty, int warp, int nwarps, int cpw) {
+                                               int nwork, unsigned *dirty, int warp, int nwarps, int cpw, int nlong = 0,
+                                               int last = 0) {
     constexpr int T = D == 3 ? 6 : 4;    // lanes per cell
     constexpr int TPW = 32 / T;          // teams per warp (3D: 5, lanes 30 and 31 own no face)
     const int lane = threadIdx.x & 31, tw = lane / T;
@@ -495,9 +514,48 @@ __device__ __forceinline__ void inner_team_run(const Prm &P, const Fld &F, doubl
     // every KS threads have columns of their own: [FaceK rows][KS], [3 NC][KS]
     double *const kcols = inner_smem + threadIdx.x / KS * (inner_smem_bytes<NP>() / sizeof(double));
     double *const dcols = kcols + inner_face_rows<NP>() * KS;
-    for (int w0 = warp * cpw; w0 < nwork; w0 += nwarps * cpw) {
-        const bool live = tw < TPW && tw < cpw && w0 + tw < nwork;
-        inner_team_cell<NP, D, RO>(P, F, dt, nit, list[live ? w0 + tw : w0], live, dirty, q, tb, kcols, dcols);
+    if constexpr (SPLIT) {
+        if (nwork <= nwarps) {  // a cell per warp: nothing to keep apart
+            if (warp < nwork)
+                inner_team_cell<NP, D, RO, false>(P, F, dt, nit, list[warp < nlong ? warp : last - (warp - nlong)],
+                                                  tw == 0, dirty, q, tb, kcols, dcols);
+            return;
+        }
+        // a unit is a warp's cells.  In a few rounds every warp takes long and
+        // short ones in turn, those past the last long unit short ones first.
+        // In many rounds what counts is that the cells at work at one time are
+        // near each other in the mesh: long and short units in one sequence,
+        // (u * rate) >> 32 of its first u long.
+        const int nshort = nwork - nlong, ulong = (nlong + cpw - 1) / cpw, units = ulong + (nshort + cpw - 1) / cpw;
+        const bool many = units > 8 * nwarps;
+        const unsigned long long rate = many ? (((unsigned long long)ulong << 32) + units - 1) / units : 0;
+        int l = warp, s = warp - ulong % nwarps;
+        if (s < 0) s += nwarps;
+        bool turn = false;
+        for (int u = warp; many ? u < units : l < ulong || s < units - ulong; u += nwarps) {
+            bool sh;
+            int x;
+            if (many) {
+                const int l0 = (int)(u * rate >> 32);
+                sh = (int)((u + 1) * rate >> 32) == l0;
+                x = sh ? u - l0 : l0;
+            } else {
+                sh = l >= ulong || (turn && s < units - ulong);
+                x = sh ? s : l;
+                if (sh) s += nwarps;
+                else l += nwarps;
+                turn = !sh;
+            }
+            const int w0 = x * cpw, m = sh ? nshort : nlong;
+            const bool live = tw < TPW && tw < cpw && w0 + tw < m;
+            const int at = live ? w0 + tw : w0;
+            inner_team_cell<NP, D, RO, true>(P, F, dt, nit, list[sh ? last - at : at], live, dirty, q, tb, kcols, dcols);
+        }
+    } else {
+        for (int w0 = warp * cpw; w0 < nwork; w0 += nwarps * cpw) {
+            const bool live = tw < TPW && tw < cpw && w0 + tw < nwork;
+            inner_team_cell<NP, D, RO, false>(P, F, dt, nit, list[live ? w0 + tw : w0], live, dirty, q, tb, kcols, dcols);
+        }
     }
 }
 
@@ -640,11 +698,12 @@ constexpr int SCAN_LIST = 32 * 11;  // a colour has at most 11 cells in a word o
 template <int NP, int D, bool EAGER, class PUT>
 __device__ __forceinline__ int scan_round(const Prm &P, const Fld &F, double dt, const unsigned *cmask,
                                           const unsigned *plain, unsigned *dirty, unsigned t, unsigned nwords,
-                                          int *slist, PUT put) {
+                                          int *slist, PUT put, const unsigned *expect = nullptr) {
     constexpr unsigned full = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
-    unsigned w = 0, pl = 0;
+    unsigned w = 0, pl = 0, lg = 0;
     if (t < nwords) {
+        if (expect) lg = __ldcg(expect + t);
         w = __ldcg(dirty + t) & __ldg(cmask + t);
         pl = __ldg(plain + t);
         if (w) atomicAnd(dirty + t, ~w);
@@ -660,7 +719,7 @@ __device__ __forceinline__ int scan_round(const Prm &P, const Fld &F, double dt,
     if (total == 0) return 0;
     for (int off = incl - mine; w; w &= w - 1u) {
         const int b = __ffs(w) - 1;
-        slist[off++] = (int)(32u * t + (unsigned)b | (pl >> b & 1u) << 31);
+        slist[off++] = (int)(32u * t + (unsigned)b | (pl >> b & 1u) << 31 | (lg >> b & 1u) << 30);
     }
     __syncwarp();
     for (int base = 0; base < total; base += 32) {
@@ -678,24 +737,20 @@ __device__ __forceinline__ int scan_round(const Prm &P, const Fld &F, double dt,
     return total;
 }
 
-template <int NP, int D>
-__device__ __forceinline__ void scan_phase(const Prm &P, const Fld &F, double dt, const unsigned *cmask,
-                                           const unsigned *plain, unsigned *dirty, int *work, int *count, int *tested,
-                                           unsigned warp, unsigned nwarps, int *slist) {
+// a phase's test by all warps of a grid: put as scan_round's; returns the
+// number of cells this warp tested
+template <int NP, int D, class PUT>
+__device__ __forceinline__ int scan_phase(const Prm &P, const Fld &F, double dt, const unsigned *cmask,
+                                          const unsigned *plain, unsigned *dirty, unsigned warp, unsigned nwarps,
+                                          int *slist, PUT put, const unsigned *expect = nullptr) {
     const unsigned lane = threadIdx.x & 31u, nwords = ((unsigned)P.ncell + 31u) / 32u;
     const unsigned gs = nwords <= 32u * nwarps ? 1u : 8u, gpi = 32u / gs;  // words per group, groups per round
     int ntest = 0;
     for (unsigned g0 = 0; (size_t)g0 * nwarps * gs < nwords; g0 += gpi) {
         const unsigned t = ((g0 + lane / gs) * nwarps + warp) * gs + lane % gs;
-        ntest += scan_round<NP, D, false>(P, F, dt, cmask, plain, dirty, t, nwords, slist,
-                                          [&](unsigned um, unsigned ln, bool u, int e) {
-                                              int at = 0;
-                                              if (ln == 0) at = atomicAdd(count, __popc(um));
-                                              at = __shfl_sync(0xffffffffu, at, 0);
-                                              if (u) work[at + __popc(um & ((1u << ln) - 1u))] = e;
-                                          });
+        ntest += scan_round<NP, D, false>(P, F, dt, cmask, plain, dirty, t, nwords, slist, put, expect);
     }
-    if (tested && lane == 0 && ntest) atomicAdd(tested, ntest);
+    return ntest;
 }
 
 template <int NP, int D>
@@ -703,7 +758,14 @@ __global__ void __launch_bounds__(TPB_RESID) k_resid_scan(Prm P, Fld F, double d
                                                           const unsigned *plain, unsigned *dirty, int *work, int *count) {
     __shared__ int slist[TPB_RESID / 32][SCAN_LIST];
     const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    scan_phase<NP, D>(P, F, dt, cmask, plain, dirty, work, count, count + 3, warp, nwarps, slist[threadIdx.x >> 5]);
+    const int ntest = scan_phase<NP, D>(P, F, dt, cmask, plain, dirty, warp, nwarps, slist[threadIdx.x >> 5],
+                                        [&](unsigned um, unsigned ln, bool u, int e) {
+                                            int at = 0;
+                                            if (ln == 0) at = atomicAdd(count, __popc(um));
+                                            at = __shfl_sync(0xffffffffu, at, 0);
+                                            if (u) work[at + __popc(um & ((1u << ln) - 1u))] = e;
+                                        });
+    if ((threadIdx.x & 31u) == 0 && ntest) atomicAdd(count + 3, ntest);
 }
 
 // The whole outer sweep loop of iter (iter.f:204-410) in one launch whose
@@ -713,7 +775,9 @@ __global__ void __launch_bounds__(TPB_RESID) k_resid_scan(Prm P, Fld F, double d
 // on counters that all threads read after the same barrier.
 struct SweepWork {
     int *wcount;      // on return: [col] worklist length of the last sweep
-    int *counts;      // two sets of three worklist lengths, for odd and even sweeps
+    // two sets of three worklist lengths, for odd and even sweeps: the
+    // expected long cells in the low half, the others in the high half
+    unsigned long long *counts;
     int *work;        // worklists, colour col at work + col * wstride
     unsigned *dirty;  // active set, one bit per cell
     const unsigned *cmask;  // the three colour masks and the plain mask
@@ -722,8 +786,9 @@ struct SweepWork {
 };
 
 // after a sweep's last barrier: its worklist lengths; true when the loop ends
-__device__ __forceinline__ bool sweep_ends(const SweepWork &W, const int *cnt, int nit, int maxout) {
-    const int n0 = __ldcg(cnt), n1 = __ldcg(cnt + 1), n2 = __ldcg(cnt + 2);
+__device__ __forceinline__ bool sweep_ends(const SweepWork &W, const unsigned long long *cnt, int nit, int maxout) {
+    auto length = [](unsigned long long v) { return (int)(v & 0xffffffffu) + (int)(v >> 32); };
+    const int n0 = length(__ldcg(cnt)), n1 = length(__ldcg(cnt + 1)), n2 = length(__ldcg(cnt + 2));
     const bool conv = (long)n0 + n1 + n2 == 0;
     if (!conv && nit < maxout) return false;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -748,19 +813,37 @@ __global__ void __launch_bounds__(KS, PDAC_INNER_MINB(NP)) k_sweep_grid(Prm P, F
     if (blockIdx.x == 0 && threadIdx.x < 6) W.counts[threadIdx.x] = 0;
     barrier();
     for (int nit = 1;; ++nit) {
-        int *const cnt = W.counts + 3 * (nit & 1), *const other = W.counts + 3 * (~nit & 1);
+        unsigned long long *const cnt = W.counts + 3 * (nit & 1), *const other = W.counts + 3 * (~nit & 1);
         for (int col = 0; col < 3; ++col) {
             int *const work = W.work + col * W.wstride;
-            scan_phase<NP, D>(P, F, dt, W.cmask + (size_t)col * nwords, W.cmask + (size_t)3 * nwords, W.dirty, work,
-                              cnt + col, nullptr, warp, nwarps, slist);
+            const int last = (int)W.wstride - 1;
+            // after the last sweep the list is read from its front
+            const bool all_long = nit == maxout;
+            scan_phase<NP, D>(P, F, dt, W.cmask + (size_t)col * nwords, W.cmask + (size_t)3 * nwords, W.dirty, warp,
+                              nwarps, slist,
+                              [&](unsigned um, unsigned ln, bool u, int e) {
+                                  const unsigned lm = __ballot_sync(0xffffffffu, u && (all_long || (e & ENTRY_LONG))), sm = um & ~lm;
+                                  unsigned long long at = 0;
+                                  if (ln == 0)
+                                      at = atomicAdd(cnt + col, (unsigned long long)__popc(sm) << 32 | (unsigned)__popc(lm));
+                                  at = __shfl_sync(0xffffffffu, at, 0);
+                                  const unsigned before = (1u << ln) - 1u;
+                                  if (lm >> ln & 1u) work[(int)(at & 0xffffffffu) + __popc(lm & before)] = e;
+                                  else if (u) work[last - (int)(at >> 32) - __popc(sm & before)] = e;
+                              },
+                              expect_long(P, W.dirty));
             __syncwarp();
             barrier();
-            const int nwork = __ldcg(cnt + col);
+            const unsigned long long lens = __ldcg(cnt + col);
+            const int nlong = (int)(lens & 0xffffffffu), nwork = nlong + (int)(lens >> 32);
             // the next sweep's lengths: last read before this sweep's first barrier
             if (col == 1 && blockIdx.x == 0 && threadIdx.x < 3) other[threadIdx.x] = 0;
-            if (nwork)
-                inner_team_run<NP, D, false>(P, F, dt, nit, work, nwork, W.dirty, warp, nwarps,
-                                             cells_per_warp<D>(nwork, nwarps));
+            if (nwork) {
+                constexpr int TPW = 32 / (D == 3 ? 6 : 4);
+                int cpw = cells_per_warp<D>(nwork, nwarps);  // a unit per warp, where they go round
+                while (cpw < TPW && (nlong + cpw - 1) / cpw + (nwork - nlong + cpw - 1) / cpw > nwarps) ++cpw;
+                inner_team_run<NP, D, false, true>(P, F, dt, nit, work, nwork, W.dirty, warp, nwarps, cpw, nlong, last);
+            }
             __syncwarp();
             barrier();
         }
@@ -803,7 +886,7 @@ __global__ void __launch_bounds__(KC, 1) k_sweep_cluster(Prm P, Fld F, double dt
     if (threadIdx.x == 0) nmine = 0;
     barrier();
     for (int nit = 1;; ++nit) {
-        int *const cnt = W.counts + 3 * (nit & 1), *const other = W.counts + 3 * (~nit & 1);
+        unsigned long long *const cnt = W.counts + 3 * (nit & 1), *const other = W.counts + 3 * (~nit & 1);
         for (int col = 0; col < 3; ++col) {
             const unsigned g = wid + KC / 32 * lane;  // this thread's group of CLUSTER words
             scan_round<NP, 2, true>(P, F, dt, W.cmask + (size_t)col * nwords, W.cmask + (size_t)3 * nwords, W.dirty,
@@ -816,7 +899,7 @@ __global__ void __launch_bounds__(KC, 1) k_sweep_cluster(Prm P, Fld F, double dt
                                     });
             __syncthreads();
             const int nwork = nmine;
-            if (threadIdx.x == 0 && nwork) base = atomicAdd(cnt + col, nwork);
+            if (threadIdx.x == 0 && nwork) base = (int)atomicAdd(cnt + col, (unsigned long long)nwork);
             if (nit == maxout && nwork) {  // the cells a loop without convergence reports
                 __syncthreads();
                 for (int q = threadIdx.x; q < nwork; q += KC) W.work[col * W.wstride + base + q] = mine[q];

@@ -58,6 +58,24 @@ def test_sweep_loop_forms_agree(kind, a, b, ns, steps):
         e.close()
 
 
+@pytest.mark.parametrize("cells_per_block", [300, 4000, 40000])
+def test_grids_of_few_blocks_agree(cells_per_block):
+    """Worklists of many rounds of a grid's warps, whose expected long and
+    short cells alternate, and of a few rounds."""
+    from pdac_b200.engine import Engine
+    from pdac_b200.setup_state import Case
+    case = Case(_deck("3d", (33, 31, 35), None, 2))
+    one, grid = Engine(case), Engine(case)
+    grid.set_tuning(dict(tile_shape=0, tile_kchunk=2, inner_grid=37, test_grid=5, coop_cells_per_block=cells_per_block))
+    for sweep in (1, 2):
+        assert one.step(sweep) == grid.step(sweep)
+        got, want = grid.download(), one.download()
+        for name in want:
+            assert np.array_equal(got[name], want[name]), f"step {sweep}: {name}"
+    one.close()
+    grid.close()
+
+
 @pytest.mark.parametrize("kind,a,b,ns", [("2d", 97, 129, 2), ("2d", 23, 31, 5), ("3d", (33, 31, 35), None, 2)])
 def test_forms_agree_on_a_loop_that_ends_unconverged(kind, a, b, ns):
     from pdac_b200.engine import Engine
