@@ -529,7 +529,7 @@ def engine_arm(args):
         calls = max(stats["rk3_calls"], 1)
         group = max(stats["rk3_ms"], key=stats["rk3_ms"].get)
         names = {"flux": "flux passes (k_rk3_mflux, k_tilde_flux*, k_htilde_flux*)", "stage": "k_rk3_stage",
-                 "wave": "k_rk3_wave (hyperplane wavefront)", "final": "k_rk3_final_rhs/phys/solve"}
+                 "wave": "k_rk3_wave_pre/tile/post (gas-enthalpy wavefront)", "final": "k_rk3_final_rhs/phys/solve"}
         gbytes = roofline.rk3_group_bytes(case.nsolid, case.ngas, dims, nfluid)
         kname = names[group]
         bytes_per_launch = gbytes[group]
@@ -549,7 +549,7 @@ def engine_arm(args):
             kname, kms = "k_inner_team", stats["inner_ms"]
             kbytes = roofline.inner_bytes(case.nsolid, case.ngas, dims, unconv)
         else:
-            kname, kms = "k_resid_test", stats["resid_ms"]
+            kname, kms = "k_resid_scan", stats["resid_ms"]
             kbytes = roofline.resid_bytes(case.nsolid, dims, tested - unconv, unconv, ncell, phases)
         bytes_per_launch = kbytes / phases
         avg_launch_s = kms / 1000.0 / phases

@@ -5,8 +5,9 @@ a batch (``pdac_gpu_batch_*`` in include/pdac_gpu.h) steps many engine
 contexts at once, each on its own stream, so that small 2D members, which
 fill a few percent of a B200 each, run side by side.  A member computes
 exactly what it computes alone: in the batch its sweep loop and wavefront
-take their multi-launch forms instead of one cooperative launch, with the
-same arithmetic, so a member of a batch produces the same bits as the same
+run on one cluster or one block where they do alone, and in their
+multi-launch forms instead of one cooperative launch, with the same
+arithmetic, so a member of a batch produces the same bits as the same
 deck run alone.
 
 :func:`member_decks` draws the members of the 2D cylindrical ensemble: the
