@@ -43,7 +43,7 @@ struct pdac_ctx {
     double *d_vfact = nullptr, *d_vfact0 = nullptr;
     double *d_app0u = nullptr, *d_app0v = nullptr, *d_app0w = nullptr;
     double *d_partial = nullptr;
-    double *d_fk = nullptr;  // face records of iter where mf cannot hold them
+    double *d_fk = nullptr;  // face records of iter (F.fk)
     int nvent = 0;
     std::string err;
     cudaEvent_t ev[16];
@@ -1094,17 +1094,13 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     F.counters = ctx->d_counters;
     // the face records of iter (solve.cuh), for the phase counts whose inner
     // loop reads them and while tilde, which rewrites the terms they are made
-    // of, does not run inside the sweeps.  In 3D they take the place of the
-    // momentum fluxes and stresses (mf and vis, neighbours in the arena),
-    // which tilde is done with when iter starts and rewrites before it reads
-    // them again; where they do not fit there (six phases) and in 2D they get
-    // memory of their own, and if there is none left the inner loop forms the
-    // terms itself
+    // of, does not run inside the sweeps.  Memory of their own: every array of
+    // the arena can be read by name after any call (pdac_gpu_get_array).  If
+    // there is none left the inner loop forms the terms itself
     F.fk = nullptr;
     if (!t1 && !cfg->implicit_fluxes && (ctx->nph <= 4 || ctx->nph == 6)) {
         const size_t need = (size_t)pdac::face_rec(ctx->nph) * (ctx->d3 ? 3 : 2) * n;
-        if (ctx->d3 && need <= stride * 12 * ctx->nph) F.fk = F.mf;
-        else if (cudaMalloc(&ctx->d_fk, need * sizeof(double)) == cudaSuccess) F.fk = ctx->d_fk;
+        if (cudaMalloc(&ctx->d_fk, need * sizeof(double)) == cudaSuccess) F.fk = ctx->d_fk;
         else (void)cudaGetLastError();
     }
     if (lt) {
