@@ -419,6 +419,18 @@ int pdac_gpu_elapsed(pdac_ctx *ctx, int a, int b, double *ms);
 int pdac_gpu_autotune(pdac_ctx *ctx, const char *cache_path, int *out, int nout);
 int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin);
 
+/* The forms a context's kernels run in, which it chooses by its mesh and the
+ * device; none of them changes a result.  Test and debugging aid.
+ * pdac_gpu_set_forms (nin >= 1; PDAC_ERR_ARG for a form the context cannot
+ * run in):
+ *   [0] the corrector's face records: 0 = when they leave as much device
+ *       memory free as the context's fields take (they are also given back
+ *       to an allocation of this library that does not fit otherwise),
+ *       1 = none.
+ * pdac_gpu_get_forms (nout >= 1): [0] 1 if the context holds face records.  */
+int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin);
+int pdac_gpu_get_forms(pdac_ctx *ctx, int *out, int nout);
+
 /* ---- ensembles of independent runs ------------------------------------ */
 /* No counterpart in the reference, which runs one domain per job (an
  * ensemble there is many jobs).  A batch advances many contexts (members:

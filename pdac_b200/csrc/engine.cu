@@ -12,6 +12,7 @@
 #include <string>
 #include <vector>
 #include <algorithm>
+#include <atomic>
 #include <condition_variable>
 #include <mutex>
 #include <thread>
@@ -43,7 +44,15 @@ struct pdac_ctx {
     double *d_vfact = nullptr, *d_vfact0 = nullptr;
     double *d_app0u = nullptr, *d_app0v = nullptr, *d_app0w = nullptr;
     double *d_partial = nullptr;
-    double *d_fk = nullptr;  // face records of iter (F.fk)
+    // face records of iter: their memory, which another context's allocation
+    // may take back between two calls (free_records; F.fk is set from it
+    // when a call that reads them starts), their size (0: this context's inner
+    // loop reads none) and whether they are switched off (pdac_gpu_set_forms)
+    double *d_fk = nullptr;
+    size_t fk_doubles = 0;
+    bool fk_off = false;
+    std::mutex fk_mu;  // held while kernels that read the records may run
+    int dev = 0;       // the device the context was created on
     int nvent = 0;
     std::string err;
     cudaEvent_t ev[16];
@@ -63,7 +72,11 @@ struct pdac_ctx {
     // failures of ftem, non-finite flag] read back once per step
     cudaGraph_t step_graph = nullptr;
     cudaGraphExec_t step_exec = nullptr;
-    long graph_gen = 0;  // bumped whenever captured launch shapes go stale (put_tuning)
+    // bumped whenever what the captured graphs hold by value goes stale (launch
+    // shapes, the records' address); the generations it_exec and step_exec were
+    // built at
+    std::atomic<long> graph_gen{0};
+    long it_gen = -1, step_gen = -1;
     long long step_launches = 0;
     int *d_status = nullptr, *h_status = nullptr;
     unsigned *d_dirty = nullptr;                 // corrector active set, one bit per cell; then as many for its expected long cells
@@ -248,6 +261,74 @@ RestCells rest_cells(const pdac_ctx *c) {
     } while (0)
 
 inline int blocks(long n, int tpb = TPB) { return (int)((n + tpb - 1) / tpb); }
+
+// ---- device memory ---------------------------------------------------------
+// The face records of iter (F.fk, solve.cuh) only save time: without them the
+// inner loop gathers the same terms, with the same results (four steps with
+// and without them: 128 x 128 x 96 with three phases 47.3 / 50.6 ms, with four
+// 68.0 / 78.5, its hills with six 120.5 / 142.6, 256 x 256 x 192 with four 407 /
+// 468).  A context takes them last in create, when they leave at least as much
+// memory free as its fields take, and any allocation of this library that does
+// not fit takes them back, from every context of the device, so that the
+// meshes, the number of contexts and the autotuner's copy that fit without
+// them still do.
+std::mutex g_records_mu;             // guards the list; taken before any context's fk_mu
+std::vector<pdac_ctx *> g_records;   // the contexts that hold records
+
+// frees the records of the contexts that pick accepts; waits for calls that
+// read them.  True if there were any
+template <class Pick>
+bool free_records(Pick pick) {
+    std::lock_guard<std::mutex> list(g_records_mu);
+    const size_t before = g_records.size();
+    g_records.erase(std::remove_if(g_records.begin(), g_records.end(),
+                                   [&](pdac_ctx *c) {
+                                       if (!pick(c)) return false;
+                                       std::lock_guard<std::mutex> lk(c->fk_mu);
+                                       cudaFree(c->d_fk);
+                                       c->d_fk = nullptr;
+                                       c->graph_gen++;
+                                       return true;
+                                   }),
+                    g_records.end());
+    return g_records.size() != before;
+}
+
+template <class T>
+cudaError_t dev_malloc(T **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    int dev = 0;
+    if (e == cudaErrorMemoryAllocation && cudaGetDevice(&dev) == cudaSuccess && free_records([dev](pdac_ctx *c) { return c->dev == dev; })) {
+        (void)cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+// the context's records, if they are wanted and there is room for them
+void take_records(pdac_ctx *ctx) {
+    std::lock_guard<std::mutex> list(g_records_mu);
+    std::lock_guard<std::mutex> lk(ctx->fk_mu);
+    if (ctx->d_fk || !ctx->fk_doubles || ctx->fk_off) return;
+    const size_t need = ctx->fk_doubles * sizeof(double);
+    size_t avail = 0, total = 0;
+    if (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail < need + ctx->arena_doubles * sizeof(double) ||
+        cudaMalloc(&ctx->d_fk, need) != cudaSuccess) {
+        (void)cudaGetLastError();
+        ctx->d_fk = nullptr;
+        return;
+    }
+    ctx->graph_gen++;
+    g_records.push_back(ctx);
+}
+
+// held by a call from before it launches kernels that read the records until
+// its stream is idle
+std::unique_lock<std::mutex> hold_records(pdac_ctx *ctx) {
+    std::unique_lock<std::mutex> lk(ctx->fk_mu);
+    ctx->F.fk = ctx->d_fk;
+    return lk;
+}
 
 // launch a kernel template instantiated for the run's phase count (gas +
 // solid classes): 2, 3, 4 and 6 phases have register-resident phase systems,
@@ -649,14 +730,14 @@ int setup_wave(pdac_ctx *ctx, const int *flag) {
         if (pos_of[c - nx * ny] >= 0) m |= pdac::WC_B;
         code[pos_of[c]] = (unsigned char)m;
     });
-    CK(cudaMalloc(&ctx->d_wave_idx, (order.size() + pos_of.size()) * sizeof(int) + code.size()));
+    CK(dev_malloc(&ctx->d_wave_idx, (order.size() + pos_of.size()) * sizeof(int) + code.size()));
     int *o = ctx->d_wave_idx, *po = o + order.size();
     unsigned char *cd = reinterpret_cast<unsigned char *>(po + pos_of.size());
     CK(cudaMemcpy(o, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(po, pos_of.data(), pos_of.size() * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(cd, code.data(), code.size(), cudaMemcpyHostToDevice));
     const size_t nrec = (size_t)(pdac::WR_YG + ctx->ng) + 1;  // the fields and pnew
-    CK(cudaMalloc(&ctx->d_wave_rec, nrec * np * sizeof(double)));
+    CK(dev_malloc(&ctx->d_wave_rec, nrec * np * sizeof(double)));
     W.order = o;
     W.pos_of = po;
     W.code = cd;
@@ -797,6 +878,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     }
     pdac_ctx *ctx = new pdac_ctx();
     ctx->cfg = *cfg;
+    CK(cudaGetDevice(&ctx->dev));
     ctx->d3 = cfg->job_type == 3;
     ctx->nx = cfg->nx; ctx->ny = ctx->d3 ? cfg->ny : 1; ctx->nz = cfg->nz;
     ctx->ncell = ctx->nx * ctx->ny * ctx->nz;
@@ -873,7 +955,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
                                                &hx, &hy, &hz};
     size_t mtot = 0;
     for (auto *v : mets) mtot += v->size();
-    CK(cudaMalloc(&ctx->metric, mtot * sizeof(double)));
+    CK(dev_malloc(&ctx->metric, mtot * sizeof(double)));
     size_t off = 0;
     std::vector<const double *> mp;
     for (auto *v : mets) {
@@ -893,7 +975,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
         hf.reserve(ftot);
         for (int q : qs)
             for (double v : *mets[q]) hf.push_back((float)v);
-        CK(cudaMalloc(&ctx->metric_f, ftot * sizeof(float)));
+        CK(dev_malloc(&ctx->metric_f, ftot * sizeof(float)));
         CK(cudaMemcpy(ctx->metric_f, hf.data(), ftot * sizeof(float), cudaMemcpyHostToDevice));
         const float *fp[11];
         size_t fo = 0;
@@ -901,7 +983,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
         P.dxf = fp[0]; P.dyf = fp[1]; P.dzf = fp[2]; P.indxf = fp[3]; P.indyf = fp[4]; P.indzf = fp[5];
         P.hxf = fp[6]; P.hyf = fp[7]; P.hzf = fp[8]; P.rf = fp[9]; P.rbf = fp[10];
     }
-    CK(cudaMalloc(&ctx->d_flag, n * sizeof(int)));
+    CK(dev_malloc(&ctx->d_flag, n * sizeof(int)));
     CK(cudaMemcpy(ctx->d_flag, cfg->flag, n * sizeof(int), cudaMemcpyHostToDevice));
     P.flag = ctx->d_flag;
     // immersed boundaries: the tables and coordinates (read-only) and the
@@ -948,12 +1030,12 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
             }
             dofs += m + 5;
         }
-        CK(cudaMalloc(&ctx->d_ibint, hint.size() * sizeof(int)));
+        CK(dev_malloc(&ctx->d_ibint, hint.size() * sizeof(int)));
         CK(cudaMemcpy(ctx->d_ibint, hint.data(), hint.size() * sizeof(int), cudaMemcpyHostToDevice));
-        CK(cudaMalloc(&ctx->d_ibdbl, hdbl.size() * sizeof(double)));
+        CK(dev_malloc(&ctx->d_ibdbl, hdbl.size() * sizeof(double)));
         CK(cudaMemcpy(ctx->d_ibdbl, hdbl.data(), hdbl.size() * sizeof(double), cudaMemcpyHostToDevice));
         ctx->ibstate_doubles = (size_t)ctx->nph * (nfp[0] + nfp[1] + nfp[2]) + (size_t)n;
-        CK(cudaMalloc(&ctx->d_ibstate, ctx->ibstate_doubles * sizeof(double)));
+        CK(dev_malloc(&ctx->d_ibstate, ctx->ibstate_doubles * sizeof(double)));
         CK(cudaMemset(ctx->d_ibstate, 0, ctx->ibstate_doubles * sizeof(double)));
         P.ib_faces = ctx->d_ibint;
         P.ib_ivf = ctx->d_ibdbl;
@@ -975,15 +1057,15 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
         std::vector<int> items;
         boundary_levels(cfg, items, ctx->blevel);
         if (!items.empty()) {
-            CK(cudaMalloc(&ctx->d_bitems, items.size() * sizeof(int)));
+            CK(dev_malloc(&ctx->d_bitems, items.size() * sizeof(int)));
             CK(cudaMemcpy(ctx->d_bitems, items.data(), items.size() * sizeof(int), cudaMemcpyHostToDevice));
         }
     }
     ctx->nvent = cfg->nvent;
     int nv = std::max(1, cfg->nvent);
-    CK(cudaMalloc(&ctx->d_vent, nv * sizeof(int)));
-    CK(cudaMalloc(&ctx->d_vfact, nv * sizeof(double)));
-    CK(cudaMalloc(&ctx->d_vfact0, nv * sizeof(double)));
+    CK(dev_malloc(&ctx->d_vent, nv * sizeof(int)));
+    CK(dev_malloc(&ctx->d_vfact, nv * sizeof(double)));
+    CK(dev_malloc(&ctx->d_vfact0, nv * sizeof(double)));
     if (cfg->nvent > 0) {
         CK(cudaMemcpy(ctx->d_vent, cfg->vent_ijk, cfg->nvent * sizeof(int), cudaMemcpyHostToDevice));
         // vent.f:176-178 initialises fact = 1 and fact0 = 0; random_switch
@@ -995,23 +1077,23 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     // a colour phase holds at most ceil(nx / 3) * ny * nz cells: for fixed
     // (j, k), (i + j + k) mod 3 takes one value on every third i
     ctx->work_stride = ((long)((ctx->nx + 2) / 3) * ctx->ny * ctx->nz + 63) / 64 * 64;
-    CK(cudaMalloc(&ctx->d_work, (size_t)3 * ctx->work_stride * sizeof(int)));
-    CK(cudaMalloc(&ctx->d_nonfinite, sizeof(int)));
+    CK(dev_malloc(&ctx->d_work, (size_t)3 * ctx->work_stride * sizeof(int)));
+    CK(dev_malloc(&ctx->d_nonfinite, sizeof(int)));
     CK(cudaMallocHost(&ctx->h_nonfinite, sizeof(int)));
-    CK(cudaMalloc(&ctx->d_status, 4 * sizeof(int)));
+    CK(dev_malloc(&ctx->d_status, 4 * sizeof(int)));
     CK(cudaMallocHost(&ctx->h_status, 4 * sizeof(int)));
-    CK(cudaMalloc(&ctx->d_wcount, 24 * sizeof(int)));
-    CK(cudaMalloc(&ctx->d_dirty, (size_t)2 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
-    CK(cudaMalloc(&ctx->d_cmask, (size_t)4 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
+    CK(dev_malloc(&ctx->d_wcount, 24 * sizeof(int)));
+    CK(dev_malloc(&ctx->d_dirty, (size_t)2 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
+    CK(dev_malloc(&ctx->d_cmask, (size_t)4 * (((size_t)n + 31) / 32) * sizeof(unsigned)));
     if (ctx->d3 && P.muscl > 0) {
-        CK(cudaMalloc(&ctx->d_simple, ((size_t)n + 31) / 32 * sizeof(unsigned)));
+        CK(dev_malloc(&ctx->d_simple, ((size_t)n + 31) / 32 * sizeof(unsigned)));
         pdac::k_simple_mask<<<blocks(((long)n + 31) / 32), TPB, 0, ctx->stream>>>(P, ctx->d_simple);
         P.simple = ctx->d_simple;
         CK(cudaMemsetAsync(ctx->d_nonfinite, 0, sizeof(int), ctx->stream));  // counts here
         pdac::k_rest_list<<<blocks(n, 256), 256, 0, ctx->stream>>>(P, ctx->d_nonfinite, nullptr);
         CK(cudaMemcpyAsync(&ctx->nrest, ctx->d_nonfinite, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        CK(cudaMalloc(&ctx->d_rest, (size_t)std::max(1, ctx->nrest) * sizeof(int)));
+        CK(dev_malloc(&ctx->d_rest, (size_t)std::max(1, ctx->nrest) * sizeof(int)));
         CK(cudaMemsetAsync(ctx->d_nonfinite, 0, sizeof(int), ctx->stream));
         pdac::k_rest_list<<<blocks(n, 256), 256, 0, ctx->stream>>>(P, ctx->d_nonfinite, ctx->d_rest);
     }
@@ -1023,9 +1105,9 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         ctx->inner_grid = nsm * 16;
     }
-    CK(cudaMalloc(&ctx->d_nit, sizeof(int)));
+    CK(dev_malloc(&ctx->d_nit, sizeof(int)));
     CK(cudaMallocHost(&ctx->h_nit, sizeof(int)));
-    CK(cudaMalloc(&ctx->d_counters, 8 * sizeof(int)));
+    CK(dev_malloc(&ctx->d_counters, 8 * sizeof(int)));
     CK(cudaMemset(ctx->d_counters, 0, 8 * sizeof(int)));
     CK(cudaMallocHost(&ctx->h_counters, 8 * sizeof(int)));
 
@@ -1080,7 +1162,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     size_t total = 0;
     for (auto &s : slots) total += stride * s.blocks;
     ctx->arena_doubles = total;
-    CK(cudaMalloc(&ctx->arena, total * sizeof(double)));
+    CK(dev_malloc(&ctx->arena, total * sizeof(double)));
     CK(cudaMemset(ctx->arena, 0, total * sizeof(double)));
     size_t o2 = 0;
     for (auto &s : slots) {
@@ -1095,14 +1177,10 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     // the face records of iter (solve.cuh), for the phase counts whose inner
     // loop reads them and while tilde, which rewrites the terms they are made
     // of, does not run inside the sweeps.  Memory of their own: every array of
-    // the arena can be read by name after any call (pdac_gpu_get_array).  If
-    // there is none left the inner loop forms the terms itself
+    // the arena can be read by name after any call (pdac_gpu_get_array)
     F.fk = nullptr;
-    if (!t1 && !cfg->implicit_fluxes && (ctx->nph <= 4 || ctx->nph == 6)) {
-        const size_t need = (size_t)pdac::face_rec(ctx->nph) * (ctx->d3 ? 3 : 2) * n;
-        if (cudaMalloc(&ctx->d_fk, need * sizeof(double)) == cudaSuccess) F.fk = ctx->d_fk;
-        else (void)cudaGetLastError();
-    }
+    if (!t1 && !cfg->implicit_fluxes && (ctx->nph <= 4 || ctx->nph == 6))
+        ctx->fk_doubles = (size_t)pdac::face_rec(ctx->nph) * (ctx->d3 ? 3 : 2) * n;
     if (lt) {
         // turbulence_setup (turbo.f:42-108): smag = lm^2 with the
         // Smagorinsky length lm = cmut delta, delta = sqrt(dz dx) in 2D and
@@ -1157,7 +1235,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
         CK(cudaMemcpy(F.delt, delt.data(), n * sizeof(double), cudaMemcpyHostToDevice));
     }
     int nq = 1 + ns + ng;
-    CK(cudaMalloc(&ctx->d_partial, (size_t)nq * 1024 * sizeof(double)));
+    CK(dev_malloc(&ctx->d_partial, (size_t)nq * 1024 * sizeof(double)));
     if (ctx->d3) CK(set_tile_attrs(ctx->P, ctx->F));
     CK(set_inner_attrs());
     if (t1) {
@@ -1190,9 +1268,9 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
             ring[b] = (dist2 > rprox2 && dist2 < rdist2) ? 1 : 0;
         }
         const size_t nm = (size_t)ntr * ns;
-        CK(cudaMalloc(&ctx->d_sinkbuf, 2 * nm * sizeof(double)));
+        CK(dev_malloc(&ctx->d_sinkbuf, 2 * nm * sizeof(double)));
         CK(cudaMemset(ctx->d_sinkbuf, 0, 2 * nm * sizeof(double)));
-        CK(cudaMalloc(&ctx->d_ring, ntr * sizeof(int)));
+        CK(dev_malloc(&ctx->d_ring, ntr * sizeof(int)));
         CK(cudaMemcpy(ctx->d_ring, ring.data(), ntr * sizeof(int), cudaMemcpyHostToDevice));
         ctx->S.massl = ctx->d_sinkbuf;
         ctx->S.mass_loss = ctx->d_sinkbuf + nm;
@@ -1201,12 +1279,14 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
         ctx->names.push_back({"massl", {ctx->S.massl, nm}});
         ctx->names.push_back({"mass_loss", {ctx->S.mass_loss, nm}});
     }
+    take_records(ctx);  // after everything the context cannot do without
     *out = ctx;
     return PDAC_OK;
 }
 
 int pdac_gpu_destroy(pdac_ctx *ctx) {
     if (!ctx) return PDAC_ERR_ARG;
+    free_records([ctx](pdac_ctx *c) { return c == ctx; });
     cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->arena);
     cudaFree(ctx->metric);
@@ -1235,7 +1315,6 @@ int pdac_gpu_destroy(pdac_ctx *ctx) {
     cudaFree(ctx->d_simple);
     cudaFree(ctx->d_rest);
     cudaFree(ctx->d_partial);
-    cudaFree(ctx->d_fk);
     cudaFree(ctx->d_sinkbuf);
     cudaFree(ctx->d_ring);
     cudaFree(ctx->d_wave_idx);
@@ -1611,6 +1690,7 @@ static int enqueue_sweep(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof) {
 // conditional node around one sweep plus k_sweep_check, which clears the
 // condition when the sweep left no unconverged cell or maxout is reached
 static int build_iter_graph(pdac_ctx *ctx, double dt) {
+    const long gen = ctx->graph_gen;
     if (ctx->it_exec) { cudaGraphExecDestroy(ctx->it_exec); ctx->it_exec = nullptr; }
     if (ctx->it_graph) { cudaGraphDestroy(ctx->it_graph); ctx->it_graph = nullptr; }
     cudaStream_t st = ctx->stream;
@@ -1644,6 +1724,7 @@ static int build_iter_graph(pdac_ctx *ctx, double dt) {
     CK(cudaGetLastError());
     CK(cudaGraphInstantiate(&ctx->it_exec, ctx->it_graph, 0));
     ctx->it_dt = dt;
+    ctx->it_gen = gen;
     return PDAC_OK;
 }
 
@@ -1667,6 +1748,7 @@ static int maxout_status(pdac_ctx *ctx, int nit);
 
 int pdac_gpu_iter(pdac_ctx *ctx, double dt, int *nit_out) {
     if (!ctx) return PDAC_ERR_ARG;
+    const auto records = hold_records(ctx);
     cudaStream_t st = ctx->stream;
     size_t n = ctx->ncell, ns = ctx->ns;
     Fld &F = ctx->F;
@@ -1714,7 +1796,7 @@ int pdac_gpu_iter(pdac_ctx *ctx, double dt, int *nit_out) {
         ctx->launches++;
     } else if (!ctx->prof) {
         // the sweep loop runs on the device; one read-back of its count
-        if (!ctx->it_exec || ctx->it_dt != dt) {
+        if (!ctx->it_exec || ctx->it_dt != dt || ctx->it_gen != ctx->graph_gen) {
             int s = build_iter_graph(ctx, dt);
             if (s) return s;
         }
@@ -1858,6 +1940,7 @@ int pdac_gpu_iter_static(pdac_ctx *ctx, double dt, int *nit_out) {
         return fail(ctx, PDAC_ERR_ARG, "iter_static: this mesh needs " + std::to_string(need) +
                                            " bytes of static scratch, the limit is " +
                                            std::to_string((size_t)PDAC_ITER_STATIC_SCRATCH_BYTES));
+    const auto records = hold_records(ctx);
     unsigned char *base = nullptr;
     int st_ = static_scratch(ctx, &base);
     if (st_) return st_;
@@ -2385,12 +2468,8 @@ void put_tuning(pdac_ctx *ctx, const Tuning &t) {
     ctx->coop_cpb = t.coop_cpb;
     if (ctx->coop_max_blocks > 0)
         ctx->coop_blocks = std::min(std::max(1, (int)((ctx->ncell + t.coop_cpb - 1) / t.coop_cpb)), ctx->coop_max_blocks);
-    if (ctx->it_exec) { cudaGraphExecDestroy(ctx->it_exec); ctx->it_exec = nullptr; }
-    if (ctx->it_graph) { cudaGraphDestroy(ctx->it_graph); ctx->it_graph = nullptr; }
     if (ctx->ex_exec) { cudaGraphExecDestroy(ctx->ex_exec); ctx->ex_exec = nullptr; }
     if (ctx->ex_graph) { cudaGraphDestroy(ctx->ex_graph); ctx->ex_graph = nullptr; }
-    if (ctx->step_exec) { cudaGraphExecDestroy(ctx->step_exec); ctx->step_exec = nullptr; }
-    if (ctx->step_graph) { cudaGraphDestroy(ctx->step_graph); ctx->step_graph = nullptr; }
     ctx->graph_gen++;
 }
 
@@ -2461,6 +2540,23 @@ int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin) {
     return PDAC_OK;
 }
 
+// forms a context runs in that its mesh does not ask for
+int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin) {
+    if (!ctx || !in || nin < 1) return PDAC_ERR_ARG;
+    if (in[0] < 0 || in[0] > 1) return fail(ctx, PDAC_ERR_ARG, "set_forms: a value is out of range");
+    ctx->fk_off = in[0] == 1;
+    if (ctx->fk_off) free_records([ctx](pdac_ctx *c) { return c == ctx; });
+    else take_records(ctx);
+    return PDAC_OK;
+}
+
+int pdac_gpu_get_forms(pdac_ctx *ctx, int *out, int nout) {
+    if (!ctx || !out || nout < 1) return PDAC_ERR_ARG;
+    const auto records = hold_records(ctx);
+    out[0] = ctx->d_fk ? 1 : 0;
+    return PDAC_OK;
+}
+
 int pdac_gpu_autotune(pdac_ctx *ctx, const char *cache_path, int *out, int nout) {
     if (!ctx || (out && nout < 0)) return PDAC_ERR_ARG;
     const std::string key = tuning_key(ctx);
@@ -2511,7 +2607,7 @@ int pdac_gpu_autotune(pdac_ctx *ctx, const char *cache_path, int *out, int nout)
     size_t nv = std::max(ctx->nvent, 1), nm = ctx->S.ntr > 0 ? (size_t)2 * ctx->S.ntr * ctx->ns : 0;
     const size_t nib = ctx->ibstate_doubles;
     const size_t snap_doubles = ctx->arena_doubles + 2 * nv + nm + nib;
-    if (status == PDAC_OK && semi && cudaMalloc(&snap, snap_doubles * sizeof(double)) != cudaSuccess) {
+    if (status == PDAC_OK && semi && dev_malloc(&snap, snap_doubles * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         snap = nullptr;
     }
@@ -2593,6 +2689,7 @@ int pdac_gpu_autotune(pdac_ctx *ctx, const char *cache_path, int *out, int nout)
         if (!status) status = s3;
         if (!status) status = cudaStreamSynchronize(st) == cudaSuccess ? PDAC_OK : fail(ctx, PDAC_ERR_CUDA, "autotune: restore");
         cudaFree(snap);
+        take_records(ctx);  // in case the copy took them
         ctx->launches = launches; ctx->sweeps = sweeps; ctx->corr_launches = corr_launches;
         ctx->work_cells = work_cells; ctx->tested_cells = tested_cells; ctx->ex_calls = ex_calls;
         ctx->corr_ms = corr_ms; ctx->resid_ms = resid_ms; ctx->inner_ms = inner_ms;
@@ -3184,12 +3281,14 @@ static int add_step_nodes(pdac_ctx *ctx, cudaGraph_t g) {
 }
 
 static int build_step_graph(pdac_ctx *ctx) {
+    const long gen = ctx->graph_gen;
     if (ctx->step_exec) { cudaGraphExecDestroy(ctx->step_exec); ctx->step_exec = nullptr; }
     if (ctx->step_graph) { cudaGraphDestroy(ctx->step_graph); ctx->step_graph = nullptr; }
     CK(cudaGraphCreate(&ctx->step_graph, 0));
     int s = add_step_nodes(ctx, ctx->step_graph);
     if (s) return s;
     CK(cudaGraphInstantiate(&ctx->step_exec, ctx->step_graph, 0));
+    ctx->step_gen = gen;
     return PDAC_OK;
 }
 
@@ -3344,9 +3443,10 @@ static int build_batch_graph(pdac_batch *b) {
     b->bgen.assign(b->m.size(), -1);
     for (size_t i = 0; i < b->m.size(); ++i) {
         if (!b->graph[i]) continue;
+        const long gen = b->m[i]->graph_gen;
         int s = add_step_nodes(b->m[i], b->bgraph);
         if (s) return s;
-        b->bgen[i] = b->m[i]->graph_gen;
+        b->bgen[i] = gen;
     }
     if (cudaGraphInstantiate(&b->bexec, b->bgraph, 0) != cudaSuccess) {
         cudaGetLastError();
@@ -3358,6 +3458,11 @@ static int build_batch_graph(pdac_batch *b) {
 int pdac_gpu_batch_step(pdac_batch *b, int sweep, int *nit, int *status) {
     if (!b) return PDAC_ERR_ARG;
     std::vector<char> launched(b->m.size(), 0);
+    // the graph members' records stay until the step is complete (the other
+    // members' iter holds theirs)
+    std::vector<std::unique_lock<std::mutex>> records;
+    for (size_t i = 0; i < b->m.size(); ++i)
+        if (b->graph[i]) records.push_back(hold_records(b->m[i]));
     bool any_graph = false;
     for (size_t i = 0; i < b->m.size(); ++i) any_graph = any_graph || b->graph[i];
     // the batch graph runs on the lead stream: it first waits for what the
@@ -3394,7 +3499,7 @@ int pdac_gpu_batch_step(pdac_batch *b, int sweep, int *nit, int *status) {
         for (size_t i = 0; i < b->m.size(); ++i) {
             if (!b->graph[i]) continue;
             pdac_ctx *c = b->m[i];
-            int s = c->step_exec ? PDAC_OK : build_step_graph(c);
+            int s = c->step_exec && c->step_gen == c->graph_gen ? PDAC_OK : build_step_graph(c);
             if (!s && (cudaStreamWaitEvent(c->stream, b->t0, 0) != cudaSuccess ||
                        cudaGraphLaunch(c->step_exec, c->stream) != cudaSuccess))
                 s = fail(c, PDAC_ERR_CUDA, "batch: step graph launch failed");

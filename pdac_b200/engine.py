@@ -75,11 +75,16 @@ EXPORTED = (
     "pdac_gpu_append_mass_check", "pdac_gpu_write_mass_loss", "pdac_gpu_read_mass_loss",
     "pdac_gpu_compute_mixture_fields", "pdac_gpu_batch_create", "pdac_gpu_batch_step", "pdac_gpu_batch_elapsed",
     "pdac_gpu_batch_last_error", "pdac_gpu_batch_destroy", "pdac_gpu_unconverged_cells",
-    "pdac_gpu_autotune", "pdac_gpu_set_tuning",
+    "pdac_gpu_autotune", "pdac_gpu_set_tuning", "pdac_gpu_set_forms", "pdac_gpu_get_forms",
 )
 
 # the launch shapes pdac_gpu_autotune / pdac_gpu_set_tuning exchange, in order
 TUNING_KEYS = ("tile_shape", "tile_kchunk", "inner_grid", "test_grid", "coop_cells_per_block")
+
+
+# the forms pdac_gpu_set_forms chooses and those pdac_gpu_get_forms reports, in order
+FORM_KEYS = ("no_records",)
+FORM_REPORT = ("records",)
 
 
 class Engine:
@@ -193,6 +198,25 @@ class Engine:
         L.pdac_gpu_set_tuning.restype = C.c_int
         arr = (C.c_int * len(TUNING_KEYS))(*[int(tuning[k]) for k in TUNING_KEYS])
         self._chk(L.pdac_gpu_set_tuning(self.h, arr, len(TUNING_KEYS)), "set_tuning")
+
+    def set_forms(self, **forms):
+        """Choose the forms the context's kernels run in (FORM_KEYS, 0 or
+        absent: as the mesh and the device ask); no result changes."""
+        L = self.L
+        L.pdac_gpu_set_forms.argtypes = [C.c_void_p, C.POINTER(C.c_int), C.c_int]
+        L.pdac_gpu_set_forms.restype = C.c_int
+        arr = (C.c_int * len(FORM_KEYS))(*[int(forms.pop(k, 0)) for k in FORM_KEYS])
+        assert not forms, f"unknown forms {sorted(forms)}"
+        self._chk(L.pdac_gpu_set_forms(self.h, arr, len(FORM_KEYS)), "set_forms")
+
+    def forms(self):
+        """The forms in use (a dict with FORM_REPORT)."""
+        L = self.L
+        L.pdac_gpu_get_forms.argtypes = [C.c_void_p, C.POINTER(C.c_int), C.c_int]
+        L.pdac_gpu_get_forms.restype = C.c_int
+        out = (C.c_int * len(FORM_REPORT))()
+        self._chk(L.pdac_gpu_get_forms(self.h, out, len(FORM_REPORT)), "get_forms")
+        return dict(zip(FORM_REPORT, list(out)))
 
     def ygas(self, dt):
         self._chk(self.L.pdac_gpu_ygas(self.h, dt), "ygas")
