@@ -423,11 +423,18 @@ int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin);
  * device; none of them changes a result.  Test and debugging aid.
  * pdac_gpu_set_forms (nin >= 1; PDAC_ERR_ARG for a form the context cannot
  * run in):
- *   [0] the corrector's face records: 0 = when they leave as much device
- *       memory free as the context's fields take (they are also given back
- *       to an allocation of this library that does not fit otherwise),
- *       1 = none.
- * pdac_gpu_get_forms (nout >= 1): [0] 1 if the context holds face records.  */
+ *   [0] the corrector's face records: 0 = when they leave an eighth of the
+ *       device's memory free (they are also given back to an allocation of
+ *       this library that does not fit otherwise), 1 = none;
+ *   [1] the explicit solver's gas-enthalpy wavefront: 0 = as the mesh asks
+ *       (3 if the device holds the tiles at once, else 2), 1 = a launch per
+ *       hyperplane, 2 = one launch over all hyperplanes, 3 = tiles, of 16 x 4
+ *       columns (j x k) in 3D, all columns (up to 256) or else 64 in 2D, 4 =
+ *       2D tiles of 64.
+ * pdac_gpu_get_forms (nout >= 1): [0] 1 if the context holds face records;
+ * [1] tiles of the wavefront (0: none), [2], [3] their columns j and k, [4]
+ * the blocks of the launch over all hyperplanes (0 and no tiles: a launch
+ * each).                                                                    */
 int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin);
 int pdac_gpu_get_forms(pdac_ctx *ctx, int *out, int nout);
 

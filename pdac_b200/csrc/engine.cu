@@ -130,10 +130,6 @@ struct pdac_ctx {
     cudaEvent_t up_done = nullptr;
     double ex_ms[4] = {0, 0, 0, 0};
     long long ex_calls = 0;
-    // gas-enthalpy wavefront on hyperplane-ordered records: the cooperative
-    // grid (0 when the device cannot co-schedule one; the wavefront then
-    // runs as one launch per hyperplane) and whether it covers the widest
-    // hyperplane
     // ground sink (isink > 0): per-column mass taken out, restart values,
     // ring mask
     pdac::Sink S{};
@@ -156,10 +152,16 @@ struct pdac_ctx {
     // shared-memory tiled 3D stencil passes: tile shape (index into
     // TILE_SHAPES) and planes per block of the march up k
     int tile_shape = 0, tile_kchunk = 32;
+    // gas-enthalpy wavefront of the explicit solver: records in tile order
     int *d_wave_idx = nullptr;    // order, pos_of, code
     double *d_wave_rec = nullptr; // records and pnew
-    int wave_tiles = 0;     // tiles of the gas-enthalpy wavefront (0: a launch per hyperplane)
-    bool wave_one = false;  // one column per thread
+    // its form (setup_wave): tiles, or (0) all hyperplanes in one launch of
+    // wave_blocks blocks, with wave_one a record per thread and hyperplane, or
+    // (0) a launch each
+    int wave_tiles = 0, wave_blocks = 0;
+    bool wave_one = false;
+    // one launch whose blocks wait for one another
+    bool wave_coop() const { return wave_tiles > 1 || wave_blocks > 0; }
 };
 
 namespace {
@@ -267,11 +269,10 @@ inline int blocks(long n, int tpb = TPB) { return (int)((n + tpb - 1) / tpb); }
 // inner loop gathers the same terms, with the same results (four steps with
 // and without them: 128 x 128 x 96 with three phases 47.3 / 50.6 ms, with four
 // 68.0 / 78.5, its hills with six 120.5 / 142.6, 256 x 256 x 192 with four 407 /
-// 468).  A context takes them last in create, when they leave at least as much
-// memory free as its fields take, and any allocation of this library that does
-// not fit takes them back, from every context of the device, so that the
-// meshes, the number of contexts and the autotuner's copy that fit without
-// them still do.
+// 468).  A context takes them last in create, from memory to spare, and any
+// allocation of this library that does not fit takes them back, from every
+// context of the device, so that the meshes, the number of contexts and the
+// autotuner's copy that fit without them still do.
 std::mutex g_records_mu;             // guards the list; taken before any context's fk_mu
 std::vector<pdac_ctx *> g_records;   // the contexts that hold records
 
@@ -305,15 +306,24 @@ cudaError_t dev_malloc(T **p, size_t bytes) {
     return e;
 }
 
+// whether an allocation that a context can do without leaves an eighth of the
+// device's memory free
+bool memory_to_spare(size_t bytes) {
+    size_t avail = 0, total = 0;
+    if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return avail >= bytes + total / 8;
+}
+
 // the context's records, if they are wanted and there is room for them
 void take_records(pdac_ctx *ctx) {
     std::lock_guard<std::mutex> list(g_records_mu);
     std::lock_guard<std::mutex> lk(ctx->fk_mu);
     if (ctx->d_fk || !ctx->fk_doubles || ctx->fk_off) return;
     const size_t need = ctx->fk_doubles * sizeof(double);
-    size_t avail = 0, total = 0;
-    if (cudaMemGetInfo(&avail, &total) != cudaSuccess || avail < need + ctx->arena_doubles * sizeof(double) ||
-        cudaMalloc(&ctx->d_fk, need) != cudaSuccess) {
+    if (!memory_to_spare(need) || cudaMalloc(&ctx->d_fk, need) != cudaSuccess) {
         (void)cudaGetLastError();
         ctx->d_fk = nullptr;
         return;
@@ -652,63 +662,60 @@ void boundary_levels(const pdac_cfg *c, std::vector<int> &items, std::vector<int
     starts.push_back((int)lev.size());
 }
 
-// The tiles and records of the explicit solver's gas-enthalpy wavefront
-// (k_rk3_wave_tile; fixed by the cell flags).  Tiles of 16 x 4 columns
-// (measured, both stages and their records, 128 x 128 x 96 / 224 x 208 x 161:
-// 16 x 4 2.0 / 5.7 ms, 8 x 8 2.3 / 6.7, 16 x 8 2.4 / 7.1, 16 x 16 2.5 / 6.9);
-// where those are more than the device holds at once (about 57000 columns),
-// tiles of 1024 and 2048 columns, several per thread.  2D meshes have one row
-// of columns: one tile up to 256 of them, which needs no exchange through L2
-// and no cooperative launch (128 x 192: 0.63 ms, three tiles of 64 0.84), else
-// tiles of 64.
-int setup_wave(pdac_ctx *ctx, const int *flag) {
+// forms of the explicit solver's gas-enthalpy wavefront (pdac_gpu_set_forms):
+// as the mesh asks, a launch per hyperplane, one launch over all hyperplanes,
+// tiles, tiles of 64 columns in 2D
+enum { WAVE_AUTO = 0, WAVE_LAUNCHES, WAVE_PLANES, WAVE_TILES, WAVE_TILES_64 };
+
+// the tiles of tt columns whose blocks the device holds at once
+int wave_room(const pdac_ctx *ctx, int tt, int nsm) {
+    int occ = 0;
+    const size_t sm = 2 * (size_t)tt * sizeof(double);
+    if (ctx->d3) (void)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<3, true>, tt, sm);
+    else (void)cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<2, true>, tt, sm);
+    return occ * nsm;
+}
+
+// The records of the wavefront (fixed by the cell flags) and the form it takes:
+// tiles of columns (j, k) if the device holds all of them at once, a thread per
+// column, else all hyperplanes in one cooperative launch, else a launch each.
+//
+// Tiles of 16 x 4 in 3D (measured, both stages and their records, 128 x 128 x
+// 96 / 224 x 208 x 161: 16 x 4 2.0 / 5.7 ms, 8 x 8 2.3 / 6.7, 16 x 8 2.4 / 7.1,
+// 16 x 16 2.5 / 6.9; whole steps of 128 x 128 x 96 9.4 ms, over hyperplanes
+// 10.1).  Above the about 57000 columns that fit, hyperplanes: several columns
+// a thread, in the best of the tiles tried, took 7.0 ms a step of 6 x 262 x 243
+// against 5.4, 16.3 / 13.4 of 9 x 500 x 300, 57.4 / 53.6 of 100 x 384 x 256.
+// 2D meshes have one row of columns: one tile up to 256 of them, which needs no
+// exchange through L2 and no cooperative launch (128 x 192: 0.63 ms, three
+// tiles of 64 0.84), else tiles of 64.
+int setup_wave(pdac_ctx *ctx, const int *flag, int form = WAVE_AUTO) {
     const int nx = ctx->nx, ny = ctx->d3 ? ctx->ny : 1, nz = ctx->nz, n = ctx->ncell;
     const int jlo = ctx->d3 ? 2 : 1, jhi = ctx->d3 ? ny - 1 : 1;
     const int ni = nx - 2, nj = jhi - jlo + 1, nk = nz - 2;
-    ctx->wave_tiles = 0;
-    if (ni < 1 || nj < 1 || nk < 1) return PDAC_OK;
+    ctx->wave_tiles = ctx->wave_blocks = 0;
+    cudaFree(ctx->d_wave_idx);
+    cudaFree(ctx->d_wave_rec);
+    ctx->d_wave_idx = nullptr;
+    ctx->d_wave_rec = nullptr;
+    ctx->W = pdac::Wave{};
+    if (form == WAVE_LAUNCHES) return PDAC_OK;
     int dev = 0, coop = 0, nsm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    auto room = [&](bool one, int threads, int tt) {
-        int occ = 0;
-        const size_t sm = 2 * (size_t)tt * sizeof(double);
-        if (ctx->d3)
-            (void)(one ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<3, true, true>, threads, sm)
-                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<3, false, true>, threads, sm));
-        else
-            (void)(one ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<2, true, true>, threads, sm)
-                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pdac::k_rk3_wave_tile<2, false, true>, threads, sm));
-        return occ * nsm;
-    };
-    const int shapes3[][2] = {{16, 4}, {32, 32}, {64, 32}}, shapes2[][2] = {{1, 64}, {1, 1024}, {1, 2048}};
-    pdac::Wave &W = ctx->W;
-    int tiles = 0;
-    bool one = true;
-    if (!ctx->d3 && nk <= 256) {
-        W.tj = 1;
-        W.tk = (nk + 31) / 32 * 32;
-        tiles = 1;  // with one column per thread
-    } else {
-        for (int q = 0; q < 3 && coop; ++q) {
-            W.tj = ctx->d3 ? shapes3[q][0] : shapes2[q][0];
-            W.tk = ctx->d3 ? shapes3[q][1] : shapes2[q][1];
-            one = W.tj * W.tk <= 256;
-            const int m = ((nj + W.tj - 1) / W.tj) * ((nk + W.tk - 1) / W.tk);
-            if (m <= room(one, std::min(512, W.tj * W.tk), W.tj * W.tk)) { tiles = m; break; }
-        }
-    }
-    if (tiles == 1 && !one) tiles = 0;  // cannot be: several columns a thread come with many tiles
-    if (!tiles) return PDAC_OK;
-    W.tt = W.tj * W.tk;
-    W.ntj = (nj + W.tj - 1) / W.tj;
-    W.steps = ni + W.tj + W.tk - 2;
-    const long long np = (long long)tiles * W.steps * W.tt;
-    if (np > 0x7fffffffLL) return PDAC_OK;
-    W.npos = (int)np;
-    std::vector<int> order(np, -1), pos_of(n, -1);
-    std::vector<unsigned char> code(np, 0);
+    const size_t rec_doubles = (size_t)(pdac::WR_YG + ctx->ng) + 1;  // the fields and pnew
+    const bool row = !ctx->d3 && nk <= 256 && form != WAVE_TILES_64;  // all columns in one tile
+    const int tj = ctx->d3 ? 16 : 1, tk = ctx->d3 ? 4 : (row ? (nk + 31) / 32 * 32 : 64);
+    const int mj = (nj + tj - 1) / tj, mk = (nk + tk - 1) / tk, steps = ni + tj + tk - 2;
+    long long np = (long long)mj * mk * steps * tj * tk;
+    bool tiles = form != WAVE_PLANES && np <= 0x7fffffffLL && (mj * mk == 1 || (coop && mj * mk <= wave_room(ctx, tj * tk, nsm)));
+    // records padded to more than half as much again: only into memory to spare
+    if (2 * np > 3LL * ni * nj * nk) tiles = tiles && memory_to_spare((size_t)np * (rec_doubles * sizeof(double) + sizeof(int) + 1));
+    if (!tiles && form >= WAVE_TILES) return fail(ctx, PDAC_ERR_ARG, "set_forms: the wavefront cannot run in these tiles");
+    pdac::Wave W{};
+    std::vector<int> order, pos_of(n, -1), start, src;
+    std::vector<unsigned char> code;
     auto each = [&](auto fn) {
         for (int k = 2; k <= nz - 1; ++k)
             for (int j = jlo; j <= jhi; ++j)
@@ -717,12 +724,53 @@ int setup_wave(pdac_ctx *ctx, const int *flag) {
                     if (flag[c] & 1) fn(c, i, j, k);
                 }
     };
-    each([&](int c, int i, int j, int k) {
-        const int J = (j - jlo) / W.tj, jl = (j - jlo) % W.tj, K = (k - 2) / W.tk, kl = (k - 2) % W.tk;
-        const int tile = J + W.ntj * K, s = (i - 2) + jl + kl, p = (tile * W.steps + s) * W.tt + jl + W.tj * kl;
-        pos_of[c] = p;
-        order[p] = c;
-    });
+    int widest = 0;
+    if (tiles) {
+        W.tj = tj;
+        W.tk = tk;
+        W.tt = tj * tk;
+        W.ntj = mj;
+        W.steps = steps;
+        order.assign(np, -1);
+        each([&](int c, int i, int j, int k) {
+            const int J = (j - jlo) / W.tj, jl = (j - jlo) % W.tj, K = (k - 2) / W.tk, kl = (k - 2) % W.tk;
+            const int tile = J + W.ntj * K, s = (i - 2) + jl + kl, p = (tile * W.steps + s) * W.tt + jl + W.tj * kl;
+            pos_of[c] = p;
+            order[p] = c;
+        });
+    } else {
+        // hyperplane d = i + j + k (i + k in 2D) after hyperplane, cell order
+        // within one; empty ones are dropped, as no cell depends on one
+        if (!coop) return form == WAVE_AUTO ? PDAC_OK : fail(ctx, PDAC_ERR_ARG, "set_forms: no cooperative launches");
+        const int dmin = 2 + jlo + 2, nd = (nx - 1) + jhi + (nz - 1) - dmin + 1;
+        std::vector<int> first(nd + 1, 0);
+        each([&](int, int i, int j, int k) { first[i + j + k - dmin + 1]++; });
+        for (int q = 0; q < nd; ++q) {
+            if (first[q + 1]) start.push_back(first[q]);
+            widest = std::max(widest, first[q + 1]);
+            first[q + 1] += first[q];
+        }
+        np = first[nd];
+        if (np == 0) return PDAC_OK;
+        W.nplanes = (int)start.size();
+        start.push_back((int)np);
+        start.push_back((int)np);  // read one past the last hyperplane
+        order.assign(np, -1);
+        std::vector<int> fill(first.begin(), first.end() - 1);
+        each([&](int c, int i, int j, int k) {
+            pos_of[c] = fill[i + j + k - dmin];
+            order[fill[i + j + k - dmin]++] = c;
+        });
+        src.assign(3 * (size_t)np, -1);
+        for (int p = 0; p < np; ++p) {
+            const int c = order[p];
+            src[p] = pos_of[c - 1];
+            if (ctx->d3) src[np + p] = pos_of[c - nx];
+            src[2 * np + p] = pos_of[c - nx * ny];
+        }
+    }
+    W.npos = (int)np;
+    code.assign(np, 0);
     each([&](int c, int, int, int) {
         int m = pdac::WC_REC;
         if (pos_of[c - 1] >= 0) m |= pdac::WC_W;
@@ -730,21 +778,43 @@ int setup_wave(pdac_ctx *ctx, const int *flag) {
         if (pos_of[c - nx * ny] >= 0) m |= pdac::WC_B;
         code[pos_of[c]] = (unsigned char)m;
     });
-    CK(dev_malloc(&ctx->d_wave_idx, (order.size() + pos_of.size()) * sizeof(int) + code.size()));
-    int *o = ctx->d_wave_idx, *po = o + order.size();
-    unsigned char *cd = reinterpret_cast<unsigned char *>(po + pos_of.size());
-    CK(cudaMemcpy(o, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(po, pos_of.data(), pos_of.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(cd, code.data(), code.size(), cudaMemcpyHostToDevice));
-    const size_t nrec = (size_t)(pdac::WR_YG + ctx->ng) + 1;  // the fields and pnew
-    CK(dev_malloc(&ctx->d_wave_rec, nrec * np * sizeof(double)));
-    W.order = o;
-    W.pos_of = po;
-    W.code = cd;
+    const size_t idx = order.size() + pos_of.size() + start.size() + src.size();
+    if (dev_malloc(&ctx->d_wave_idx, idx * sizeof(int) + code.size()) != cudaSuccess ||
+        dev_malloc(&ctx->d_wave_rec, rec_doubles * np * sizeof(double)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        cudaFree(ctx->d_wave_idx);
+        ctx->d_wave_idx = nullptr;
+        return form == WAVE_AUTO ? PDAC_OK : fail(ctx, PDAC_ERR_CUDA, "set_forms: no memory for the wavefront's records");
+    }
+    int *at = ctx->d_wave_idx;
+    auto put = [&](const std::vector<int> &v) -> int * {
+        int *const d = at;
+        at += v.size();
+        return v.empty() || cudaMemcpy(d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess ? d : nullptr;
+    };
+    W.order = put(order);
+    W.pos_of = put(pos_of);
+    W.start = put(start);
+    W.src = put(src);
+    if (!W.order || !W.pos_of || !W.start || !W.src) return fail(ctx, PDAC_ERR_CUDA, "the wavefront's tables");
+    CK(cudaMemcpy(at, code.data(), code.size(), cudaMemcpyHostToDevice));
+    W.code = reinterpret_cast<unsigned char *>(at);
     W.rec = ctx->d_wave_rec;
-    W.pnew = ctx->d_wave_rec + (nrec - 1) * np;
-    ctx->wave_tiles = tiles;
-    ctx->wave_one = one;
+    W.pnew = ctx->d_wave_rec + (rec_doubles - 1) * np;
+    ctx->W = W;
+    ctx->wave_tiles = tiles ? mj * mk : 0;
+    if (!tiles) {  // a record per thread and hyperplane where the device holds enough threads
+        int occ1 = 0, occn = 0;
+        if (ctx->d3) {
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, pdac::k_rk3_wave_planes<3, true>, TPB, 0));
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occn, pdac::k_rk3_wave_planes<3, false>, TPB, 0));
+        } else {
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, pdac::k_rk3_wave_planes<2, true>, TPB, 0));
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occn, pdac::k_rk3_wave_planes<2, false>, TPB, 0));
+        }
+        ctx->wave_one = blocks(widest) <= occ1 * nsm;
+        ctx->wave_blocks = ctx->wave_one ? blocks(widest) : occn * nsm;
+    }
     return PDAC_OK;
 }
 
@@ -2223,11 +2293,12 @@ static long long enqueue_explicit(pdac_ctx *ctx, double dt, cudaStream_t st, boo
         else PHASE_LAUNCH_D(nph, pdac::k_rk3_stage, 2, blocks(n), TPB, st, P, F, K, dt, stage);
         L++;
         mark();
-        // gas-enthalpy wavefront: records, one launch over all tiles,
-        // scatter of the results; in a batch, where a cooperative launch is
-        // not allowed, meshes of several tiles take a launch per hyperplane
-        // i + j + k = d of the interior (2 <= i <= nx - 1 ...), in increasing d
-        if (ctx->wave_tiles == 1 || (ctx->wave_tiles > 1 && ctx->allow_coop)) {
+        // gas-enthalpy wavefront: records, one launch over all tiles or
+        // hyperplanes, scatter of the results; where a cooperative launch is
+        // not allowed (in a batch) and there are several tiles, a launch per
+        // hyperplane i + j + k = d of the interior (2 <= i <= nx - 1 ...), in
+        // increasing d
+        if (ctx->wave_tiles == 1 || (ctx->wave_coop() && ctx->allow_coop)) {
             const pdac::Wave &W = ctx->W;
             const int rb = blocks(W.npos);
             int *gave_up = ctx->d_counters + 6;
@@ -2235,24 +2306,27 @@ static long long enqueue_explicit(pdac_ctx *ctx, double dt, cudaStream_t st, boo
             cudaLaunchAttribute at[1];
             at[0].id = cudaLaunchAttributeCooperative;
             at[0].val.cooperative = 1;
-            lc.gridDim = dim3(ctx->wave_tiles);
-            lc.blockDim = dim3(std::min(512, W.tt));
+            lc.gridDim = dim3(ctx->wave_tiles ? ctx->wave_tiles : ctx->wave_blocks);
+            lc.blockDim = dim3(ctx->wave_tiles ? W.tt : TPB);
             lc.dynamicSmemBytes = 2 * (size_t)W.tt * sizeof(double);
             lc.stream = st;
             lc.attrs = at;
-            const bool multi = ctx->wave_tiles > 1;
-            lc.numAttrs = multi ? 1 : 0;
+            lc.numAttrs = ctx->wave_coop() ? 1 : 0;
+            auto wave = [&](auto kernel) { cudaLaunchKernelEx(&lc, kernel, P, W, dt, stage, gave_up); };
+            auto planes = [&](auto kernel) { cudaLaunchKernelEx(&lc, kernel, P, W, dt, stage); };
             if (ctx->d3) {
                 pdac::k_rk3_wave_pre<3><<<blocks(n), TPB, 0, st>>>(P, F, K, W, dt, stage);
-                if (!multi) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<3, true, false>, P, W, dt, stage, gave_up);
-                else if (ctx->wave_one) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<3, true, true>, P, W, dt, stage, gave_up);
-                else cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<3, false, true>, P, W, dt, stage, gave_up);
+                if (ctx->wave_tiles == 1) wave(pdac::k_rk3_wave_tile<3, false>);
+                else if (ctx->wave_tiles) wave(pdac::k_rk3_wave_tile<3, true>);
+                else if (ctx->wave_one) planes(pdac::k_rk3_wave_planes<3, true>);
+                else planes(pdac::k_rk3_wave_planes<3, false>);
                 pdac::k_rk3_wave_post<3><<<rb, TPB, 0, st>>>(P, F, K, W, stage);
             } else {
                 pdac::k_rk3_wave_pre<2><<<blocks(n), TPB, 0, st>>>(P, F, K, W, dt, stage);
-                if (!multi) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<2, true, false>, P, W, dt, stage, gave_up);
-                else if (ctx->wave_one) cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<2, true, true>, P, W, dt, stage, gave_up);
-                else cudaLaunchKernelEx(&lc, pdac::k_rk3_wave_tile<2, false, true>, P, W, dt, stage, gave_up);
+                if (ctx->wave_tiles == 1) wave(pdac::k_rk3_wave_tile<2, false>);
+                else if (ctx->wave_tiles) wave(pdac::k_rk3_wave_tile<2, true>);
+                else if (ctx->wave_one) planes(pdac::k_rk3_wave_planes<2, true>);
+                else planes(pdac::k_rk3_wave_planes<2, false>);
                 pdac::k_rk3_wave_post<2><<<rb, TPB, 0, st>>>(P, F, K, W, stage);
             }
             L += 3;
@@ -2314,7 +2388,7 @@ int pdac_gpu_explicit_iter(pdac_ctx *ctx, double dt) {
     cudaStream_t st = ctx->stream;
     CK(cudaEventRecord(ctx->ev[6], st));
     std::unique_lock<std::mutex> lk(coop_lock(), std::defer_lock);
-    if (ctx->wave_tiles > 1 && ctx->allow_coop) lk.lock();  // until the stream is idle below
+    if (ctx->wave_coop() && ctx->allow_coop) lk.lock();  // until the stream is idle below
     if (ctx->prof) {
         ctx->launches += enqueue_explicit(ctx, dt, st, true);
         CK(cudaGetLastError());
@@ -2543,7 +2617,17 @@ int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin) {
 // forms a context runs in that its mesh does not ask for
 int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin) {
     if (!ctx || !in || nin < 1) return PDAC_ERR_ARG;
-    if (in[0] < 0 || in[0] > 1) return fail(ctx, PDAC_ERR_ARG, "set_forms: a value is out of range");
+    const int wave = nin > 1 ? in[1] : 0;
+    if (in[0] < 0 || in[0] > 1 || wave < 0 || wave > (ctx->d3 ? WAVE_TILES : WAVE_TILES_64) || (wave && ctx->ti != 1))
+        return fail(ctx, PDAC_ERR_ARG, "set_forms: a value is out of range");
+    if (ctx->ti == 1) {
+        std::vector<int> flag(ctx->ncell);
+        CK(cudaMemcpy(flag.data(), ctx->d_flag, flag.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        CK(cudaStreamSynchronize(ctx->stream));
+        ctx->ex_dt = -1.0;  // explicit_iter's graph is built again
+        int s = setup_wave(ctx, flag.data(), wave);
+        if (s) return s;
+    }
     ctx->fk_off = in[0] == 1;
     if (ctx->fk_off) free_records([ctx](pdac_ctx *c) { return c == ctx; });
     else take_records(ctx);
@@ -2553,7 +2637,8 @@ int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin) {
 int pdac_gpu_get_forms(pdac_ctx *ctx, int *out, int nout) {
     if (!ctx || !out || nout < 1) return PDAC_ERR_ARG;
     const auto records = hold_records(ctx);
-    out[0] = ctx->d_fk ? 1 : 0;
+    const int v[] = {ctx->d_fk ? 1 : 0, ctx->wave_tiles, ctx->W.tj, ctx->W.tk, ctx->wave_blocks};
+    for (int q = 0; q < nout && q < (int)(sizeof v / sizeof *v); ++q) out[q] = v[q];
     return PDAC_OK;
 }
 

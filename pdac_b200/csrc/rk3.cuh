@@ -638,13 +638,20 @@ __global__ void k_rk3_wave(Prm P, Fld F, RkF K, double dt, int stage, int d, int
 // jl - kl of its column in step s, so a step is a hyperplane of the tile, and
 // its records lie one after the other: record (tile, s, t) at (tile steps +
 // s) tt + t.
+// Meshes whose columns do not fit (setup_wave) take k_rk3_wave_planes over
+// records in hyperplane order, without padding.
 struct Wave {
     const int *order;           // record position -> cell, -1 where there is none
     const int *pos_of;          // cell -> record position, -1 for cells without a record
     const unsigned char *code;  // per position: WC_REC a record, WC_W/S/B its neighbour's pressure is the wavefront's
     double *rec;                // [WR_YG + ng][npos]
     double *pnew;               // new pressure per record
-    int npos, tj, tk, tt, ntj, steps;
+    int npos;
+    int tj, tk, tt, ntj, steps;  // tiles
+    // hyperplanes: records start[q] .. start[q + 1] - 1 of hyperplane q, and per
+    // record the W / S / B neighbour's ([3][npos]; -1: none)
+    const int *start, *src;
+    int nplanes;
 };
 enum { WC_REC = 1, WC_W = 2, WC_S = 4, WC_B = 8 };
 // record fields; the wavefront's results (WR_O*) are stored in record order
@@ -806,11 +813,10 @@ constexpr int WAVE_LOOKS = 1 << 22;  // the limit of one wait: a second or two
 // word holds WAVE_EMPTY from k_rk3_wave_pre until its record is solved.  Each
 // wait is bounded all the same; one that runs out sets *gave_up, on which the
 // other waits give up too and every block leaves after its next barrier.
-// ONE: a thread per column, which loads the next step's record while this one
-// is solved; else a thread takes several columns in turn.
-// MULTI: there is more than one tile.
-template <int D, bool ONE, bool MULTI>
-__global__ void __launch_bounds__(ONE ? 256 : 512) k_rk3_wave_tile(Prm P, Wave W, double dt, int stage, int *gave_up) {
+// A thread per column, which loads the next step's record while this one is
+// solved.  MULTI: there is more than one tile.
+template <int D, bool MULTI>
+__global__ void __launch_bounds__(256) k_rk3_wave_tile(Prm P, Wave W, double dt, int stage, int *gave_up) {
     extern __shared__ double sp[];  // [2][tt]
     const int tt = W.tt, tile = blockIdx.x, steps = W.steps;
     const double a1dt = (stage == 1 ? 1.0 : 0.25) * dt, a2dt = (stage == 1 ? 0.0 : 0.25) * dt;
@@ -828,65 +834,94 @@ __global__ void __launch_bounds__(ONE ? 256 : 512) k_rk3_wave_tile(Prm P, Wave W
         }
         return __longlong_as_double((long long)x);
     };
-    if (ONE) {
-        const int t = threadIdx.x, jl = t % W.tj, kl = t / W.tj;
-        const bool south = jl == 0, below = kl == 0;
-        int pos = base + t, code = W.code[pos], code1 = steps > 1 ? W.code[pos + tt] : 0;
-        unsigned long long es = WAVE_EMPTY, eb = WAVE_EMPTY;  // looked for one step ahead
-        double pown = 0.0;
-        // step s on record v while the next one arrives in w
-        auto step = [&](int s, WaveIn &v, WaveIn &w) {
-            const int npos = pos + tt, code2 = s + 2 < steps ? W.code[npos + tt] : 0;
-            unsigned long long ns = WAVE_EMPTY, nb = WAVE_EMPTY;
-            if (code1 & WC_REC) wave_load<D>(P, W, npos, w);
-            if (MULTI && (code1 & WC_S) && south) ns = wave_look(W.pnew + npos + off_s);
-            if (MULTI && (code1 & WC_B) && below) nb = wave_look(W.pnew + npos + off_b);
-            bool lost = false;
-            if (code & WC_REC) {
-                const double *prev = sp + ((s + 1) & 1) * tt;
-                double ps = v.ps, pb = v.pb;
-                if (code & WC_S) ps = MULTI && south ? wait(W.pnew + pos + off_s, es, lost) : prev[t - 1];
-                if (code & WC_B) pb = MULTI && below ? wait(W.pnew + pos + off_b, eb, lost) : prev[t - W.tj];
-                pown = wave_solve<D, MULTI>(P, W, v, pos, code & WC_W ? pown : v.pw, ps, pb, a1dt, a2dt, stage);
-                sp[(s & 1) * tt + t] = pown;
-            }
-            pos = npos;
-            code = code1;
-            code1 = code2;
-            es = ns;
-            eb = nb;
-            if (MULTI) return __syncthreads_or(lost) != 0;
-            __syncthreads();
-            return false;
-        };
-        WaveIn v, w;
-        if (code & WC_REC) wave_load<D>(P, W, pos, v);
+    const int t = threadIdx.x, jl = t % W.tj, kl = t / W.tj;
+    const bool south = jl == 0, below = kl == 0;
+    int pos = base + t, code = W.code[pos], code1 = steps > 1 ? W.code[pos + tt] : 0;
+    unsigned long long es = WAVE_EMPTY, eb = WAVE_EMPTY;  // looked for one step ahead
+    double pown = 0.0;
+    // step s on record v while the next one arrives in w
+    auto step = [&](int s, WaveIn &v, WaveIn &w) {
+        const int npos = pos + tt, code2 = s + 2 < steps ? W.code[npos + tt] : 0;
+        unsigned long long ns = WAVE_EMPTY, nb = WAVE_EMPTY;
+        if (code1 & WC_REC) wave_load<D>(P, W, npos, w);
+        if (MULTI && (code1 & WC_S) && south) ns = wave_look(W.pnew + npos + off_s);
+        if (MULTI && (code1 & WC_B) && below) nb = wave_look(W.pnew + npos + off_b);
         bool lost = false;
-        for (int s = 0; s < steps && !lost; s += 2) {
-            lost = step(s, v, w);
-            if (!lost && s + 1 < steps) lost = step(s + 1, w, v);
+        if (code & WC_REC) {
+            const double *prev = sp + ((s + 1) & 1) * tt;
+            double ps = v.ps, pb = v.pb;
+            if (code & WC_S) ps = MULTI && south ? wait(W.pnew + pos + off_s, es, lost) : prev[t - 1];
+            if (code & WC_B) pb = MULTI && below ? wait(W.pnew + pos + off_b, eb, lost) : prev[t - W.tj];
+            pown = wave_solve<D, MULTI>(P, W, v, pos, code & WC_W ? pown : v.pw, ps, pb, a1dt, a2dt, stage);
+            sp[(s & 1) * tt + t] = pown;
         }
-        if (lost && t == 0) atomicExch(gave_up, 1);
+        pos = npos;
+        code = code1;
+        code1 = code2;
+        es = ns;
+        eb = nb;
+        if (MULTI) return __syncthreads_or(lost) != 0;
+        __syncthreads();
+        return false;
+    };
+    WaveIn v, w;
+    if (code & WC_REC) wave_load<D>(P, W, pos, v);
+    bool lost = false;
+    for (int s = 0; s < steps && !lost; s += 2) {
+        lost = step(s, v, w);
+        if (!lost && s + 1 < steps) lost = step(s + 1, w, v);
+    }
+    if (lost && t == 0) atomicExch(gave_up, 1);
+}
+
+// every hyperplane of a stage in one cooperative launch over the records: a
+// grid-wide barrier separates the hyperplanes (all blocks are resident, so it
+// always completes) and the neighbour pressures of the previous one are read
+// past L1.  What bounds it is the barrier, 3 of the 4.6 us of a hyperplane of
+// 128 x 128 x 96.  Whole steps of 100 x 384 x 256 53.6 ms (a launch each 65.8),
+// 5 x 700 x 600 18.4 (40.3).  ONE: the grid covers the widest hyperplane, so a
+// thread holds at most one record of each and loads the next one before the
+// barrier.
+template <int D, bool ONE>
+__global__ void __launch_bounds__(128) k_rk3_wave_planes(Prm P, Wave W, double dt, int stage) {
+    cooperative_groups::grid_group g = cooperative_groups::this_grid();
+    const int nthr = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t np = W.npos;
+    const double a1dt = (stage == 1 ? 1.0 : 0.25) * dt, a2dt = (stage == 1 ? 0.0 : 0.25) * dt;
+    auto solve = [&](const WaveIn &v, int pos, int sw, int ss, int sb) {
+        const double pw = sw >= 0 ? __ldcg(W.pnew + sw) : v.pw, pb = sb >= 0 ? __ldcg(W.pnew + sb) : v.pb;
+        const double ps = D == 3 && ss >= 0 ? __ldcg(W.pnew + ss) : v.ps;
+        wave_solve<D, true>(P, W, v, pos, pw, ps, pb, a1dt, a2dt, stage);
+    };
+    if (ONE) {
+        WaveIn v;
+        int pos = W.start[0] + tid, sw = -1, ss = -1, sb = -1;
+        bool have = pos < W.start[1];
+        auto load = [&] {
+            wave_load<D>(P, W, pos, v);
+            sw = W.src[pos];
+            if (D == 3) ss = W.src[np + pos];
+            sb = W.src[2 * np + pos];
+        };
+        if (have) load();
+        for (int q = 0; q < W.nplanes; ++q) {
+            if (have) solve(v, pos, sw, ss, sb);
+            if (q + 1 < W.nplanes) {
+                pos = W.start[q + 1] + tid;
+                have = pos < W.start[q + 2];
+                if (have) load();
+            }
+            g.sync();
+        }
     } else {
-        for (int s = 0; s < steps; ++s) {
-            bool lost = false;
-            for (int t = threadIdx.x; t < tt; t += blockDim.x) {
-                const int pos = base + s * tt + t, code = W.code[pos];
-                if (!(code & WC_REC)) continue;
-                const int jl = t % W.tj, kl = t / W.tj;
+        for (int q = 0; q < W.nplanes; ++q) {
+            const int end = W.start[q + 1];
+            for (int pos = W.start[q] + tid; pos < end; pos += nthr) {
                 WaveIn v;
                 wave_load<D>(P, W, pos, v);
-                const double *prev = sp + ((s + 1) & 1) * tt;
-                double ps = v.ps, pb = v.pb;
-                if (code & WC_S) ps = jl == 0 ? wait(W.pnew + pos + off_s, WAVE_EMPTY, lost) : prev[t - 1];
-                if (code & WC_B) pb = kl == 0 ? wait(W.pnew + pos + off_b, WAVE_EMPTY, lost) : prev[t - W.tj];
-                sp[(s & 1) * tt + t] =
-                    wave_solve<D, MULTI>(P, W, v, pos, code & WC_W ? prev[t] : v.pw, ps, pb, a1dt, a2dt, stage);
+                solve(v, pos, W.src[pos], D == 3 ? W.src[np + pos] : -1, W.src[2 * np + pos]);
             }
-            if (__syncthreads_or(lost)) {
-                if (threadIdx.x == 0) atomicExch(gave_up, 1);
-                return;
-            }
+            g.sync();
         }
     }
 }
