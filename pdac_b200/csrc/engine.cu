@@ -2872,8 +2872,7 @@ int pdac_gpu_read_restart(pdac_ctx *ctx, const char *path, double *time, int *nf
         // kernels and captured graphs carry the gas table by value
         for (int ig = 0; ig < ctx->ng; ++ig) ctx->cfg.gas_type[ig] = ctx->P.gas_type[ig] = gt[ig];
         set_gas_tables(ctx);
-        if (ctx->it_exec) { cudaGraphExecDestroy(ctx->it_exec); ctx->it_exec = nullptr; }
-        if (ctx->it_graph) { cudaGraphDestroy(ctx->it_graph); ctx->it_graph = nullptr; }
+        ctx->graph_gen++;
         if (ctx->ex_exec) { cudaGraphExecDestroy(ctx->ex_exec); ctx->ex_exec = nullptr; }
         if (ctx->ex_graph) { cudaGraphDestroy(ctx->ex_graph); ctx->ex_graph = nullptr; }
     }
