@@ -115,10 +115,13 @@ struct pdac_ctx {
     // graph of one explicit_iter, instantiated for one dt
     int ti = 0;
     RkF K{};
-    cudaGraph_t ex_graph = nullptr;
-    cudaGraphExec_t ex_exec = nullptr;
-    double ex_dt = 0.0;
-    long long ex_launches = 0;  // kernel launches of one explicit_iter
+    struct ExGraph {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        double dt = 0.0;
+        long gen = -1;           // the graph_gen it was built at
+        long long launches = 0;  // kernel launches of one explicit_iter
+    } ex[2];                     // the wavefront in launches, in the context's form
     // profiling of explicit_iter: marks between its kernel groups and the
     // accumulated device ms of the groups [flux passes, stage kernels,
     // gas-enthalpy wavefronts, final rhs + coefficients + solve]
@@ -925,8 +928,8 @@ static int setup_sweep_loop(pdac_ctx *ctx) {
 
 // Held while a cooperative grid of this library is in flight on a device:
 // contexts may be stepped from several host threads, and two such grids at
-// once could each hold part of the device and wait for the rest.  iter takes
-// the graph form instead of waiting.
+// once could each hold part of the device and wait for the rest.  iter and
+// explicit_iter take a form of separate launches instead of waiting.
 static std::mutex &coop_lock() {
     static std::mutex mu[64];
     int dev = 0;
@@ -1377,8 +1380,10 @@ int pdac_gpu_destroy(pdac_ctx *ctx) {
     cudaFree(ctx->d_dirty);
     if (ctx->it_exec) cudaGraphExecDestroy(ctx->it_exec);
     if (ctx->it_graph) cudaGraphDestroy(ctx->it_graph);
-    if (ctx->ex_exec) cudaGraphExecDestroy(ctx->ex_exec);
-    if (ctx->ex_graph) cudaGraphDestroy(ctx->ex_graph);
+    for (auto &g : ctx->ex) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        if (g.graph) cudaGraphDestroy(g.graph);
+    }
     cudaFree(ctx->d_nit);
     cudaFreeHost(ctx->h_nit);
     cudaFree(ctx->d_cmask);
@@ -2243,7 +2248,7 @@ int pdac_gpu_sgss(pdac_ctx *ctx) {
 // the kernels of one explicit_iter on stream st; returns their count.  With
 // prof, events xev[0..8] mark the group boundaries: flux pass, stage 1,
 // wavefront 1, flux pass, stage 2, wavefront 2, flux pass, final kernels
-static long long enqueue_explicit(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof) {
+static long long enqueue_explicit(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof, bool own) {
     int q = 0;
     auto mark = [&]() { if (prof) cudaEventRecord(ctx->xev[q++], st); };
     const Prm &P = ctx->P;
@@ -2294,11 +2299,11 @@ static long long enqueue_explicit(pdac_ctx *ctx, double dt, cudaStream_t st, boo
         L++;
         mark();
         // gas-enthalpy wavefront: records, one launch over all tiles or
-        // hyperplanes, scatter of the results; where a cooperative launch is
-        // not allowed (in a batch) and there are several tiles, a launch per
-        // hyperplane i + j + k = d of the interior (2 <= i <= nx - 1 ...), in
-        // increasing d
-        if (ctx->wave_tiles == 1 || (ctx->wave_coop() && ctx->allow_coop)) {
+        // hyperplanes, scatter of the results (own); where a cooperative launch
+        // is not allowed (in a batch, or beside another one) and there are
+        // several tiles, a launch per hyperplane i + j + k = d of the interior
+        // (2 <= i <= nx - 1 ...), in increasing d
+        if (own) {
             const pdac::Wave &W = ctx->W;
             const int rb = blocks(W.npos);
             int *gave_up = ctx->d_counters + 6;
@@ -2367,18 +2372,19 @@ static long long enqueue_explicit(pdac_ctx *ctx, double dt, cudaStream_t st, boo
 }
 
 // explicit_iter as one graph for time step dt
-static int build_explicit_graph(pdac_ctx *ctx, double dt) {
-    if (ctx->ex_exec) { cudaGraphExecDestroy(ctx->ex_exec); ctx->ex_exec = nullptr; }
-    if (ctx->ex_graph) { cudaGraphDestroy(ctx->ex_graph); ctx->ex_graph = nullptr; }
+static int build_explicit_graph(pdac_ctx *ctx, double dt, bool own) {
+    auto &g = ctx->ex[own];
+    if (g.exec) { cudaGraphExecDestroy(g.exec); g.exec = nullptr; }
+    if (g.graph) { cudaGraphDestroy(g.graph); g.graph = nullptr; }
     cudaStream_t st = ctx->stream;
+    g.gen = ctx->graph_gen;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
-    long long L = enqueue_explicit(ctx, dt, st, false);
-    cudaError_t e = cudaStreamEndCapture(st, &ctx->ex_graph);
+    g.launches = enqueue_explicit(ctx, dt, st, false, own);
+    cudaError_t e = cudaStreamEndCapture(st, &g.graph);
     if (e != cudaSuccess) return fail(ctx, PDAC_ERR_CUDA, std::string("explicit_iter graph capture: ") + cudaGetErrorString(e));
     CK(cudaGetLastError());
-    CK(cudaGraphInstantiate(&ctx->ex_exec, ctx->ex_graph, 0));
-    ctx->ex_dt = dt;
-    ctx->ex_launches = L;
+    CK(cudaGraphInstantiate(&g.exec, g.graph, 0));
+    g.dt = dt;
     return PDAC_OK;
 }
 
@@ -2387,18 +2393,24 @@ int pdac_gpu_explicit_iter(pdac_ctx *ctx, double dt) {
     if (ctx->ti != 1) return fail(ctx, PDAC_ERR_CONFIG, "explicit_iter: the context runs time_integration = 0");
     cudaStream_t st = ctx->stream;
     CK(cudaEventRecord(ctx->ev[6], st));
-    std::unique_lock<std::mutex> lk(coop_lock(), std::defer_lock);
-    if (ctx->wave_coop() && ctx->allow_coop) lk.lock();  // until the stream is idle below
+    // the wavefront in the context's own form (else a launch per hyperplane)
+    bool own = ctx->wave_tiles == 1;
+    std::unique_lock<std::mutex> lk;
+    if (ctx->wave_coop() && ctx->allow_coop) {
+        lk = std::unique_lock<std::mutex>(coop_lock(), std::try_to_lock);  // until the stream is idle below
+        own = lk.owns_lock();
+    }
     if (ctx->prof) {
-        ctx->launches += enqueue_explicit(ctx, dt, st, true);
+        ctx->launches += enqueue_explicit(ctx, dt, st, true, own);
         CK(cudaGetLastError());
     } else {
-        if (!ctx->ex_exec || ctx->ex_dt != dt) {
-            int s = build_explicit_graph(ctx, dt);
+        const auto &g = ctx->ex[own];
+        if (!g.exec || g.dt != dt || g.gen != ctx->graph_gen) {
+            int s = build_explicit_graph(ctx, dt, own);
             if (s) return s;
         }
-        CK(cudaGraphLaunch(ctx->ex_exec, st));
-        ctx->launches += ctx->ex_launches;
+        CK(cudaGraphLaunch(g.exec, st));
+        ctx->launches += g.launches;
     }
     CK(cudaEventRecord(ctx->ev[7], st));
     CK(cudaMemcpyAsync(ctx->h_counters + 1, ctx->d_counters + 1, 6 * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -2542,8 +2554,6 @@ void put_tuning(pdac_ctx *ctx, const Tuning &t) {
     ctx->coop_cpb = t.coop_cpb;
     if (ctx->coop_max_blocks > 0)
         ctx->coop_blocks = std::min(std::max(1, (int)((ctx->ncell + t.coop_cpb - 1) / t.coop_cpb)), ctx->coop_max_blocks);
-    if (ctx->ex_exec) { cudaGraphExecDestroy(ctx->ex_exec); ctx->ex_exec = nullptr; }
-    if (ctx->ex_graph) { cudaGraphDestroy(ctx->ex_graph); ctx->ex_graph = nullptr; }
     ctx->graph_gen++;
 }
 
@@ -2624,7 +2634,7 @@ int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin) {
         std::vector<int> flag(ctx->ncell);
         CK(cudaMemcpy(flag.data(), ctx->d_flag, flag.size() * sizeof(int), cudaMemcpyDeviceToHost));
         CK(cudaStreamSynchronize(ctx->stream));
-        ctx->ex_dt = -1.0;  // explicit_iter's graph is built again
+        ctx->graph_gen++;
         int s = setup_wave(ctx, flag.data(), wave);
         if (s) return s;
     }
@@ -2873,8 +2883,6 @@ int pdac_gpu_read_restart(pdac_ctx *ctx, const char *path, double *time, int *nf
         for (int ig = 0; ig < ctx->ng; ++ig) ctx->cfg.gas_type[ig] = ctx->P.gas_type[ig] = gt[ig];
         set_gas_tables(ctx);
         ctx->graph_gen++;
-        if (ctx->ex_exec) { cudaGraphExecDestroy(ctx->ex_exec); ctx->ex_exec = nullptr; }
-        if (ctx->ex_graph) { cudaGraphDestroy(ctx->ex_graph); ctx->ex_graph = nullptr; }
     }
     std::vector<double> buf(n);
     for (auto &a : restart_arrays(ctx)) {
@@ -3447,10 +3455,7 @@ static void batch_free(pdac_batch *b) {
     }
     b->go.notify_all();
     for (auto &t : b->th) t.join();
-    for (pdac_ctx *c : b->m) {
-        c->allow_coop = true;
-        c->ex_dt = -1.0;
-    }
+    for (pdac_ctx *c : b->m) c->allow_coop = true;
     for (auto e : b->fin) if (e) cudaEventDestroy(e);
     if (b->bexec) cudaGraphExecDestroy(b->bexec);
     if (b->bgraph) cudaGraphDestroy(b->bgraph);
@@ -3482,12 +3487,8 @@ int pdac_gpu_batch_create(pdac_ctx *const *members, int nmember, int nthreads, p
         nthread_members += b->graph[i] ? 0 : 1;
     }
     int nt = nthreads > 0 ? std::min(nthreads, nthread_members) : nthread_members;
-    // members take the non-cooperative paths while in the batch (the
-    // explicit_iter graph, built with the cooperative wavefront, is rebuilt)
-    for (pdac_ctx *c : b->m) {
-        c->allow_coop = false;
-        c->ex_dt = -1.0;
-    }
+    // members take the non-cooperative paths while in the batch
+    for (pdac_ctx *c : b->m) c->allow_coop = false;
     b->nit.assign(nmember, 0);
     b->status.assign(nmember, 0);
     b->fin.assign(nmember, nullptr);
