@@ -430,7 +430,10 @@ int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin);
  *       (3 if the device holds the tiles at once, else 2), 1 = a launch per
  *       hyperplane, 2 = one launch over all hyperplanes, 3 = tiles, of 16 x 4
  *       columns (j x k) in 3D, all columns (up to 256) or else 64 in 2D, 4 =
- *       2D tiles of 64.
+ *       2D tiles of 64;
+ *   [2] how often a tile of the wavefront looks for another tile's pressure
+ *       before it gives up (PDAC_ERR_TIMEOUT): 0 = the default, a second or
+ *       two.
  * pdac_gpu_get_forms (nout >= 1): [0] 1 if the context holds face records;
  * [1] tiles of the wavefront (0: none), [2], [3] their columns j and k, [4]
  * the blocks of the launch over all hyperplanes (0 and no tiles: a launch

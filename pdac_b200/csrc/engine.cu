@@ -163,6 +163,7 @@ struct pdac_ctx {
     // (0) a launch each
     int wave_tiles = 0, wave_blocks = 0;
     bool wave_one = false;
+    int wave_looks = pdac::WAVE_LOOKS;  // the limit of a tile's waits
     // one launch whose blocks wait for one another
     bool wave_coop() const { return wave_tiles > 1 || wave_blocks > 0; }
 };
@@ -773,6 +774,7 @@ int setup_wave(pdac_ctx *ctx, const int *flag, int form = WAVE_AUTO) {
         }
     }
     W.npos = (int)np;
+    W.looks = ctx->wave_looks;
     code.assign(np, 0);
     each([&](int c, int, int, int) {
         int m = pdac::WC_REC;
@@ -2627,14 +2629,16 @@ int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin) {
 // forms a context runs in that its mesh does not ask for
 int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin) {
     if (!ctx || !in || nin < 1) return PDAC_ERR_ARG;
-    const int wave = nin > 1 ? in[1] : 0;
-    if (in[0] < 0 || in[0] > 1 || wave < 0 || wave > (ctx->d3 ? WAVE_TILES : WAVE_TILES_64) || (wave && ctx->ti != 1))
+    const int wave = nin > 1 ? in[1] : 0, looks = nin > 2 ? in[2] : 0;
+    if (in[0] < 0 || in[0] > 1 || wave < 0 || wave > (ctx->d3 ? WAVE_TILES : WAVE_TILES_64) || (wave && ctx->ti != 1) ||
+        looks < 0 || looks > pdac::WAVE_LOOKS)
         return fail(ctx, PDAC_ERR_ARG, "set_forms: a value is out of range");
     if (ctx->ti == 1) {
         std::vector<int> flag(ctx->ncell);
         CK(cudaMemcpy(flag.data(), ctx->d_flag, flag.size() * sizeof(int), cudaMemcpyDeviceToHost));
         CK(cudaStreamSynchronize(ctx->stream));
         ctx->graph_gen++;
+        ctx->wave_looks = looks ? looks : pdac::WAVE_LOOKS;
         int s = setup_wave(ctx, flag.data(), wave);
         if (s) return s;
     }

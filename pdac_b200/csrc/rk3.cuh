@@ -640,6 +640,7 @@ __global__ void k_rk3_wave(Prm P, Fld F, RkF K, double dt, int stage, int d, int
 // s) tt + t.
 // Meshes whose columns do not fit (setup_wave) take k_rk3_wave_planes over
 // records in hyperplane order, without padding.
+constexpr int WAVE_LOOKS = 1 << 22;  // the limit of one wait: a second or two
 struct Wave {
     const int *order;           // record position -> cell, -1 where there is none
     const int *pos_of;          // cell -> record position, -1 for cells without a record
@@ -648,6 +649,7 @@ struct Wave {
     double *pnew;               // new pressure per record
     int npos;
     int tj, tk, tt, ntj, steps;  // tiles
+    int looks;                   // the limit of a tile's wait for a pressure (WAVE_LOOKS)
     // hyperplanes: records start[q] .. start[q + 1] - 1 of hyperplane q, and per
     // record the W / S / B neighbour's ([3][npos]; -1: none)
     const int *start, *src;
@@ -791,7 +793,6 @@ __device__ __forceinline__ double wave_solve(const Prm &P, const Wave &W, const 
     return p;
 }
 
-constexpr int WAVE_LOOKS = 1 << 22;  // the limit of one wait: a second or two
 
 // The wavefront of a stage in one launch, a block per tile.  The west
 // pressure of a cell is its thread's previous one, the south and bottom ones
@@ -827,7 +828,7 @@ __global__ void __launch_bounds__(256) k_rk3_wave_tile(Prm P, Wave W, double dt,
     auto wait = [&](const double *p, unsigned long long x, bool &lost) {
         for (int q = 0; x == WAVE_EMPTY; ++q) {
             x = wave_look(p);
-            if (q >= WAVE_LOOKS || ((q & 1023) == 1023 && *(volatile int *)gave_up)) {
+            if (x == WAVE_EMPTY && (q >= W.looks || ((q & 1023) == 1023 && *(volatile int *)gave_up))) {
                 lost = true;
                 break;
             }
