@@ -433,11 +433,15 @@ int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin);
  *       2D tiles of 64;
  *   [2] how often a tile of the wavefront looks for another tile's pressure
  *       before it gives up (PDAC_ERR_TIMEOUT): 0 = the default, a second or
- *       two.
+ *       two;
+ *   [3] the corrector's sweep loop: 0 = as the mesh asks, 1 = one launch on a
+ *       thread-block cluster (2D, up to 131072 cells), 2 = one cooperative
+ *       launch, 3 = a graph of launches.
  * pdac_gpu_get_forms (nout >= 1): [0] 1 if the context holds face records;
  * [1] tiles of the wavefront (0: none), [2], [3] their columns j and k, [4]
  * the blocks of the launch over all hyperplanes (0 and no tiles: a launch
- * each).                                                                    */
+ * each), [5] the form the last pdac_gpu_iter's sweep loop ran in (4: the host
+ * loop of profiling; 0: none yet).                                          */
 int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin);
 int pdac_gpu_get_forms(pdac_ctx *ctx, int *out, int nout);
 

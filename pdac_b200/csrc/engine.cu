@@ -99,6 +99,8 @@ struct pdac_ctx {
     // resident at once), else (both 0) the graph
     int coop_blocks = 0, coop_cpb = 1024, coop_max_blocks = 0;
     int cluster_blocks = 0;
+    int sweep_form = 0;              // SWEEP_AUTO, or the one pdac_gpu_set_forms chose
+    int last_form = 0;               // the one the last iter took
     // grid of the residual-test kernels (0: half the inner-loop grid)
     int test_grid = 0;
     // cooperative launches (the sweep loop, the explicit solver's wavefront)
@@ -897,6 +899,17 @@ static cudaError_t sweep_loop_room(int nsm, int &grid_blocks, int &clusters) {
     return cudaOccupancyMaxActiveClusters(&clusters, pdac::k_sweep_cluster<NP>, &lc);
 }
 
+// the forms of the sweep loop (pdac_gpu_set_forms): as the mesh asks, a
+// cluster, a cooperative grid, a graph of launches; profiling's host loop
+enum { SWEEP_AUTO = 0, SWEEP_CLUSTER, SWEEP_GRID, SWEEP_GRAPH, SWEEP_HOST };
+
+// the blocks of the cooperative grid for the context's cells per block
+static int coop_grid(const pdac_ctx *ctx) {
+    if (ctx->sweep_form == SWEEP_CLUSTER || ctx->sweep_form == SWEEP_GRAPH) return 0;
+    const int want = std::max(1, (int)((ctx->ncell + ctx->coop_cpb - 1) / ctx->coop_cpb));
+    return std::min(want, ctx->coop_max_blocks);
+}
+
 // The form of the sweep loop.  One launch whose blocks stay resident spares
 // each colour phase its two launches, which the barriers between the residual
 // tests and the inner loop replace: a cluster for the 2D meshes above, a
@@ -919,12 +932,15 @@ static int setup_sweep_loop(pdac_ctx *ctx) {
         case 6: CK((ctx->d3 ? sweep_loop_room<6, 3> : sweep_loop_room<6, 2>)(nsm, room, clusters)); break;
         default: CK((ctx->d3 ? sweep_loop_room<0, 3> : sweep_loop_room<0, 2>)(nsm, room, clusters)); break;
     }
-    if (!ctx->d3 && (long)ctx->ncell <= PDAC_CLUSTER_MAX_CELLS && clusters > 0) ctx->cluster_blocks = pdac::CLUSTER;
-    if (!coop) return PDAC_OK;
-    ctx->coop_cpb = ctx->d3 ? 64 : 1024;
-    ctx->coop_max_blocks = room;
-    const int want = std::max(1, (int)((ctx->ncell + ctx->coop_cpb - 1) / ctx->coop_cpb));
-    ctx->coop_blocks = std::min(want, ctx->coop_max_blocks);
+    const bool cluster = !ctx->d3 && (long)ctx->ncell <= PDAC_CLUSTER_MAX_CELLS && clusters > 0;
+    if ((ctx->sweep_form == SWEEP_CLUSTER && !cluster) || (ctx->sweep_form == SWEEP_GRID && (!coop || room < 1))) {
+        ctx->sweep_form = SWEEP_AUTO;
+        (void)setup_sweep_loop(ctx);
+        return fail(ctx, PDAC_ERR_ARG, "set_forms: the sweep loop cannot run in this form");
+    }
+    if (cluster && ctx->sweep_form <= SWEEP_CLUSTER) ctx->cluster_blocks = pdac::CLUSTER;
+    ctx->coop_max_blocks = coop ? room : 0;
+    ctx->coop_blocks = coop_grid(ctx);
     return PDAC_OK;
 }
 
@@ -1317,6 +1333,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
         int st = setup_wave(ctx, cfg->flag);
         if (st) return st;
     } else {
+        ctx->coop_cpb = ctx->d3 ? 64 : 1024;
         int st = setup_sweep_loop(ctx);
         if (st) return st;
     }
@@ -1863,6 +1880,7 @@ int pdac_gpu_iter(pdac_ctx *ctx, double dt, int *nit_out) {
             one = lk.owns_lock();
         }
     }
+    ctx->last_form = one ? (ctx->cluster_blocks > 0 ? SWEEP_CLUSTER : SWEEP_GRID) : (ctx->prof ? SWEEP_HOST : SWEEP_GRAPH);
     if (one) {
         CK(launch_sweep_loop(ctx, dt, st));
         CK(cudaMemcpyAsync(ctx->h_nit, ctx->d_nit, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -2554,8 +2572,7 @@ void put_tuning(pdac_ctx *ctx, const Tuning &t) {
     ctx->inner_grid = t.inner_grid;
     ctx->test_grid = t.test_grid;
     ctx->coop_cpb = t.coop_cpb;
-    if (ctx->coop_max_blocks > 0)
-        ctx->coop_blocks = std::min(std::max(1, (int)((ctx->ncell + t.coop_cpb - 1) / t.coop_cpb)), ctx->coop_max_blocks);
+    ctx->coop_blocks = coop_grid(ctx);
     ctx->graph_gen++;
 }
 
@@ -2629,9 +2646,9 @@ int pdac_gpu_set_tuning(pdac_ctx *ctx, const int *in, int nin) {
 // forms a context runs in that its mesh does not ask for
 int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin) {
     if (!ctx || !in || nin < 1) return PDAC_ERR_ARG;
-    const int wave = nin > 1 ? in[1] : 0, looks = nin > 2 ? in[2] : 0;
+    const int wave = nin > 1 ? in[1] : 0, looks = nin > 2 ? in[2] : 0, sweep = nin > 3 ? in[3] : 0;
     if (in[0] < 0 || in[0] > 1 || wave < 0 || wave > (ctx->d3 ? WAVE_TILES : WAVE_TILES_64) || (wave && ctx->ti != 1) ||
-        looks < 0 || looks > pdac::WAVE_LOOKS)
+        looks < 0 || looks > pdac::WAVE_LOOKS || sweep < 0 || sweep > SWEEP_GRAPH || (sweep && ctx->ti != 0))
         return fail(ctx, PDAC_ERR_ARG, "set_forms: a value is out of range");
     if (ctx->ti == 1) {
         std::vector<int> flag(ctx->ncell);
@@ -2640,6 +2657,12 @@ int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin) {
         ctx->graph_gen++;
         ctx->wave_looks = looks ? looks : pdac::WAVE_LOOKS;
         int s = setup_wave(ctx, flag.data(), wave);
+        if (s) return s;
+    }
+    else {
+        ctx->graph_gen++;
+        ctx->sweep_form = sweep;
+        int s = setup_sweep_loop(ctx);
         if (s) return s;
     }
     ctx->fk_off = in[0] == 1;
@@ -2651,7 +2674,8 @@ int pdac_gpu_set_forms(pdac_ctx *ctx, const int *in, int nin) {
 int pdac_gpu_get_forms(pdac_ctx *ctx, int *out, int nout) {
     if (!ctx || !out || nout < 1) return PDAC_ERR_ARG;
     const auto records = hold_records(ctx);
-    const int v[] = {ctx->d_fk ? 1 : 0, ctx->wave_tiles, ctx->W.tj, ctx->W.tk, ctx->wave_blocks};
+    const int v[] = {ctx->d_fk ? 1 : 0, ctx->wave_tiles, ctx->W.tj, ctx->W.tk, ctx->wave_blocks,
+                     ctx->last_form};
     for (int q = 0; q < nout && q < (int)(sizeof v / sizeof *v); ++q) out[q] = v[q];
     return PDAC_OK;
 }
@@ -2754,7 +2778,7 @@ int pdac_gpu_autotune(pdac_ctx *ctx, const char *cache_path, int *out, int nout)
                                   : fail(ctx, PDAC_ERR_CUDA, "autotune: device query");
         const bool one_launch = !ctx->cfg.implicit_fluxes && !ctx->cfg.implicit_enthalpy;
         const bool cluster = one_launch && ctx->cluster_blocks > 0;  // nothing to tune
-        const bool coop = one_launch && ctx->coop_max_blocks > 0 && ctx->allow_coop;
+        const bool coop = one_launch && ctx->coop_blocks > 0 && ctx->allow_coop;
         float best_ms = 1e30f;
         if (!status && coop && !cluster) {
             for (int cpb : {64, 256, 1024, 4096}) {

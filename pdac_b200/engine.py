@@ -83,8 +83,8 @@ TUNING_KEYS = ("tile_shape", "tile_kchunk", "inner_grid", "test_grid", "coop_cel
 
 
 # the forms pdac_gpu_set_forms chooses and those pdac_gpu_get_forms reports, in order
-FORM_KEYS = ("no_records", "wave", "wave_looks")
-FORM_REPORT = ("records", "wave_tiles", "wave_tj", "wave_tk", "wave_blocks")
+FORM_KEYS = ("no_records", "wave", "wave_looks", "sweep")
+FORM_REPORT = ("records", "wave_tiles", "wave_tj", "wave_tk", "wave_blocks", "sweep")
 
 
 class Engine:
