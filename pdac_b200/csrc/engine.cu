@@ -409,9 +409,8 @@ static cudaError_t set_inner_attrs() {
     return e;
 }
 
-// the specific-heat tables of the run's gases (hcapgs.f:33-85, the
-// polynomials of hcapg1) in their order; again when a restart file brings
-// other gases
+// the specific-heat and viscosity tables of the run's gases (hcapgs.f:33-85,
+// visc.f:37-148) in their order; again when a restart file brings other gases
 void set_gas_tables(pdac_ctx *ctx) {
     static const double cp[7][4] = {
         {2.811e1, -3.68e-6, 1.746e-5, -1.065e-8}, {3.115e1, -1.357e-2, 2.680e-5, -1.168e-8},

@@ -94,7 +94,7 @@ __global__ void k_restart_derive(Prm P, Fld F) {
     for (int is = 1; is <= P.ns; ++is) rls = rls + SOL(F.rlk, c, is) * P.inrl[is];
     F.ep[c] = 1.0 - rls;
     double hc = 0.0;
-    for (int ig = 0; ig < P.ng; ++ig) hc = hc + hcapg1(P, P.gas_type[ig], F.tg[c]) * yg[ig];
+    for (int ig = 0; ig < P.ng; ++ig) hc = hc + hcap(P, ig, F.tg[c]) * yg[ig];
     F.cg[c] = hc;
 }
 

@@ -22,7 +22,7 @@ __global__ void k_mixture(Prm P, Fld F) {
     // mixture_temperature (derived.f:269-296)
     const double tg = F.tg[c];
     double cgas = 0.0;
-    for (int ig = 0; ig < ng; ++ig) cgas = hcapg1(P, P.gas_type[ig], tg) * GAS(F.ygc, c, ig) + cgas;
+    for (int ig = 0; ig < ng; ++ig) cgas = hcap(P, ig, tg) * GAS(F.ygc, c, ig) + cgas;
     double sts = 0.0, scp = 0.0;
     for (int is = 1; is <= ns; ++is) {
         const double rl = F.rlk[(is - 1) * n + c];

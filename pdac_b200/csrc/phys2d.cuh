@@ -468,23 +468,6 @@ __device__ __forceinline__ void viscon(const Prm &P, const Fld &F, int c, double
     }
 }
 
-// hcapgs.f:33-85, for one reference gas type g (1..7)
-__device__ __forceinline__ double hcapg1(const Prm &P, int g, double tg) {
-    double t1 = (P.icpc <= 1) ? P.tref : tg, t2 = t1 * t1, t3 = t1 * t2, c;
-    switch (g) {
-    case 1: c = (2.811e1 - 3.68e-6 * t1 + 1.746e-5 * t2 - 1.065e-8 * t3); break;
-    case 2: c = (3.115e1 - 1.357e-2 * t1 + 2.680e-5 * t2 - 1.168e-8 * t3); break;
-    case 3: c = (1.980e1 + 7.344e-2 * t1 - 5.602e-5 * t2 + 1.715e-8 * t3); break;
-    case 4: c = (2.714e1 + 9.274e-3 * t1 - 1.381e-5 * t2 + 7.645e-9 * t3); break;
-    case 5: c = (3.224e1 + 1.924e-3 * t1 + 1.055e-5 * t2 - 3.596e-9 * t3); break;
-    case 6: c = (3.0413e1 - 1.059e-2 * t1 + 2.458e-5 * t2 - 1.135e-8 * t3); break;
-    default: c = (2.385e1 + 6.699e-2 * t1 - 4.961e-5 * t2 + 1.328e-8 * t3); break;
-    }
-    c = c / P.gmw[g];
-    if (P.icpc == 0) { if (g == 5) c = 1810.0; if (g == 6) c = 1004.0; }
-    return c;
-}
-
 // eosg.f:114-137
 __device__ __forceinline__ double thermal_eosg(const Prm &P, double tg, double p, const double *xg) {
     double mg = 0;
@@ -500,12 +483,17 @@ __device__ __forceinline__ void mole(const Prm &P, double *xg, const double *yg)
     for (int ig = 0; ig < P.ng; ++ig) xg[ig] = yg[ig] / P.gmw[P.gas_type[ig]] * molinv;
 }
 
-// hcapgs.f:33-85 for gas ig of the run: hcapg1's polynomial with the signs in
-// the coefficients, its powers given
+// hcapgs.f:33-85 for gas ig of the run: the polynomial of its type
+// (set_gas_tables), of temperature t1 and its powers
 __device__ __forceinline__ double hcap_of(const Prm &P, int ig, double t1, double t2, double t3) {
     double c = P.hcp[ig][0] + P.hcp[ig][1] * t1 + P.hcp[ig][2] * t2 + P.hcp[ig][3] * t3;
     c = pdac_fp::div_by(c, P.hmw[ig]);
     return P.hfix[ig] != 0.0 ? P.hfix[ig] : c;
+}
+
+__device__ __forceinline__ double hcap(const Prm &P, int ig, double tg) {
+    const double t1 = (P.icpc <= 1) ? P.tref : tg, t2 = t1 * t1;
+    return hcap_of(P, ig, t1, t2, t1 * t2);
 }
 
 // the cell's gas mass fractions, in registers (constant indices)
