@@ -260,10 +260,17 @@ template <int NP>
 __host__ __device__ constexpr size_t inner_smem_bytes() {
     return (size_t)(inner_face_rows<NP>() + inner_dens_rows<NP>()) * KS * sizeof(double);
 }
+// The most cells of one colour in 32 consecutive ones, whatever their flags: a
+// row of nx cells has one on every third i, so 32 cells over rows of at least 5
+// have 14 at most (11 where the rows' first and last cells are not fluid, as on
+// the meshes of the reference, whose frame is a boundary).
+constexpr int WORD_CELLS = 14;
+constexpr int SCAN_LIST = 32 * WORD_CELLS;  // a warp's list of the candidates of 32 words
 // the sweep loops', which hold the warps' scan lists in the same place
 template <int NP>
 __host__ __device__ constexpr size_t sweep_smem_bytes(int threads = KS) {
-    return (size_t)threads / KS * (inner_smem_bytes<NP>() > KS / 32 * 352 * sizeof(int) ? inner_smem_bytes<NP>() : KS / 32 * 352 * sizeof(int));
+    constexpr size_t lists = KS / 32 * SCAN_LIST * sizeof(int);
+    return (size_t)threads / KS * (inner_smem_bytes<NP>() > lists ? inner_smem_bytes<NP>() : lists);
 }
 
 // A worklist entry is a cell, with the top bit set for a plain one: a cell
@@ -690,7 +697,6 @@ __device__ __forceinline__ bool test_cell(const Prm &P, const Fld &F, double dt,
 // groups of eight (one 32-byte sector).  slist: SCAN_LIST ints per warp.
 // Collecting and testing in one pass took the two launches' fixed cost
 // (about 12 us) down to one's.
-constexpr int SCAN_LIST = 32 * 11;  // a colour has at most 11 cells in a word of 32
 
 // one warp's round: lane's word t (of words) of the active set under its
 // colour mask, its candidates tested; put(um, lane, u, e) takes the unconverged
@@ -868,7 +874,7 @@ __global__ void __launch_bounds__(KS, PDAC_INNER_MINB(NP)) k_sweep_grid(Prm P, F
 constexpr int CLUSTER = 16, KC = 256;  // blocks; their threads, each with a word of the active set at most
 template <int NP>
 __host__ __device__ constexpr size_t cluster_smem_bytes() {
-    return sweep_smem_bytes<NP>(KC) + KC * 11 * sizeof(int);
+    return sweep_smem_bytes<NP>(KC) + KC * WORD_CELLS * sizeof(int);
 }
 template <int NP>
 __global__ void __launch_bounds__(KC, 1) k_sweep_cluster(Prm P, Fld F, double dt, SweepWork W, int maxout) {
