@@ -225,8 +225,6 @@ cudaError_t launch_mom_tile(const pdac::Prm &P, const pdac::Fld &F, int nph, int
     }
 }
 
-// kernel launches of one momentum-flux pass of form shape
-inline int mom_launches(int shape) { return shape == 0 ? 2 : 1; }
 
 cudaError_t set_tile_attrs(const pdac::Prm &P, const pdac::Fld &F) {
     for (int s = 0; s < N_TILE_SHAPES; ++s) {
@@ -243,6 +241,12 @@ const int TPB_TEAM = 128;
 int fail(pdac_ctx *c, int code, const std::string &msg) {
     if (c) c->err = msg;
     return code;
+}
+
+// kernel launches of one momentum-flux pass (launch_mom_tile)
+int mom_launches(const pdac_ctx *c) {
+    if (c->tile_shape != 0 && !c->P.immb) return 1;
+    return c->P.simple ? 1 + (c->nrest > 0) : 1;
 }
 
 // the general passes' cells of a context, and kernel launches over a 3D
@@ -1691,7 +1695,7 @@ static int enqueue_tilde(pdac_ctx *ctx, double dt, cudaStream_t st) {
         STENCIL_LAUNCH(ctx, ctx->nph, st, pdac::k_visc3d<true>, pdac::k_visc3d<false>, );
         if (ctx->P.mixed) CK(launch_mom_tile<float>(ctx->P, F, ctx->nph, ctx->tile_shape, ctx->tile_kchunk, st, rest_cells(ctx)));
         else CK(launch_mom_tile<double>(ctx->P, F, ctx->nph, ctx->tile_shape, ctx->tile_kchunk, st, rest_cells(ctx)));
-        ctx->launches += mom_launches(ctx->tile_shape);
+        ctx->launches += mom_launches(ctx);
         PHASE_LAUNCH(ctx->nph, pdac::k_tilde3d, blocks(n), TPB, st, ctx->P, F, dt, ctx->d_app0u, ctx->d_app0v, ctx->d_app0w);
         ctx->launches++;
     } else {
@@ -1802,7 +1806,7 @@ static int build_iter_graph(pdac_ctx *ctx, double dt) {
     CK(cudaGraphAddNode(&node, ctx->it_graph, nullptr, 0, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     CK(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    // kernels of one sweep: the nine of the colour phases, the check, and
+    // kernels of one sweep: the six of the colour phases, the check, and
     // those the implicit modes add (counted by their enqueue functions,
     // which run here only to record them)
     const long long before = ctx->launches;
@@ -1859,12 +1863,11 @@ int pdac_gpu_iter(pdac_ctx *ctx, double dt, int *nit_out) {
     if (ctx->d3) {
         PHASE_LAUNCH(nph, pdac::k_predictor3d, blocks(n), TPB, st, ctx->P, F, dt);
         STENCIL_LAUNCH(ctx, 1, st, pdac::k_mflux_init3d<true>, pdac::k_mflux_init3d<false>, dt PDAC_COMMA);
-        ctx->launches--;  // counted below
     } else {
         PHASE_LAUNCH(nph, pdac::k_predictor2d, blocks(n), TPB, st, ctx->P, F, dt);
-        pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);
+        pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt), ctx->launches++;
     }
-    ctx->launches += 2;
+    ctx->launches++;
     CK(cudaGetLastError());
     // every cell is tested in the first sweep
     CK(cudaMemsetAsync(ctx->d_dirty, 0xff, 2 * ((n + 31) / 32) * sizeof(unsigned), st));
@@ -2053,12 +2056,11 @@ int pdac_gpu_iter_static(pdac_ctx *ctx, double dt, int *nit_out) {
     if (ctx->d3) {
         PHASE_LAUNCH(nph, pdac::k_predictor3d, blocks(n), TPB, st, ctx->P, F, dt);
         STENCIL_LAUNCH(ctx, 1, st, pdac::k_mflux_init3d<true>, pdac::k_mflux_init3d<false>, dt PDAC_COMMA);
-        ctx->launches--;  // counted below
     } else {
         PHASE_LAUNCH(nph, pdac::k_predictor2d, blocks(n), TPB, st, ctx->P, F, dt);
-        pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);
+        pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt), ctx->launches++;
     }
-    ctx->launches += 2;
+    ctx->launches++;
     CK(cudaGetLastError());
     CK(cudaMemsetAsync(dirty, 0xff, nwords * sizeof(unsigned), st));
     // the context's own worklist lengths describe an earlier pdac_gpu_iter
@@ -2219,13 +2221,12 @@ int pdac_gpu_initialize_fieldn(pdac_ctx *ctx) {
         PHASE_LAUNCH_D(ctx->nph, pdac::k_rk3_fieldn, 3, blocks(n), TPB, st, ctx->P, F, ctx->K, ctx->cfg.dt);
         if (int s = accumulate_viscosities(ctx, st)) return s;
         STENCIL_LAUNCH(ctx, ctx->nph, st, pdac::k_visc3d<true>, pdac::k_visc3d<false>, );
-        ctx->launches--;  // counted below
     } else {
         PHASE_LAUNCH_D(ctx->nph, pdac::k_rk3_fieldn, 2, blocks(n), TPB, st, ctx->P, F, ctx->K, ctx->cfg.dt);
         if (int s = accumulate_viscosities(ctx, st)) return s;
-        pdac::k_visc2d<<<blocks((long)n * (ns + 1)), TPB, 0, st>>>(ctx->P, F);
+        pdac::k_visc2d<<<blocks((long)n * (ns + 1)), TPB, 0, st>>>(ctx->P, F), ctx->launches++;
     }
-    ctx->launches += 2;
+    ctx->launches++;
     CK(cudaGetLastError());
     CK(cudaEventRecord(ctx->ev[3], st));
     return PDAC_OK;
@@ -2295,7 +2296,7 @@ static long long enqueue_explicit(pdac_ctx *ctx, double dt, cudaStream_t st, boo
             }
             L += ctx->launches - before;
             ctx->launches = before;  // the caller adds L
-            L += mom_launches(ctx->tile_shape);
+            L += mom_launches(ctx);
         } else {
             if (P.mixed) {
                 pdac::k_rk3_mflux<2, float, false><<<blocks(n), TPB, 0, st>>>(P, F, nullptr, 0);
@@ -3293,14 +3294,13 @@ static int enqueue_step_pre(pdac_ctx *ctx, double dt, cudaStream_t st) {
     if (ctx->d3) {
         PHASE_LAUNCH(nph, pdac::k_predictor3d, blocks(n), TPB, st, ctx->P, F, dt);
         STENCIL_LAUNCH(ctx, 1, st, pdac::k_mflux_init3d<true>, pdac::k_mflux_init3d<false>, dt PDAC_COMMA);
-        ctx->launches--;  // counted below
     } else {
         PHASE_LAUNCH(nph, pdac::k_predictor2d, blocks(n), TPB, st, ctx->P, F, dt);
-        pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt);
+        pdac::k_mflux_init2d<<<blocks(n), TPB, 0, st>>>(ctx->P, F, dt), ctx->launches++;
     }
     CK(cudaMemsetAsync(ctx->d_dirty, 0xff, 2 * ((n + 31) / 32) * sizeof(unsigned), st));
     pdac::k_set_int<<<1, 1, 0, st>>>(ctx->d_nit, 1);
-    ctx->launches += 3;
+    ctx->launches += 2;
     CK(cudaGetLastError());
     return PDAC_OK;
 }
