@@ -52,7 +52,7 @@ struct pdac_ctx {
     size_t fk_doubles = 0;
     bool fk_off = false;
     std::mutex fk_mu;  // held while kernels that read the records may run
-    int dev = 0;       // the device the context was created on
+    int dev = 0, nsm = 148;  // the device the context was created on and its SMs
     int nvent = 0;
     std::string err;
     cudaEvent_t ev[16];
@@ -973,6 +973,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     pdac_ctx *ctx = new pdac_ctx();
     ctx->cfg = *cfg;
     CK(cudaGetDevice(&ctx->dev));
+    CK(cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->dev));
     ctx->d3 = cfg->job_type == 3;
     ctx->nx = cfg->nx; ctx->ny = ctx->d3 ? cfg->ny : 1; ctx->nz = cfg->nz;
     ctx->ncell = ctx->nx * ctx->ny * ctx->nz;
@@ -1193,12 +1194,7 @@ int pdac_gpu_create(const pdac_cfg *cfg, pdac_ctx **out) {
     }
     pdac::k_colour_masks<<<blocks(((long)n + 31) / 32), TPB, 0, ctx->stream>>>(P, ctx->d_cmask);
     CK(cudaGetLastError());
-    {
-        int dev = 0, nsm = 148;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        ctx->inner_grid = nsm * 16;
-    }
+    ctx->inner_grid = ctx->nsm * 16;
     CK(dev_malloc(&ctx->d_nit, sizeof(int)));
     CK(cudaMallocHost(&ctx->h_nit, sizeof(int)));
     CK(dev_malloc(&ctx->d_counters, 8 * sizeof(int)));
@@ -1736,7 +1732,7 @@ static long long sweep_kernels(const pdac_ctx *) { return 7; }
 // warps k_inner_team may spread a short worklist over: those resident at
 // once, or none beyond the packed ones for a member of a batch
 static int inner_spread(const pdac_ctx *ctx) {
-    return ctx->allow_coop ? 148 * PDAC_INNER_MINB(ctx->nph) * (pdac::KS / 32) : 1;
+    return ctx->allow_coop ? ctx->nsm * PDAC_INNER_MINB(ctx->nph) * (pdac::KS / 32) : 1;
 }
 
 static int enqueue_sweep(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof) {
