@@ -263,8 +263,8 @@ int pdac_gpu_unconverged_cells(pdac_ctx *ctx, int *ijk, long *n_inout);
  * allocations, or whose memory accounting admits only the buffers it
  * created.  Limits and rules:
  *  - the mesh must fit: 256 + 2 * (4 * ceil(nx / 3) * ny * nz rounded
- *    up to 256) + 4 * ceil(nx * ny * nz / 32) bytes
- *    <= PDAC_ITER_STATIC_SCRATCH_BYTES, else the
+ *    up to 256) + 4 * ceil(nx * ny * nz / 32) bytes (one of the two
+ *    lists is kept free) <= PDAC_ITER_STATIC_SCRATCH_BYTES, else the
  *    call returns PDAC_ERR_ARG with the sizes in pdac_gpu_last_error;
  *  - the context's device must be current; the first call on a device looks
  *    up the array's address once (cudaGetSymbolAddress), so make that first
@@ -394,9 +394,8 @@ int pdac_gpu_elapsed(pdac_ctx *ctx, int a, int b, double *ms);
 /* ---- launch-shape autotuner (no counterpart in the reference) ---------- */
 /* The launch shapes of the engine's tunable kernels, as five ints:
  *   [0] form of the 3D momentum-flux pass: 0 = one thread per (cell,
- *       phase) and component (three launches), 1..4 = the shared-memory
- *       tiled pass with 32 x 4, 32 x 8, 16 x 8 or 64 x 2 cells (i x j) per
- *       block;
+ *       phase, component), 1..4 = the shared-memory tiled pass with 32 x 4,
+ *       32 x 8, 16 x 8 or 64 x 2 cells (i x j) per block;
  *   [1] planes of a tiled block's march up k;
  *   [2] blocks of the corrector's inner-loop kernel;
  *   [3] blocks of its residual-test kernel;

@@ -1752,8 +1752,8 @@ static int enqueue_sweep(pdac_ctx *ctx, double dt, cudaStream_t st, bool prof) {
     const long team_threads = (nthr + (ctx->d3 ? 4 : 7)) / (ctx->d3 ? 5 : 8) * 32;
     const int g = std::min(ctx->inner_grid, blocks(team_threads, TPB_TEAM));
     unsigned *dirty = ctx->d_dirty;
-    // [col] worklist length, [3 + col] cells tested, [6 + col] candidates, of colour col
-    CK(cudaMemsetAsync(ctx->d_wcount, 0, 9 * sizeof(int), st));
+    // [col] worklist length, [3 + col] cells tested, of colour col
+    CK(cudaMemsetAsync(ctx->d_wcount, 0, 6 * sizeof(int), st));
     for (int col = 0; col < 3; ++col) {
         int *cnt = ctx->d_wcount + col;
         if (prof) CK(cudaEventRecord(ctx->cev[3 * col], st));
@@ -1986,11 +1986,11 @@ int pdac_gpu_unconverged_cells(pdac_ctx *ctx, int *ijk, long *n_inout) {
 // counters, worklist, active-set flags) in one fixed static device array
 // instead of the context's buffers; the call allocates nothing.
 //
-// Layout of the static array: bytes [0, 256) hold the nine int counters
-// (worklist length, tested cells and candidates per colour) and the sweep
-// number (int 12), then the
-// worklist and the candidate list (one int per cell of the largest colour
-// phase each, 256-aligned lengths), then the active set (one bit per cell).
+// Layout of the static array: bytes [0, 256) hold the six int counters
+// (worklist length and tested cells per colour) and the sweep number (int 12),
+// then the worklist (one int per cell of the largest colour phase, a 256-aligned
+// length) and as much again that no kernel uses (the call's stated limit counts
+// it), then the active set (one bit per cell).
 // The counters must be zero when a colour phase starts: the call clears them
 // itself on its stream before every sweep, and sets every active-set bit
 // before the first sweep, so no part of the array has to start at zero.
@@ -2066,7 +2066,7 @@ int pdac_gpu_iter_static(pdac_ctx *ctx, double dt, int *nit_out) {
     for (nit = 1; nit <= ctx->cfg.maxout; ++nit) {
         *ctx->h_nit = nit;
         CK(cudaMemcpyAsync(dnit, ctx->h_nit, sizeof(int), cudaMemcpyHostToDevice, st));
-        CK(cudaMemsetAsync(wcount, 0, 9 * sizeof(int), st));
+        CK(cudaMemsetAsync(wcount, 0, 6 * sizeof(int), st));
         for (int col = 0; col < 3; ++col) {
             int *cnt = wcount + col;
             const unsigned *cmask = ctx->d_cmask + (size_t)col * nwords;

@@ -249,7 +249,7 @@ __device__ __forceinline__ void face_assemble(const Prm &P, KT &K, DT &Dk, int s
 
 // the inner loop's shared memory, allocated at launch (dynamic): FaceK
 // columns for up to six phases, then DensK columns up to
-// PDAC_INNER_SHD_MAXP phases (64.5 KB per block at six phases)
+// PDAC_INNER_SHD_MAXP phases (34 KB per block at four phases, 54 at six)
 template <int NP>
 __host__ __device__ constexpr int inner_face_rows() { return (NP > 0 && NP <= 6) ? FaceK<NP, true>::N : 0; }
 template <int NP>
@@ -304,7 +304,7 @@ __device__ __forceinline__ void inner_team_cell(const Prm &P, const Fld &F, doub
                                                 unsigned *dirty, int q, int tb, double *kcols, double *dcols) {
     constexpr unsigned full = 0xffffffffu;
     constexpr int NC = Sys<NP>::M - 1;   // phase capacity
-    constexpr bool SH = inner_face_rows<NP>() > 0;   // FaceK in shared memory (40 KB per block at NP = 6)
+    constexpr bool SH = inner_face_rows<NP>() > 0;   // FaceK in shared memory (22 KB per block at NP = 4, 36 KB at 6)
     constexpr bool SHD = inner_dens_rows<NP>() > 0;  // DensK too (12 KB at NP = 4, 18 KB at NP = 6)
     constexpr int NAX = D == 3 ? 3 : 2;  // axes; lanes q < NAX own the minus faces
     const int nph = nphases<NP>(P), ns = nph - 1;
@@ -532,7 +532,11 @@ __device__ __forceinline__ void inner_team_run(const Prm &P, const Fld &F, doubl
         // short ones in turn, those past the last long unit short ones first.
         // In many rounds what counts is that the cells at work at one time are
         // near each other in the mesh: long and short units in one sequence,
-        // (u * rate) >> 32 of its first u long.
+        // (u * rate) >> 32 of its first u long.  Four steps with the line at
+        // eight rounds, at three, in turns throughout and in one sequence
+        // throughout: 128 x 128 x 96 67.4 / 68.4 / 67.4 / 68.5 ms, its hills
+        // with six phases 120.3 / 120.8 / 120.1 / 123.7, 256 x 256 x 192 405.4
+        // / 404.7 / 407.7 / 403.4.
         const int nshort = nwork - nlong, ulong = (nlong + cpw - 1) / cpw, units = ulong + (nshort + cpw - 1) / cpw;
         const bool many = units > 8 * nwarps;
         const unsigned long long rate = many ? (((unsigned long long)ulong << 32) + units - 1) / units : 0;
