@@ -340,8 +340,8 @@ def measured_peaks():
 
 def profiled_traffic(workload, kernel, algorithmic_bytes):
     """DRAM bytes per launch of `kernel` from a committed ncu capture, and
-    how it was obtained: the capture's own figure on its workload; on another
-    workload its DRAM/algorithmic ratio times this launch's algorithmic bytes
+    how it was obtained: the capture's own figure on a captured workload; on
+    another the DRAM/algorithmic ratio times this launch's algorithmic bytes
     where that ratio was found the same at two sizes; else None."""
     p = os.path.join(ROOT, "profiles", "traffic.json")
     if not os.path.exists(p):
@@ -349,13 +349,14 @@ def profiled_traffic(workload, kernel, algorithmic_bytes):
     d = json.load(open(p)).get(kernel)
     if not d:
         return None, "no capture"
-    if d.get("workload") == workload:
-        return d["bytes_per_launch"], f"ncu on {workload}, mean of {d['launches']} launches"
-    if d.get("proportional"):
+    own = d["workloads"].get(workload)
+    if own:
+        return own["bytes_per_launch"], f"ncu on {workload}, mean over {own['launches']} launches"
+    if d["proportional"]:
         return (d["dram_per_algorithmic"] * algorithmic_bytes,
-                f"{d['dram_per_algorithmic']:.2f} x algorithmic bytes, the DRAM/algorithmic ratio of ncu on "
-                f"{d['workload']} ({d['launches']} launches); {d['evidence']}")
-    return None, f"not scaled from {d['workload']}: {d['why_not']}"
+                f"{d['dram_per_algorithmic']:.2f} x algorithmic bytes, the DRAM/algorithmic ratio of ncu captures "
+                f"({d['evidence']})")
+    return None, f"not scaled from {', '.join(d['workloads'])}: {d['why_not']}"
 
 
 # ---------------------------------------------------------------------------
@@ -555,6 +556,8 @@ def engine_arm(args):
         avg_launch_s = kms / 1000.0 / phases
         achieved = bytes_per_launch / avg_launch_s / 1e9
         rdetail = {"launches": phases,
+                   "route": "kernel timed in launches (host sweep loop, the steps of measured_on); the timed steps run "
+                            "the same cell bodies inside one launch of the sweep loop",
                    "corrector_ms": {"resid": stats["resid_ms"], "inner": stats["inner_ms"]},
                    "unconverged_cell_visits": unconv, "tested_cell_visits": tested,
                    "fluid_cell_visits": sweeps_cells, "measured_on": measured_on}
