@@ -98,4 +98,51 @@ def test_a_context_that_fits_without_records_is_created(tmp_path):
     ref.close()
 
 
+def test_records_are_taken_back_from_a_context_that_another_thread_steps():
+    """The allocation waits for the running iter; the steps around it have the
+    bits of a context stepped alone."""
+    import threading
+
+    import torch
+    from pdac_b200.engine import Engine
+    case = _case("3d", 5, nx=64, ny=60, nz=56)
+    steps = 12
+    alone = Engine(case)
+    nit = [alone.step(s) for s in range(1, steps + 1)]
+    rec_bytes = 84 * 8 * case.ncell
+    free = lambda: torch.cuda.mem_get_info()[0]
+    first = Engine(case)
+    first.step(1)
+    before = free()
+    second = Engine(case)
+    takes = before - free() - rec_bytes
+    second.close()
+    alone.set_forms(no_records=1)
+    fill = torch.empty(free() - (takes - rec_bytes // 2), dtype=torch.uint8, device="cuda")
+    got, go = [], threading.Event()
+
+    def work():
+        for s in range(2, steps + 1):
+            got.append(first.step(s))
+            go.set()
+
+    t = threading.Thread(target=work)
+    try:
+        assert first.forms()["records"] == 1
+        t.start()
+        go.wait()
+        second = Engine(case)
+        t.join()
+        assert first.forms()["records"] == 0 and second.step(1) == nit[0]
+        second.close()
+    finally:
+        t.join()
+        del fill
+        torch.cuda.empty_cache()
+    assert got == nit[1:]
+    _same(first, alone)
+    first.close()
+    alone.close()
+
+
 ARENA_SAMPLE = ("p", "mf", "vis", "appu", "appv", "appw")
